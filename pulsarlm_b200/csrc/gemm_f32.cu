@@ -2,20 +2,37 @@
 //
 // CUDA-core FMAs only: no tensor cores, no TF32. Each output element is one chain
 // of fmaf over k = 0 .. K-1 in ascending order, whatever M is, so a token's row
-// does not depend on what else is in the batch or on how a prompt was cut.
+// does not depend on what else is in the batch or on how a prompt was cut. All kernels
+// below make that same chain, so their results are equal bit for bit and which of them
+// runs is a matter of time alone.
 #include "common.cuh"
+
+#include "mma_helpers.cuh"
 
 namespace {
 
+struct GemmF32Params {
+    const float* a;
+    const float* w;
+    float* c;
+    int m, n, k, lda, ldw, ldc, accumulate;
+};
+
+__device__ __forceinline__ void put(const GemmF32Params& p, int row, int col, float v) {
+    if (row < p.m && col < p.n) {
+        float* dst = p.c + static_cast<int64_t>(row) * p.ldc + col;
+        *dst = p.accumulate ? *dst + v : v;
+    }
+}
+
+// ---------------------------------------------------------------------------- any address and stride
+// 256 threads; thread (ty, tx) of a 16x16 grid owns a 4x4 block of the 64x64 tile. For operands whose
+// rows do not start on 16 bytes.
 constexpr int kTileM = 64;
 constexpr int kTileN = 64;
 constexpr int kTileK = 16;
 
-// 256 threads; thread (ty, tx) of a 16x16 grid owns a 4x4 block of the 64x64 tile.
-// Optional `accumulate`: C += product (used to add into the fp32 residual stream).
-__global__ void __launch_bounds__(256)
-gemm_f32_kernel(const float* __restrict__ a, const float* __restrict__ w, float* __restrict__ c, int m, int n,
-                int k, int lda, int ldw, int ldc, int accumulate) {
+__global__ void __launch_bounds__(256) gemm_f32_any_kernel(const GemmF32Params p) {
     __shared__ float as[kTileK][kTileM + 1];
     __shared__ float ws[kTileK][kTileN + 1];
     const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
@@ -30,7 +47,7 @@ gemm_f32_kernel(const float* __restrict__ a, const float* __restrict__ w, float*
         }
     }
 
-    for (int k0 = 0; k0 < k; k0 += kTileK) {
+    for (int k0 = 0; k0 < p.k; k0 += kTileK) {
         // 64 rows x 16 k of each operand: 1024 elements, 4 per thread; consecutive
         // threads read consecutive k of one row.
 #pragma unroll
@@ -38,8 +55,8 @@ gemm_f32_kernel(const float* __restrict__ a, const float* __restrict__ w, float*
             const int e = threadIdx.x + i * 256;
             const int row = e / kTileK, kk = e % kTileK;
             const int gk = k0 + kk;
-            as[kk][row] = (m0 + row < m && gk < k) ? a[static_cast<int64_t>(m0 + row) * lda + gk] : 0.0f;
-            ws[kk][row] = (n0 + row < n && gk < k) ? w[static_cast<int64_t>(n0 + row) * ldw + gk] : 0.0f;
+            as[kk][row] = (m0 + row < p.m && gk < p.k) ? p.a[static_cast<int64_t>(m0 + row) * p.lda + gk] : 0.0f;
+            ws[kk][row] = (n0 + row < p.n && gk < p.k) ? p.w[static_cast<int64_t>(n0 + row) * p.ldw + gk] : 0.0f;
         }
         __syncthreads();
 #pragma unroll
@@ -60,22 +77,315 @@ gemm_f32_kernel(const float* __restrict__ a, const float* __restrict__ w, float*
         }
         __syncthreads();
     }
-
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const int row = m0 + ty * 4 + i;
-        if (row >= m) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            put(p, m0 + ty * 4 + i, n0 + tx * 4 + j, acc[i][j]);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------- tiles
+// Two chains a step: fma.rn.f32x2 rounds each half as fmaf does.
+__device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ uint64_t twice(float v) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+    return r;
+}
+
+// Rows of four floats along k, zeros past the operand's rows and past k.
+__device__ __forceinline__ float4 load_row4(const float* base, int ld, int row, int rows, int gk, int k) {
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (row < rows) {
+        const float* src = base + static_cast<int64_t>(row) * ld + gk;
+        if (gk + 3 < k) {
+            v = *reinterpret_cast<const float4*>(src);
+        } else {
+            if (gk < k) v.x = src[0];
+            if (gk + 1 < k) v.y = src[1];
+            if (gk + 2 < k) v.z = src[2];
+        }
+    }
+    return v;
+}
+
+// A BM x BN tile per CTA, RM rows x RN columns a thread (both in runs of four), both operands in shared memory
+// with k outermost, the next 16 k in registers meanwhile. A thread reads its RM + RN operands of a k
+// AHEAD k before their fmafs. What bounds it: shared memory hands a warp one operand a lane and cycle while the
+// SM's four schedulers do four fmafs a lane and cycle, so RM x RN / (RM + RN) has to stay above four (8 x 16: 5.3;
+// 8 x 8: 4; 4 x 8: 2.7, for products of few tiles, where more warps count more).
+template <int BM, int BN, int RM, int RN, int AHEAD, int CTAS>
+__global__ void __launch_bounds__(BM * BN / (RM * RN), CTAS) gemm_f32_tile_kernel(const GemmF32Params p) {
+    constexpr int kThreads = BM * BN / (RM * RN);
+    constexpr int BK = 16;
+    constexpr int kLdA = BM + 4, kLdW = BN + 4;
+    constexpr int kTx = BN / RN;
+    constexpr int kTy = BM / RM;
+    constexpr int kLoadsA = BM * BK / 4 / kThreads, kLoadsW = BN * BK / 4 / kThreads;
+    constexpr int kBufs = AHEAD + 1;
+    static_assert(kLoadsA >= 1 && kLoadsW >= 1 && kTx * kTy == kThreads && RM % 4 == 0 && RN % 4 == 0, "tile");
+    extern __shared__ __align__(16) float tile_smem[];
+    float (*as)[BK][kLdA] = reinterpret_cast<float (*)[BK][kLdA]>(tile_smem);
+    float (*ws)[BK][kLdW] = reinterpret_cast<float (*)[BK][kLdW]>(tile_smem + 2 * BK * kLdA);
+    const int tid = threadIdx.x;
+    const int tx = tid % kTx, ty = tid / kTx;
+    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+
+    uint64_t acc[RM][RN / 2];
+#pragma unroll
+    for (int i = 0; i < RM; ++i) {
+#pragma unroll
+        for (int j = 0; j < RN / 2; ++j) {
+            acc[i][j] = 0;
+        }
+    }
+    float4 la[kLoadsA], lw[kLoadsW];
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < kLoadsA; ++i) {
+            const int e = tid + i * kThreads;
+            la[i] = load_row4(p.a, p.lda, m0 + e / 4, p.m, k0 + (e % 4) * 4, p.k);
+        }
+#pragma unroll
+        for (int i = 0; i < kLoadsW; ++i) {
+            const int e = tid + i * kThreads;
+            lw[i] = load_row4(p.w, p.ldw, n0 + e / 4, p.n, k0 + (e % 4) * 4, p.k);
+        }
+    };
+    auto stash = [&](int buffer) {
+#pragma unroll
+        for (int i = 0; i < kLoadsA; ++i) {
+            const int e = tid + i * kThreads, row = e / 4, kk = (e % 4) * 4;
+            as[buffer][kk][row] = la[i].x;
+            as[buffer][kk + 1][row] = la[i].y;
+            as[buffer][kk + 2][row] = la[i].z;
+            as[buffer][kk + 3][row] = la[i].w;
+        }
+#pragma unroll
+        for (int i = 0; i < kLoadsW; ++i) {
+            const int e = tid + i * kThreads, row = e / 4, kk = (e % 4) * 4;
+            ws[buffer][kk][row] = lw[i].x;
+            ws[buffer][kk + 1][row] = lw[i].y;
+            ws[buffer][kk + 2][row] = lw[i].z;
+            ws[buffer][kk + 3][row] = lw[i].w;
+        }
+    };
+    fetch(0);
+    stash(0);
+    __syncthreads();
+    int buffer = 0;
+    for (int k0 = 0; k0 < p.k; k0 += BK, buffer ^= 1) {
+        const bool more = k0 + BK < p.k;
+        if (more) {
+            fetch(k0 + BK);
+        }
+        ulonglong2 wf[kBufs][RN / 4];
+        float4 af[kBufs][RM / 4];
+        auto pick = [&](int which, int kk) {
+#pragma unroll
+            for (int j = 0; j < RN / 4; ++j) {
+                wf[which][j] = *reinterpret_cast<const ulonglong2*>(&ws[buffer][kk][j * (BN / (RN / 4)) + tx * 4]);
+            }
+#pragma unroll
+            for (int i4 = 0; i4 < RM / 4; ++i4) {
+                af[which][i4] = *reinterpret_cast<const float4*>(&as[buffer][kk][i4 * (BM / (RM / 4)) + ty * 4]);
+            }
+        };
+#pragma unroll
+        for (int kk = 0; kk < AHEAD; ++kk) {
+            pick(kk, kk);
+        }
+#pragma unroll
+        for (int kk = 0; kk < BK; ++kk) {
+            const int now = kk % kBufs;
+            if (kk + AHEAD < BK) {
+                pick((kk + AHEAD) % kBufs, kk + AHEAD);
+            }
+#pragma unroll
+            for (int i4 = 0; i4 < RM / 4; ++i4) {
+                const float4 av = af[now][i4];
+                const float a4[4] = {av.x, av.y, av.z, av.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint64_t a2 = twice(a4[i]);
+#pragma unroll
+                    for (int j = 0; j < RN / 4; ++j) {
+                        fma2(acc[i4 * 4 + i][2 * j], a2, wf[now][j].x);
+                        fma2(acc[i4 * 4 + i][2 * j + 1], a2, wf[now][j].y);
+                    }
+                }
+            }
+        }
+        if (more) {
+            stash(buffer ^ 1);  // (last read a round ago; the round's barrier came since)
+        }
+        __syncthreads();
+    }
+    const bool vec = (p.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(p.c) & 15) == 0;
+#pragma unroll
+    for (int i = 0; i < RM; ++i) {
+        const int row = m0 + (i / 4) * (BM / (RM / 4)) + ty * 4 + i % 4;
+        if (row >= p.m) {
             continue;
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int col = n0 + tx * 4 + j;
-            if (col < n) {
-                float* dst = c + static_cast<int64_t>(row) * ldc + col;
-                *dst = accumulate ? *dst + acc[i][j] : acc[i][j];
+        for (int run = 0; run < RN / 4; ++run) {
+            const int col = n0 + run * (BN / (RN / 4)) + tx * 4;
+            float v[4];
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(v[0]), "=f"(v[1]) : "l"(acc[i][2 * run]));
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(v[2]), "=f"(v[3]) : "l"(acc[i][2 * run + 1]));
+            if (vec && col + 3 < p.n) {
+                float4* dst = reinterpret_cast<float4*>(p.c + static_cast<int64_t>(row) * p.ldc + col);
+                float4 r = make_float4(v[0], v[1], v[2], v[3]);
+                if (p.accumulate) {
+                    const float4 old = *dst;
+                    r = make_float4(old.x + r.x, old.y + r.y, old.z + r.z, old.w + r.w);
+                }
+                *dst = r;
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    put(p, row, col + j, v[j]);
+                }
             }
         }
     }
+}
+
+template <int BM, int BN, int RM, int RN, int AHEAD, int CTAS>
+void launch_tile(const GemmF32Params& p, cudaStream_t stream) {
+    constexpr int kSmem = 2 * 16 * (BM + 4 + BN + 4) * static_cast<int>(sizeof(float));
+    static_assert(kSmem <= 48 * 1024, "needs no opt-in");
+    gemm_f32_tile_kernel<BM, BN, RM, RN, AHEAD, CTAS>
+        <<<dim3((p.m + BM - 1) / BM, (p.n + BN - 1) / BN), BM * BN / (RM * RN), kSmem, stream>>>(p);
+}
+
+// ---------------------------------------------------------------------------- few rows
+// A few rows of A against a stream of weights: 16 weight rows a CTA, TM x RM rows of A, a thread one weight
+// row and RM rows of A. Both operands arrive by cp.async, `stages` pieces of 128 k in flight, and are read
+// sixteen (RM == 4: eight) k ahead of the fmafs. What bounds it: the weights' stream where N is large, the chain
+// of K dependent fmafs (4 cycles each) where K is.
+constexpr int kFewN = 16;
+constexpr int kFewK = 128;
+constexpr int kFewLd = kFewK + 4;  // (rows 4 banks apart: eight rows' 16-byte reads meet no bank twice)
+
+template <int TM, int RM>
+__global__ void __launch_bounds__(kFewN * TM) gemm_f32_few_kernel(const GemmF32Params p, const int stages) {
+    constexpr int BM = TM * RM;
+    constexpr int kThreads = kFewN * TM;
+    constexpr int kStageFloats = (kFewN + BM) * kFewLd;
+    constexpr int kAhead = RM == 4 ? 2 : 4;  // 16-byte groups of k read ahead
+    extern __shared__ __align__(16) float few_smem[];
+    const int tid = threadIdx.x;
+    const int col = tid % kFewN, tm = tid / kFewN;
+    const int n0 = blockIdx.x * kFewN, m0 = blockIdx.y * BM;
+    const int pieces = (p.k + kFewK - 1) / kFewK;
+
+    // This thread's copies: 16 bytes at column (tid % 32) * 4 of every (kThreads / 32)-th row.
+    const int load_row = tid / 32, load_k = (tid % 32) * 4;
+    auto load = [&](int piece, int slot) {
+        float* stage = few_smem + slot * kStageFloats + load_row * kFewLd + load_k;
+        const int gk = piece * kFewK + load_k;
+        const int left = max(0, min(4, p.k - gk)) * 4;
+        const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(stage));
+#pragma unroll
+        for (int i = 0; i < (kFewN + BM) / (kThreads / 32); ++i) {
+            const int row = load_row + i * (kThreads / 32);
+            const bool weight = row < kFewN;
+            const int at = weight ? n0 + row : m0 + row - kFewN;
+            const bool there = left > 0 && (weight ? at < p.n : at < p.m);
+            const float* base = weight ? p.w : p.a;
+            // (past the operand nothing is read: the address is then its first, with no bytes)
+            const float* from = there ? base + static_cast<int64_t>(at) * (weight ? p.ldw : p.lda) + gk : base;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                             dst + i * (kThreads / 32) * kFewLd * static_cast<int>(sizeof(float))),
+                         "l"(from), "r"(there ? left : 0)
+                         : "memory");
+        }
+    };
+    for (int s = 0; s < stages - 1; ++s) {
+        if (s < pieces) {
+            load(s, s);
+        }
+        cp_async_commit();
+    }
+    float acc[RM];
+#pragma unroll
+    for (int i = 0; i < RM; ++i) {
+        acc[i] = 0.0f;
+    }
+    int slot = 0, next_slot = stages - 1;
+    for (int piece = 0; piece < pieces; ++piece) {
+        // The group of this piece is the oldest of stages - 1 in flight.
+        if (stages == 8) {
+            cp_async_wait<6>();
+        } else {
+            cp_async_wait<2>();
+        }
+        __syncthreads();
+        if (piece + stages - 1 < pieces) {
+            load(piece + stages - 1, next_slot);  // (into the stage that was read before the barrier)
+        }
+        cp_async_commit();
+        next_slot = next_slot + 1 == stages ? 0 : next_slot + 1;
+        const float* stage = few_smem + slot * kStageFloats;
+        slot = slot + 1 == stages ? 0 : slot + 1;
+        const float4* w4 = reinterpret_cast<const float4*>(stage + col * kFewLd);
+        const float4* a4 = reinterpret_cast<const float4*>(stage + (kFewN + tm * RM) * kFewLd);
+        float4 w[2][kAhead], a[2][RM][kAhead];
+        auto fetch = [&](int which, int group) {
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j) {
+                w[which][j] = w4[group * kAhead + j];
+#pragma unroll
+                for (int i = 0; i < RM; ++i) {
+                    a[which][i][j] = a4[i * (kFewLd / 4) + group * kAhead + j];
+                }
+            }
+        };
+        fetch(0, 0);
+        constexpr int kGroups = kFewK / 4 / kAhead;
+#pragma unroll
+        for (int group = 0; group < kGroups; ++group) {
+            const int now = group & 1;
+            if (group + 1 < kGroups) {
+                fetch(now ^ 1, group + 1);
+            }
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j) {
+#pragma unroll
+                for (int i = 0; i < RM; ++i) acc[i] = fmaf(a[now][i][j].x, w[now][j].x, acc[i]);
+#pragma unroll
+                for (int i = 0; i < RM; ++i) acc[i] = fmaf(a[now][i][j].y, w[now][j].y, acc[i]);
+#pragma unroll
+                for (int i = 0; i < RM; ++i) acc[i] = fmaf(a[now][i][j].z, w[now][j].z, acc[i]);
+#pragma unroll
+                for (int i = 0; i < RM; ++i) acc[i] = fmaf(a[now][i][j].w, w[now][j].w, acc[i]);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < RM; ++i) {
+        put(p, m0 + tm * RM + i, n0 + col, acc[i]);
+    }
+}
+
+template <int TM, int RM>
+cudaError_t launch_few(const GemmF32Params& p, cudaStream_t stream) {
+    const dim3 grid((p.n + kFewN - 1) / kFewN, (p.m + TM * RM - 1) / (TM * RM));
+    // A CTA alone on its SM keeps eight pieces in flight; where SMs hold several, four each (8 KB of weights a piece).
+    const int stages = static_cast<int64_t>(grid.x) * grid.y <= 148 ? 8 : 4;
+    const int smem = stages * (kFewN + TM * RM) * kFewLd * static_cast<int>(sizeof(float));
+    const cudaError_t set = cudaFuncSetAttribute(gemm_f32_few_kernel<TM, RM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (set != cudaSuccess) {
+        return set;
+    }
+    gemm_f32_few_kernel<TM, RM><<<grid, kFewN * TM, smem, stream>>>(p, stages);
+    return cudaGetLastError();
 }
 
 }  // namespace
@@ -88,9 +398,46 @@ PL_API int pl_gemm_f32(const float* a, const float* w, float* c, int m, int n, i
     if (m == 0) {
         return 0;
     }
-    const dim3 grid((n + kTileN - 1) / kTileN, (m + kTileM - 1) / kTileM);
-    PL_REQUIRE(grid.y <= 65535, "gemm_f32: m=%d is too large for one launch", m);
-    gemm_f32_kernel<<<grid, 256, 0, stream>>>(a, w, c, m, n, k, lda, ldw, ldc, accumulate);
+    PL_REQUIRE((m + kTileM - 1) / kTileM <= 65535, "gemm_f32: m=%d is too large for one launch", m);
+    const GemmF32Params p{a, w, c, m, n, k, lda, ldw, ldc, accumulate};
+    const bool rows16 = (lda & 3) == 0 && (ldw & 3) == 0 &&
+        ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
+    // Where the lines lie (us, measured alone with a cold L2; shapes N x K; the 64 x 64 tiles with a 4 x 4 block a
+    // thread that ran every size before are the last figure of each row):
+    //   2048 x 8192, 8 rows: few 44, 64 x 64 tiles 412, before 939; 16384 x 2048: 54, 134, 281
+    //   3072 x 2048, 64 rows (768 few CTAs): few 60, tiles 105; 128 rows (1,536): 102, 105, 221
+    //   16384 x 2048, 64 rows (2,048): few 228, tiles 139
+    //   2048 x 8192, 509 rows: 64 x 64 tiles 524 (256 of them), 128 x 64 tiles 516 (128), 128 x 128 tiles 868 (64)
+    //   3072 x 2048, 509 rows: 197 (384), 225 (192), 223 (96); 16384 x 2048: 852, 693, 733, before 1580
+    //   32000 x 2048, 509 rows: 1681, 1345, 1253 (1,000 tiles)
+    const int64_t few_ctas = static_cast<int64_t>((n + kFewN - 1) / kFewN) * ((m + 31) / 32);
+    const int64_t tiles64 = static_cast<int64_t>((m + 63) / 64) * ((n + 63) / 64);
+    const int64_t tiles128x64 = static_cast<int64_t>((m + 127) / 128) * ((n + 63) / 64);
+    const bool padded = 2 * tiles128x64 > tiles64 + tiles64 / 4;  // (128-row tiles that would be a fifth empty and more)
+    cudaError_t few = cudaSuccess;
+    if (!rows16) {
+        const dim3 grid((n + kTileN - 1) / kTileN, (m + kTileM - 1) / kTileM);
+        gemm_f32_any_kernel<<<grid, 256, 0, stream>>>(p);
+    } else if (m <= 4) {
+        few = launch_few<4, 1>(p, stream);
+    } else if (m <= 8 && few_ctas <= 148) {
+        few = launch_few<8, 1>(p, stream);
+    } else if (m <= 8 || (m <= 16 && n < 8192)) {
+        few = launch_few<4, 2>(p, stream);
+    } else if (m <= 16) {
+        few = launch_few<8, 2>(p, stream);
+    } else if (m <= 32 || few_ctas <= 768) {
+        few = launch_few<8, 4>(p, stream);
+    } else if (padded || tiles64 <= 148 || (tiles128x64 > 148 && tiles64 <= 448)) {
+        launch_tile<64, 64, 4, 8, 1, 4>(p, stream);
+    } else if (tiles128x64 < 1500) {
+        launch_tile<128, 64, 8, 8, 1, 3>(p, stream);
+    } else {
+        launch_tile<128, 128, 8, 16, 2, 2>(p, stream);
+    }
+    if (few != cudaSuccess) {
+        return pl_fail(3, "gemm_f32: launch failed: %s", cudaGetErrorString(few));
+    }
     PL_CHECK_LAUNCH("gemm_f32");
     return 0;
 }

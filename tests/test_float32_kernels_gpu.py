@@ -1,0 +1,105 @@
+"""The float32 engine's product and attention: every form of a kernel makes the same chain of sums, so forms are
+compared bit for bit, and one of them with float64."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _ops():
+    from pulsarlm_b200.kernels import ops
+
+    ops.require_device()
+    return ops
+
+
+# Rows of A around every form's edges, K with and without a last piece of its own, N off the tiles and below one.
+@pytest.mark.parametrize("m", [1, 4, 5, 8, 9, 16, 17, 32, 33, 65, 129, 300])
+@pytest.mark.parametrize("n,k", [(24, 4), (7, 132), (2500, 260), (8200, 64), (33000, 20)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_every_form_of_the_product_gives_the_same_bits(m, n, k, accumulate):
+    ops = _ops()
+    gen = torch.Generator(device=DEV).manual_seed(m + n + k)
+    a = torch.randn((m, k), generator=gen, device=DEV)
+    w = torch.randn((n, k), generator=gen, device=DEV)
+    off = torch.zeros((m, k + 1), device=DEV)
+    off[:, 1:] = a                                       # (rows that start on no 16 bytes take the general form)
+    got = torch.full((m, n), 0.5, device=DEV)
+    want = got.clone()
+    ops.gemm_f32(a, w, got, accumulate=accumulate)
+    ops.gemm_f32(off[:, 1:], w, want, accumulate=accumulate)
+    assert torch.equal(got, want)
+    exact = a.double() @ w.double().t() + (0.5 if accumulate else 0.0)
+    # k roundings of partial sums no larger than sum |a| |w|
+    bound = (k + 2) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t() + 1.0)
+    assert bool(((got.double() - exact).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("heads,kv,dim", [(8, 2, 64), (3, 3, 20), (16, 1, 128), (5, 1, 36)])
+@pytest.mark.parametrize("portions", [[1] * 3 + [5], [1] * 40 + [90, 1], [150]])
+@pytest.mark.parametrize("options", [{}, {"window": 37}, {"window": 37, "keep_first": 5},
+                                     {"softcap": 3.0, "sinks": True, "gate": True, "bias": True, "slopes": True}])
+def test_staged_attention_gives_the_bits_of_the_plain_walk(heads, kv, dim, portions, options):
+    """The plain walk is reached by asking for attention mass. Requests of several lengths, single tokens beside
+    portions, a page that holds NaN in the values of tokens no query may see."""
+    ops = _ops()
+    gen = torch.Generator().manual_seed(heads * dim + len(portions))
+    page = 16
+    before = [int(torch.randint(0, 100, (1,), generator=gen)) for _ in portions]
+    widths = [-(-(b + n + 3) // page) for b, n in zip(before, portions)]
+    n_pages = sum(widths) + 1
+    order = torch.randperm(n_pages, generator=gen).tolist()
+    table = torch.full((len(portions), max(widths)), -1, dtype=torch.int32)
+    for e, w in enumerate(widths):
+        table[e, :w] = torch.tensor([order.pop() for _ in range(w)], dtype=torch.int32)
+    pools = torch.randn((2, n_pages, kv, page, dim), generator=gen)
+    for e, (b, n) in enumerate(zip(before, portions)):  # (places past the last token are not written yet)
+        for j in range(b + n, widths[e] * page):
+            pools[:, table[e, j // page], :, j % page] = float("nan")
+    pools = pools.to(DEV)
+    tokens = sum(portions)
+    pos = torch.tensor([b + i for b, n in zip(before, portions) for i in range(n)], dtype=torch.int32, device=DEV)
+    entry = torch.tensor([e for e, n in enumerate(portions) for _ in range(n)], dtype=torch.int32, device=DEV)
+    q = torch.randn((tokens, heads, dim), generator=gen).to(DEV)
+    more = {}
+    if options.get("sinks"):
+        more["sinks"] = torch.randn(heads, generator=gen).to(DEV)
+        more["gate"] = torch.randn((tokens, heads), generator=gen).to(DEV)
+        more["distance_bias"] = torch.randn((heads, 50), generator=gen).to(DEV)
+        more["distance_slopes"] = torch.rand(heads, generator=gen).to(DEV) * 0.1
+    args = (pools[0], pools[1], table.to(DEV), pos, entry)
+    scale = dim ** -0.5
+    common = dict(softcap=options.get("softcap", 0.0), keep_first=options.get("keep_first", 0), **more)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    got, want = torch.empty_like(q), torch.empty_like(q)
+    ops.attention_simt(q, *args, got, page, options.get("window"), scale, status, **common)
+    mass, weight = torch.zeros((n_pages, heads), device=DEV), torch.zeros(n_pages, device=DEV)
+    ops.attention_simt(q, *args, want, page, options.get("window"), scale, status, mass, weight, **common)
+    assert int(status.item()) == 0 and bool(torch.isfinite(want).all())
+    assert torch.equal(got, want)
+    one = torch.empty_like(q[-1:])   # (a token alone takes another form than among many)
+    if "gate" in common:
+        common["gate"] = common["gate"][-1:]
+    ops.attention_simt(q[-1:], *args[:3], pos[-1:], entry[-1:], one, page, options.get("window"), scale, status, **common)
+    assert torch.equal(one, want[-1:])
+
+
+def test_a_page_outside_the_pool_is_flagged_and_its_keys_are_left_out():
+    ops = _ops()
+    pools = torch.randn((2, 4, 1, 16, 64), device=DEV)
+    q = torch.randn((70, 2, 64), device=DEV)
+    pos = torch.arange(70, dtype=torch.int32, device=DEV) % 48
+    entry = torch.zeros(70, dtype=torch.int32, device=DEV)
+    table = torch.tensor([[0, 9, 2]], dtype=torch.int32, device=DEV)
+    for rows in (slice(0, 70), slice(20, 24)):
+        status = torch.zeros(1, dtype=torch.int32, device=DEV)
+        got, want = torch.empty_like(q[rows]), torch.empty_like(q[rows])
+        ops.attention_simt(q[rows], pools[0], pools[1], table, pos[rows], entry[rows], got, 16, None, 0.125, status)
+        assert int(status.item()) == 4
+        mass, weight = torch.zeros((4, 2), device=DEV), torch.zeros(4, device=DEV)
+        ops.attention_simt(q[rows], pools[0], pools[1], table, pos[rows], entry[rows], want, 16, None, 0.125, None, mass, weight)
+        assert torch.equal(got, want)
