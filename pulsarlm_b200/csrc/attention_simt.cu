@@ -12,6 +12,8 @@
 // attn_scalar_kernel, pulsarlm-core/src/kernels/paged_common.cu:26-137.
 #include "common.cuh"
 
+#include "mma_helpers.cuh"
+
 namespace {
 
 constexpr int kMaxAcc = 16;      // head_dim <= 512
@@ -227,6 +229,315 @@ __global__ void attention_simt_kernel(const scalar_t* __restrict__ q, int64_t q_
     }
 }
 
+// The same walk for the float32 engine with the keys and values of a chunk in shared memory, every sum in the
+// order of the kernel above (their results are equal bit for bit). A CTA takes `run` neighbouring tokens of
+// one kv head; a warp takes P of their (token, head) pairs, so a key or value read from shared memory serves P
+// of them, and chunks arrive by cp.async two ahead. Neighbours of other requests are walked one request after
+// the other. What bounds the kernel above is the time a load takes to answer, once per key; here it is the operands
+// that shared memory hands out (1.25 a fmaf of the scores at P = 4), with few CTAs the chain of a chunk's phases. 32
+// heads of 64 over 8 kv heads, cold caches: 509 tokens of one prompt 779 -> 164 us, 8 single tokens of 600 keys
+// 413 -> 36 us. (With the head size known to the compiler a single token's walk is a quarter shorter; four pairs a
+// warp then take 132 registers, one CTA an SM instead of two, 195 us: those keep it a number.)
+constexpr int kStagedDim = 128;
+constexpr int kStagedStages = 3;
+constexpr int kOffsetRing = kStagedStages + 1;  // (where a chunk lies is known a step before its copies set out)
+
+struct StagedParams {
+    const float* q;
+    int64_t q_row_stride;
+    const float* k_pool;
+    const float* v_pool;
+    int64_t page_stride, head_stride;
+    int page_size, n_pages;
+    const int32_t* table;
+    int table_width;
+    const int32_t* pos;
+    const int32_t* entry;
+    float* out;
+    int64_t out_row_stride;
+    int n_tokens, group, head_dim, window, run;
+    float scale, softcap;
+    const float* sinks;
+    const float* gate;
+    int64_t gate_row_stride;
+    const float* distance_bias;
+    int bias_rows;
+    const float* distance_slopes;
+    int keep_first;
+    int32_t* status;
+};
+
+inline int staged_smem_bytes(int pairs, int head_dim) {
+    const int floats = pairs * head_dim + pairs * 32 + kStagedStages * 32 * (2 * head_dim + 4);
+    return floats * 4 + kOffsetRing * 32 * 8;
+}
+
+template <int P, int ACC, int DIM>
+__global__ void attention_f32_staged_kernel(const StagedParams a) {
+    extern __shared__ __align__(16) float staged_smem[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int hd = DIM > 0 ? DIM : a.head_dim, group = a.group;   // (DIM: a head size known to the compiler, or 0)
+    const int pairs = a.run * group;
+    const int k_ld = hd + 4;                             // (rows 4 banks apart: a lane reads a key of its own)
+    float* qs = staged_smem;                             // [pairs][hd]
+    float* ps = qs + pairs * hd;                         // [pairs][32]
+    float* ks = ps + pairs * 32;                         // [stages][32][hd + 4]
+    float* vs = ks + kStagedStages * 32 * k_ld;          // [stages][32][hd]
+    int64_t* offsets = reinterpret_cast<int64_t*>(vs + kStagedStages * 32 * hd);  // [stages + 1][32]
+    const int kv_head = blockIdx.y;
+    // (the last tokens of a prompt have the longest walks: they start first)
+    const int t_begin = static_cast<int>(gridDim.x - 1 - blockIdx.x) * a.run;
+    const int t_end = min(t_begin + a.run, a.n_tokens);
+
+    for (int idx = tid; idx < (t_end - t_begin) * group * hd; idx += blockDim.x) {
+        const int pair = idx / hd, d = idx - pair * hd;
+        qs[idx] = a.q[(t_begin + pair / group) * a.q_row_stride + static_cast<int64_t>(kv_head * group + pair % group) * hd + d];
+    }
+
+    for (int seg = t_begin; seg < t_end;) {
+        const int e = a.entry[seg];
+        int seg_end = seg, p_max = -1, first_min = INT_MAX;
+        while (seg_end < t_end && a.entry[seg_end] == e) {
+            const int p = a.pos[seg_end];
+            p_max = max(p_max, p);
+            first_min = min(first_min, a.window > 0 ? max(0, p - a.window + 1) : 0);
+            ++seg_end;
+        }
+        const PlTileWalk walk(first_min, a.keep_first, 32);
+        const int chunks = walk.count(p_max, 32);
+        const int32_t* row = a.table + static_cast<int64_t>(e) * a.table_width;
+
+        // Where the 32 keys of the walk's place w lie (-1: no page, or past the last key), by the first warp; the
+        // page is asked for a step before it is needed.
+        auto ask = [&](int w) {
+            const int j = w < chunks ? walk.tile(w) * 32 + lane : INT_MAX;
+            return warp == 0 && j <= p_max ? row[j / a.page_size] : -1;
+        };
+        auto locate = [&](int w, int page) {
+            if (warp == 0 && w < chunks) {
+                const int j = walk.tile(w) * 32 + lane;
+                offsets[w % kOffsetRing * 32 + lane] = page >= 0 && page < a.n_pages
+                    ? page * a.page_stride + kv_head * a.head_stride + static_cast<int64_t>(j % a.page_size) * hd : -1;
+            }
+        };
+        auto load = [&](int w) {
+            if (w < chunks) {
+                const int64_t* where = offsets + w % kOffsetRing * 32;
+                const int stage = w % kStagedStages, per = hd / 4;
+                for (int idx = tid; idx < 32 * per; idx += blockDim.x) {
+                    const int key = idx / per, c = (idx - key * per) * 4;
+                    const int64_t offset = where[key];
+                    const bool there = offset >= 0;
+                    cp_async_16_or_zero(ks + (stage * 32 + key) * k_ld + c, a.k_pool + (there ? offset + c : 0), there);
+                    cp_async_16_or_zero(vs + (stage * 32 + key) * hd + c, a.v_pool + (there ? offset + c : 0), there);
+                }
+            }
+            cp_async_commit();
+        };
+
+        int position[P], first[P];
+        bool mine[P];
+        float m[P], l[P], acc[P][ACC];
+#pragma unroll
+        for (int i = 0; i < P; ++i) {
+            const int pair = warp * P + i;
+            const int t = t_begin + pair / group;
+            mine[i] = pair < pairs && t >= seg && t < seg_end;
+            position[i] = mine[i] ? a.pos[t] : -1;
+            first[i] = a.window > 0 ? max(0, position[i] - a.window + 1) : 0;
+            m[i] = -INFINITY;
+            l[i] = 0.0f;
+#pragma unroll
+            for (int n = 0; n < ACC; ++n) {
+                acc[i][n] = 0.0f;
+            }
+        }
+
+        __syncthreads();  // (the queries are there; nothing of an earlier request's chunks is read any more)
+        locate(0, ask(0));
+        locate(1, ask(1));
+        locate(2, ask(2));
+        int page = ask(3);
+        __syncthreads();
+        load(0);
+        load(1);
+        for (int w = 0; w < chunks; ++w) {
+            cp_async_wait<1>();
+            __syncthreads();  // the chunk has landed, and the one before it was read by everyone
+            locate(w + 3, page);
+            page = ask(w + 4);
+            load(w + 2);
+            const int chunk = walk.tile(w), base = chunk * 32, j = base + lane;
+            bool takes[P], any = false;
+#pragma unroll
+            for (int i = 0; i < P; ++i) {
+                const PlTileWalk own(first[i], a.keep_first, 32);
+                takes[i] = mine[i] && (chunk < own.head || chunk >= own.start) && base <= position[i];
+                any = any || takes[i];
+            }
+            if (!any) {
+                continue;
+            }
+            const int stage = w % kStagedStages;
+            const float* krow = ks + (stage * 32 + lane) * k_ld;
+            const bool paged = offsets[w % kOffsetRing * 32 + lane] >= 0;
+            float s[P];
+#pragma unroll
+            for (int i = 0; i < P; ++i) {
+                s[i] = 0.0f;
+            }
+#pragma unroll(DIM > 0 ? DIM / 4 : 4)
+            for (int d = 0; d < hd; d += 4) {
+                const float4 kv = *reinterpret_cast<const float4*>(krow + d);
+#pragma unroll
+                for (int i = 0; i < P; ++i) {
+                    // (a pair past the CTA's last reads another's query: nothing is made of it)
+                    const float4 qv = *reinterpret_cast<const float4*>(qs + min(warp * P + i, pairs - 1) * hd + d);
+                    s[i] = fmaf(qv.x, kv.x, s[i]);
+                    s[i] = fmaf(qv.y, kv.y, s[i]);
+                    s[i] = fmaf(qv.z, kv.z, s[i]);
+                    s[i] = fmaf(qv.w, kv.w, s[i]);
+                }
+            }
+            uint32_t seen_keys[P];
+            bool whole = true;
+#pragma unroll
+            for (int i = 0; i < P; ++i) {
+                const int h = kv_head * group + (warp * P + i) % group;
+                const bool reach = takes[i] && (j >= first[i] || j < a.keep_first) && j <= position[i];
+                if (reach && !paged && a.status != nullptr) {
+                    atomicOr(a.status, 4);
+                }
+                const bool valid = reach && paged;
+                float score = -INFINITY;
+                if (valid) {
+                    score = s[i] * a.scale;
+                    if (a.softcap > 0.0f) {
+                        score = a.softcap * tanhf(score / a.softcap);
+                    }
+                    if (a.distance_bias != nullptr) {
+                        score += a.distance_bias[static_cast<int64_t>(h) * a.bias_rows + min(position[i] - j, a.bias_rows - 1)];
+                    }
+                    if (a.distance_slopes != nullptr) {
+                        score = fmaf(-a.distance_slopes[h], static_cast<float>(position[i] - j), score);
+                    }
+                }
+                seen_keys[i] = __ballot_sync(0xffffffffu, valid);
+                whole = whole && (!takes[i] || seen_keys[i] == 0xffffffffu);
+                float pw = 0.0f;
+                if (takes[i]) {
+                    const float m_new = fmaxf(m[i], pl_warp_max(score));
+                    const bool seen = m_new > -INFINITY;  // (-inf only if a bad block table hid every key so far)
+                    const float corr = seen ? expf(m[i] - m_new) : 1.0f;
+                    pw = valid && seen ? expf(score - m_new) : 0.0f;
+                    l[i] = l[i] * corr + pl_warp_sum(pw);
+#pragma unroll
+                    for (int n = 0; n < ACC; ++n) {
+                        acc[i][n] *= corr;
+                    }
+                    m[i] = m_new;
+                }
+                if (warp * P + i < pairs) {
+                    ps[(warp * P + i) * 32 + lane] = pw;
+                }
+            }
+            __syncwarp();
+            const float* vrows = vs + stage * 32 * hd;
+            auto weigh = [&](int jj, const float (&pj)[P], bool check) {
+                float v[ACC];
+#pragma unroll
+                for (int n = 0; n < ACC; ++n) {
+                    const int d = lane + 32 * n;
+                    v[n] = d < hd ? vrows[jj * hd + d] : 0.0f;
+                }
+#pragma unroll
+                for (int i = 0; i < P; ++i) {
+                    if (takes[i] && (!check || (seen_keys[i] >> jj & 1))) {
+#pragma unroll
+                        for (int n = 0; n < ACC; ++n) {
+                            acc[i][n] = fmaf(pj[i], v[n], acc[i][n]);
+                        }
+                    }
+                }
+            };
+#pragma unroll(P == 1 ? 8 : 2)
+            for (int j4 = 0; j4 < 32; j4 += 4) {
+                float4 p4[P];
+#pragma unroll
+                for (int i = 0; i < P; ++i) {
+                    p4[i] = *reinterpret_cast<const float4*>(ps + min(warp * P + i, pairs - 1) * 32 + j4);
+                }
+                float pj[4][P];
+#pragma unroll
+                for (int i = 0; i < P; ++i) {
+                    pj[0][i] = p4[i].x;
+                    pj[1][i] = p4[i].y;
+                    pj[2][i] = p4[i].z;
+                    pj[3][i] = p4[i].w;
+                }
+                if (whole) {
+#pragma unroll
+                    for (int n = 0; n < 4; ++n) {
+                        weigh(j4 + n, pj[n], false);
+                    }
+                } else {
+#pragma unroll
+                    for (int n = 0; n < 4; ++n) {
+                        weigh(j4 + n, pj[n], true);
+                    }
+                }
+            }
+            __syncwarp();  // (the weights are written anew in the next chunk)
+        }
+        cp_async_wait<0>();
+
+#pragma unroll
+        for (int i = 0; i < P; ++i) {
+            if (!mine[i]) {
+                continue;
+            }
+            const int t = t_begin + (warp * P + i) / group, h = kv_head * group + (warp * P + i) % group;
+            if (a.sinks != nullptr) {
+                const float sink = a.sinks[h];
+                const float m_new = fmaxf(m[i], sink);
+                const float corr = m[i] > -INFINITY ? expf(m[i] - m_new) : 0.0f;
+                l[i] = l[i] * corr + expf(sink - m_new);
+#pragma unroll
+                for (int n = 0; n < ACC; ++n) {
+                    acc[i][n] *= corr;
+                }
+            }
+            float inv = l[i] > 0.0f ? 1.0f / l[i] : 0.0f;
+            if (a.gate != nullptr) {
+                inv *= 1.0f / (1.0f + expf(-a.gate[t * a.gate_row_stride + h]));
+            }
+            float* orow = a.out + t * a.out_row_stride + static_cast<int64_t>(h) * hd;
+#pragma unroll
+            for (int n = 0; n < ACC; ++n) {
+                const int d = lane + 32 * n;
+                if (d < hd) {
+                    orow[d] = acc[i][n] * inv;
+                }
+            }
+        }
+        seg = seg_end;
+    }
+}
+
+template <int P, int ACC, int DIM>
+cudaError_t launch_staged(const StagedParams& a, int n_kv_heads, cudaStream_t stream) {
+    const int pairs = a.run * a.group;
+    const int warps = (pairs + P - 1) / P;
+    const int smem = staged_smem_bytes(pairs, a.head_dim);
+    auto kernel = attention_f32_staged_kernel<P, ACC, DIM>;
+    const cudaError_t set = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (set != cudaSuccess) {
+        return set;
+    }
+    kernel<<<dim3((a.n_tokens + a.run - 1) / a.run, n_kv_heads), warps * 32, smem, stream>>>(a);
+    return cudaGetLastError();
+}
+
 }  // namespace
 
 // q [T, n_heads, head_dim] with q_row_stride elements between tokens; out likewise
@@ -267,6 +578,32 @@ PL_API int pl_attention_simt(const void* q, int64_t q_row_stride, const void* k_
         return 0;
     }
     const int group = n_heads / n_kv_heads;
+    // The staged form takes float32 rows of whole 16-byte pieces up to 128, up to 16 heads a kv head, no mass. Up to
+    // 64 tokens a CTA has one token and a warp one head of it (nothing is shared between a step's single tokens, and a
+    // short portion's few CTAs finish soonest so); beyond, as many neighbouring tokens as make 32 pairs.
+    if (dtype == PL_F32 && mass_sum == nullptr && head_dim % 4 == 0 && head_dim <= kStagedDim && group <= 16 &&
+        page_stride % 4 == 0 && head_stride % 4 == 0 &&
+        ((reinterpret_cast<uintptr_t>(k_pool) | reinterpret_cast<uintptr_t>(v_pool)) & 15) == 0) {
+        const bool few = n_tokens <= 64;
+        const StagedParams a{static_cast<const float*>(q), q_row_stride, static_cast<const float*>(k_pool),
+                             static_cast<const float*>(v_pool), page_stride, head_stride, page_size, n_pages, table,
+                             table_width, pos, entry, static_cast<float*>(out), out_row_stride, n_tokens, group, head_dim,
+                             window, few ? 1 : 32 / group, scale, softcap, sinks, static_cast<const float*>(gate),
+                             gate_row_stride, distance_bias, bias_rows, distance_slopes, keep_first > 0 ? keep_first : 0,
+                             status};
+        const cudaError_t failed =
+            few ? (head_dim == 64    ? launch_staged<1, 2, 64>(a, n_kv_heads, stream)
+                   : head_dim == 128 ? launch_staged<1, 4, 128>(a, n_kv_heads, stream)
+                   : head_dim <= 64  ? launch_staged<1, 2, 0>(a, n_kv_heads, stream)
+                                     : launch_staged<1, 4, 0>(a, n_kv_heads, stream))
+                : (head_dim <= 64 ? launch_staged<4, 2, 0>(a, n_kv_heads, stream)
+                                  : launch_staged<4, 4, 0>(a, n_kv_heads, stream));
+        if (failed != cudaSuccess) {
+            return pl_fail(3, "attention: launch failed: %s", cudaGetErrorString(failed));
+        }
+        PL_CHECK_LAUNCH("attention");
+        return 0;
+    }
     const int warps = group < 8 ? group : 8;
     const size_t smem = static_cast<size_t>(warps) * head_dim * sizeof(float);
     const dim3 grid(n_tokens, n_kv_heads);
