@@ -1,0 +1,450 @@
+// Delta rules over prompt portions in chunks of 16 tokens, bfloat16 engine: what the two recurrent mixers
+// (gated_delta.cu, delta_rule.cu) share.
+//
+// A token's update of a head's state S [dim, vdim] is S <- diag(g) S + k z^T with a row z that itself reads the old
+// state. Over a chunk that starts from S0 the rows solve a unit lower triangular system whose right-hand side
+// is linear in S0 (the WY form of Householder products: Bischof and Van Loan 1987; for delta rules Yang et al.
+// 2024), so with matrices that do not know S0
+//
+//   Z = Zi + Wm S0        [16, vdim]      O = Oi + Qg S0 + M Z      S <- diag(gC) S0 + Kd^T Z (+ Kv^T V)
+//
+// A first kernel makes Zi, Wm, Qg, M, Kd, gC (Oi, Kv) of all chunks side by side, all in fp32, decays between two tokens
+// as running products (never as quotients, nor as differences of long sums of logarithms). The kernel below walks the
+// chunks: one chain step per 16 tokens instead of one per token. A CTA has a head's 16 value columns; warp w of
+// dim / 16 has their 16 state rows from 16 w on, transposed, in the accumulators of m16n8k16 products: that layout is
+// also the A operand's, so the state goes from one product into the next without leaving registers. Every product
+// multiplies fp32 numbers as three bfloat16 terms each (six of the nine products of terms; the rest is below
+// fp32's last bit). The warps' shares of S0's products meet in shared memory, one barrier a chunk; all else
+// lies in the scratch in the order the lanes read it.
+#pragma once
+
+#include "common.cuh"
+
+#include "mma_helpers.cuh"
+
+namespace {
+
+constexpr int kDeltaChunk = 16;
+constexpr int kDeltaWindow = 128;  // chunks of an entry in one pass of the two kernels (bounds the scratch)
+constexpr int kDeltaCols = 16;     // value columns of a CTA of the walk
+
+// Where a chunk's matrices lie in its scratch, in floats. All of it in fragment order. A matrix that is an operand (wm, qg,
+// kd, kv by 16 state rows, m) is three bfloat16 terms: 384 floats, per term the 16 bytes that a lane reads of two 16 x 8 tiles.
+// Of the results' starts (zi, oi) and the packed values (vv) a lane reads 16 bytes per tile of 16 columns.
+struct DeltaChunkLayout {
+    int wm, qg, kd, kv, m, zi, oi, vv, g, floats;
+    __host__ __device__ constexpr DeltaChunkLayout(int dim, int vdim, bool general)
+    : wm(0), qg(24 * dim), kd(48 * dim), kv(72 * dim), m(general ? 96 * dim : 72 * dim), zi(m + 384), oi(zi + 16 * vdim),
+      vv(oi + (general ? 16 * vdim : 0)), g(vv + (general ? 8 * vdim : 0)), floats(g + dim) {}
+};
+
+// While a chunk is put together in shared memory the operands are fp32: 256 floats per 16 state rows, and 256 for m. Every tile
+// of 128 floats takes kStagedTile there, so that a column's places meet fewer banks twice (all starts are whole tiles).
+constexpr int kStagedTile = 136;
+struct DeltaStageLayout {
+    int wm, qg, kd, kv, m, zi, oi, vv, g, floats;
+    __host__ __device__ constexpr DeltaStageLayout(int dim, int vdim, bool general)
+    : wm(0), qg(tiles(16 * dim)), kd(tiles(32 * dim)), kv(tiles(48 * dim)), m(general ? tiles(64 * dim) : kv), zi(m + tiles(256)),
+      oi(zi + tiles(16 * vdim)), vv(oi + (general ? tiles(16 * vdim) : 0)), g(vv + (general ? tiles(8 * vdim) : 0)),
+      floats(g + dim) {}
+    __host__ __device__ static constexpr int tiles(int n) { return n / 128 * kStagedTile; }
+};
+
+// Places in shared memory, each a base of one index and a fixed distance for the other. Element (token t, channel d) of a
+// [16, dim] operand whose k axis is the channel (Wm, Qg) ...
+__device__ __forceinline__ int place_of_channel(int d) {
+    return (d >> 4) * 2 * kStagedTile + (((d & 7) >> 1) << 2) + ((d >> 3 & 1) << 1) + (d & 1);
+}
+__host__ __device__ constexpr int at_token(int t) { return (t >> 3) * kStagedTile + (t & 7) * 16; }
+// ... or the token (Kd, Kv); (for channel 4 l + 32 h + r with r < 4: place_of_quad(l) + at_quad(h, r) more)
+__device__ __forceinline__ int place_of_source(int s) { return (((s & 7) >> 1) << 2) + ((s >> 3) << 1) + (s & 1); }
+__device__ __forceinline__ int place_of_quad(int l) { return (l >> 1) * kStagedTile + (l & 1) * 64; }
+__host__ __device__ constexpr int at_quad(int h, int r) { return h * 4 * kStagedTile + r * 16; }
+// Element (t, s) of M: place_of_source(s) + at_token(t). Element (t, column c) of a result, and the packed values' 32 bits of
+// tokens t, t + 1.
+__device__ __forceinline__ int place_of_column(int c) { return (c >> 4) * 2 * kStagedTile + (c & 7) * 16 + ((c >> 3 & 1) << 1); }
+__host__ __device__ constexpr int at_result(int t) { return (t >> 3) * kStagedTile + ((t & 7) >> 1) * 4 + (t & 1); }
+__device__ __forceinline__ int place_of_value(int c) { return (c >> 4) * kStagedTile + (c & 7) * 16 + (c >> 3 & 1); }
+__host__ __device__ constexpr int at_value(int t) { return ((t & 7) >> 1) * 4 + 2 * (t >> 3); }
+// A channel of gC: 16 floats per 16 state rows, four per lane & 3.
+__device__ __forceinline__ int place_of_decay(int d) {
+    return (d >> 4) * 16 + ((d & 7) >> 1) * 4 + (d >> 3 & 1) * 2 + (d & 1);
+}
+
+// Two fp32 numbers as three pairs of bfloat16.
+__device__ __forceinline__ void three_pairs(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+    hi = pack_bf16(x, y);
+    const float rx = x - __uint_as_float(hi << 16), ry = y - __uint_as_float(hi & 0xffff0000u);
+    mid = pack_bf16(rx, ry);
+    lo = pack_bf16(rx - __uint_as_float(mid << 16), ry - __uint_as_float(mid & 0xffff0000u));
+}
+
+// What was put together leaves for the scratch: the operands (all that comes before zi) as three terms, the others as
+// they are.
+__device__ __forceinline__ void send_chunk(const float* out, float* scratch, const DeltaStageLayout& at, int dim) {
+    const float4* src = reinterpret_cast<const float4*>(out);
+    uint4* dst = reinterpret_cast<uint4*>(scratch);
+    const int groups = at.zi / (2 * kStagedTile);    // (16 state rows of an operand, or m: two tiles)
+    for (int idx = threadIdx.x; idx < groups * 32; idx += blockDim.x) {
+        const int group = idx >> 5, lane = idx & 31;
+        const float4 a = src[group * (kStagedTile / 2) + lane], b = src[group * (kStagedTile / 2) + kStagedTile / 4 + lane];
+        uint4 hi, mid, lo;
+        three_pairs(a.x, a.y, hi.x, mid.x, lo.x);
+        three_pairs(a.z, a.w, hi.y, mid.y, lo.y);
+        three_pairs(b.x, b.y, hi.z, mid.z, lo.z);
+        three_pairs(b.z, b.w, hi.w, mid.w, lo.w);
+        uint4* to = dst + group * 96 + lane;
+        to[0] = hi;
+        to[32] = mid;
+        to[64] = lo;
+    }
+    float4* tail = reinterpret_cast<float4*>(scratch) + groups * 96;
+    const int tiles = (at.g - at.zi) / kStagedTile;
+    for (int idx = threadIdx.x; idx < tiles * 32 + dim / 4; idx += blockDim.x) {
+        tail[idx] = src[at.zi / 4 + idx + min(idx >> 5, tiles) * ((kStagedTile - 128) / 4)];
+    }
+}
+
+// values[i], i < 16, of a whole warp's lanes, summed: the lanes 2 i and 2 i + 1 get sum i.
+__device__ __forceinline__ float sum_over_warp(float (&values)[16]) {
+    const int lane = threadIdx.x & 31;
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const bool upper = lane & 16;
+        const float give = upper ? values[i] : values[i + 8], keep = upper ? values[i + 8] : values[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
+    }
+#pragma unroll
+    for (int n = 4; n >= 1; n >>= 1) {
+        const bool upper = lane & (2 * n);
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            const float give = upper ? v[i] : v[i + n], keep = upper ? v[i + n] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * n);
+        }
+    }
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+// values[i], i < 16, of the eight lanes that share lane >> 3, summed: lane l of them gets sums 2 (l & 7) and the next.
+__device__ __forceinline__ void sum_over_eight(float (&values)[16], float& even, float& odd) {
+    const int l = threadIdx.x & 7;
+    float a[8], b[4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const bool upper = l & 4;
+        const float give = upper ? values[i] : values[i + 8], keep = upper ? values[i + 8] : values[i];
+        a[i] = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const bool upper = l & 2;
+        const float give = upper ? a[i] : a[i + 4], keep = upper ? a[i + 4] : a[i];
+        b[i] = keep + __shfl_xor_sync(0xffffffffu, give, 2);
+    }
+    const bool upper = l & 1;
+    const float give0 = upper ? b[0] : b[2], give1 = upper ? b[1] : b[3];
+    even = (upper ? b[2] : b[0]) + __shfl_xor_sync(0xffffffffu, give0, 1);
+    odd = (upper ? b[3] : b[1]) + __shfl_xor_sync(0xffffffffu, give1, 1);
+}
+
+// Chunks of an entry of `count` rows in pass `pass`.
+__device__ __forceinline__ int delta_chunks_of(int count, int pass) {
+    return max(0, min((count + kDeltaChunk - 1) / kDeltaChunk - pass * kDeltaWindow, kDeltaWindow));
+}
+
+// The entry and its chunk that scratch slot `slot` of this pass belongs to; false past the last. (By a whole warp.)
+__device__ __forceinline__ bool delta_find_chunk(const int32_t* counts, int n_entries, int pass, int slot, int& entry,
+                                                 int& chunk) {
+    const int lane = threadIdx.x & 31;
+    int before = 0;
+    for (int base = 0; base < n_entries; base += 32) {
+        const int mine = base + lane < n_entries ? delta_chunks_of(counts[base + lane], pass) : 0;
+        int upto = mine;
+#pragma unroll
+        for (int offset = 1; offset < 32; offset <<= 1) {
+            const int other = __shfl_up_sync(0xffffffffu, upto, offset);
+            upto += lane >= offset ? other : 0;
+        }
+        const uint32_t past = __ballot_sync(0xffffffffu, before + upto > slot);
+        if (past != 0) {
+            const int who = __ffs(past) - 1;
+            entry = base + who;
+            chunk = slot - before - __shfl_sync(0xffffffffu, upto - mine, who);
+            return true;
+        }
+        before += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    return false;
+}
+
+// Chunks before entry `entry` in this pass. (By a whole warp.)
+__device__ __forceinline__ int delta_chunks_before(const int32_t* counts, int entry, int pass) {
+    int sum = 0;
+    for (int e = threadIdx.x & 31; e < entry; e += 32) {
+        sum += delta_chunks_of(counts[e], pass);
+    }
+#pragma unroll
+    for (int offset = 16; offset > 0; offset >>= 1) {
+        sum += __shfl_xor_sync(0xffffffffu, sum, offset);
+    }
+    return sum;
+}
+
+struct DeltaChainParams {
+    const float* scratch;
+    float* state;
+    const int32_t* first_rows;
+    const int32_t* counts;
+    const int32_t* slots;
+    float* o_raw;
+    int n_heads, vdim, pass;
+};
+
+struct TermsA {
+    uint32_t t[3][4];  // hi, mid, lo
+};
+struct TermsB {
+    uint4 t[3];        // two tiles' registers of each term
+};
+__device__ __forceinline__ void terms_of(TermsA& a, const float (&lo8)[4], const float (&hi8)[4]) {
+    three_pairs(lo8[0], lo8[1], a.t[0][0], a.t[1][0], a.t[2][0]);
+    three_pairs(lo8[2], lo8[3], a.t[0][1], a.t[1][1], a.t[2][1]);
+    three_pairs(hi8[0], hi8[1], a.t[0][2], a.t[1][2], a.t[2][2]);
+    three_pairs(hi8[2], hi8[3], a.t[0][3], a.t[1][3], a.t[2][3]);
+}
+// d0, d1 += a b's two tiles, the small products first.
+__device__ __forceinline__ void mma_terms(float (&d0)[4], float (&d1)[4], const TermsA& a, const TermsB& b) {
+    constexpr int kA[6] = {2, 0, 1, 1, 0, 0}, kB[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        mma_bf16(d0, a.t[kA[i]], b.t[kB[i]].x, b.t[kB[i]].y);
+        mma_bf16(d1, a.t[kA[i]], b.t[kB[i]].z, b.t[kB[i]].w);
+    }
+}
+
+// What a lane needs of a chunk, a chunk ahead of its use in registers (through shared memory it would pass the same ports
+// twice, which bound a first form of this kernel).
+template <bool GENERAL>
+struct DeltaLane {
+    TermsB wm, qg, kd, m, kv;
+    float4 zi[2], oi, g;
+    uint4 vv;
+};
+
+// grid (entries, heads, vdim / 16), NW = dim / 16 warps. On the path from a chunk to the next are only Z's products, their sum
+// over the warps, and the state's update; O's products fill the waits between and are added up a chunk later.
+template <int NW, bool GENERAL>
+__global__ void __launch_bounds__(NW * 32) delta_chain_kernel(const DeltaChainParams p) {
+    pl_grid_trigger();
+    pl_grid_wait();
+    constexpr int kDim = NW * 16;
+    __shared__ float4 shares[2][4][NW][32];  // by chunk parity: two tiles of Z, two of O
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int e = blockIdx.x, head = blockIdx.y, ct = blockIdx.z;
+    const int count = p.counts[e];
+    const int n_chunks = delta_chunks_of(count, p.pass);
+    if (n_chunks == 0) {
+        return;
+    }
+    const DeltaChunkLayout at(kDim, p.vdim, GENERAL);
+    constexpr DeltaChunkLayout kAt(kDim, 0, GENERAL);  // (the places up to zi hold for any vdim)
+    const int64_t step = static_cast<int64_t>(p.n_heads) * at.floats;
+    const float* chunk0 = p.scratch + (static_cast<int64_t>(delta_chunks_before(p.counts, e, p.pass)) * p.n_heads + head) * at.floats;
+    const float* src = chunk0 + w * 384 + lane * 4;
+    const float* src_m = chunk0 + kAt.m + lane * 4;
+    const float* src_zi = chunk0 + kAt.zi + (ct * 2 * 32 + lane) * 4;
+    const float* src_oi = chunk0 + at.oi + ((ct * 2 + w) * 32 + lane) * 4;
+    const float* src_vv = chunk0 + at.vv + (ct * 32 + lane) * 4;
+    const float* src_g = chunk0 + at.g + w * 16 + (lane & 3) * 4;
+    auto fetch = [&](DeltaLane<GENERAL>& in) {
+        auto terms = [](TermsB& b, const float* from) {
+#pragma unroll
+            for (int term = 0; term < 3; ++term) {
+                b.t[term] = *reinterpret_cast<const uint4*>(from + term * 128);
+            }
+        };
+        terms(in.wm, src);
+        terms(in.qg, src + kAt.qg);
+        terms(in.kd, src + kAt.kd);
+        in.zi[0] = *reinterpret_cast<const float4*>(src_zi);
+        in.zi[1] = *reinterpret_cast<const float4*>(src_zi + 128);
+        in.g = *reinterpret_cast<const float4*>(src_g);
+        if (w < 2) {
+            terms(in.m, src_m);
+        }
+        if constexpr (GENERAL) {
+            terms(in.kv, src + kAt.kv);
+            in.vv = *reinterpret_cast<const uint4*>(src_vv);
+            if (w < 2) {
+                in.oi = *reinterpret_cast<const float4*>(src_oi);
+            }
+            src_vv += step;
+            src_oi += step;
+        }
+        src += step;
+        src_m += step;
+        src_zi += step;
+        src_g += step;
+    };
+    DeltaLane<GENERAL> even = {}, odd = {};
+    fetch(even);
+
+    // S transposed: s[j][r] is column ct * 16 + lane / 4 (+ 8 for r >= 2), row w * 16 + 8 j + (lane % 4) * 2 + r % 2.
+    float s[2][4];
+    float* corner = p.state + ((static_cast<int64_t>(p.slots[e]) * p.n_heads + head) * kDim + w * 16 + (lane & 3) * 2) * p.vdim +
+        ct * kDeltaCols + (lane >> 2);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            s[j][r] = corner[static_cast<int64_t>(8 * j + (r & 1)) * p.vdim + (r >> 1) * 8];
+        }
+    }
+    // This lane's outputs: columns lane / 4 and 8 on, tokens 8 w + (lane % 4) * 2 and the next (of the first two warps).
+    const int rows = count - p.pass * kDeltaWindow * kDeltaChunk;
+    const int64_t o_stride = static_cast<int64_t>(p.n_heads) * p.vdim;
+    int token = w * 8 + (lane & 3) * 2;
+    float* dst = p.o_raw + (p.first_rows[e] + p.pass * kDeltaWindow * kDeltaChunk + token) * o_stride +
+        static_cast<int64_t>(head) * p.vdim + ct * kDeltaCols + (lane >> 2);
+    float o[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    auto finish = [&](int parity) {
+#pragma unroll
+        for (int other = 0; other < NW; ++other) {
+            const float4 part = shares[parity][2 + w][other][lane];
+            o[0] += part.x;
+            o[1] += part.y;
+            o[2] += part.z;
+            o[3] += part.w;
+        }
+        if (token < rows) {
+            dst[0] = o[0];
+            dst[8] = o[2];
+        }
+        if (token + 1 < rows) {
+            dst[o_stride] = o[1];
+            dst[o_stride + 8] = o[3];
+        }
+        token += kDeltaChunk;
+        dst += kDeltaChunk * o_stride;
+    };
+
+    auto advance = [&](const DeltaLane<GENERAL>& in, DeltaLane<GENERAL>& ahead, int c, const int parity) {
+        if (c + 1 < n_chunks) {
+            fetch(ahead);
+        }
+        TermsA a, az;
+        terms_of(a, s[0], s[1]);
+        float d[2][4] = {};
+        mma_terms(d[0], d[1], a, in.wm);  // this warp's rows' share of S0's part of Z
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            shares[parity][j][w][lane] = make_float4(d[j][0], d[j][1], d[j][2], d[j][3]);
+        }
+        const float decay[2][2] = {{in.g.x, in.g.y}, {in.g.z, in.g.w}};
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                s[j][r] *= decay[j][r & 1];
+            }
+        }
+        if constexpr (GENERAL) {  // + Kv^T V: the values are bfloat16 as they are
+            const uint32_t v[4] = {in.vv.x, in.vv.y, in.vv.z, in.vv.w};
+#pragma unroll
+            for (int term = 2; term >= 0; --term) {
+                mma_bf16(s[0], v, in.kv.t[term].x, in.kv.t[term].y);
+                mma_bf16(s[1], v, in.kv.t[term].z, in.kv.t[term].w);
+            }
+        }
+        __syncthreads();
+        float z[2][4];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            z[j][0] = in.zi[j].x;
+            z[j][1] = in.zi[j].y;
+            z[j][2] = in.zi[j].z;
+            z[j][3] = in.zi[j].w;
+#pragma unroll
+            for (int other = 0; other < NW; ++other) {
+                const float4 part = shares[parity][j][other][lane];
+                z[j][0] += part.x;
+                z[j][1] += part.y;
+                z[j][2] += part.z;
+                z[j][3] += part.w;
+            }
+        }
+        float q[2][4] = {};
+        mma_terms(q[0], q[1], a, in.qg);  // (and of O: made while the sums of Z come in, read after the next barrier)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            shares[parity][2 + j][w][lane] = make_float4(q[j][0], q[j][1], q[j][2], q[j][3]);
+        }
+        terms_of(az, z[0], z[1]);
+        mma_terms(s[0], s[1], az, in.kd);
+        if (w < 2) {
+            if (c > 0) {
+                finish(parity ^ 1);  // the chunk before: its shares were written before this chunk's barrier
+            }
+            float half[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            if constexpr (GENERAL) {
+                o[0] = in.oi.x;
+                o[1] = in.oi.y;
+                o[2] = in.oi.z;
+                o[3] = in.oi.w;
+            } else {
+                o[0] = o[1] = o[2] = o[3] = 0.0f;
+            }
+            constexpr int kA[6] = {2, 0, 1, 1, 0, 0}, kB[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+            for (int i = 0; i < 6; ++i) {
+                const uint4 b = in.m.t[kB[i]];
+                mma_bf16(i % 2 ? o : half, az.t[kA[i]], w == 0 ? b.x : b.z, w == 0 ? b.y : b.w);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                o[i] += half[i];
+            }
+        }
+    };
+    for (int c = 0; c < n_chunks; c += 2) {
+        advance(even, odd, c, 0);
+        if (c + 1 < n_chunks) {
+            advance(odd, even, c + 1, 1);
+        }
+    }
+    __syncthreads();
+    if (w < 2) {
+        finish((n_chunks - 1) & 1);
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            corner[static_cast<int64_t>(8 * j + (r & 1)) * p.vdim + (r >> 1) * 8] = s[j][r];
+        }
+    }
+}
+
+template <int NW, bool GENERAL>
+cudaError_t launch_delta_chain(const DeltaChainParams& p, int n_entries, cudaStream_t stream) {
+    return pl_launch_overlapped(delta_chain_kernel<NW, GENERAL>, dim3(n_entries, p.n_heads, p.vdim / kDeltaCols), dim3(NW * 32), 0,
+                                stream, p);
+}
+
+// Whether a step's portions go in chunks: bfloat16, sizes that fill the fragments, and more than a few tokens an
+// entry.
+inline bool delta_takes_chunks(int n_tokens, int n_entries, int dim, int vdim, int dtype) {
+    return dtype == PL_BF16 && (dim == 32 || dim == 64 || dim == 128) && vdim % kDeltaCols == 0 && vdim <= 256 &&
+        n_tokens > 2 * n_entries && n_tokens - n_entries >= 32;
+}
+// Slots for chunks in a pass, and passes, at most.
+inline int64_t delta_chunk_slots(int n_tokens, int n_entries) {
+    const int64_t all = static_cast<int64_t>(n_tokens) / kDeltaChunk + n_entries;
+    const int64_t most = static_cast<int64_t>(n_entries) * kDeltaWindow;
+    return all < most ? all : most;
+}
+inline int delta_passes(int n_tokens) { return (n_tokens + kDeltaWindow * kDeltaChunk - 1) / (kDeltaWindow * kDeltaChunk); }
+
+}  // namespace

@@ -29,6 +29,7 @@
 // busy and takes about a microsecond a token whatever the width.
 #include "common.cuh"
 
+#include "delta_chunks.cuh"
 #include "mma_helpers.cuh"
 
 namespace {
@@ -403,6 +404,286 @@ void launch_scan(const ScanParams& p, dim3 grid, int threads, size_t smem, cudaS
     }
 }
 
+// ---------------------------------------------------------------------------- portions in chunks
+// The matrices of one chunk (delta_chunks.cuh) of one head, by a CTA. What a token removes, z_t = S_{t-1}^T u_t, is the row
+// that the chunk solves for (Z is its negative): with p = a * u, G_t the product of the decays up to token t of the chunk and
+// e_ts that of the tokens after s up to t,
+//   Lk_ts = sum_i u_ti e_(t-1)si k_si, Lp_ts likewise with p (s < t);  Mk_ts = sum_i r_ti e_tsi k_si, M_ts with p (s <= t)
+//   (I + Lp) X = (G_(t-1) u | Lk v):  Wm and Zi are -X's two parts;  Oi = Mk v,  Qg = G r,  Kd_s = e_15,s p_s,
+//   Kv_s = e_15,s k_s,  gC = G_15.
+// A column of X is one thread's. Rows past the portion's last decay by 1 and add nothing.
+struct RuleChunkParams {
+    ScanParams in;
+    int n_entries, pass;
+    float* scratch;
+};
+
+template <int DIM>
+constexpr int rule_chunk_smem() {
+    return (5 * 16 * (DIM + 4) + 4 * 256 + DeltaStageLayout(DIM, DIM, true).floats) * 4;
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(128) delta_rule_chunk_kernel(const RuleChunkParams c) {
+    pl_grid_trigger();
+    pl_grid_wait();
+    constexpr int kLd = DIM + 4;
+    const ScanParams& p = c.in;
+    extern __shared__ __align__(16) float chunk_smem[];
+    float* su = chunk_smem;          // [16][kLd] each
+    float* sk = su + 16 * kLd;
+    float* sp = sk + 16 * kLd;
+    float* sr = sp + 16 * kLd;
+    float* sw = sr + 16 * kLd;       // a token's decay
+    float* Lp = sw + 16 * kLd;       // [16][16]
+    float* Lk = Lp + 256;
+    float* M = Lk + 256;
+    float* Mk = M + 256;
+    float* out = Mk + 256;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int head = blockIdx.y;
+    int e, chunk;
+    if (!delta_find_chunk(p.counts, c.n_entries, c.pass, blockIdx.x, e, chunk)) {
+        return;
+    }
+    const int done = (c.pass * kDeltaWindow + chunk) * kDeltaChunk;
+    const int n = min(kDeltaChunk, p.counts[e] - done);
+    const int64_t t0 = p.first_rows[e] + done;
+    const int64_t hoff = static_cast<int64_t>(head) * DIM;
+    const __nv_bfloat16* r = static_cast<const __nv_bfloat16*>(p.r) + hoff;
+    const __nv_bfloat16* k = static_cast<const __nv_bfloat16*>(p.k) + hoff;
+    const __nv_bfloat16* v = static_cast<const __nv_bfloat16*>(p.v) + hoff;
+    const __nv_bfloat16* a_pre = static_cast<const __nv_bfloat16*>(p.a_pre) + hoff;
+    const __nv_bfloat16* w_pre = static_cast<const __nv_bfloat16*>(p.w_pre) + hoff;
+
+    // A warp has four tokens, a lane DIM / 32 channels of each. All of a lane's loads set out before anything is stored.
+    constexpr int kPer = DIM / 32;
+    float kv[4][kPer], rv[4][kPer], av[4][kPer], wv[4][kPer], w0[kPer], a0[kPer], sums[16];
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        w0[j] = p.w0[hoff + lane + 32 * j];
+        a0[j] = p.a0[hoff + lane + 32 * j];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int t = warp * 4 + q;
+        const bool there = t < n;
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const int i = lane + 32 * j;
+            kv[q][j] = there ? pl_load(k + (t0 + t) * p.row_stride + i) : 0.0f;
+            rv[q][j] = there ? pl_load(r + (t0 + t) * p.row_stride + i) : 0.0f;
+            av[q][j] = there ? pl_load(a_pre + (t0 + t) * p.row_stride + i) : 0.0f;
+            wv[q][j] = there ? pl_load(w_pre + (t0 + t) * p.w_row_stride + i) : 0.0f;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const bool there = warp * 4 + q < n;
+        sums[q] = sums[4 + q] = sums[8 + q] = sums[12 + q] = 0.0f;
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            av[q][j] = there ? sigmoid_f32(av[q][j] + a0[j]) * kv[q][j] : 0.0f;  // (times the unit factor: a u)
+            wv[q][j] = there ? expf(-p.decay_scale * sigmoid_f32(wv[q][j] + w0[j])) : 1.0f;
+            sums[q] = fmaf(kv[q][j], kv[q][j], sums[q]);
+            sums[4 + q] = fmaf(rv[q][j], kv[q][j], sums[4 + q]);
+            sums[8 + q] = fmaf(rv[q][j], av[q][j], sums[8 + q]);
+        }
+    }
+    const float sum = sum_over_warp(sums);
+    const float inv = 1.0f / sqrtf(fabsf(sum) + p.unit_eps);  // (read of the lanes below 8)
+    const float inv_mine = __shfl_sync(0xffffffffu, inv, lane & 7);
+    if (lane >= 8 && lane < 24) {
+        const int t = warp * 4 + (lane >> 1 & 3);
+        (lane < 16 ? Mk : M)[t * 16 + t] = lane < 16 ? sum : sum * inv_mine;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int t = warp * 4 + q;
+        const float unit = __shfl_sync(0xffffffffu, inv, 2 * q);
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const int i = lane + 32 * j;
+            su[t * kLd + i] = kv[q][j] * unit;
+            sk[t * kLd + i] = kv[q][j];
+            sp[t * kLd + i] = av[q][j] * unit;
+            sr[t * kLd + i] = rv[q][j];
+            sw[t * kLd + i] = wv[q][j];
+        }
+        if (lane > t && lane < 16) {
+            M[t * 16 + lane] = 0.0f;
+            Mk[t * 16 + lane] = 0.0f;
+        }
+    }
+    // This thread's column of the values, if it has one, for later (128 threads, 2 DIM columns in all: one at most).
+    __nv_bfloat16 column[16];
+    const int early = tid - DIM % 128;
+    const bool values = early >= 0 && early < DIM;
+#pragma unroll
+    for (int t = 0; t < 16; ++t) {
+        column[t] = values && t < n ? v[(t0 + t) * p.row_stride + early] : __float2bfloat16_rn(0.0f);
+    }
+    __syncthreads();
+    // Token s of the chunk is eight lanes', DIM / 8 channels each: its key and what it removes decay from token to token in
+    // registers and meet every later u (before that token's decay) and r (after it) on the way.
+    constexpr DeltaChunkLayout sent(DIM, DIM, true);
+    constexpr DeltaStageLayout at(DIM, DIM, true);
+    {
+        constexpr int kQuads = DIM / 32;
+        const int s = warp + (lane >> 3) * 4, first = (lane & 7) * 4;
+        const int mine = place_of_source(s) + place_of_quad(lane & 7);
+        float xk[kQuads][4], xp[kQuads][4], lk[16], lp[16], mk[16], mp[16];
+        auto quad = [&](const float* rows, int t, int h, float (&to)[4]) {
+            const float4 v4 = *reinterpret_cast<const float4*>(rows + t * kLd + first + 32 * h);
+            to[0] = v4.x;
+            to[1] = v4.y;
+            to[2] = v4.z;
+            to[3] = v4.w;
+        };
+#pragma unroll
+        for (int h = 0; h < kQuads; ++h) {
+            quad(sk, s, h, xk[h]);
+            quad(sp, s, h, xp[h]);
+        }
+        lk[0] = lp[0] = mk[0] = mp[0] = 0.0f;
+#pragma unroll
+        for (int t = 1; t < 16; ++t) {
+            lk[t] = lp[t] = mk[t] = mp[t] = 0.0f;
+            if (t > s) {
+#pragma unroll
+                for (int h = 0; h < kQuads; ++h) {
+                    float u[4], r4[4], w4[4];
+                    quad(su, t, h, u);
+                    quad(sr, t, h, r4);
+                    quad(sw, t, h, w4);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        lk[t] = fmaf(u[j], xk[h][j], lk[t]);
+                        lp[t] = fmaf(u[j], xp[h][j], lp[t]);
+                        xk[h][j] *= w4[j];
+                        xp[h][j] *= w4[j];
+                        mk[t] = fmaf(r4[j], xk[h][j], mk[t]);
+                        mp[t] = fmaf(r4[j], xp[h][j], mp[t]);
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < kQuads; ++h) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                out[at.kd + mine + at_quad(h, j)] = xp[h][j];
+                out[at.kv + mine + at_quad(h, j)] = xk[h][j];
+            }
+        }
+        float a[2][4];
+        sum_over_eight(lk, a[0][0], a[1][0]);
+        sum_over_eight(lp, a[0][1], a[1][1]);
+        sum_over_eight(mk, a[0][2], a[1][2]);
+        sum_over_eight(mp, a[0][3], a[1][3]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int t = 2 * (lane & 7) + j;
+            Lk[t * 16 + s] = a[j][0];
+            Lp[t * 16 + s] = a[j][1];
+            if (t > s) {
+                Mk[t * 16 + s] = a[j][2];
+                M[t * 16 + s] = a[j][3];
+            }
+        }
+    }
+    __syncthreads();
+    for (int j = tid; j < 2 * DIM; j += 128) {
+        float x[16];
+        const int col = j - DIM;
+        const int mine = j < DIM ? place_of_channel(j) : place_of_column(col);
+        if (j < DIM) {
+            float G = 1.0f;
+#pragma unroll
+            for (int t = 0; t < 16; ++t) {
+                x[t] = G * su[t * kLd + j];
+                G *= sw[t * kLd + j];
+                out[at.qg + mine + at_token(t)] = G * sr[t * kLd + j];
+            }
+            out[at.g + place_of_decay(j)] = G;
+        } else {
+            float vv[16], o[16];
+#pragma unroll
+            for (int t = 0; t < 16; ++t) {
+                vv[t] = __bfloat162float(column[t]);
+            }
+            // the values as an A operand: lane (column % 8) * 4 + pair of tokens % 4, register column / 8 + 2 (token / 8)
+            uint32_t* packed = reinterpret_cast<uint32_t*>(out);
+#pragma unroll
+            for (int t = 0; t < 16; ++t) {
+                float z = 0.0f;
+                o[t] = Mk[t * 16 + t] * vv[t];
+                float lrow[16], mrow[16];
+#pragma unroll
+                for (int s = 0; s < t; s += 4) {
+                    *reinterpret_cast<float4*>(lrow + s) = *reinterpret_cast<const float4*>(Lk + t * 16 + s);
+                    *reinterpret_cast<float4*>(mrow + s) = *reinterpret_cast<const float4*>(Mk + t * 16 + s);
+                }
+#pragma unroll
+                for (int s = 0; s < t; ++s) {
+                    z = fmaf(lrow[s], vv[s], z);
+                    o[t] = fmaf(mrow[s], vv[s], o[t]);
+                }
+                x[t] = z;
+            }
+#pragma unroll
+            for (int t = 0; t < 16; t += 2) {
+                *reinterpret_cast<float2*>(out + at.oi + mine + at_result(t)) = make_float2(o[t], o[t + 1]);
+                const __nv_bfloat162 two(column[t], column[t + 1]);
+                packed[at.vv + place_of_value(col) + at_value(t)] = *reinterpret_cast<const uint32_t*>(&two);
+            }
+        }
+#pragma unroll
+        for (int t = 1; t < 16; ++t) {
+            float row[16];
+#pragma unroll
+            for (int s = 0; s < t; s += 4) {
+                *reinterpret_cast<float4*>(row + s) = *reinterpret_cast<const float4*>(Lp + t * 16 + s);
+            }
+#pragma unroll
+            for (int s = 0; s < t; ++s) {
+                x[t] = fmaf(-row[s], x[s], x[t]);
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < 16; t += 2) {
+            if (j < DIM) {
+                out[at.wm + mine + at_token(t)] = -x[t];
+                out[at.wm + mine + at_token(t + 1)] = -x[t + 1];
+            } else {
+                *reinterpret_cast<float2*>(out + at.zi + mine + at_result(t)) = make_float2(-x[t], -x[t + 1]);
+            }
+        }
+    }
+    for (int idx = tid; idx < 256; idx += 128) {
+        out[at.m + place_of_source(idx % 16) + at_token(idx / 16)] = M[idx];
+    }
+    __syncthreads();
+    send_chunk(out, c.scratch + (static_cast<int64_t>(blockIdx.x) * p.n_heads + head) * sent.floats, at, DIM);
+}
+
+template <int DIM>
+cudaError_t launch_rule_chunks(const RuleChunkParams& c, int64_t slots, cudaStream_t stream) {
+    constexpr int kSmem = rule_chunk_smem<DIM>();
+    const cudaError_t set = cudaFuncSetAttribute(delta_rule_chunk_kernel<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    if (set != cudaSuccess) {
+        return set;
+    }
+    const cudaError_t made = pl_launch_overlapped(delta_rule_chunk_kernel<DIM>, dim3(static_cast<unsigned>(slots), c.in.n_heads),
+                                                  dim3(128), kSmem, stream, c);
+    if (made != cudaSuccess) {
+        return made;
+    }
+    const DeltaChainParams chain{c.scratch, c.in.state, c.in.first_rows, c.in.counts, c.in.slots, c.in.o_raw, c.in.n_heads,
+                                 DIM, c.pass};
+    return launch_delta_chain<DIM / 16, true>(chain, c.n_entries, stream);
+}
+
 // A warp per (token, head): out = o * rsqrt(mean(o^2) + eps) * norm * sigmoid(g).
 template <typename scalar_t>
 __global__ void delta_rule_finish_kernel(const float* __restrict__ o_raw, const scalar_t* __restrict__ g,
@@ -500,6 +781,51 @@ PL_API int pl_delta_rule(const void* r, const void* k, const void* v, const void
                              0, stream, static_cast<const float*>(o_raw), static_cast<const scalar_t*>(g), row_stride,
                              norm, static_cast<scalar_t*>(out), out_row_stride, n_tokens, n_heads, dim, eps);
     });
+    PL_CHECK_LAUNCH("delta_rule_finish");
+    return 0;
+}
+
+// Floats of scratch that pl_delta_rule_chunks needs, 0 where the step's portions are walked token by token.
+PL_API int64_t pl_delta_rule_chunk_floats(int n_tokens, int n_entries, int n_heads, int dim, int dtype) {
+    if (n_tokens <= 0 || n_entries <= 0 || n_heads <= 0 || !delta_takes_chunks(n_tokens, n_entries, dim, dim, dtype)) {
+        return 0;
+    }
+    return delta_chunk_slots(n_tokens, n_entries) * n_heads * DeltaChunkLayout(dim, dim, true).floats;
+}
+
+// pl_delta_rule in chunks of 16 tokens (bfloat16). scratch: pl_delta_rule_chunk_floats floats on 16 bytes.
+PL_API int pl_delta_rule_chunks(const void* r, const void* k, const void* v, const void* g, const void* a_pre,
+                                int64_t row_stride, const void* w_pre, int64_t w_row_stride, const float* w0,
+                                const float* a0, const float* norm, float* state, const int32_t* first_rows,
+                                const int32_t* counts, const int32_t* slots, float* o_raw, float* scratch, void* out,
+                                int64_t out_row_stride, int n_tokens, int n_entries, int n_heads, int dim,
+                                float decay_scale, float unit_eps, float eps, cudaStream_t stream) {
+    PL_REQUIRE(n_heads > 0 && n_heads <= 65535, "delta_rule: bad heads=%d", n_heads);
+    PL_REQUIRE(delta_takes_chunks(n_tokens, n_entries, dim, dim, PL_BF16),
+               "delta_rule: tokens=%d entries=%d dim=%d do not go in chunks", n_tokens, n_entries, dim);
+    PL_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 15) == 0, "delta_rule: the scratch must start on 16 bytes");
+    RuleChunkParams c = {};
+    ScanParams& p = c.in;
+    p.r = r; p.k = k; p.v = v; p.a_pre = a_pre; p.row_stride = row_stride;
+    p.w_pre = w_pre; p.w_row_stride = w_row_stride; p.w0 = w0; p.a0 = a0; p.state = state;
+    p.first_rows = first_rows; p.counts = counts; p.slots = slots; p.o_raw = o_raw;
+    p.n_heads = n_heads; p.dim = dim; p.decay_scale = decay_scale; p.unit_eps = unit_eps;
+    c.n_entries = n_entries;
+    c.scratch = scratch;
+    const int64_t n_slots = delta_chunk_slots(n_tokens, n_entries);
+    cudaError_t made = cudaSuccess;
+    for (c.pass = 0; c.pass < delta_passes(n_tokens) && made == cudaSuccess; ++c.pass) {
+        made = dim == 32 ? launch_rule_chunks<32>(c, n_slots, stream)
+             : dim == 64 ? launch_rule_chunks<64>(c, n_slots, stream)
+                         : launch_rule_chunks<128>(c, n_slots, stream);
+    }
+    if (made != cudaSuccess) {
+        return pl_fail(3, "delta_rule: launch failed: %s", cudaGetErrorString(made));
+    }
+    const int64_t pairs = static_cast<int64_t>(n_tokens) * n_heads;
+    pl_launch_overlapped(delta_rule_finish_kernel<__nv_bfloat16>, dim3(static_cast<unsigned>((pairs + 3) / 4)), dim3(128),
+                         0, stream, static_cast<const float*>(o_raw), static_cast<const __nv_bfloat16*>(g), row_stride,
+                         norm, static_cast<__nv_bfloat16*>(out), out_row_stride, n_tokens, n_heads, dim, eps);
     PL_CHECK_LAUNCH("delta_rule_finish");
     return 0;
 }

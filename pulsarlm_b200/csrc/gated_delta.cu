@@ -24,6 +24,7 @@
 // or on the rest of the batch.
 #include "common.cuh"
 
+#include "delta_chunks.cuh"
 #include "mma_helpers.cuh"
 
 namespace {
@@ -665,6 +666,247 @@ __global__ void __launch_bounds__(128) gated_delta_scan_static_single_kernel(con
     }
 }
 
+// ---------------------------------------------------------------------------- portions in chunks
+// The matrices of one chunk (delta_chunks.cuh) of one head, by a CTA: with G_t the product of the decays up to token
+// t of the chunk and e_ts that of the tokens after s up to t,
+//   L_ts = b_t sum_i k^_ti e_tsi k^_si (s < t),  M_ts = sum_i q^_ti e_tsi k^_si (s <= t)
+//   (I + L) X = b (G k^ | v):  Wm = -X's first part, Zi the second;  Qg = G q^,  Kd_s = e_15,s k^_s,  gC = G_15.
+// A column of X is one thread's. Rows past the portion's last decay by 1 and add nothing.
+struct GatedChunkParams {
+    GatedDeltaParams in;
+    int n_entries, pass;
+    float* scratch;
+};
+
+template <int DIM>
+constexpr int gated_chunk_smem(int vdim) {
+    return (3 * 16 * (DIM + 4) + 2 * 256 + 16 + DeltaStageLayout(DIM, vdim, false).floats) * 4;
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(128) gated_delta_chunk_kernel(const GatedChunkParams c) {
+    pl_grid_trigger();
+    pl_grid_wait();
+    constexpr int kLd = DIM + 4;
+    const GatedDeltaParams& p = c.in;
+    extern __shared__ __align__(16) float chunk_smem[];
+    float* sk = chunk_smem;          // [16][kLd] each
+    float* sq = sk + 16 * kLd;
+    float* sg = sq + 16 * kLd;       // a token's decay
+    float* L = sg + 16 * kLd;        // [16][16] b_t L_ts
+    float* M = L + 256;
+    float* sb = M + 256;             // [16]
+    float* out = sb + 16;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int head = blockIdx.y;
+    int e, chunk;
+    if (!delta_find_chunk(p.counts, c.n_entries, c.pass, blockIdx.x, e, chunk)) {
+        return;
+    }
+    const int done = (c.pass * kDeltaWindow + chunk) * kDeltaChunk;
+    const int n = min(kDeltaChunk, p.counts[e] - done);
+    const int64_t t0 = p.first_rows[e] + done;
+    const int qk_head = head / (p.n_heads / p.qk_heads);
+    const __nv_bfloat16* q = static_cast<const __nv_bfloat16*>(p.q) + static_cast<int64_t>(qk_head) * DIM;
+    const __nv_bfloat16* k = static_cast<const __nv_bfloat16*>(p.k) + static_cast<int64_t>(qk_head) * DIM;
+    const __nv_bfloat16* v = static_cast<const __nv_bfloat16*>(p.v) + static_cast<int64_t>(head) * p.vdim;
+    const __nv_bfloat16* a_pre = static_cast<const __nv_bfloat16*>(p.a_pre) + static_cast<int64_t>(head) * DIM;
+    const __nv_bfloat16* b_pre = static_cast<const __nv_bfloat16*>(p.b_pre) + head;
+    const float rate = expf(p.a_log[head]);
+
+    // A warp has four tokens, a lane DIM / 32 channels of each. All of a lane's loads set out before anything is stored.
+    constexpr int kPer = DIM / 32;
+    float qv[4][kPer], kv[4][kPer], gv[4][kPer], bias[kPer], sums[16];
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        bias[j] = p.dt_bias[static_cast<int64_t>(head) * DIM + lane + 32 * j];
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int t = warp * 4 + r;
+        const bool there = t < n;
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const int i = lane + 32 * j;
+            qv[r][j] = there ? pl_load(q + (t0 + t) * p.qkv_stride + i) : 0.0f;
+            kv[r][j] = there ? pl_load(k + (t0 + t) * p.qkv_stride + i) : 0.0f;
+            gv[r][j] = there ? pl_load(a_pre + (t0 + t) * p.a_stride + i) : 0.0f;
+        }
+    }
+    // (lanes 2 r, 2 r + 1 of every eight: token r's b)
+    const int mine_t = warp * 4 + (lane >> 1 & 3);
+    float b = mine_t < n ? pl_load(b_pre + (t0 + mine_t) * p.b_stride) : 0.0f;
+    b = mine_t < n ? 1.0f / (1.0f + expf(-b)) : 0.0f;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        sums[r] = sums[4 + r] = sums[8 + r] = sums[12 + r] = 0.0f;
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            sums[r] = fmaf(qv[r][j], qv[r][j], sums[r]);
+            sums[4 + r] = fmaf(kv[r][j], kv[r][j], sums[4 + r]);
+            sums[8 + r] = fmaf(qv[r][j], kv[r][j], sums[8 + r]);
+            gv[r][j] = warp * 4 + r < n ? expf(-rate * softplus_f32(gv[r][j] + bias[j])) : 1.0f;
+        }
+    }
+    const float sum = sum_over_warp(sums);
+    const float inv = (lane < 8 ? p.q_scale : 1.0f) / sqrtf(fabsf(sum) + p.unit_eps);  // (read of the lanes below 16)
+    const float inv_qk = __shfl_sync(0xffffffffu, inv, lane & 7) * __shfl_sync(0xffffffffu, inv, 8 + (lane & 7));
+    if (lane >= 16 && lane < 24) {
+        const int t = warp * 4 + (lane >> 1 & 3);
+        M[t * 16 + t] = sum * inv_qk;
+        sb[t] = b;
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int t = warp * 4 + r;
+        const float inv_q = __shfl_sync(0xffffffffu, inv, 2 * r), inv_k = __shfl_sync(0xffffffffu, inv, 8 + 2 * r);
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const int i = lane + 32 * j;
+            sq[t * kLd + i] = qv[r][j] * inv_q;
+            sk[t * kLd + i] = kv[r][j] * inv_k;
+            sg[t * kLd + i] = gv[r][j];
+        }
+        if (lane > t && lane < 16) {
+            M[t * 16 + lane] = 0.0f;
+        }
+    }
+    // This thread's first column of the values, if it has one, for later.
+    __nv_bfloat16 column[16];
+    const int early = tid - DIM % 128;
+    const bool values = early >= 0 && early < p.vdim;
+#pragma unroll
+    for (int t = 0; t < 16; ++t) {
+        column[t] = values && t < n ? v[(t0 + t) * p.qkv_stride + early] : __float2bfloat16_rn(0.0f);
+    }
+    __syncthreads();
+    // Token s of the chunk is eight lanes', DIM / 8 channels each: its key decays from token to token in registers and meets
+    // every later key and query on the way (rows s, s + 4, s + 8, s + 12 share a warp).
+    const DeltaChunkLayout sent(DIM, p.vdim, false);
+    const DeltaStageLayout at(DIM, p.vdim, false);
+    {
+        constexpr int kQuads = DIM / 32;
+        const int s = warp + (lane >> 3) * 4, first = (lane & 7) * 4;
+        const int mine = place_of_source(s) + place_of_quad(lane & 7);
+        float x[kQuads][4], l[16], m[16];
+#pragma unroll
+        for (int h = 0; h < kQuads; ++h) {
+            const float4 v4 = *reinterpret_cast<const float4*>(sk + s * kLd + first + 32 * h);
+            x[h][0] = v4.x;
+            x[h][1] = v4.y;
+            x[h][2] = v4.z;
+            x[h][3] = v4.w;
+        }
+        l[0] = m[0] = 0.0f;
+#pragma unroll
+        for (int t = 1; t < 16; ++t) {
+            l[t] = m[t] = 0.0f;
+            if (t > s) {
+#pragma unroll
+                for (int h = 0; h < kQuads; ++h) {
+                    const float4 g = *reinterpret_cast<const float4*>(sg + t * kLd + first + 32 * h);
+                    const float4 a = *reinterpret_cast<const float4*>(sk + t * kLd + first + 32 * h);
+                    const float4 d = *reinterpret_cast<const float4*>(sq + t * kLd + first + 32 * h);
+                    x[h][0] *= g.x;
+                    x[h][1] *= g.y;
+                    x[h][2] *= g.z;
+                    x[h][3] *= g.w;
+                    l[t] = fmaf(a.x, x[h][0], fmaf(a.y, x[h][1], fmaf(a.z, x[h][2], fmaf(a.w, x[h][3], l[t]))));
+                    m[t] = fmaf(d.x, x[h][0], fmaf(d.y, x[h][1], fmaf(d.z, x[h][2], fmaf(d.w, x[h][3], m[t]))));
+                }
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < kQuads; ++h) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                out[at.kd + mine + at_quad(h, r)] = x[h][r];
+            }
+        }
+        float l0, l1, m0, m1;
+        sum_over_eight(l, l0, l1);
+        sum_over_eight(m, m0, m1);
+        const int t = 2 * (lane & 7);
+        L[t * 16 + s] = sb[t] * l0;
+        L[(t + 1) * 16 + s] = sb[t + 1] * l1;
+        if (t > s) {
+            M[t * 16 + s] = m0;
+        }
+        if (t + 1 > s) {
+            M[(t + 1) * 16 + s] = m1;
+        }
+    }
+    __syncthreads();
+    for (int j = tid; j < DIM + p.vdim; j += 128) {
+        float x[16];
+        const int mine = j < DIM ? place_of_channel(j) : place_of_column(j - DIM);
+        if (j < DIM) {
+            float G = 1.0f;
+#pragma unroll
+            for (int t = 0; t < 16; ++t) {
+                G *= sg[t * kLd + j];
+                x[t] = sb[t] * (G * sk[t * kLd + j]);
+                out[at.qg + mine + at_token(t)] = G * sq[t * kLd + j];
+            }
+            out[at.g + place_of_decay(j)] = G;
+        } else {
+#pragma unroll
+            for (int t = 0; t < 16; ++t) {
+                x[t] = j - DIM == early ? __bfloat162float(column[t])
+                     : t < n            ? pl_load(v + (t0 + t) * p.qkv_stride + j - DIM)
+                                        : 0.0f;
+            }
+#pragma unroll
+            for (int t = 0; t < 16; ++t) {
+                x[t] *= sb[t];
+            }
+        }
+#pragma unroll
+        for (int t = 1; t < 16; ++t) {
+            float row[16];
+#pragma unroll
+            for (int s = 0; s < t; s += 4) {
+                *reinterpret_cast<float4*>(row + s) = *reinterpret_cast<const float4*>(L + t * 16 + s);
+            }
+#pragma unroll
+            for (int s = 0; s < t; ++s) {
+                x[t] = fmaf(-row[s], x[s], x[t]);
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < 16; t += 2) {
+            if (j < DIM) {
+                out[at.wm + mine + at_token(t)] = -x[t];
+                out[at.wm + mine + at_token(t + 1)] = -x[t + 1];
+            } else {
+                *reinterpret_cast<float2*>(out + at.zi + mine + at_result(t)) = make_float2(x[t], x[t + 1]);
+            }
+        }
+    }
+    for (int idx = tid; idx < 256; idx += 128) {
+        out[at.m + place_of_source(idx % 16) + at_token(idx / 16)] = M[idx];
+    }
+    __syncthreads();
+    send_chunk(out, c.scratch + (static_cast<int64_t>(blockIdx.x) * p.n_heads + head) * sent.floats, at, DIM);
+}
+
+template <int DIM>
+cudaError_t launch_gated_chunks(const GatedChunkParams& c, int64_t slots, cudaStream_t stream) {
+    const int smem = gated_chunk_smem<DIM>(c.in.vdim);
+    const cudaError_t set = cudaFuncSetAttribute(gated_delta_chunk_kernel<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (set != cudaSuccess) {
+        return set;
+    }
+    const cudaError_t made = pl_launch_overlapped(gated_delta_chunk_kernel<DIM>, dim3(static_cast<unsigned>(slots), c.in.n_heads),
+                                                  dim3(128), smem, stream, c);
+    if (made != cudaSuccess) {
+        return made;
+    }
+    const DeltaChainParams chain{c.scratch, c.in.state, c.in.first_rows, c.in.counts, c.in.slots, c.in.o_raw, c.in.n_heads,
+                                 c.in.vdim, c.pass};
+    return launch_delta_chain<DIM / 16, false>(chain, c.n_entries, stream);
+}
+
 // A warp per (token, head): the head's norm over vdim, its weight and the gate.
 template <typename scalar_t>
 __global__ void gated_delta_finish_kernel(const float* __restrict__ o_raw, const float* __restrict__ norm,
@@ -804,6 +1046,53 @@ PL_API int pl_gated_delta(const void* q, const void* k, const void* v, int64_t q
                              static_cast<scalar_t*>(out), out_stride, n_pairs, n_heads, vdim, eps);
     });
 #undef PL_SCAN_STATIC
+    PL_CHECK_LAUNCH("gated_delta");
+    return 0;
+}
+
+// Floats of scratch that pl_gated_delta_chunks needs, 0 where the step's portions are walked token by token.
+PL_API int64_t pl_gated_delta_chunk_floats(int n_tokens, int n_entries, int n_heads, int dim, int vdim, int dtype) {
+    if (n_tokens <= 0 || n_entries <= 0 || n_heads <= 0 || !delta_takes_chunks(n_tokens, n_entries, dim, vdim, dtype)) {
+        return 0;
+    }
+    return delta_chunk_slots(n_tokens, n_entries) * n_heads * DeltaChunkLayout(dim, vdim, false).floats;
+}
+
+// pl_gated_delta in chunks of 16 tokens (bfloat16). scratch: pl_gated_delta_chunk_floats floats on 16 bytes.
+PL_API int pl_gated_delta_chunks(const void* q, const void* k, const void* v, int64_t qkv_stride, const void* b_pre,
+                                 int64_t b_stride, const void* a_pre, int64_t a_stride, const void* gate_pre,
+                                 int64_t gate_stride, const float* a_log, const float* dt_bias, const float* norm,
+                                 float* state, const int32_t* first_rows, const int32_t* counts, const int32_t* slots,
+                                 float* o_raw, float* scratch, void* out, int64_t out_stride, int n_tokens,
+                                 int n_entries, int n_heads, int qk_heads, int dim, int vdim, float unit_eps,
+                                 float q_scale, float eps, cudaStream_t stream) {
+    PL_REQUIRE(qk_heads > 0 && n_heads > 0 && n_heads % qk_heads == 0 && n_heads <= 65535,
+               "gated_delta: bad heads=%d qk_heads=%d", n_heads, qk_heads);
+    PL_REQUIRE(delta_takes_chunks(n_tokens, n_entries, dim, vdim, PL_BF16),
+               "gated_delta: tokens=%d entries=%d dim=%d vdim=%d do not go in chunks", n_tokens, n_entries, dim, vdim);
+    PL_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 15) == 0, "gated_delta: the scratch must start on 16 bytes");
+    GatedChunkParams c = {};
+    GatedDeltaParams& p = c.in;
+    p.q = q; p.k = k; p.v = v; p.qkv_stride = qkv_stride; p.b_pre = b_pre; p.b_stride = b_stride; p.a_pre = a_pre;
+    p.a_stride = a_stride; p.a_log = a_log; p.dt_bias = dt_bias; p.state = state; p.first_rows = first_rows;
+    p.counts = counts; p.slots = slots; p.o_raw = o_raw; p.n_heads = n_heads; p.qk_heads = qk_heads; p.dim = dim;
+    p.vdim = vdim; p.unit_eps = unit_eps; p.q_scale = q_scale;
+    c.n_entries = n_entries;
+    c.scratch = scratch;
+    const int64_t n_slots = delta_chunk_slots(n_tokens, n_entries);
+    cudaError_t made = cudaSuccess;
+    for (c.pass = 0; c.pass < delta_passes(n_tokens) && made == cudaSuccess; ++c.pass) {
+        made = dim == 32 ? launch_gated_chunks<32>(c, n_slots, stream)
+             : dim == 64 ? launch_gated_chunks<64>(c, n_slots, stream)
+                         : launch_gated_chunks<128>(c, n_slots, stream);
+    }
+    if (made != cudaSuccess) {
+        return pl_fail(3, "gated_delta: launch failed: %s", cudaGetErrorString(made));
+    }
+    const int n_pairs = n_tokens * n_heads;
+    pl_launch_overlapped(gated_delta_finish_kernel<__nv_bfloat16>, dim3((n_pairs + 3) / 4), dim3(128), 0, stream,
+                         static_cast<const float*>(o_raw), norm, static_cast<const __nv_bfloat16*>(gate_pre), gate_stride,
+                         static_cast<__nv_bfloat16*>(out), out_stride, n_pairs, n_heads, vdim, eps);
     PL_CHECK_LAUNCH("gated_delta");
     return 0;
 }

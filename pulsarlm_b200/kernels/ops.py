@@ -43,6 +43,8 @@ _SIGNATURES = {
     "pl_short_conv_state": [_PTR, _PTR, _PTR, _PTR, _I32, _I32, _I32, _I32, _PTR],
     "pl_delta_rule": [_PTR, _PTR, _PTR, _PTR, _PTR, _I64, _PTR, _I64, _PTR, _PTR, _PTR, _PTR, _PTR, _PTR, _PTR, _PTR,
                       _PTR, _I64, _I32, _I32, _I32, _I32, _F32, _F32, _F32, _I32, _PTR],
+    "pl_delta_rule_chunks": [_PTR, _PTR, _PTR, _PTR, _PTR, _I64, _PTR, _I64, _PTR, _PTR, _PTR, _PTR, _PTR, _PTR, _PTR, _PTR,
+                             _PTR, _PTR, _I64, _I32, _I32, _I32, _I32, _F32, _F32, _F32, _PTR],
     "pl_norm_write_paged": [_PTR, _I64, _PTR, _F32, _PTR, _PTR, _PTR, _I32, _PTR, _I64, _I32, _I32, _I32, _I32, _I32,
                             _PTR, _PTR],
     "pl_take_tokens": [_PTR, _PTR, _PTR, _I32, _I32, _PTR, _PTR],
@@ -103,6 +105,8 @@ _SIGNATURES = {
     "pl_short_conv_state_strided": [_PTR, _I64, _PTR, _PTR, _PTR, _I32, _I32, _I32, _I32, _PTR],
     "pl_gated_delta": [_PTR, _PTR, _PTR, _I64, _PTR, _I64, _PTR, _I64, _PTR, _I64, _PTR, _PTR, _PTR, _PTR, _PTR, _PTR,
                        _PTR, _PTR, _PTR, _I64, _I32, _I32, _I32, _I32, _I32, _I32, _F32, _F32, _F32, _I32, _PTR],
+    "pl_gated_delta_chunks": [_PTR, _PTR, _PTR, _I64, _PTR, _I64, _PTR, _I64, _PTR, _I64, _PTR, _PTR, _PTR, _PTR, _PTR, _PTR,
+                              _PTR, _PTR, _PTR, _PTR, _I64, _I32, _I32, _I32, _I32, _I32, _I32, _F32, _F32, _F32, _PTR],
     "pl_moe_route": [_PTR, _I64, _PTR, _PTR, _PTR, _PTR, _PTR, _I32, _I32, _I32, _I32, _I32, _I32, _I32, _I32, _I32, _PTR,
                      _I32, _PTR],
     "pl_moe_up": [_PTR, _I64, _PTR, _PTR, _PTR, _I32, _I32, _I32, _I32, _I32, _I32, _I32, _PTR],
@@ -178,6 +182,10 @@ def library() -> ctypes.CDLL:
         lib.pl_attention_decode_scratch_floats.restype = _I64
         lib.pl_attention_prefill_scratch_floats.argtypes = [_I32, _I32, _I32, _I32]
         lib.pl_attention_prefill_scratch_floats.restype = _I64
+        lib.pl_gated_delta_chunk_floats.argtypes = [_I32, _I32, _I32, _I32, _I32, _I32]
+        lib.pl_gated_delta_chunk_floats.restype = _I64
+        lib.pl_delta_rule_chunk_floats.argtypes = [_I32, _I32, _I32, _I32, _I32]
+        lib.pl_delta_rule_chunk_floats.restype = _I64
         lib.pl_set_overlap.argtypes = [_I32]
         lib.pl_set_overlap.restype = _I32
         if os.environ.get("PULSARLM_B200_OVERLAP", "1") == "0":
@@ -454,6 +462,9 @@ def short_conv_state(h: torch.Tensor, entry: torch.Tensor, slots: torch.Tensor, 
           _stream())
 
 
+_DELTA_PASS_TOKENS = 2048  # tokens of an entry in one pass of the chunked scans (csrc/delta_chunks.cuh)
+
+
 def delta_rule(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tensor, a_pre: torch.Tensor,
                w_pre: torch.Tensor, w0: torch.Tensor, a0: torch.Tensor, norm: torch.Tensor, state: torch.Tensor,
                first_rows: torch.Tensor, counts: torch.Tensor, slots: torch.Tensor, out: torch.Tensor, n_heads: int,
@@ -473,11 +484,19 @@ def delta_rule(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tenso
     n_entries = first_rows.numel()
     tokens = r.shape[0]
     assert counts.numel() == n_entries and slots.numel() >= n_entries
-    o_raw = torch.empty((tokens, width), dtype=torch.float32, device=out.device)  # (the scan's output before the norm)
+    global _launches
+    floats = library().pl_delta_rule_chunk_floats(tokens, n_entries, n_heads, dim, _code(out.dtype))
+    # (the scan's output before the norm, and what the chunks of a bfloat16 portion need)
+    o_raw = torch.empty(tokens * width + floats, dtype=torch.float32, device=out.device)
+    if floats:  # a chunk of tokens a step of the scan instead of a token
+        _call("pl_delta_rule_chunks", _p(r), _p(k), _p(v), _p(g), _p(a_pre), stride, _p(w_pre), w_pre.stride(0), _p(w0), _p(a0),
+              _p(norm), _p(state), _p(first_rows), _p(counts), _p(slots), _p(o_raw), _p(o_raw) + 4 * tokens * width, _p(out),
+              out.stride(0), tokens, n_entries, n_heads, dim, float(decay_scale), float(unit_eps), float(eps), _stream())
+        _launches += 2 * -(-tokens // _DELTA_PASS_TOKENS)
+        return
     _call("pl_delta_rule", _p(r), _p(k), _p(v), _p(g), _p(a_pre), stride, _p(w_pre), w_pre.stride(0), _p(w0), _p(a0),
           _p(norm), _p(state), _p(first_rows), _p(counts), _p(slots), _p(o_raw), _p(out), out.stride(0), tokens,
           n_entries, n_heads, dim, float(decay_scale), float(unit_eps), float(eps), _code(out.dtype), _stream())
-    global _launches
     _launches += 1  # (two kernels)
 
 
@@ -608,16 +627,25 @@ def gated_delta(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b_pre: torch.
     assert state.dtype == torch.float32 and state.is_contiguous() and state.shape[1:] == (n_heads, dim, vdim)
     n_entries = first_rows.numel()
     assert counts.numel() == n_entries and slots.numel() >= n_entries
-    o_raw = torch.empty((tokens, n_heads * vdim), dtype=torch.float32, device=out.device)
 
     def stride(t):
         return t.stride(0) if tokens > 1 else t.shape[1]
 
+    global _launches
+    floats = library().pl_gated_delta_chunk_floats(tokens, n_entries, n_heads, dim, vdim, _code(out.dtype))
+    # (the scan's output before the norm, and what the chunks of a bfloat16 portion need)
+    o_raw = torch.empty(tokens * n_heads * vdim + floats, dtype=torch.float32, device=out.device)
+    if floats:  # a chunk of tokens a step of the scan instead of a token
+        _call("pl_gated_delta_chunks", _p(q), _p(k), _p(v), stride(q), _p(b_pre), stride(b_pre), _p(a_pre), stride(a_pre),
+              _p(gate_pre), stride(gate_pre), _p(a_log), _p(dt_bias), _p(norm), _p(state), _p(first_rows), _p(counts),
+              _p(slots), _p(o_raw), _p(o_raw) + 4 * tokens * n_heads * vdim, _p(out), stride(out), tokens, n_entries, n_heads,
+              qk_heads, dim, vdim, float(unit_eps), float(q_scale), float(eps), _stream())
+        _launches += 2 * -(-tokens // _DELTA_PASS_TOKENS)
+        return
     _call("pl_gated_delta", _p(q), _p(k), _p(v), stride(q), _p(b_pre), stride(b_pre), _p(a_pre), stride(a_pre),
           _p(gate_pre), stride(gate_pre), _p(a_log), _p(dt_bias), _p(norm), _p(state), _p(first_rows), _p(counts),
           _p(slots), _p(o_raw), _p(out), stride(out), tokens, n_entries, n_heads, qk_heads, dim, vdim, float(unit_eps),
           float(q_scale), float(eps), _code(out.dtype), _stream())
-    global _launches
     _launches += 1  # (two kernels)
 
 
