@@ -433,6 +433,61 @@ cudaError_t launch_delta_chain(const DeltaChainParams& p, int n_entries, cudaStr
                                 stream, p);
 }
 
+// The heads' norm over vdim, its weight and the gate: out = o * rsqrt(mean(o^2) + eps) * norm * sigmoid(gate), four values a
+// lane, LANES lanes a (token, head). norm_stride: distance between heads' norm weights (0: all heads have the same).
+template <int LANES>
+__global__ void __launch_bounds__(256) delta_finish_kernel(const float* __restrict__ o_raw, const float* __restrict__ norm,
+                                                           int norm_stride, const __nv_bfloat16* __restrict__ gate_pre,
+                                                           int64_t gate_stride, __nv_bfloat16* __restrict__ out,
+                                                           int64_t out_stride, int n_tokens, int n_heads, int vdim, float eps) {
+    pl_grid_trigger();
+    const int64_t pair = (static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x) / LANES;
+    const int d = threadIdx.x % LANES * 4;
+    const int t = static_cast<int>(pair / n_heads), h = static_cast<int>(pair % n_heads);
+    const bool there = t < n_tokens && d < vdim;
+    float4 weight = make_float4(0.0f, 0.0f, 0.0f, 0.0f), o = weight, g = weight;
+    if (there) {
+        weight = *reinterpret_cast<const float4*>(norm + h * norm_stride + d);
+    }
+    pl_grid_wait();
+    if (there) {
+        o = *reinterpret_cast<const float4*>(o_raw + pair * vdim + d);
+        g = pl_load4(gate_pre + t * gate_stride + h * vdim + d);
+    }
+    float square = fmaf(o.x, o.x, fmaf(o.y, o.y, fmaf(o.z, o.z, o.w * o.w)));
+#pragma unroll
+    for (int offset = LANES / 2; offset > 0; offset >>= 1) {
+        square += __shfl_xor_sync(0xffffffffu, square, offset);
+    }
+    if (there) {
+        const float factor = 1.0f / sqrtf(square / static_cast<float>(vdim) + eps);
+        const float4 r = make_float4(o.x * factor * weight.x * (1.0f / (1.0f + expf(-g.x))),
+                                     o.y * factor * weight.y * (1.0f / (1.0f + expf(-g.y))),
+                                     o.z * factor * weight.z * (1.0f / (1.0f + expf(-g.z))),
+                                     o.w * factor * weight.w * (1.0f / (1.0f + expf(-g.w))));
+        pl_store4(out + t * out_stride + h * vdim + d, r);
+    }
+}
+
+// Whether its loads of four values start where they have to.
+inline bool delta_finish_supports(const float* norm, const void* gate_pre, int64_t gate_stride, const void* out,
+                                  int64_t out_stride, int vdim) {
+    return vdim % 4 == 0 && vdim <= 128 && gate_stride % 4 == 0 && out_stride % 4 == 0 &&
+        (reinterpret_cast<uintptr_t>(norm) & 15) == 0 &&
+        ((reinterpret_cast<uintptr_t>(gate_pre) | reinterpret_cast<uintptr_t>(out)) & 7) == 0;
+}
+inline void launch_delta_finish(const float* o_raw, const float* norm, int norm_stride, const void* gate_pre, int64_t gate_stride,
+                                void* out, int64_t out_stride, int n_tokens, int n_heads, int vdim, float eps,
+                                cudaStream_t stream) {
+    const int lanes = vdim <= 16 ? 4 : vdim <= 32 ? 8 : vdim <= 64 ? 16 : 32;
+    const int64_t threads = static_cast<int64_t>(n_tokens) * n_heads * lanes;
+    auto kernel = lanes == 4 ? delta_finish_kernel<4> : lanes == 8 ? delta_finish_kernel<8>
+                : lanes == 16 ? delta_finish_kernel<16> : delta_finish_kernel<32>;
+    pl_launch_overlapped(kernel, dim3(static_cast<unsigned>((threads + 255) / 256)), dim3(256), 0, stream, o_raw, norm, norm_stride,
+                         static_cast<const __nv_bfloat16*>(gate_pre), gate_stride, static_cast<__nv_bfloat16*>(out), out_stride,
+                         n_tokens, n_heads, vdim, eps);
+}
+
 // Whether a step's portions go in chunks: bfloat16, sizes that fill the fragments, and more than a few tokens an
 // entry.
 inline bool delta_takes_chunks(int n_tokens, int n_entries, int dim, int vdim, int dtype) {

@@ -459,6 +459,7 @@ __global__ void __launch_bounds__(128) delta_rule_chunk_kernel(const RuleChunkPa
     // A warp has four tokens, a lane DIM / 32 channels of each. All of a lane's loads set out before anything is stored.
     constexpr int kPer = DIM / 32;
     float kv[4][kPer], rv[4][kPer], av[4][kPer], wv[4][kPer], w0[kPer], a0[kPer], sums[16];
+    const int64_t from = (t0 + warp * 4) * p.row_stride + lane, from_w = (t0 + warp * 4) * p.w_row_stride + lane;
 #pragma unroll
     for (int j = 0; j < kPer; ++j) {
         w0[j] = p.w0[hoff + lane + 32 * j];
@@ -470,11 +471,10 @@ __global__ void __launch_bounds__(128) delta_rule_chunk_kernel(const RuleChunkPa
         const bool there = t < n;
 #pragma unroll
         for (int j = 0; j < kPer; ++j) {
-            const int i = lane + 32 * j;
-            kv[q][j] = there ? pl_load(k + (t0 + t) * p.row_stride + i) : 0.0f;
-            rv[q][j] = there ? pl_load(r + (t0 + t) * p.row_stride + i) : 0.0f;
-            av[q][j] = there ? pl_load(a_pre + (t0 + t) * p.row_stride + i) : 0.0f;
-            wv[q][j] = there ? pl_load(w_pre + (t0 + t) * p.w_row_stride + i) : 0.0f;
+            kv[q][j] = there ? pl_load(k + from + q * p.row_stride + 32 * j) : 0.0f;
+            rv[q][j] = there ? pl_load(r + from + q * p.row_stride + 32 * j) : 0.0f;
+            av[q][j] = there ? pl_load(a_pre + from + q * p.row_stride + 32 * j) : 0.0f;
+            wv[q][j] = there ? pl_load(w_pre + from_w + q * p.w_row_stride + 32 * j) : 0.0f;
         }
     }
 #pragma unroll
@@ -519,9 +519,10 @@ __global__ void __launch_bounds__(128) delta_rule_chunk_kernel(const RuleChunkPa
     __nv_bfloat16 column[16];
     const int early = tid - DIM % 128;
     const bool values = early >= 0 && early < DIM;
+    const __nv_bfloat16* v_column = v + t0 * p.row_stride + early;
 #pragma unroll
-    for (int t = 0; t < 16; ++t) {
-        column[t] = values && t < n ? v[(t0 + t) * p.row_stride + early] : __float2bfloat16_rn(0.0f);
+    for (int t = 0; t < 16; ++t, v_column += p.row_stride) {
+        column[t] = values && t < n ? *v_column : __float2bfloat16_rn(0.0f);
     }
     __syncthreads();
     // Token s of the chunk is eight lanes', DIM / 8 channels each: its key and what it removes decay from token to token in
@@ -821,6 +822,11 @@ PL_API int pl_delta_rule_chunks(const void* r, const void* k, const void* v, con
     }
     if (made != cudaSuccess) {
         return pl_fail(3, "delta_rule: launch failed: %s", cudaGetErrorString(made));
+    }
+    if (delta_finish_supports(norm, g, row_stride, out, out_row_stride, dim)) {
+        launch_delta_finish(o_raw, norm, dim, g, row_stride, out, out_row_stride, n_tokens, n_heads, dim, eps, stream);
+        PL_CHECK_LAUNCH("delta_rule_finish");
+        return 0;
     }
     const int64_t pairs = static_cast<int64_t>(n_tokens) * n_heads;
     pl_launch_overlapped(delta_rule_finish_kernel<__nv_bfloat16>, dim3(static_cast<unsigned>((pairs + 3) / 4)), dim3(128),

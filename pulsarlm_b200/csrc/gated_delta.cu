@@ -717,6 +717,9 @@ __global__ void __launch_bounds__(128) gated_delta_chunk_kernel(const GatedChunk
     // A warp has four tokens, a lane DIM / 32 channels of each. All of a lane's loads set out before anything is stored.
     constexpr int kPer = DIM / 32;
     float qv[4][kPer], kv[4][kPer], gv[4][kPer], bias[kPer], sums[16];
+    const __nv_bfloat16* q_rows = q + (t0 + warp * 4) * p.qkv_stride + lane;
+    const __nv_bfloat16* k_rows = k + (t0 + warp * 4) * p.qkv_stride + lane;
+    const __nv_bfloat16* a_rows = a_pre + (t0 + warp * 4) * p.a_stride + lane;
 #pragma unroll
     for (int j = 0; j < kPer; ++j) {
         bias[j] = p.dt_bias[static_cast<int64_t>(head) * DIM + lane + 32 * j];
@@ -727,10 +730,9 @@ __global__ void __launch_bounds__(128) gated_delta_chunk_kernel(const GatedChunk
         const bool there = t < n;
 #pragma unroll
         for (int j = 0; j < kPer; ++j) {
-            const int i = lane + 32 * j;
-            qv[r][j] = there ? pl_load(q + (t0 + t) * p.qkv_stride + i) : 0.0f;
-            kv[r][j] = there ? pl_load(k + (t0 + t) * p.qkv_stride + i) : 0.0f;
-            gv[r][j] = there ? pl_load(a_pre + (t0 + t) * p.a_stride + i) : 0.0f;
+            qv[r][j] = there ? pl_load(q_rows + r * p.qkv_stride + 32 * j) : 0.0f;
+            kv[r][j] = there ? pl_load(k_rows + r * p.qkv_stride + 32 * j) : 0.0f;
+            gv[r][j] = there ? pl_load(a_rows + r * p.a_stride + 32 * j) : 0.0f;
         }
     }
     // (lanes 2 r, 2 r + 1 of every eight: token r's b)
@@ -775,9 +777,10 @@ __global__ void __launch_bounds__(128) gated_delta_chunk_kernel(const GatedChunk
     __nv_bfloat16 column[16];
     const int early = tid - DIM % 128;
     const bool values = early >= 0 && early < p.vdim;
+    const __nv_bfloat16* v_column = v + t0 * p.qkv_stride + early;
 #pragma unroll
-    for (int t = 0; t < 16; ++t) {
-        column[t] = values && t < n ? v[(t0 + t) * p.qkv_stride + early] : __float2bfloat16_rn(0.0f);
+    for (int t = 0; t < 16; ++t, v_column += p.qkv_stride) {
+        column[t] = values && t < n ? *v_column : __float2bfloat16_rn(0.0f);
     }
     __syncthreads();
     // Token s of the chunk is eight lanes', DIM / 8 channels each: its key decays from token to token in registers and meets
@@ -1088,6 +1091,11 @@ PL_API int pl_gated_delta_chunks(const void* q, const void* k, const void* v, in
     }
     if (made != cudaSuccess) {
         return pl_fail(3, "gated_delta: launch failed: %s", cudaGetErrorString(made));
+    }
+    if (delta_finish_supports(norm, gate_pre, gate_stride, out, out_stride, vdim)) {
+        launch_delta_finish(o_raw, norm, 0, gate_pre, gate_stride, out, out_stride, n_tokens, n_heads, vdim, eps, stream);
+        PL_CHECK_LAUNCH("gated_delta");
+        return 0;
     }
     const int n_pairs = n_tokens * n_heads;
     pl_launch_overlapped(gated_delta_finish_kernel<__nv_bfloat16>, dim3((n_pairs + 3) / 4), dim3(128), 0, stream,

@@ -93,7 +93,7 @@ __global__ void short_conv_kernel(const scalar_t* __restrict__ h, const float* _
 // rows of 4 * 128 channels with the earlier inputs in registers, so a row of h is read once
 // instead of `taps` times and the weights once a block. Same products in the same order as the
 // kernel above: same bits.
-constexpr int kRowsPerBlock = 16;
+constexpr int kRowsPerBlock = 8;
 
 template <typename scalar_t, int TAPS>
 __global__ void __launch_bounds__(128) short_conv_rows_kernel(
@@ -116,39 +116,52 @@ __global__ void __launch_bounds__(128) short_conv_rows_kernel(
         }
     }
     pl_grid_wait();
-    float4 window[REACH > 0 ? REACH : 1];  // the inputs before the row at hand, oldest first
-    float4 last = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    int last_entry = -1;
-    for (int t = t0; t < min(t0 + kRowsPerBlock, n_tokens); ++t) {
-        const int e = entry[t];
-        if (t == t0) {
-            int inside = 0;
-            while (inside < REACH && t - inside - 1 >= 0 && entry[t - inside - 1] == e) {
-                ++inside;
-            }
-            const scalar_t* old = state + static_cast<int64_t>(slots[e]) * REACH * width;
+    // All of the block's rows set out before the first is worked on (one load's time to answer a block, not a row).
+    const int n = min(kRowsPerBlock, n_tokens - t0);
+    float4 rows[kRowsPerBlock];
+    int entries[kRowsPerBlock];
 #pragma unroll
-            for (int j = 0; j < REACH; ++j) {
-                const int back = REACH - j;
-                window[j] = back <= inside ? pl_load4(h + static_cast<int64_t>(t - back) * h_stride + c)
-                                           : pl_load4(old + static_cast<int64_t>(REACH - (back - inside)) * width + c);
-            }
-        } else if (e != last_entry) {
-            const scalar_t* old = state + static_cast<int64_t>(slots[e]) * REACH * width;
+    for (int i = 0; i < kRowsPerBlock; ++i) {
+        const int t = t0 + min(i, n - 1);
+        rows[i] = pl_load4(h + static_cast<int64_t>(t) * h_stride + c);
+        entries[i] = entry[t];
+    }
+    // The inputs before the first row, oldest first: rows of its sequence in this step, or the state's.
+    float4 window[REACH];
+    {
+        int inside = 0;
+        while (inside < REACH && t0 - inside - 1 >= 0 && entry[t0 - inside - 1] == entries[0]) {
+            ++inside;
+        }
+        const scalar_t* old = state + static_cast<int64_t>(slots[entries[0]]) * REACH * width;
 #pragma unroll
-            for (int j = 0; j < REACH; ++j) {
-                window[j] = pl_load4(old + static_cast<int64_t>(j) * width + c);
-            }
-        } else {
+        for (int j = 0; j < REACH; ++j) {
+            const int back = REACH - j;
+            window[j] = back <= inside ? pl_load4(h + static_cast<int64_t>(t0 - back) * h_stride + c)
+                                       : pl_load4(old + static_cast<int64_t>(REACH - (back - inside)) * width + c);
+        }
+    }
 #pragma unroll
-            for (int j = 0; j + 1 < REACH; ++j) {
-                window[j] = window[j + 1];
-            }
-            if (REACH > 0) {
-                window[REACH - 1] = last;
+    for (int i = 0; i < kRowsPerBlock; ++i) {
+        if (i >= n) {
+            break;
+        }
+        if (i > 0) {
+            if (entries[i] != entries[i - 1]) {
+                const scalar_t* old = state + static_cast<int64_t>(slots[entries[i]]) * REACH * width;
+#pragma unroll
+                for (int j = 0; j < REACH; ++j) {
+                    window[j] = pl_load4(old + static_cast<int64_t>(j) * width + c);
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j + 1 < REACH; ++j) {
+                    window[j] = window[j + 1];
+                }
+                window[REACH - 1] = rows[i - 1];
             }
         }
-        const float4 own = pl_load4(h + static_cast<int64_t>(t) * h_stride + c);
+        const float4 own = rows[i];
         float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
         for (int j = 0; j < REACH; ++j) {
@@ -161,9 +174,7 @@ __global__ void __launch_bounds__(128) short_conv_rows_kernel(
         acc.y = fmaf(w[1][REACH], own.y, acc.y);
         acc.z = fmaf(w[2][REACH], own.z, acc.z);
         acc.w = fmaf(w[3][REACH], own.w, acc.w);
-        pl_store4(out + static_cast<int64_t>(t) * width + c, conv_result(own, acc, residual, act));
-        last = own;
-        last_entry = e;
+        pl_store4(out + static_cast<int64_t>(t0 + i) * width + c, conv_result(own, acc, residual, act));
     }
 }
 
@@ -233,11 +244,14 @@ __global__ void short_conv_state_kernel(const scalar_t* __restrict__ h, const in
     const int t = blockIdx.x;
     const int e = entry[t];
     const int reach = taps - 1;
+    // (lane i looks at row t - reach + i, 31 rows at most: one load's time for all neighbours)
+    const int near = t - reach + static_cast<int>(threadIdx.x & 31);
+    const uint32_t same = __ballot_sync(0xffffffffu, near >= 0 && near < n_tokens && near <= t + reach && entry[near] == e);
     int before = 0, after = 0;
-    while (before < reach && t - before - 1 >= 0 && entry[t - before - 1] == e) {
+    while (before < reach && (same >> (reach - before - 1) & 1)) {
         ++before;
     }
-    while (after < reach && t + after + 1 < n_tokens && entry[t + after + 1] == e) {
+    while (after < reach && (same >> (reach + after + 1) & 1)) {
         ++after;
     }
     scalar_t* mine = state + static_cast<int64_t>(slots[e]) * reach * width;
@@ -245,6 +259,15 @@ __global__ void short_conv_state_kernel(const scalar_t* __restrict__ h, const in
     if (before == reach || after == reach || before + 1 + after >= reach) {
         // A portion of at least `reach` rows: each of its last `reach` rows writes itself.
         if (after < reach) {
+            constexpr int kPer = 16 / sizeof(scalar_t);
+            scalar_t* to = mine + static_cast<int64_t>(reach - 1 - after) * width;
+            const scalar_t* from = h + static_cast<int64_t>(t) * h_stride;
+            if (width % kPer == 0 && ((reinterpret_cast<uintptr_t>(to) | reinterpret_cast<uintptr_t>(from)) & 15) == 0) {
+                for (int c = threadIdx.x * kPer; c < width; c += blockDim.x * kPer) {
+                    *reinterpret_cast<uint4*>(to + c) = *reinterpret_cast<const uint4*>(from + c);
+                }
+                return;
+            }
             for (int c = threadIdx.x; c < width; c += blockDim.x) {
                 mine[static_cast<int64_t>(reach - 1 - after) * width + c] = h[static_cast<int64_t>(t) * h_stride + c];
             }
