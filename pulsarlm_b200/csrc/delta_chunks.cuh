@@ -488,11 +488,11 @@ inline void launch_delta_finish(const float* o_raw, const float* norm, int norm_
                          n_tokens, n_heads, vdim, eps);
 }
 
-// Whether a step's portions go in chunks: bfloat16, sizes that fill the fragments, and more than a few tokens an
-// entry.
+// Whether a step's portions go in chunks: bfloat16, sizes that fill the fragments, and more tokens than one an entry by
+// what two chunks hold (a walk takes a third of a microsecond a token, a pass of two kernels about ten).
 inline bool delta_takes_chunks(int n_tokens, int n_entries, int dim, int vdim, int dtype) {
     return dtype == PL_BF16 && (dim == 32 || dim == 64 || dim == 128) && vdim % kDeltaCols == 0 && vdim <= 256 &&
-        n_tokens > 2 * n_entries && n_tokens - n_entries >= 32;
+        n_tokens - n_entries >= 32;
 }
 // Slots for chunks in a pass, and passes, at most.
 inline int64_t delta_chunk_slots(int n_tokens, int n_entries) {

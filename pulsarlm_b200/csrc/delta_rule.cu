@@ -30,6 +30,7 @@
 #include "common.cuh"
 
 #include "delta_chunks.cuh"
+#include "delta_step.cuh"
 #include "mma_helpers.cuh"
 
 namespace {
@@ -685,6 +686,66 @@ cudaError_t launch_rule_chunks(const RuleChunkParams& c, int64_t slots, cudaStre
     return launch_delta_chain<DIM / 16, true>(chain, c.n_entries, stream);
 }
 
+// ---------------------------------------------------------------------------- steps of single tokens
+struct RuleStepParams {
+    ScanParams in;
+    const __nv_bfloat16* g;
+    const float* norm;
+    __nv_bfloat16* out;
+    int64_t out_stride;
+    float eps;
+};
+
+template <int DIM>
+__global__ void __launch_bounds__(kStepThreads) delta_rule_step_kernel(const RuleStepParams c) {
+    pl_grid_trigger();
+    pl_grid_wait();
+    __shared__ __align__(16) DeltaStepShared<DIM, DIM> s;
+    const ScanParams& p = c.in;
+    const int e = blockIdx.x, head = blockIdx.y, i = threadIdx.x;
+    const int count = p.counts[e];
+    if (count == 0) {
+        return;
+    }
+    const int64_t first = p.first_rows[e], hoff = static_cast<int64_t>(head) * DIM;
+    const __nv_bfloat16* r = static_cast<const __nv_bfloat16*>(p.r) + hoff + i;
+    const __nv_bfloat16* k = static_cast<const __nv_bfloat16*>(p.k) + hoff + i;
+    const __nv_bfloat16* v = static_cast<const __nv_bfloat16*>(p.v) + hoff + i;
+    const __nv_bfloat16* a_pre = static_cast<const __nv_bfloat16*>(p.a_pre) + hoff + i;
+    const __nv_bfloat16* w_pre = static_cast<const __nv_bfloat16*>(p.w_pre) + hoff + i;
+    float* state = p.state + (static_cast<int64_t>(p.slots[e]) * p.n_heads + head) * DIM * DIM;
+    const float w0 = i < DIM ? p.w0[hoff + i] : 0.0f, a0 = i < DIM ? p.a0[hoff + i] : 0.0f;
+    auto vectors = [&](int t) {
+        const int64_t row = first + t;
+        float kv = 0.0f, removal = 0.0f;
+        if (i < DIM) {
+            kv = pl_load(k + row * p.row_stride);
+            removal = sigmoid_f32(pl_load(a_pre + row * p.row_stride) + a0);
+            s.q[i] = pl_load(r + row * p.row_stride);
+            s.g[i] = expf(-p.decay_scale * sigmoid_f32(pl_load(w_pre + row * p.w_row_stride) + w0));
+            s.k[i] = kv;
+            s.v[i] = pl_load(v + row * p.row_stride);
+        }
+        const float2 squares = step_vector_sums<DIM, DIM>(s, kv * kv, 0.0f);
+        if (i < DIM) {
+            const float u = kv * (1.0f / sqrtf(squares.x + p.unit_eps));
+            s.x[i] = u;
+            s.p[i] = removal * u;
+        }
+    };
+    auto store = [&](int t, int column, float4 o) {
+        const int64_t row = first + t;
+        const __nv_bfloat16* gate = c.g + row * p.row_stride + hoff + column;
+        __nv_bfloat16* out = c.out + row * c.out_stride + hoff + column;
+        const float values[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            pl_store(out + j, values[j] * c.norm[hoff + column + j] * sigmoid_f32(pl_load(gate + j)));
+        }
+    };
+    delta_step_walk<DIM, DIM, true>(s, state, count, c.eps, vectors, store);
+}
+
 // A warp per (token, head): out = o * rsqrt(mean(o^2) + eps) * norm * sigmoid(g).
 template <typename scalar_t>
 __global__ void delta_rule_finish_kernel(const float* __restrict__ o_raw, const scalar_t* __restrict__ g,
@@ -774,6 +835,16 @@ PL_API int pl_delta_rule(const void* r, const void* k, const void* v, const void
     const size_t smem = static_cast<size_t>(2 * dim + p.chunk * 5 * dim + p.chunk * threads) * sizeof(float) +
         2 * raw_bytes;
     const dim3 grid(n_entries, n_heads, col_blocks);
+    // bfloat16 steps of single tokens: the form with a whole head's state in a CTA's registers and the norm behind
+    // it. float32 keeps the walk, whose bits do not depend on how a prompt was cut.
+    if (dtype == PL_BF16 && n_tokens == n_entries && (dim == 32 || dim == 64 || dim == 128) && aligned(state)) {
+        const RuleStepParams c{p, static_cast<const __nv_bfloat16*>(g), norm, static_cast<__nv_bfloat16*>(out), out_row_stride,
+                               eps};
+        auto kernel = dim == 32 ? delta_rule_step_kernel<32> : dim == 64 ? delta_rule_step_kernel<64> : delta_rule_step_kernel<128>;
+        pl_launch_overlapped(kernel, dim3(n_entries, n_heads), dim3(kStepThreads), 0, stream, c);
+        PL_CHECK_LAUNCH("delta_rule");
+        return 0;
+    }
     PL_DISPATCH_DTYPE(dtype, "delta_rule", {
         launch_scan<scalar_t>(p, grid, threads, smem, stream);
         PL_CHECK_LAUNCH("delta_rule");

@@ -1,0 +1,140 @@
+// Delta rules in steps of single tokens, bfloat16 engine: what the two
+// recurrent mixers (gated_delta.cu, delta_rule.cu) share. A CTA has a whole head of one entry: its state [DIM, VDIM]
+// lies in the threads' registers (four neighbouring columns, DIM * VDIM / 1024 rows each), so it is read once with 16-byte
+// loads and written once, and the head's norm, its weight and the gate follow in the same kernel. What bounds it is the
+// state's stream: 64 entries of 32 heads of 64 x 64 are 67 MB. The forms for longer portions give a head to several CTAs
+// (that is what one entry's few heads need) which all make the token's vectors anew and leave the norm to a second kernel.
+#pragma once
+
+#include "common.cuh"
+
+namespace {
+
+constexpr int kStepThreads = 256;
+
+// A token's vectors of a head, made by the first DIM threads, and its scalars.
+template <int DIM, int VDIM>
+struct DeltaStepShared {
+    float q[DIM];            // meets the new state
+    float x[DIM];            // meets the old one
+    float g[DIM];            // decays it
+    float p[DIM], k[DIM];    // (general rule: removed, written)
+    float v[VDIM];
+    float sums[kStepThreads / 32][VDIM];
+    float b;                 // (last: everything before it starts on 16 bytes)
+};
+
+// parts[c] over all row groups for this thread's columns, in every thread.
+template <int DIM, int VDIM>
+__device__ __forceinline__ float4 step_column_sums(DeltaStepShared<DIM, VDIM>& s, float4 part) {
+    constexpr int kQuads = VDIM / 4;
+#pragma unroll
+    for (int offset = 16; offset >= kQuads; offset >>= 1) {
+        part.x += __shfl_xor_sync(0xffffffffu, part.x, offset);
+        part.y += __shfl_xor_sync(0xffffffffu, part.y, offset);
+        part.z += __shfl_xor_sync(0xffffffffu, part.z, offset);
+        part.w += __shfl_xor_sync(0xffffffffu, part.w, offset);
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, quad = threadIdx.x % kQuads;
+    if (lane < kQuads) {
+        *reinterpret_cast<float4*>(&s.sums[warp][quad * 4]) = part;
+    }
+    __syncthreads();
+    float4 total = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (int w = 0; w < kStepThreads / 32; ++w) {
+        const float4 v = *reinterpret_cast<const float4*>(&s.sums[w][quad * 4]);
+        total.x += v.x;
+        total.y += v.y;
+        total.z += v.z;
+        total.w += v.w;
+    }
+    __syncthreads();
+    return total;
+}
+
+// Walks `count` tokens of one entry and head; VECTORS(t) fills s.q .. s.b of token t (all threads call it; what it wrote
+// is read after a barrier here); OUT(t, column, value, factor) takes the four outputs of a thread of the first row group.
+template <int DIM, int VDIM, bool GENERAL, typename Vectors, typename Out>
+__device__ __forceinline__ void delta_step_walk(DeltaStepShared<DIM, VDIM>& s, float* state, int count, float eps,
+                                                const Vectors& vectors, const Out& store) {
+    constexpr int kQuads = VDIM / 4, kGroups = kStepThreads / kQuads, kRows = DIM / kGroups;
+    static_assert(kRows >= 1 && kRows * kGroups == DIM, "rows of a thread");
+    const int quad = threadIdx.x % kQuads, group = threadIdx.x / kQuads;
+    float4 S[kRows];
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+        S[r] = *reinterpret_cast<const float4*>(state + (group + r * kGroups) * VDIM + quad * 4);
+    }
+    for (int t = 0; t < count; ++t) {
+        vectors(t);
+        __syncthreads();
+        float4 part = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+            const int i = group + r * kGroups;
+            const float x = s.x[i];
+            if constexpr (!GENERAL) {
+                const float g = s.g[i];
+                S[r] = make_float4(S[r].x * g, S[r].y * g, S[r].z * g, S[r].w * g);
+            }
+            part = make_float4(fmaf(S[r].x, x, part.x), fmaf(S[r].y, x, part.y), fmaf(S[r].z, x, part.z), fmaf(S[r].w, x, part.w));
+        }
+        const float4 dot = step_column_sums<DIM, VDIM>(s, part);
+        const float4 v = *reinterpret_cast<const float4*>(&s.v[quad * 4]);
+        const float b = s.b;
+        const float4 u = make_float4(b * (v.x - dot.x), b * (v.y - dot.y), b * (v.z - dot.z), b * (v.w - dot.w));
+        part = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+            const int i = group + r * kGroups;
+            if constexpr (GENERAL) {
+                const float g = s.g[i], p = -s.p[i], k = s.k[i];
+                S[r] = make_float4(fmaf(k, v.x, fmaf(p, dot.x, g * S[r].x)), fmaf(k, v.y, fmaf(p, dot.y, g * S[r].y)),
+                                   fmaf(k, v.z, fmaf(p, dot.z, g * S[r].z)), fmaf(k, v.w, fmaf(p, dot.w, g * S[r].w)));
+            } else {
+                const float x = s.x[i];
+                S[r] = make_float4(fmaf(x, u.x, S[r].x), fmaf(x, u.y, S[r].y), fmaf(x, u.z, S[r].z), fmaf(x, u.w, S[r].w));
+            }
+            const float q = s.q[i];
+            part = make_float4(fmaf(S[r].x, q, part.x), fmaf(S[r].y, q, part.y), fmaf(S[r].z, q, part.z), fmaf(S[r].w, q, part.w));
+        }
+        const float4 o = step_column_sums<DIM, VDIM>(s, part);
+        // the head's norm: the first row group's lanes hold every column once
+        float square = fmaf(o.x, o.x, fmaf(o.y, o.y, fmaf(o.z, o.z, o.w * o.w)));
+#pragma unroll
+        for (int offset = kQuads / 2; offset > 0; offset >>= 1) {
+            square += __shfl_xor_sync(0xffffffffu, square, offset);
+        }
+        if (group == 0) {
+            const float factor = 1.0f / sqrtf(square / static_cast<float>(VDIM) + eps);
+            store(t, quad * 4, make_float4(o.x * factor, o.y * factor, o.z * factor, o.w * factor));
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+        *reinterpret_cast<float4*>(state + (group + r * kGroups) * VDIM + quad * 4) = S[r];
+    }
+}
+
+// The sums over the first DIM threads of two values each, in all of them (and nothing of use in the others).
+template <int DIM, int VDIM>
+__device__ __forceinline__ float2 step_vector_sums(DeltaStepShared<DIM, VDIM>& s, float a, float b) {
+    const int warp = threadIdx.x >> 5;
+    a = pl_warp_sum(a);
+    b = pl_warp_sum(b);
+    if ((threadIdx.x & 31) == 0 && warp < DIM / 32) {
+        s.sums[0][2 * warp] = a;
+        s.sums[0][2 * warp + 1] = b;
+    }
+    __syncthreads();
+    a = b = 0.0f;
+#pragma unroll
+    for (int w = 0; w < DIM / 32; ++w) {
+        a += s.sums[0][2 * w];
+        b += s.sums[0][2 * w + 1];
+    }
+    return make_float2(a, b);
+}
+
+}  // namespace

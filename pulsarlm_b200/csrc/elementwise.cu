@@ -36,6 +36,32 @@ __global__ void embed_kernel(const scalar_t* __restrict__ table, const int32_t* 
     }
 }
 
+// The same four values a load, for rows of whole pieces (a thread of the kernel above had a load's time to answer per
+// element: 2,048 rows of 4,096 took 20.4 us, 8 rows 11).
+template <typename scalar_t>
+__global__ void embed_vec_kernel(const scalar_t* __restrict__ table, const int32_t* __restrict__ tokens,
+                                 float* __restrict__ x, int hidden, int vocab, float scale, int32_t* status) {
+    pl_grid_trigger();
+    pl_grid_wait();
+    const int t = blockIdx.x;
+    const int token = tokens[t];
+    const bool known = token >= 0 && token < vocab;
+    if (!known && threadIdx.x == 0 && status != nullptr) {
+        atomicOr(status, 1);
+    }
+    const scalar_t* src = table + (known ? static_cast<int64_t>(token) * hidden : 0);
+    float* row = x + static_cast<int64_t>(t) * hidden;
+#pragma unroll 4
+    for (int i = 4 * threadIdx.x; i < hidden; i += 4 * blockDim.x) {
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (known) {
+            v = pl_load4(src + i);
+            v = make_float4(v.x * scale, v.y * scale, v.z * scale, v.w * scale);
+        }
+        *reinterpret_cast<float4*>(row + i) = v;
+    }
+}
+
 // tokens[i] = ids[source[i]] where source[i] >= 0 (other rows keep what the host wrote).
 __global__ void take_tokens_kernel(int32_t* __restrict__ tokens, const int32_t* __restrict__ source,
                                    const int32_t* __restrict__ ids, int n, int n_ids, int32_t* status) {
@@ -243,6 +269,14 @@ PL_API int pl_embed(const void* table, const int32_t* tokens, float* x, int n_to
         return 0;
     }
     const int threads = hidden >= 1024 ? 256 : 128;
+    if (hidden % 4 == 0 && ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(x)) & 15) == 0) {
+        PL_DISPATCH_DTYPE(dtype, "embed", {
+            pl_launch_overlapped(embed_vec_kernel<scalar_t>, n_tokens, threads, 0, stream,
+                                 static_cast<const scalar_t*>(table), tokens, x, hidden, vocab, scale, status);
+        });
+        PL_CHECK_LAUNCH("embed");
+        return 0;
+    }
     PL_DISPATCH_DTYPE(dtype, "embed", {
         pl_launch_overlapped(embed_kernel<scalar_t>, n_tokens, threads, 0, stream,
                              static_cast<const scalar_t*>(table), tokens, x, hidden, vocab, scale, status);

@@ -25,6 +25,7 @@
 #include "common.cuh"
 
 #include "delta_chunks.cuh"
+#include "delta_step.cuh"
 #include "mma_helpers.cuh"
 
 namespace {
@@ -910,6 +911,78 @@ cudaError_t launch_gated_chunks(const GatedChunkParams& c, int64_t slots, cudaSt
     return launch_delta_chain<DIM / 16, false>(chain, c.n_entries, stream);
 }
 
+// ---------------------------------------------------------------------------- steps of single tokens
+struct GatedStepParams {
+    GatedDeltaParams in;
+    const __nv_bfloat16* gate_pre;
+    int64_t gate_stride;
+    const float* norm;
+    __nv_bfloat16* out;
+    int64_t out_stride;
+    float eps;
+};
+
+template <int DIM, int VDIM>
+__global__ void __launch_bounds__(kStepThreads) gated_delta_step_kernel(const GatedStepParams c) {
+    pl_grid_trigger();
+    pl_grid_wait();
+    __shared__ __align__(16) DeltaStepShared<DIM, VDIM> s;
+    const GatedDeltaParams& p = c.in;
+    const int e = blockIdx.x, head = blockIdx.y, i = threadIdx.x;
+    const int count = p.counts[e];
+    if (count == 0) {
+        return;
+    }
+    const int64_t first = p.first_rows[e];
+    const int qk_head = head / (p.n_heads / p.qk_heads);
+    const __nv_bfloat16* q = static_cast<const __nv_bfloat16*>(p.q) + static_cast<int64_t>(qk_head) * DIM + i;
+    const __nv_bfloat16* k = static_cast<const __nv_bfloat16*>(p.k) + static_cast<int64_t>(qk_head) * DIM + i;
+    const __nv_bfloat16* v = static_cast<const __nv_bfloat16*>(p.v) + static_cast<int64_t>(head) * VDIM + i;
+    const __nv_bfloat16* a_pre = static_cast<const __nv_bfloat16*>(p.a_pre) + static_cast<int64_t>(head) * DIM + i;
+    const __nv_bfloat16* b_pre = static_cast<const __nv_bfloat16*>(p.b_pre) + head;
+    float* state = p.state + (static_cast<int64_t>(p.slots[e]) * p.n_heads + head) * DIM * VDIM;
+    const float rate = expf(p.a_log[head]);
+    const float bias = i < DIM ? p.dt_bias[static_cast<int64_t>(head) * DIM + i] : 0.0f;
+    auto vectors = [&](int t) {
+        const int64_t row = first + t;
+        float qv = 0.0f, kv = 0.0f;
+        if (i < DIM) {
+            qv = pl_load(q + row * p.qkv_stride);
+            kv = pl_load(k + row * p.qkv_stride);
+            s.g[i] = expf(-rate * softplus_f32(pl_load(a_pre + row * p.a_stride) + bias));
+        }
+        if (i < VDIM) {
+            s.v[i] = pl_load(v + row * p.qkv_stride);
+        }
+        if (i == kStepThreads - 1) {
+            s.b = 1.0f / (1.0f + expf(-pl_load(b_pre + row * p.b_stride)));
+        }
+        const float2 squares = step_vector_sums<DIM, VDIM>(s, qv * qv, kv * kv);
+        if (i < DIM) {
+            s.q[i] = qv * (p.q_scale / sqrtf(squares.x + p.unit_eps));
+            s.x[i] = kv * (1.0f / sqrtf(squares.y + p.unit_eps));
+        }
+    };
+    auto store = [&](int t, int column, float4 o) {
+        const int64_t row = first + t;
+        const __nv_bfloat16* gate = c.gate_pre + row * c.gate_stride + static_cast<int64_t>(head) * VDIM + column;
+        __nv_bfloat16* out = c.out + row * c.out_stride + static_cast<int64_t>(head) * VDIM + column;
+        const float values[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            pl_store(out + j, values[j] * c.norm[column + j] * (1.0f / (1.0f + expf(-pl_load(gate + j)))));
+        }
+    };
+    delta_step_walk<DIM, VDIM, false>(s, state, count, c.eps, vectors, store);
+}
+
+template <int DIM>
+void launch_gated_step(const GatedStepParams& c, int n_entries, cudaStream_t stream) {
+    auto kernel = c.in.vdim == 32 ? gated_delta_step_kernel<DIM, 32>
+                : c.in.vdim == 64 ? gated_delta_step_kernel<DIM, 64> : gated_delta_step_kernel<DIM, 128>;
+    pl_launch_overlapped(kernel, dim3(n_entries, c.in.n_heads), dim3(kStepThreads), 0, stream, c);
+}
+
 // A warp per (token, head): the head's norm over vdim, its weight and the gate.
 template <typename scalar_t>
 __global__ void gated_delta_finish_kernel(const float* __restrict__ o_raw, const float* __restrict__ norm,
@@ -1010,6 +1083,22 @@ PL_API int pl_gated_delta(const void* q, const void* k, const void* v, int64_t q
     p.counts = counts; p.slots = slots; p.o_raw = o_raw; p.n_heads = n_heads; p.qk_heads = qk_heads; p.dim = dim;
     p.vdim = vdim; p.parts = parts; p.cols = cols; p.chunk = chunk; p.async_loads = async_loads; p.unit_eps = unit_eps; p.q_scale = q_scale;
     const dim3 grid(n_entries, n_heads, (vdim + cols - 1) / cols);
+    // bfloat16 steps of single tokens: the form with a whole head's state in a CTA's registers and the norm behind it (64 entries of 32 heads of
+    // 64 x 64: 48 -> 17 us). float32 keeps the walk, whose bits do not depend on how a prompt was cut.
+    if (n_tokens == n_entries && dtype == PL_BF16 && (dim == 32 || dim == 64 || dim == 128) && (vdim == 32 || vdim == 64 || vdim == 128) &&
+        (reinterpret_cast<uintptr_t>(state) & 15) == 0) {
+        const GatedStepParams c{p, static_cast<const __nv_bfloat16*>(gate_pre), gate_stride, norm,
+                                static_cast<__nv_bfloat16*>(out), out_stride, eps};
+        if (dim == 32) {
+            launch_gated_step<32>(c, n_entries, stream);
+        } else if (dim == 64) {
+            launch_gated_step<64>(c, n_entries, stream);
+        } else {
+            launch_gated_step<128>(c, n_entries, stream);
+        }
+        PL_CHECK_LAUNCH("gated_delta");
+        return 0;
+    }
     const int n_pairs = n_tokens * n_heads;
 #define PL_SCAN_STATIC(D, P)                                                                                        \
     do {                                                                                                               \

@@ -1,5 +1,5 @@
-"""Delta rules over bfloat16 portions: sixteen tokens a step of the scan beside the walk token by token, both against
-float64 on the same inputs."""
+"""Delta rules in bfloat16: portions sixteen tokens a step of the scan beside the walk token by token, and steps of single
+tokens, all against float64 on the same inputs."""
 
 from __future__ import annotations
 
@@ -29,7 +29,8 @@ def _rel(got, want):
 
 
 # Portions shorter than a chunk, of whole chunks, one more and one less, one past the pass of 128 chunks, singles between.
-LENGTHS = [[33], [1, 48, 1, 17, 15], [16, 0, 31], [2081], [5] * 12]
+# Steps of single tokens have a form of their own (the last two; an entry may bring none or two).
+LENGTHS = [[33], [1, 48, 1, 17, 15], [16, 0, 31], [2081], [5] * 12, [1] * 7, [2, 0, 1]]
 
 
 def _both(ops, monkeypatch, name, call):
