@@ -117,6 +117,7 @@ _SIGNATURES = {
                                _I64, _I64, _I32, _I32, _PTR, _I32, _I32, _I32, _I32, _I32, _I32, _I32, _I32, _PTR,
                                _PTR, _F32, _I32, _PTR, _PTR],
     "pl_moe_gate_up": [_PTR, _I64, _PTR, _PTR, _PTR, _I32, _I32, _I32, _I32, _I32, _I32, _F32, _PTR, _I32, _PTR],
+    "pl_moe_down_by_expert": [_PTR, _PTR, _PTR, _PTR, _PTR, _PTR, _PTR, _PTR, _I32, _I32, _I32, _I32, _I32, _I32, _PTR],
     "pl_moe_down": [_PTR, _PTR, _PTR, _PTR, _PTR, _PTR, _PTR, _I32, _I32, _I32, _I32, _I32, _I32, _PTR],
     "pl_moe_sort": [_PTR, _I32, _I32, _PTR, _PTR, _PTR, _PTR],
     "pl_moe_gather": [_PTR, _I64, _PTR, _PTR, _I32, _I32, _I32, _I32, _PTR],
@@ -182,6 +183,8 @@ def library() -> ctypes.CDLL:
         lib.pl_attention_decode_scratch_floats.restype = _I64
         lib.pl_attention_prefill_scratch_floats.argtypes = [_I32, _I32, _I32, _I32]
         lib.pl_attention_prefill_scratch_floats.restype = _I64
+        lib.pl_moe_down_scratch_floats.argtypes = [_I32, _I32, _I32, _I32, _I32, _I32, _PTR]
+        lib.pl_moe_down_scratch_floats.restype = _I64
         lib.pl_gated_delta_chunk_floats.argtypes = [_I32, _I32, _I32, _I32, _I32, _I32]
         lib.pl_gated_delta_chunk_floats.restype = _I64
         lib.pl_delta_rule_chunk_floats.argtypes = [_I32, _I32, _I32, _I32, _I32]
@@ -717,6 +720,14 @@ def moe_down(act: torch.Tensor, down: torch.Tensor, ids: torch.Tensor, weights: 
     assert act.is_contiguous() and act.shape == (tokens * top, ff) and out.is_contiguous()
     assert weights is None or (weights.dtype == torch.float32 and weights.is_contiguous() and weights.shape == ids.shape)
     assert also is None or (also.shape == out.shape and also.is_contiguous() and also.dtype == out.dtype)
+    floats = library().pl_moe_down_scratch_floats(tokens, hidden, ff, top, n_experts, _code(out.dtype), _p(down))
+    if floats:  # (experts that several tokens chose: their weights once, the pairs' products in fp32 in between)
+        y = torch.empty(floats, dtype=torch.float32, device=out.device)
+        _call("pl_moe_down_by_expert", _p(act), _p(down), _p(ids), _p(weights), _p(also), _p(also_weights), _p(y), _p(out), tokens,
+              hidden, ff, top, n_experts, _code(out.dtype), _stream())
+        global _launches
+        _launches += 1  # (two kernels)
+        return
     _call("pl_moe_down", _p(act), _p(down), _p(ids), _p(weights), _p(also), _p(also_weights), _p(out), tokens, hidden, ff, top,
           n_experts, _code(out.dtype), _stream())
 

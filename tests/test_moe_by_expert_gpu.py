@@ -1,0 +1,74 @@
+"""Experts' products by expert against the same products a token at a time (the kernels that go pair by pair): equal bits, as
+both make each sum in the same order. Sorting and gathering against what they say; routing against a token at a time."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+# (hidden, ff: whole and partial blocks of features and channels, rows of partial warps; 12 and 20 values are no whole pieces in
+# bfloat16, 8,192 too wide for four rows at once, and 4,096 in float32: those go pair by pair)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("hidden,ff", [(8, 8), (264, 72), (12, 20), (1024, 200), (8192, 16), (4096, 16)])
+@pytest.mark.parametrize("tokens,top,experts", [(2, 1, 4), (9, 4, 6), (23, 2, 3), (128, 8, 16)])
+def test_products_by_expert_have_the_bits_of_pair_by_pair(dtype, hidden, ff, tokens, top, experts):
+    from pulsarlm_b200.kernels import ops
+
+    ops.require_device()
+    g = torch.Generator(device=DEV).manual_seed(1)
+    draw = lambda *shape: torch.randn(shape, generator=g, device=DEV)
+    h = draw(tokens, hidden + 8).to(dtype)[:, :hidden]
+    gate_up, down = (draw(experts, 2 * ff, hidden) / 16).to(dtype), (draw(experts, hidden, ff) / 16).to(dtype)
+    up = gate_up[:, :ff].contiguous()
+    ids = torch.randint(0, experts, (tokens, top), generator=g, device=DEV, dtype=torch.int32)
+    ids[0, 0], ids[-1, -1] = -1, experts  # (nobody's)
+    weights, also, also_weights = draw(tokens, top), draw(tokens, hidden).to(dtype), draw(tokens)
+
+    def run(a, b):
+        """Tokens a to b, in one call of each."""
+        n = slice(a, b)
+        acts = [torch.zeros(((b - a) * top, ff), dtype=dtype, device=DEV) for _ in range(3)]
+        ops.moe_gate_up(h[n], gate_up, ids[n], acts[0])
+        ops.moe_gate_up(h[n], gate_up, ids[n], acts[1], 2.0, weights[n])
+        ops.moe_up(h[n], up, ids[n], acts[2], "gelu")
+        outs = [torch.empty((b - a, hidden), dtype=dtype, device=DEV) for _ in range(2)]
+        ops.moe_down(acts[0], down, ids[n], weights[n], also[n], outs[0], also_weights[n])
+        ops.moe_down(acts[0], down, ids[n], None, None, outs[1])
+        return [x.view(b - a, -1) for x in acts + outs]
+
+    whole, single = run(0, tokens), [run(t, t + 1) for t in range(tokens)]
+    for i, got in enumerate(whole):
+        assert torch.equal(got, torch.cat([s[i] for s in single])), i
+
+
+@pytest.mark.parametrize("pairs,experts", [(1, 1), (1000, 33), (8192, 32), (8193, 300), (20000, 5)])
+def test_sorted_pairs_and_their_rows(pairs, experts):
+    from pulsarlm_b200.kernels import ops
+
+    ops.require_device()
+    ids = torch.randint(0, experts, (pairs, 1), device=DEV, dtype=torch.int32)
+    ends, row_of_pair, pair_of_row = ops.moe_sort(ids, experts)
+    assert torch.equal(ends.long(), torch.bincount(ids.flatten().long(), minlength=experts).cumsum(0))
+    assert torch.equal(pair_of_row.long()[row_of_pair.long()], torch.arange(pairs, device=DEV))
+    assert torch.equal(ids.flatten()[pair_of_row.long()], ids.flatten().sort().values)
+    x = torch.randn((pairs, 40), device=DEV)
+    for rows in (x, x[:, :33], x.to(torch.bfloat16)):
+        assert torch.equal(ops.moe_gather(rows, pair_of_row, 1), rows[pair_of_row.long()])
+
+
+@pytest.mark.parametrize("hidden,experts", [(1024, 32), (260, 7), (64, 129)])
+def test_routes_of_many_tokens_are_those_of_one(hidden, experts):
+    from pulsarlm_b200.kernels import ops
+
+    ops.require_device()
+    h, router = torch.randn((259, hidden), device=DEV), torch.randn((experts + 1, hidden), device=DEV)
+    shared = torch.empty(259, device=DEV)
+    ids, weights = ops.moe_route(h, router, None, 4, 1, 1, False, 1, True, shared)
+    for t in (0, 7, 8, 258):
+        gate = torch.empty(1, device=DEV)
+        one_ids, one_weights = ops.moe_route(h[t : t + 1], router, None, 4, 1, 1, False, 1, True, gate)
+        assert torch.equal(one_ids[0], ids[t]) and torch.equal(one_weights[0], weights[t]) and torch.equal(gate[0], shared[t])
