@@ -27,6 +27,11 @@
 // scan is the chain from one token's state to the next (a dot product over a column, the
 // shuffles that add its lanes' shares, the update): a prompt of one request keeps a few SMs
 // busy and takes about a microsecond a token whatever the width.
+//
+// float32 and head sizes off the list below take this walk for every step. bfloat16 with heads of 32, 64 or 128 has two
+// more forms: portions in chunks of 16 tokens (delta_chunks.cuh), steps of single tokens with a whole head a CTA
+// (delta_step.cuh). The forms' sums have different orders, so in bfloat16 a prompt's cut moves the state by fp32
+// roundings; whatever else a batch holds does not, but for which form a step takes.
 #include "common.cuh"
 
 #include "delta_chunks.cuh"
@@ -836,7 +841,8 @@ PL_API int pl_delta_rule(const void* r, const void* k, const void* v, const void
         2 * raw_bytes;
     const dim3 grid(n_entries, n_heads, col_blocks);
     // bfloat16 steps of single tokens: the form with a whole head's state in a CTA's registers and the norm behind
-    // it. float32 keeps the walk, whose bits do not depend on how a prompt was cut.
+    // it (the same state's stream as the rule with a decay per channel, where 64 entries of 32 heads of 64 x 64 went from
+    // 48 to 20.3 us). float32 keeps the walk, whose bits do not depend on how a prompt was cut.
     if (dtype == PL_BF16 && n_tokens == n_entries && (dim == 32 || dim == 64 || dim == 128) && aligned(state)) {
         const RuleStepParams c{p, static_cast<const __nv_bfloat16*>(g), norm, static_cast<__nv_bfloat16*>(out), out_row_stride,
                                eps};

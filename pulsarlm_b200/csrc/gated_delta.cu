@@ -22,6 +22,11 @@
 // the gate and rounds once. The order of every sum depends on the sizes alone, so a token's
 // result depends on the tokens before it only: not on how the prompt was cut, on the chunks
 // or on the rest of the batch.
+//
+// float32 and sizes off the list below take this walk for every step. bfloat16 with key channels 32, 64 or 128 a head has
+// two more forms: portions in chunks of 16 tokens (delta_chunks.cuh), steps of single tokens with a whole head a CTA
+// (delta_step.cuh). The forms' sums have different orders, so in bfloat16 a prompt's cut moves the state by fp32
+// roundings; whatever else a batch holds does not, but for which form a step takes.
 #include "common.cuh"
 
 #include "delta_chunks.cuh"
@@ -1083,8 +1088,9 @@ PL_API int pl_gated_delta(const void* q, const void* k, const void* v, int64_t q
     p.counts = counts; p.slots = slots; p.o_raw = o_raw; p.n_heads = n_heads; p.qk_heads = qk_heads; p.dim = dim;
     p.vdim = vdim; p.parts = parts; p.cols = cols; p.chunk = chunk; p.async_loads = async_loads; p.unit_eps = unit_eps; p.q_scale = q_scale;
     const dim3 grid(n_entries, n_heads, (vdim + cols - 1) / cols);
-    // bfloat16 steps of single tokens: the form with a whole head's state in a CTA's registers and the norm behind it (64 entries of 32 heads of
-    // 64 x 64: 48 -> 17 us). float32 keeps the walk, whose bits do not depend on how a prompt was cut.
+    // bfloat16 steps of single tokens: the form with a whole head's state in a CTA's registers and the norm behind it (64
+    // entries of 32 heads of 64 x 64: the walk's 43 us and the norm's 5 become 20.3). float32 keeps the walk, whose bits do
+    // not depend on how a prompt was cut.
     if (n_tokens == n_entries && dtype == PL_BF16 && (dim == 32 || dim == 64 || dim == 128) && (vdim == 32 || vdim == 64 || vdim == 128) &&
         (reinterpret_cast<uintptr_t>(state) & 15) == 0) {
         const GatedStepParams c{p, static_cast<const __nv_bfloat16*>(gate_pre), gate_stride, norm,
