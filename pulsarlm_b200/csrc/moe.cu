@@ -620,11 +620,14 @@ __global__ void moe_down_kernel(const scalar_t* __restrict__ act, const scalar_t
 // that chose it, up to four at a time, so an expert's weights come through once and not once per pair. Bound by these bytes;
 // what held the kernels above back is that a warp has one row's worth of loads at a time in flight and none before its
 // vector is staged: here the weights run through a ring in shared memory. 8 tokens of 4 of 32 experts of 2 x 1,024 x 2,048
-// (21 experts chosen, bfloat16): gate_up the same 40 us (176 MB), down and the sum over a token's experts 34.0 -> 28.4 us
-// (88 MB); with registers in the ring's place (two CTAs an SM) it was slower than pair by pair, 103 us for the whole block
-// against 88. Every sum is made as by the kernels above: the same bits.
+// (21 experts chosen, bfloat16), the whole block with router and shared expert: pair by pair 87.7 to 91.8 us, this 80.6 (down
+// and the sum over a token's experts 34.0 -> 28 us of 88 MB; gate_up stays near 40 of 176 MB). Two pieces deep with four CTAs an SM;
+// three with three: 84.2, four with two: 91.9, half the rows a warp and twice the CTAs: 82; registers in the ring's place: 103.
+// Every sum is made as by the kernels above: the same bits.
 constexpr int kExpertPairs = 1024;  // pairs of a step at most
 constexpr int kPairsAtOnce = 4;
+constexpr int kExpertFeatures = 4;  // a warp's
+constexpr int kExpertCtas = 4;      // an SM's, at least
 
 // The pairs that chose expert e, in any order; their number. (By the whole block.)
 __device__ __forceinline__ int pairs_of_expert(const int32_t* __restrict__ ids, int n_pairs, int e, int32_t* list, int* count) {
@@ -668,7 +671,7 @@ __device__ __forceinline__ void ring_copy(void* to, const void* from) {
 // ROWS rows of weights on their way through a lane's own places in shared memory, kStages pieces of 16 bytes deep for each row:
 // the loads in flight cost no registers and start before the vectors are there. (A lane reads what it copied itself: its own
 // wait is enough.)
-constexpr int kStages = 3;
+constexpr int kStages = 2;
 template <typename scalar_t, int ROWS>
 struct WeightRing {
     static constexpr int kCount = Vec<scalar_t>::kCount;
@@ -742,7 +745,7 @@ struct WeightRing {
 
 // Block (feature block, expert). GATED: act = unit(gate . h, up . h), rows [gate; up]; else act = a(up . h).
 template <typename scalar_t, bool GATED, bool CLAMPED>
-__global__ void __launch_bounds__(128, 3) moe_up_by_expert_kernel(const scalar_t* __restrict__ h, int64_t h_stride,
+__global__ void __launch_bounds__(128, kExpertCtas) moe_up_by_expert_kernel(const scalar_t* __restrict__ h, int64_t h_stride,
                                                                const scalar_t* __restrict__ weights, const int32_t* __restrict__ ids,
                                                                scalar_t* __restrict__ act, int n_pairs, int hidden, int ff, int top,
                                                                const float* __restrict__ in_weights, float limit, int activation) {
@@ -757,9 +760,9 @@ __global__ void __launch_bounds__(128, 3) moe_up_by_expert_kernel(const scalar_t
         return;
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    constexpr int kRows = GATED ? 2 * kFeaturesPerWarp : kFeaturesPerWarp;
+    constexpr int kRows = GATED ? 2 * kExpertFeatures : kExpertFeatures;
     const scalar_t* mine = weights + static_cast<int64_t>(e) * (GATED ? 2 : 1) * ff * hidden;
-    const int f0 = (blockIdx.x * 4 + warp) * kFeaturesPerWarp;
+    const int f0 = (blockIdx.x * 4 + warp) * kExpertFeatures;
     WeightRing<scalar_t, kRows> ring;
     ring.places = reinterpret_cast<uint4*>(staged + warp * WeightRing<scalar_t, kRows>::kBytes) + lane;
     ring.lane = lane;
@@ -767,8 +770,8 @@ __global__ void __launch_bounds__(128, 3) moe_up_by_expert_kernel(const scalar_t
     scalar_t* rows = reinterpret_cast<scalar_t*>(staged + 4 * WeightRing<scalar_t, kRows>::kBytes);  // [kPairsAtOnce][hidden]
 #pragma unroll
     for (int r = 0; r < kRows; ++r) {
-        const int f = min(f0 + r % kFeaturesPerWarp, ff - 1);
-        ring.w[r] = mine + static_cast<int64_t>(r < kFeaturesPerWarp ? f : ff + f) * hidden;
+        const int f = min(f0 + r % kExpertFeatures, ff - 1);
+        ring.w[r] = mine + static_cast<int64_t>(r < kExpertFeatures ? f : ff + f) * hidden;
     }
     for (int base = 0; base < n_mine; base += kPairsAtOnce) {
         const int here = min(kPairsAtOnce, n_mine - base);
@@ -792,16 +795,16 @@ __global__ void __launch_bounds__(128, 3) moe_up_by_expert_kernel(const scalar_t
                 const int pair = list[base + k];
                 const float in_weight = CLAMPED && in_weights != nullptr ? in_weights[pair] : 1.0f;
 #pragma unroll
-                for (int r = 0; r < kFeaturesPerWarp; ++r) {
+                for (int r = 0; r < kExpertFeatures; ++r) {
                     if (lane == r && f0 + r < ff) {
                         float value;
                         if constexpr (!GATED) {
                             value = pl_plain_activation(sums[r][k], activation);
                         } else if constexpr (CLAMPED) {
                             value = pl_clamped_unit<sizeof(scalar_t) == 4>(in_weight * sums[r][k],
-                                                                           in_weight * sums[r + kFeaturesPerWarp][k], limit);
+                                                                           in_weight * sums[r + kExpertFeatures][k], limit);
                         } else {
-                            value = silu_f32(sums[r][k]) * sums[r + kFeaturesPerWarp][k];
+                            value = silu_f32(sums[r][k]) * sums[r + kExpertFeatures][k];
                         }
                         pl_store(act + static_cast<int64_t>(pair) * ff + f0 + r, value);
                     }
@@ -820,7 +823,7 @@ __global__ void __launch_bounds__(128, 3) moe_up_by_expert_kernel(const scalar_t
 // Block (channel block, expert): y[pair, c] = down_e[c] . act[pair], fp32.
 constexpr int kDownRows = 8;
 template <typename scalar_t>
-__global__ void __launch_bounds__(128, 3) moe_down_by_expert_kernel(const scalar_t* __restrict__ act, const scalar_t* __restrict__ down,
+__global__ void __launch_bounds__(128, kExpertCtas) moe_down_by_expert_kernel(const scalar_t* __restrict__ act, const scalar_t* __restrict__ down,
                                                                  const int32_t* __restrict__ ids, float* __restrict__ y, int n_pairs,
                                                                  int hidden, int ff) {
     pl_grid_trigger();
@@ -920,7 +923,7 @@ inline size_t by_expert_bytes(int row, int width, int rows_per_warp) {
 inline bool moe_goes_by_expert(int n_tokens, int top, int n_experts, int row, int width, const void* weights) {
     const int64_t pairs = static_cast<int64_t>(n_tokens) * top;
     return n_tokens >= 2 && 2 * pairs >= n_experts && pairs <= kExpertPairs && n_experts <= 65535 && row <= 65536 &&
-        row * width % 16 == 0 && by_expert_bytes(row, width, 2 * kFeaturesPerWarp) <= 104 * 1024 &&
+        row * width % 16 == 0 && by_expert_bytes(row, width, kDownRows) <= 104 * 1024 &&
         (reinterpret_cast<uintptr_t>(weights) & 15) == 0;
 }
 
@@ -1156,10 +1159,10 @@ PL_API int pl_moe_gate_up(const void* h, int64_t h_stride, const void* gate_up, 
     const int warps = 4;
     if (moe_goes_by_expert(n_tokens, top, n_experts, hidden, dtype == PL_F32 ? 4 : 2, gate_up)) {
         PL_DISPATCH_DTYPE(dtype, "moe_gate_up", {
-            const size_t rows = by_expert_bytes(hidden, sizeof(scalar_t), 2 * kFeaturesPerWarp);
+            const size_t rows = by_expert_bytes(hidden, sizeof(scalar_t), 2 * kExpertFeatures);
             auto kernel = clamped ? moe_up_by_expert_kernel<scalar_t, true, true> : moe_up_by_expert_kernel<scalar_t, true, false>;
             allow_smem(kernel, rows);
-            pl_launch_overlapped(kernel, dim3((ff + warps * kFeaturesPerWarp - 1) / (warps * kFeaturesPerWarp), n_experts),
+            pl_launch_overlapped(kernel, dim3((ff + warps * kExpertFeatures - 1) / (warps * kExpertFeatures), n_experts),
                                  dim3(warps * 32), rows, stream, static_cast<const scalar_t*>(h), h_stride,
                                  static_cast<const scalar_t*>(gate_up), ids, static_cast<scalar_t*>(act), n_tokens * top, hidden, ff,
                                  top, in_weights, limit, 0);
@@ -1198,10 +1201,10 @@ PL_API int pl_moe_up(const void* h, int64_t h_stride, const void* up, const int3
     const int warps = 4;
     if (moe_goes_by_expert(n_tokens, top, n_experts, hidden, dtype == PL_F32 ? 4 : 2, up)) {
         PL_DISPATCH_DTYPE(dtype, "moe_up", {
-            const size_t rows = by_expert_bytes(hidden, sizeof(scalar_t), kFeaturesPerWarp);
+            const size_t rows = by_expert_bytes(hidden, sizeof(scalar_t), kExpertFeatures);
             auto kernel = moe_up_by_expert_kernel<scalar_t, false, false>;
             allow_smem(kernel, rows);
-            pl_launch_overlapped(kernel, dim3((ff + warps * kFeaturesPerWarp - 1) / (warps * kFeaturesPerWarp), n_experts),
+            pl_launch_overlapped(kernel, dim3((ff + warps * kExpertFeatures - 1) / (warps * kExpertFeatures), n_experts),
                                  dim3(warps * 32), rows, stream, static_cast<const scalar_t*>(h), h_stride,
                                  static_cast<const scalar_t*>(up), ids, static_cast<scalar_t*>(act), n_tokens * top, hidden, ff, top,
                                  static_cast<const float*>(nullptr), 0.0f, activation);
