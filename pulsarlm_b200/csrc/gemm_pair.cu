@@ -16,6 +16,10 @@
 // issues the MMAs for the pair and commits them to both CTAs' barriers
 // (`tcgen05.commit ... multicast::cluster`), and owns (in both CTAs) the tensor
 // memory allocation; warps 2-5 read their CTA's accumulator rows and store them.
+// A chunk of 32 tokens leaves through shared memory in rows of 128 features, 16 bytes a store (a store of two bytes a lane
+// and token was what bound tiles of few k blocks: 2,048 tokens by 32,000 rows of 2,048 took 271.6 us, now 159.7; gated,
+// 16,384 rows, 131.1 and now 96.2; 28,672 rows of 4,096, bound by the MMAs, 307 and now 306).
+// Tiles are 256 tokens high, or 192 where that leaves less of a round idle (tile_tokens below).
 // Two accumulators let the epilogue of one tile overlap the MMAs of the next; the
 // second CTA's epilogue releases an accumulator by arriving on the first CTA's barrier.
 // A pair is persistent and takes every P-th whole tile (P pairs), token tiles fastest:
@@ -28,8 +32,8 @@
 // Gated mode: W holds two stacked matrices, gate over up ([2N, K]), and the kernel
 // writes silu(gate x) * (up x) ([T, N]). A CTA's 128 rows are then 64 gate rows over
 // the 64 up rows of the same features (two TMA boxes per stage); in the epilogue the
-// warps that hold the up rows pass them through shared memory to the warps that hold
-// the gate rows, which round both to bfloat16 (as a product that stored them would)
+// warps that hold gate and up rows hand each other half of a chunk through shared memory,
+// round both to bfloat16 (as a product that stored them would)
 // and apply the activation (or the clamped unit of gate_units.cuh: a build of its own).
 //
 // Every wait on an mbarrier is bounded: after the limit the CTA raises bit 8 of the
@@ -38,19 +42,21 @@
 //
 // The reference leaves these products to a library (`at::linear`,
 // pulsarlm-core/src/engine/model/llama.cpp:67-69, 81, 91, 93).
+#include <type_traits>
+
 #include "gate_units.cuh"
 #include "tcgen05_helpers.cuh"
 
 namespace {
 
 constexpr int kTileM = 128;    // features per CTA, 256 per pair
-constexpr int kPairN = 256;    // tokens per tile, 128 loaded by each CTA
+constexpr int kMostTokens = 256;  // tokens per tile (kPairN: this or 192), half of them loaded by each CTA
 constexpr int kBlockK = 64;
 constexpr int kThreads = 192;
 constexpr int kStages = 6;
 constexpr int kBytesA = kTileM * kBlockK * 2;
-constexpr int kBytesB = (kPairN / 2) * kBlockK * 2;
-constexpr int kStageBytes = kBytesA + kBytesB;  // per CTA
+// Per CTA.
+__host__ __device__ constexpr int stage_bytes(int tokens) { return kBytesA + tokens / 2 * kBlockK * 2; }
 
 struct PairParams {
     void* y;  // [T, N] bf16 or fp32
@@ -116,12 +122,47 @@ __device__ __forceinline__ void arrive_on_first(uint64_t* bar) {
 constexpr int kGateRow = 17;  // 16 token columns handed over per thread and chunk, padded against bank conflicts
 constexpr int kGateBytes = 2 * 2 * (kTileM / 2) * kGateRow * 4;  // two buffers of [gate side, up side][64][17] floats
 
+// An epilogue's chunk of 32 tokens on its way out: [32][PER features] of fp32 at most, two of them.
+constexpr int out_bytes(int per) { return 2 * 32 * per * 4; }
+
+template <typename T>
+__device__ __forceinline__ T out_value(float v) {
+    if constexpr (sizeof(T) == 4) {
+        return v;
+    } else {
+        return __float2bfloat16_rn(v);
+    }
+}
+
+// Rows t0 .. of a chunk [32][PER] in shared memory to y, 16 bytes a store where rows start on 16 bytes (by 128 threads).
+template <int PER, typename T>
+__device__ __forceinline__ void store_rows(const T* rows, T* y, int64_t ldy, int t0, int t_end, int n0, int n_end, bool vectors,
+                                           int thread) {
+    constexpr int kPer16 = 16 / sizeof(T), kLanes = PER / kPer16;
+#pragma unroll
+    for (int i = 0; i < 32 * kLanes / 128; ++i) {
+        const int at = thread + 128 * i, t = t0 + at / kLanes, n = n0 + at % kLanes * kPer16;
+        if (t < t_end && n < n_end) {
+            const T* from = rows + at * kPer16;
+            T* to = y + t * ldy + n;
+            if (vectors && n + kPer16 <= n_end) {
+                *reinterpret_cast<uint4*>(to) = *reinterpret_cast<const uint4*>(from);
+            } else {
+                for (int e = 0; e < kPer16 && n + e < n_end; ++e) {
+                    to[e] = from[e];
+                }
+            }
+        }
+    }
+}
+
 // GATED: 0 the product alone, 1 silu(gate) * up, 2 the clamped unit of gate and up.
-template <int GATED>
+template <int GATED, int kPairN>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                  const PairParams p) {
-    constexpr uint32_t kColumns = 2 * kPairN;  // two accumulators
+    constexpr uint32_t kColumns = 2 * kMostTokens;  // two accumulators, kPairN columns of each half (a power of two is allotted)
+    constexpr int kStageBytes = stage_bytes(kPairN);
     constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kPairN >> 3) << 17) |
         (static_cast<uint32_t>((2 * kTileM) >> 4) << 24);
 
@@ -130,6 +171,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                                                             ~static_cast<uintptr_t>(1023));
     float* handover = reinterpret_cast<float*>(tiles + kStages * kStageBytes);  // gated: [2][2][64][17]
     constexpr int kPer = GATED ? kTileM / 2 : kTileM;      // output features per CTA and tile
+    unsigned char* leaving = tiles + kStages * kStageBytes + (GATED ? kGateBytes : 0);  // [2][32][kPer]
     __shared__ __align__(8) uint64_t full_bar[kStages];   // waited on in the first CTA only
     __shared__ __align__(8) uint64_t empty_bar[kStages];
     __shared__ __align__(8) uint64_t acc_full[2];
@@ -211,7 +253,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                 break;
             }
             tcgen05_fence_after();
-            const uint32_t tmem_d = tmem_base + acc * kPairN;
+            const uint32_t tmem_d = tmem_base + acc * kMostTokens;
             for (int kb = 0; kb < p.k_blocks; ++kb) {
                 if (!mbar_wait(&full_bar[stage], phase, &abort_flag)) {
                     ok = false;
@@ -245,16 +287,26 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         // ------------------------------------------------ epilogue (warps 2..5, both CTAs)
         const int lane_group = warp & 3;  // the tensor-memory lanes a warp may read: 32 * (warp % 4)
         const int feature = lane_group * 32 + lane;
+        const int thread = (warp - 2) * 32 + lane;
+        const bool vectors = p.ldy * (p.out_f32 ? 4 : 2) % 16 == 0 && (reinterpret_cast<uintptr_t>(p.y) & 15) == 0;
         for (int tile = tile_begin; tile < tile_end; tile += tile_step) {
             const int run = (tile - tile_begin) / tile_step;
             const int acc = run & 1;
-            if (!mbar_wait(&acc_full[acc], (run >> 1) & 1u, &abort_flag)) {
+            // (All four warps go on or none does: they meet at barriers below. Behind this one the last tile's chunks
+            // have left.)
+            int go = mbar_wait(&acc_full[acc], (run >> 1) & 1u, &abort_flag) ? 1 : 0;
+            asm volatile(
+                "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %0, 0;\n\tbarrier.cta.red.and.pred q, 1, 128, p;\n\t"
+                "selp.b32 %0, 1, 0, q;\n\t}"
+                : "+r"(go)::"memory");
+            if (!go) {
                 break;
             }
             tcgen05_fence_after();
+            const int n_first = (tile / p.t_tiles) * (2 * kPer) + rank * kPer;
             const int n = (tile / p.t_tiles) * (2 * kPer) + rank * kPer + (GATED ? feature % kPer : feature);
             const int t0 = (tile % p.t_tiles) * kPairN;
-            const uint32_t tmem_row = tmem_base + (static_cast<uint32_t>(lane_group * 32) << 16) + acc * kPairN;
+            const uint32_t tmem_row = tmem_base + (static_cast<uint32_t>(lane_group * 32) << 16) + acc * kMostTokens;
 #pragma unroll 1
             for (int c0 = 0; c0 < kPairN && t0 + c0 < p.t; c0 += 32) {
                 uint32_t v[32];
@@ -270,7 +322,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                         (is_up ? 0 : kPer * kGateRow) + (feature % kPer) * kGateRow;
 #pragma unroll
                     for (int c = 0; c < 16; ++c) {
-                        buffer[c] = __uint_as_float(v[(16 - mine) + c]);  // the half the partner finishes
+                        buffer[c] = __uint_as_float(is_up ? v[c] : v[16 + c]);  // the half the partner finishes
                     }
                     asm volatile("bar.sync 1, 128;" ::: "memory");  // (two buffers: one barrier per chunk is enough)
                     if (n < p.n) {
@@ -285,37 +337,46 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                         }
 #pragma unroll
                         for (int c = 0; c < 16; ++c) {
-                            const float own = __uint_as_float(v[mine + c]);
+                            const float own = __uint_as_float(is_up ? v[16 + c] : v[c]);
                             // both products rounded as a product that stored them would round them
                             const float g = __bfloat162float(__float2bfloat16_rn(is_up ? other[c] : own));
                             const float u = __bfloat162float(__float2bfloat16_rn(is_up ? own : other[c]));
                             act[c] = GATED == 2 ? pl_clamped_unit<false>(g, u, p.limit) : __fdividef(g, 1.0f + __expf(-g)) * u;
                         }
+                        auto put = [&](auto* rows) {
+                            using T = std::remove_reference_t<decltype(*rows)>;
 #pragma unroll
-                        for (int c = 0; c < 16; ++c) {
-                            const int t = t0 + c0 + mine + c;
-                            if (t < p.t) {
-                                if (p.out_f32) {
-                                    static_cast<float*>(p.y)[t * p.ldy + n] = act[c];
-                                } else {
-                                    static_cast<__nv_bfloat16*>(p.y)[t * p.ldy + n] = __float2bfloat16_rn(act[c]);
-                                }
+                            for (int c = 0; c < 16; ++c) {
+                                rows[(mine + c) * kPer + feature % kPer] = out_value<T>(act[c]);
                             }
+                        };
+                        if (p.out_f32) {
+                            put(reinterpret_cast<float*>(leaving) + ((c0 >> 5) & 1) * 32 * kPer);
+                        } else {
+                            put(reinterpret_cast<__nv_bfloat16*>(leaving) + ((c0 >> 5) & 1) * 32 * kPer);
                         }
                     }
-                } else if (n < p.n) {
+                } else {
+                    auto put = [&](auto* rows) {
+                        using T = std::remove_reference_t<decltype(*rows)>;
 #pragma unroll
-                    for (int c = 0; c < 32; ++c) {
-                        const int t = t0 + c0 + c;
-                        if (t < p.t) {
-                            if (p.out_f32) {
-                                static_cast<float*>(p.y)[t * p.ldy + n] = __uint_as_float(v[c]);
-                            } else {
-                                static_cast<__nv_bfloat16*>(p.y)[t * p.ldy + n] =
-                                    __float2bfloat16_rn(__uint_as_float(v[c]));
-                            }
+                        for (int c = 0; c < 32; ++c) {
+                            rows[c * kPer + feature] = out_value<T>(__uint_as_float(v[c]));
                         }
+                    };
+                    if (p.out_f32) {
+                        put(reinterpret_cast<float*>(leaving) + ((c0 >> 5) & 1) * 32 * kPer);
+                    } else {
+                        put(reinterpret_cast<__nv_bfloat16*>(leaving) + ((c0 >> 5) & 1) * 32 * kPer);
                     }
+                }
+                asm volatile("bar.sync 1, 128;" ::: "memory");  // (two chunks' places: one barrier per chunk is enough)
+                if (p.out_f32) {
+                    store_rows<kPer>(reinterpret_cast<const float*>(leaving) + ((c0 >> 5) & 1) * 32 * kPer,
+                                     static_cast<float*>(p.y), p.ldy, t0 + c0, p.t, n_first, p.n, vectors, thread);
+                } else {
+                    store_rows<kPer>(reinterpret_cast<const __nv_bfloat16*>(leaving) + ((c0 >> 5) & 1) * 32 * kPer,
+                                     static_cast<__nv_bfloat16*>(p.y), p.ldy, t0 + c0, p.t, n_first, p.n, vectors, thread);
                 }
             }
             tcgen05_fence_before();
@@ -371,13 +432,14 @@ PL_API int pl_gemm_bf16_pair_supports(int t, int n, int k, int64_t ldx, int64_t 
 
 namespace {
 
-template <int GATED>
+template <int GATED, int TOKENS>
 int launch_pair(const CUtensorMap& map_w, const CUtensorMap& map_x, const PairParams& p, int used_pairs,
                 cudaStream_t stream) {
-    constexpr int smem = kStages * kStageBytes + (GATED ? kGateBytes : 0) + 1024;
+    constexpr int smem =
+        kStages * stage_bytes(TOKENS) + (GATED ? kGateBytes : 0) + out_bytes(GATED ? kTileM / 2 : kTileM) + 1024;
     static bool configured = false;
     if (!configured) {
-        const cudaError_t err = cudaFuncSetAttribute(gemm_pair_kernel<GATED>,
+        const cudaError_t err = cudaFuncSetAttribute(gemm_pair_kernel<GATED, TOKENS>,
                                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (err != cudaSuccess) {
             return pl_fail(3, "gemm_bf16_pair: cannot set shared memory size: %s", cudaGetErrorString(err));
@@ -398,11 +460,24 @@ int launch_pair(const CUtensorMap& map_w, const CUtensorMap& map_x, const PairPa
     attributes[1].val.programmaticStreamSerializationAllowed = 1;
     config.attrs = attributes;
     config.numAttrs = pl_overlap_enabled() ? 2 : 1;
-    const cudaError_t err = cudaLaunchKernelEx(&config, gemm_pair_kernel<GATED>, map_w, map_x, p);
+    const cudaError_t err = cudaLaunchKernelEx(&config, gemm_pair_kernel<GATED, TOKENS>, map_w, map_x, p);
     if (err != cudaSuccess) {
         return pl_fail(3, "gemm_bf16_pair: launch failed: %s", cudaGetErrorString(err));
     }
     return 0;
+}
+
+// Tokens of a tile: 256, or 192 where the pairs' rounds of tiles then take less time: a round of 192 takes 0.82 of one of
+// 256 (0.235 us a k block against 0.277 in few rounds, 0.79 in many). Gated, 16,384 rows of 2,048: 552 tokens 45.1 against
+// 51.2 us, 1,536 tokens 77.8 against 84.0, 512 tokens 45.1 against 41.0, 2,048 tokens 102.4 against 96.2; 28,672 rows of
+// 4,096: 552 tokens 104.4 against 120.8, 1,024 tokens 180.2 against 162.0.
+int tile_tokens(int t, int n_tiles) {
+    const int64_t pairs = pair_count();
+    auto rounds = [&](int tokens) {
+        const int64_t tiles = static_cast<int64_t>(n_tiles) * ((t + tokens - 1) / tokens);
+        return (tiles + pairs - 1) / pairs;
+    };
+    return rounds(192) * 41 < rounds(256) * 50 ? 192 : 256;
 }
 
 }  // namespace
@@ -427,7 +502,8 @@ static int run_pair(const void* x, const void* w, void* y, int t, int n, int k, 
                                   gated ? kTileM / 2 : kTileM, kBlockK)) {
         return code;
     }
-    if (const int code = make_map(&map_x, x, t, k, ldx, kPairN / 2, kBlockK)) {
+    const int tokens = tile_tokens(t, (n + per_pair - 1) / per_pair);
+    if (const int code = make_map(&map_x, x, t, k, ldx, tokens / 2, kBlockK)) {
         return code;
     }
     PairParams p;
@@ -439,14 +515,19 @@ static int run_pair(const void* x, const void* w, void* y, int t, int n, int k, 
     p.out_f32 = out_f32;
     p.limit = limit;
     p.n_tiles = (n + per_pair - 1) / per_pair;
-    p.t_tiles = (t + kPairN - 1) / kPairN;
+    p.t_tiles = (t + tokens - 1) / tokens;
     p.k_blocks = (k + kBlockK - 1) / kBlockK;
     p.total_tiles = p.n_tiles * p.t_tiles;
     const int used_pairs = p.total_tiles < pair_count() ? p.total_tiles : pair_count();
     p.status = status;
-    return gated == 2 ? launch_pair<2>(map_w, map_x, p, used_pairs, stream)
-        : gated       ? launch_pair<1>(map_w, map_x, p, used_pairs, stream)
-                      : launch_pair<0>(map_w, map_x, p, used_pairs, stream);
+    if (tokens == 192) {
+        return gated == 2 ? launch_pair<2, 192>(map_w, map_x, p, used_pairs, stream)
+            : gated       ? launch_pair<1, 192>(map_w, map_x, p, used_pairs, stream)
+                          : launch_pair<0, 192>(map_w, map_x, p, used_pairs, stream);
+    }
+    return gated == 2 ? launch_pair<2, 256>(map_w, map_x, p, used_pairs, stream)
+        : gated       ? launch_pair<1, 256>(map_w, map_x, p, used_pairs, stream)
+                      : launch_pair<0, 256>(map_w, map_x, p, used_pairs, stream);
 }
 
 PL_API int pl_gemm_bf16_pair(const void* x, const void* w, void* y, int t, int n, int k, int64_t ldx, int64_t ldw,

@@ -1,0 +1,76 @@
+"""Products on pairs of SMs, both heights of their tiles, and what leaves them: whole numbers whose sums fp32 holds exactly, so
+fp32 outputs are the products and bfloat16 ones their nearest values."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _operands(t, n, k, pad):
+    g = torch.Generator(device=DEV).manual_seed(t + n + k)
+    draw = lambda *shape: torch.randint(-3, 4, shape, generator=g, device=DEV).to(torch.bfloat16)
+    return draw(t, k + pad)[:, :k], draw(n, k + pad)[:, :k]
+
+
+# (tokens: ends of chunks of 32 and of tiles of 192 and 256, several tiles a pair; features: rows that are no whole 16 bytes, ends of
+# CTAs' and pairs' shares)
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("t", [1, 31, 192, 193, 257, 552, 1100])
+@pytest.mark.parametrize("n,k,pad", [(5, 8, 0), (130, 72, 8), (256, 64, 0), (20003, 200, 0), (8200, 136, 16)])
+def test_whole_numbers_come_out_exactly(out_dtype, t, n, k, pad):
+    from pulsarlm_b200.kernels import ops
+
+    ops.require_device()
+    x, w = _operands(t, n, k, pad)
+    want = (x.float() @ w.float().t())  # (sums of at most 200 * 9: exact in any order and in TF32's products too)
+    for wide in (0, 3):  # (a matrix with rows further apart: not on 16 bytes)
+        out = torch.full((t, n + wide), 7.0, dtype=out_dtype, device=DEV)
+        ops.gemm_bf16(x, w, out[:, :n], kernel="pair")
+        assert torch.equal(out[:, :n], want.to(out_dtype)) and bool((out[:, n:] == 7.0).all())
+
+
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("limit", [None, 5.0])
+@pytest.mark.parametrize("t", [1, 193, 552])
+@pytest.mark.parametrize("n,k", [(5, 8), (130, 72), (10240, 64)])
+def test_gated_products(out_dtype, limit, t, n, k):
+    from pulsarlm_b200.kernels import ops
+
+    ops.require_device()
+    x, w = _operands(t, 2 * n, k, 0)
+    w = w / 8
+    both = (x.float() @ w.float().t()).to(torch.bfloat16)
+    if limit is None:
+        g, u = both.double().split(n, dim=1)
+        want = g / (1 + torch.exp(-g)) * u
+    else:  # (the same unit, of a product that was written)
+        want = torch.empty((t, n), dtype=torch.bfloat16, device=DEV)
+        ops.gated_act(both, want, "clamped", limit)
+        want = want.double()
+    got = torch.full((t, n + 3), 7.0, dtype=out_dtype, device=DEV)
+    ops.gemm_bf16(x, w, got[:, :n], kernel="pair", gated=True, limit=limit)
+    # (fp32: __expf's stated error of 2 + 1.16 |g| units of 2^-23, |g| at most 81, and a few roundings: 2^-16; bfloat16 on one
+    # side or both: half a place each, 2^-8 together)
+    rel = 2.0**-16 if out_dtype == torch.float32 and limit is None else 2.0**-8
+    assert bool(((got[:, :n].double() - want).abs() <= rel * want.abs() + 1e-30).all()) and bool((got[:, n:] == 7.0).all())
+
+
+@pytest.mark.parametrize("t,inter,k,own", [(507, 14336, 64, False), (508, 14336, 64, True), (1024, 8192, 64, True), (191, 65536, 64, False)])
+def test_gate_up_is_the_same_on_either_route(t, inter, k, own):  # (3 x 74 tiles of 65,536 values are the line)
+    from pulsarlm_b200.kernels import ops
+    from pulsarlm_b200.parts import linear
+
+    ops.require_device()
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:  # (where the line lies depends on the SMs)
+        assert (linear.own_kernel_for(t, 2 * inter, torch.device(DEV), k, gated=True) == "pair") == own
+    x, w = _operands(t, 2 * inter, k, 0)
+    w = w / 8
+    want = torch.empty((t, inter), dtype=torch.bfloat16, device=DEV)
+    ops.swiglu((x.float() @ w.float().t()).to(torch.bfloat16), want)
+    got = linear.gated_linear(x, w)
+    # (the same rounded products; two forms of one quotient, each rounded to bfloat16: a place apart at most)
+    assert bool(((got.float() - want.float()).abs() <= 2.0**-7 * want.float().abs() + 1e-30).all())
