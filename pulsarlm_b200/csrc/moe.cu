@@ -415,6 +415,22 @@ __device__ __forceinline__ void warp_dots_two(const scalar_t* __restrict__ w0, c
     }
 }
 
+// n values to shared memory as fp32 (by the whole block), four a load where they start on four: a value a load makes a
+// chain of sixteen and more loads' times out of a row of 2,048.
+template <typename scalar_t>
+__device__ __forceinline__ void stage_row(const scalar_t* __restrict__ from, float* __restrict__ to, int n) {
+    if ((n & 3) == 0 && (reinterpret_cast<uintptr_t>(from) & (4 * sizeof(scalar_t) - 1)) == 0) {
+#pragma unroll 4
+        for (int i = 4 * threadIdx.x; i < n; i += 4 * blockDim.x) {
+            *reinterpret_cast<float4*>(to + i) = pl_load4(from + i);
+        }
+        return;
+    }
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        to[i] = pl_load(from + i);
+    }
+}
+
 constexpr int kFeaturesPerWarp = 4;
 
 template <int N>
@@ -431,7 +447,7 @@ __global__ void moe_gate_up_kernel(const scalar_t* __restrict__ h, int64_t h_str
                                    int vectors, const float* __restrict__ in_weights, float limit) {
     pl_grid_trigger();
     pl_grid_wait();
-    extern __shared__ float row[];  // [hidden]
+    extern __shared__ __align__(16) float row[];  // [hidden]
     const int pair = blockIdx.x;
     const int t = pair / top;
     const int e = ids[pair];
@@ -440,9 +456,7 @@ __global__ void moe_gate_up_kernel(const scalar_t* __restrict__ h, int64_t h_str
     auto unit = [&](float g, float u) {
         return CLAMPED ? pl_clamped_unit<sizeof(scalar_t) == 4>(in_weight * g, in_weight * u, limit) : silu_f32(g) * u;
     };
-    for (int i = threadIdx.x; i < hidden; i += blockDim.x) {
-        row[i] = pl_load(h + t * h_stride + i);
-    }
+    stage_row(h + t * h_stride, row, hidden);
     __syncthreads();
     if (e < 0 || e >= n_experts) {
         return;
@@ -482,14 +496,12 @@ __global__ void moe_up_kernel(const scalar_t* __restrict__ h, int64_t h_stride, 
                               int n_experts, int vectors, int activation) {
     pl_grid_trigger();
     pl_grid_wait();
-    extern __shared__ float row[];  // [hidden]
+    extern __shared__ __align__(16) float row[];  // [hidden]
     const int pair = blockIdx.x;
     const int t = pair / top;
     const int e = ids[pair];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-    for (int i = threadIdx.x; i < hidden; i += blockDim.x) {
-        row[i] = pl_load(h + t * h_stride + i);
-    }
+    stage_row(h + t * h_stride, row, hidden);
     __syncthreads();
     if (e < 0 || e >= n_experts) {
         return;
@@ -529,12 +541,10 @@ __global__ void moe_down_kernel(const scalar_t* __restrict__ act, const scalar_t
                                 scalar_t* __restrict__ out, int hidden, int ff, int top, int n_experts, int vectors) {
     pl_grid_trigger();
     pl_grid_wait();
-    extern __shared__ float rows[];  // [top][ff]
+    extern __shared__ __align__(16) float rows[];  // [top][ff]
     const int t = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-    for (int i = threadIdx.x; i < top * ff; i += blockDim.x) {
-        rows[i] = pl_load(act + static_cast<int64_t>(t) * top * ff + i);
-    }
+    stage_row(act + static_cast<int64_t>(t) * top * ff, rows, top * ff);
     __syncthreads();
     const int c0 = (blockIdx.y * warps + warp) * kChannelsPerWarp;
     if (c0 + kChannelsPerWarp <= hidden) {
@@ -620,8 +630,9 @@ __global__ void moe_down_kernel(const scalar_t* __restrict__ act, const scalar_t
 // that chose it, up to four at a time, so an expert's weights come through once and not once per pair. Bound by these bytes;
 // what held the kernels above back is that a warp has one row's worth of loads at a time in flight and none before its
 // vector is staged: here the weights run through a ring in shared memory. 8 tokens of 4 of 32 experts of 2 x 1,024 x 2,048
-// (21 experts chosen, bfloat16), the whole block with router and shared expert: pair by pair 87.7 to 91.8 us, this 80.6 (down
-// and the sum over a token's experts 34.0 -> 28 us of 88 MB; gate_up stays near 40 of 176 MB). Two pieces deep with four CTAs an SM;
+// (21 experts chosen, bfloat16), the whole block with router and shared expert: pair by pair 86.4 to 91.8 us, this 76.1 (down
+// and the sum over a token's experts 34.0 -> 25.7 us of 88 MB, gate_up 40.2 -> 38.3 of 176 MB). With the tokens' rows
+// staged a value a load 80.6, of which the other forms' times: two pieces deep with four CTAs an SM, as here;
 // three with three: 84.2, four with two: 91.9, half the rows a warp and twice the CTAs: 82; registers in the ring's place: 103.
 // Every sum is made as by the kernels above: the same bits.
 constexpr int kExpertPairs = 1024;  // pairs of a step at most
@@ -743,6 +754,25 @@ struct WeightRing {
     }
 };
 
+// Rows row(0) .. row(here - 1) of n values (whole 16-byte pieces) one behind the other in shared memory, by the whole block.
+template <typename scalar_t, typename Row>
+__device__ __forceinline__ void stage_rows(scalar_t* __restrict__ to, int n, int here, bool vectors, Row row) {
+    if (vectors) {
+        constexpr int kCount = Vec<scalar_t>::kCount;
+        const int pieces = n / kCount;
+#pragma unroll 4
+        for (int i = threadIdx.x; i < here * pieces; i += 128) {
+            const int k = i / pieces;
+            reinterpret_cast<uint4*>(to)[i] = *reinterpret_cast<const uint4*>(row(k) + (i - k * pieces) * kCount);
+        }
+        return;
+    }
+    for (int i = threadIdx.x; i < here * n; i += 128) {
+        const int k = i / n;
+        to[i] = row(k)[i - k * n];
+    }
+}
+
 // Block (feature block, expert). GATED: act = unit(gate . h, up . h), rows [gate; up]; else act = a(up . h).
 template <typename scalar_t, bool GATED, bool CLAMPED>
 __global__ void __launch_bounds__(128, kExpertCtas) moe_up_by_expert_kernel(const scalar_t* __restrict__ h, int64_t h_stride,
@@ -773,18 +803,14 @@ __global__ void __launch_bounds__(128, kExpertCtas) moe_up_by_expert_kernel(cons
         const int f = min(f0 + r % kExpertFeatures, ff - 1);
         ring.w[r] = mine + static_cast<int64_t>(r < kExpertFeatures ? f : ff + f) * hidden;
     }
+    const bool vectors = h_stride * sizeof(scalar_t) % 16 == 0 && (reinterpret_cast<uintptr_t>(h) & 15) == 0;
     for (int base = 0; base < n_mine; base += kPairsAtOnce) {
         const int here = min(kPairsAtOnce, n_mine - base);
         if (base > 0) {
             __syncthreads();
         }
         ring.start();
-        for (int k = 0; k < here; ++k) {
-            const scalar_t* src = h + static_cast<int64_t>(list[base + k] / top) * h_stride;
-            for (int i = threadIdx.x; i < hidden; i += 128) {
-                rows[k * hidden + i] = src[i];
-            }
-        }
+        stage_rows<scalar_t>(rows, hidden, here, vectors, [&](int k) { return h + static_cast<int64_t>(list[base + k] / top) * h_stride; });
         __syncthreads();
         auto finish = [&](auto number) {
             constexpr int N = decltype(number)::value;
@@ -847,18 +873,14 @@ __global__ void __launch_bounds__(128, kExpertCtas) moe_down_by_expert_kernel(co
     for (int r = 0; r < kDownRows; ++r) {
         ring.w[r] = down + (static_cast<int64_t>(e) * hidden + min(c0 + r, hidden - 1)) * ff;
     }
+    const bool vectors = (reinterpret_cast<uintptr_t>(act) & 15) == 0;
     for (int base = 0; base < n_mine; base += kPairsAtOnce) {
         const int here = min(kPairsAtOnce, n_mine - base);
         if (base > 0) {
             __syncthreads();
         }
         ring.start();
-        for (int k = 0; k < here; ++k) {
-            const scalar_t* src = act + static_cast<int64_t>(list[base + k]) * ff;
-            for (int i = threadIdx.x; i < ff; i += 128) {
-                rows[k * ff + i] = src[i];
-            }
-        }
+        stage_rows<scalar_t>(rows, ff, here, vectors, [&](int k) { return act + static_cast<int64_t>(list[base + k]) * ff; });
         __syncthreads();
         auto finish = [&](auto number) {
             constexpr int N = decltype(number)::value;

@@ -12,16 +12,18 @@ DEV = "cuda:0"
 
 # (hidden, ff: whole and partial blocks of features and channels, rows of partial warps; 12 and 20 values are no whole pieces in
 # bfloat16, 8,192 too wide for four rows at once, and 4,096 in float32: those go pair by pair)
+# (pad: rows of h on 16 bytes, and not)
+@pytest.mark.parametrize("pad", [8, 3])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("hidden,ff", [(8, 8), (264, 72), (12, 20), (1024, 200), (8192, 16), (4096, 16)])
 @pytest.mark.parametrize("tokens,top,experts", [(2, 1, 4), (9, 4, 6), (23, 2, 3), (128, 8, 16)])
-def test_products_by_expert_have_the_bits_of_pair_by_pair(dtype, hidden, ff, tokens, top, experts):
+def test_products_by_expert_have_the_bits_of_pair_by_pair(pad, dtype, hidden, ff, tokens, top, experts):
     from pulsarlm_b200.kernels import ops
 
     ops.require_device()
     g = torch.Generator(device=DEV).manual_seed(1)
     draw = lambda *shape: torch.randn(shape, generator=g, device=DEV)
-    h = draw(tokens, hidden + 8).to(dtype)[:, :hidden]
+    h = draw(tokens, hidden + pad).to(dtype)[:, :hidden]
     gate_up, down = (draw(experts, 2 * ff, hidden) / 16).to(dtype), (draw(experts, hidden, ff) / 16).to(dtype)
     up = gate_up[:, :ff].contiguous()
     ids = torch.randint(0, experts, (tokens, top), generator=g, device=DEV, dtype=torch.int32)
