@@ -117,7 +117,7 @@ __device__ __forceinline__ float4 load_row4(const float* base, int ld, int row, 
 // with k outermost, the next 16 k in registers meanwhile. A thread reads its RM + RN operands of a k
 // AHEAD k before their fmafs. What bounds it: shared memory hands a warp one operand a lane and cycle while the
 // SM's four schedulers do four fmafs a lane and cycle, so RM x RN / (RM + RN) has to stay above four (8 x 16: 5.3;
-// 8 x 8: 4; 4 x 8: 2.7, for products of few tiles, where more warps count more).
+// 8 x 8: 4). For products of hundreds of rows and many tiles: 16384 x 2048, 509 rows 690 us (50 TFLOP/s).
 template <int BM, int BN, int RM, int RN, int AHEAD, int CTAS>
 __global__ void __launch_bounds__(BM * BN / (RM * RN), CTAS) gemm_f32_tile_kernel(const GemmF32Params p) {
     constexpr int kThreads = BM * BN / (RM * RN);
@@ -257,54 +257,62 @@ __global__ void __launch_bounds__(BM * BN / (RM * RN), CTAS) gemm_f32_tile_kerne
 }
 
 template <int BM, int BN, int RM, int RN, int AHEAD, int CTAS>
-void launch_tile(const GemmF32Params& p, cudaStream_t stream) {
+cudaError_t launch_tile(const GemmF32Params& p, cudaStream_t stream) {
     constexpr int kSmem = 2 * 16 * (BM + 4 + BN + 4) * static_cast<int>(sizeof(float));
     static_assert(kSmem <= 48 * 1024, "needs no opt-in");
     gemm_f32_tile_kernel<BM, BN, RM, RN, AHEAD, CTAS>
         <<<dim3((p.m + BM - 1) / BM, (p.n + BN - 1) / BN), BM * BN / (RM * RN), kSmem, stream>>>(p);
+    return cudaGetLastError();
 }
 
-// ---------------------------------------------------------------------------- few rows
-// A few rows of A against a stream of weights: 16 weight rows a CTA, TM x RM rows of A, a thread one weight
-// row and RM rows of A. Both operands arrive by cp.async, `stages` pieces of 128 k in flight, and are read
-// sixteen (RM == 4: eight) k ahead of the fmafs. What bounds it: the weights' stream where N is large, the chain
-// of K dependent fmafs (4 cycles each) where K is.
-constexpr int kFewN = 16;
-constexpr int kFewK = 128;
-constexpr int kFewLd = kFewK + 4;  // (rows 4 banks apart: eight rows' 16-byte reads meet no bank twice)
-
-template <int TM, int RM>
-__global__ void __launch_bounds__(kFewN * TM) gemm_f32_few_kernel(const GemmF32Params p, const int stages) {
-    constexpr int BM = TM * RM;
-    constexpr int kThreads = kFewN * TM;
-    constexpr int kStageFloats = (kFewN + BM) * kFewLd;
-    constexpr int kAhead = RM == 4 ? 2 : 4;  // 16-byte groups of k read ahead
-    extern __shared__ __align__(16) float few_smem[];
+// ---------------------------------------------------------------------------- rows along k
+// LN * CN weight rows and TM * RM rows of A a CTA, CN x RM of them a thread (weight rows LN apart, so that neighbours
+// of a warp read neighbouring ones). Both operands arrive by cp.async as they lie, `stages` pieces of BK k in flight, and
+// are read four k a load, AHEAD loads before their fmafs: no transposed copy, no registers held for it. What bounds it:
+// the weights' stream where N is large and rows are few; shared memory's four bytes a lane and cycle (CN + RM operands
+// for CN * RM fmafs) where rows are many; the chain of K dependent fmafs where a CTA is alone on its SM. So tiles grow
+// with the rows, and with the columns once the SMs are full (form_for below). 16384 x 2048 and 8 / 16 / 32 / 300 rows:
+// 40 / 50 / 76 / 488 us; with one weight row a thread and, above, 64 x 64 tiles through registers 51 / 90 / 130 / 589.
+template <int LN, int CN, int TM, int RM, int BK, int AHEAD, int CTAS>
+__global__ void __launch_bounds__(LN * TM, CTAS) gemm_f32_rows_kernel(const GemmF32Params p, const int stages) {
+    constexpr int BN = LN * CN, BM = TM * RM;
+    constexpr int kThreads = LN * TM;
+    constexpr int kLd = BK + 4;  // (rows 4 banks apart: eight rows' 16-byte reads meet no bank twice)
+    constexpr int kStageFloats = (BN + BM) * kLd;
+    constexpr int kLanes = BK / 4, kRows = kThreads / kLanes;  // threads that copy a row's piece, rows copied at a time
+    static_assert(kThreads % kLanes == 0 && BK / 4 > AHEAD, "tile");
+    extern __shared__ __align__(16) float rows_smem[];
     const int tid = threadIdx.x;
-    const int col = tid % kFewN, tm = tid / kFewN;
-    const int n0 = blockIdx.x * kFewN, m0 = blockIdx.y * BM;
-    const int pieces = (p.k + kFewK - 1) / kFewK;
+    const int col = tid % LN, tm = tid / LN;
+    const int n0 = blockIdx.x * BN, m0 = blockIdx.y * BM;
+    const int pieces = (p.k + BK - 1) / BK;
 
-    // This thread's copies: 16 bytes at column (tid % 32) * 4 of every (kThreads / 32)-th row.
-    const int load_row = tid / 32, load_k = (tid % 32) * 4;
+    const int load_row = tid / kLanes, load_k = (tid % kLanes) * 4;
     auto load = [&](int piece, int slot) {
-        float* stage = few_smem + slot * kStageFloats + load_row * kFewLd + load_k;
-        const int gk = piece * kFewK + load_k;
-        const int left = max(0, min(4, p.k - gk)) * 4;
-        const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(stage));
-#pragma unroll
-        for (int i = 0; i < (kFewN + BM) / (kThreads / 32); ++i) {
-            const int row = load_row + i * (kThreads / 32);
-            const bool weight = row < kFewN;
-            const int at = weight ? n0 + row : m0 + row - kFewN;
-            const bool there = left > 0 && (weight ? at < p.n : at < p.m);
-            const float* base = weight ? p.w : p.a;
-            // (past the operand nothing is read: the address is then its first, with no bytes)
-            const float* from = there ? base + static_cast<int64_t>(at) * (weight ? p.ldw : p.lda) + gk : base;
+        const int gk = piece * BK + load_k;
+        const int bytes = max(0, min(4, p.k - gk)) * 4;
+        const int from = bytes > 0 ? gk : 0;  // (past k nothing is read, nor rows of A past the last; weight rows past
+                                              // the last read it, and put() drops what comes of them)
+        const uint32_t dst = static_cast<uint32_t>(
+            __cvta_generic_to_shared(rows_smem + slot * kStageFloats + load_row * kLd + load_k));
+        auto copy = [&](int i, const float* src, int bytes) {
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
-                             dst + i * (kThreads / 32) * kFewLd * static_cast<int>(sizeof(float))),
-                         "l"(from), "r"(there ? left : 0)
+                             dst + i * kLd * static_cast<int>(sizeof(float))),
+                         "l"(src + from), "r"(bytes)
                          : "memory");
+        };
+#pragma unroll
+        for (int i = 0; i < BN; i += kRows) {
+            if (BN % kRows == 0 || i + load_row < BN) {
+                copy(i, p.w + static_cast<int64_t>(min(n0 + i + load_row, p.n - 1)) * p.ldw, bytes);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < BM; i += kRows) {
+            if (BM % kRows == 0 || i + load_row < BM) {
+                const int row = m0 + i + load_row;
+                copy(BN + i, p.a + static_cast<int64_t>(min(row, p.m - 1)) * p.lda, row < p.m ? bytes : 0);
+            }
         }
     };
     for (int s = 0; s < stages - 1; ++s) {
@@ -313,18 +321,25 @@ __global__ void __launch_bounds__(kFewN * TM) gemm_f32_few_kernel(const GemmF32P
         }
         cp_async_commit();
     }
-    float acc[RM];
+    float acc[RM][CN];
 #pragma unroll
     for (int i = 0; i < RM; ++i) {
-        acc[i] = 0.0f;
+#pragma unroll
+        for (int j = 0; j < CN; ++j) {
+            acc[i][j] = 0.0f;
+        }
     }
     int slot = 0, next_slot = stages - 1;
     for (int piece = 0; piece < pieces; ++piece) {
         // The group of this piece is the oldest of stages - 1 in flight.
         if (stages == 8) {
             cp_async_wait<6>();
-        } else {
+        } else if (stages == 6) {
+            cp_async_wait<4>();
+        } else if (stages == 4) {
             cp_async_wait<2>();
+        } else {
+            cp_async_wait<1>();
         }
         __syncthreads();
         if (piece + stages - 1 < pieces) {
@@ -332,60 +347,139 @@ __global__ void __launch_bounds__(kFewN * TM) gemm_f32_few_kernel(const GemmF32P
         }
         cp_async_commit();
         next_slot = next_slot + 1 == stages ? 0 : next_slot + 1;
-        const float* stage = few_smem + slot * kStageFloats;
+        const float* stage = rows_smem + slot * kStageFloats;
         slot = slot + 1 == stages ? 0 : slot + 1;
-        const float4* w4 = reinterpret_cast<const float4*>(stage + col * kFewLd);
-        const float4* a4 = reinterpret_cast<const float4*>(stage + (kFewN + tm * RM) * kFewLd);
-        float4 w[2][kAhead], a[2][RM][kAhead];
+        const float* w_at = stage + col * kLd;
+        const float* a_at = stage + (BN + tm * RM) * kLd;
+        float4 w[AHEAD + 1][CN], a[AHEAD + 1][RM];
         auto fetch = [&](int which, int group) {
 #pragma unroll
-            for (int j = 0; j < kAhead; ++j) {
-                w[which][j] = w4[group * kAhead + j];
+            for (int j = 0; j < CN; ++j) {
+                w[which][j] = *reinterpret_cast<const float4*>(w_at + j * LN * kLd + group * 4);
+            }
 #pragma unroll
-                for (int i = 0; i < RM; ++i) {
-                    a[which][i][j] = a4[i * (kFewLd / 4) + group * kAhead + j];
-                }
+            for (int i = 0; i < RM; ++i) {
+                a[which][i] = *reinterpret_cast<const float4*>(a_at + i * kLd + group * 4);
             }
         };
-        fetch(0, 0);
-        constexpr int kGroups = kFewK / 4 / kAhead;
 #pragma unroll
-        for (int group = 0; group < kGroups; ++group) {
-            const int now = group & 1;
-            if (group + 1 < kGroups) {
-                fetch(now ^ 1, group + 1);
+        for (int group = 0; group < AHEAD; ++group) {
+            fetch(group, group);
+        }
+#pragma unroll
+        for (int group = 0; group < BK / 4; ++group) {
+            const int now = group % (AHEAD + 1);
+            if (group + AHEAD < BK / 4) {
+                fetch((group + AHEAD) % (AHEAD + 1), group + AHEAD);
             }
 #pragma unroll
-            for (int j = 0; j < kAhead; ++j) {
+            for (int i = 0; i < RM; ++i) {
 #pragma unroll
-                for (int i = 0; i < RM; ++i) acc[i] = fmaf(a[now][i][j].x, w[now][j].x, acc[i]);
+                for (int j = 0; j < CN; ++j) {
+                    acc[i][j] = fmaf(a[now][i].x, w[now][j].x, acc[i][j]);
+                }
+            }
 #pragma unroll
-                for (int i = 0; i < RM; ++i) acc[i] = fmaf(a[now][i][j].y, w[now][j].y, acc[i]);
+            for (int i = 0; i < RM; ++i) {
 #pragma unroll
-                for (int i = 0; i < RM; ++i) acc[i] = fmaf(a[now][i][j].z, w[now][j].z, acc[i]);
+                for (int j = 0; j < CN; ++j) {
+                    acc[i][j] = fmaf(a[now][i].y, w[now][j].y, acc[i][j]);
+                }
+            }
 #pragma unroll
-                for (int i = 0; i < RM; ++i) acc[i] = fmaf(a[now][i][j].w, w[now][j].w, acc[i]);
+            for (int i = 0; i < RM; ++i) {
+#pragma unroll
+                for (int j = 0; j < CN; ++j) {
+                    acc[i][j] = fmaf(a[now][i].z, w[now][j].z, acc[i][j]);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < RM; ++i) {
+#pragma unroll
+                for (int j = 0; j < CN; ++j) {
+                    acc[i][j] = fmaf(a[now][i].w, w[now][j].w, acc[i][j]);
+                }
             }
         }
     }
 #pragma unroll
     for (int i = 0; i < RM; ++i) {
-        put(p, m0 + tm * RM + i, n0 + col, acc[i]);
+#pragma unroll
+        for (int j = 0; j < CN; ++j) {
+            put(p, m0 + tm * RM + i, n0 + col + j * LN, acc[i][j]);
+        }
     }
 }
 
-template <int TM, int RM>
-cudaError_t launch_few(const GemmF32Params& p, cudaStream_t stream) {
-    const dim3 grid((p.n + kFewN - 1) / kFewN, (p.m + TM * RM - 1) / (TM * RM));
-    // A CTA alone on its SM keeps eight pieces in flight; where SMs hold several, four each (8 KB of weights a piece).
-    const int stages = static_cast<int64_t>(grid.x) * grid.y <= 148 ? 8 : 4;
-    const int smem = stages * (kFewN + TM * RM) * kFewLd * static_cast<int>(sizeof(float));
-    const cudaError_t set = pl_allow_smem<gemm_f32_few_kernel<TM, RM>>(8 * (kFewN + TM * RM) * kFewLd * static_cast<int>(sizeof(float)));
+// A CTA alone on its SM keeps ALONE pieces in flight, one among others SHARED.
+template <int LN, int CN, int TM, int RM, int BK, int AHEAD, int ALONE, int SHARED, int CTAS = 1>
+cudaError_t launch_rows(const GemmF32Params& p, cudaStream_t stream) {
+    constexpr int BN = LN * CN, BM = TM * RM;
+    constexpr int kStage = (BN + BM) * (BK + 4) * static_cast<int>(sizeof(float));
+    static_assert(ALONE * kStage <= 227 * 1024 && SHARED <= ALONE, "stages");
+    const dim3 grid((p.n + BN - 1) / BN, (p.m + BM - 1) / BM);
+    const int stages = static_cast<int64_t>(grid.x) * grid.y <= 148 ? ALONE : SHARED;
+    const cudaError_t set = pl_allow_smem<gemm_f32_rows_kernel<LN, CN, TM, RM, BK, AHEAD, CTAS>>(ALONE * kStage);
     if (set != cudaSuccess) {
         return set;
     }
-    gemm_f32_few_kernel<TM, RM><<<grid, kFewN * TM, smem, stream>>>(p, stages);
+    gemm_f32_rows_kernel<LN, CN, TM, RM, BK, AHEAD, CTAS><<<grid, LN * TM, stages * kStage, stream>>>(p, stages);
     return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------- which form
+// A form's tile, how many of its CTAs an SM holds, the time of a CTA alone on its SM and what each further one adds, in ps a k.
+// Measured with weights that are not in L2, 2048 to 32000 columns of 2048 to 8192 k. What is chosen decides time alone.
+// Picked form / the one before these (us): 8 rows, 12288 x 2048: 32 / 47; 16 rows,
+// 8192 x 2048: 33 / 59; 32 rows, 6144 x 4096: 90 / 119; 64 rows, 4096 x 2048: 47 / 69; 128 rows, 3072 x 2048: 76 / 99;
+// 200 rows, 2048 x 8192: 301 / 389; 300 rows, 32000 x 2048: 904 / 1065; 700 rows, 4096 x 2048: 281 / 312. Within 4 % of
+// even: up to 4 rows of 4096 columns and fewer, 509 rows of 16384 and 32000 (the 128-row tiles as before).
+struct Form {
+    int rows, columns, resident, alone, more;
+    cudaError_t (*launch)(const GemmF32Params&, cudaStream_t);
+};
+const Form kForms[] = {
+    {1, 32, 3, 5700, 2900, launch_rows<32, 1, 1, 1, 128, 4, 4, 4>},
+    {2, 16, 2, 4060, 1500, launch_rows<16, 1, 2, 1, 128, 4, 8, 8>},
+    {2, 32, 3, 5700, 2900, launch_rows<32, 1, 1, 2, 128, 4, 4, 4>},
+    {4, 16, 5, 4030, 1600, launch_rows<16, 1, 4, 1, 128, 4, 8, 4>},
+    {4, 32, 5, 9000, 2500, launch_rows<16, 2, 2, 2, 64, 2, 4, 4>},
+    {8, 16, 4, 4800, 3300, launch_rows<16, 1, 4, 2, 128, 4, 8, 4>},
+    {8, 32, 5, 9100, 3500, launch_rows<16, 2, 4, 2, 64, 2, 4, 4>},
+    {16, 16, 3, 6800, 6300, launch_rows<16, 1, 8, 2, 128, 4, 8, 4>},
+    {16, 32, 2, 10500, 7500, launch_rows<16, 2, 8, 2, 64, 2, 8, 8>},
+    {16, 32, 4, 13100, 4000, launch_rows<16, 2, 4, 4, 64, 2, 4, 4>},
+    {16, 64, 2, 20100, 4200, launch_rows<16, 4, 4, 4, 64, 1, 4, 4>},
+    {32, 16, 2, 9800, 8300, launch_rows<16, 1, 8, 4, 128, 2, 4, 4>},
+    {32, 32, 1, 14000, 14000, launch_rows<16, 2, 8, 4, 128, 1, 4, 4>},
+    {32, 32, 3, 15100, 9500, launch_rows<16, 2, 8, 4, 64, 2, 4, 4>},
+    {32, 64, 2, 23000, 15600, launch_rows<16, 4, 8, 4, 64, 1, 4, 4>},
+    {32, 64, 2, 36600, 400, launch_rows<16, 4, 4, 8, 32, 1, 6, 6>},
+    {64, 64, 4, 37000, 24300, launch_rows<16, 4, 8, 8, 32, 1, 3, 3, 2>},
+    {128, 64, 3, 62500, 39000, launch_tile<128, 64, 8, 8, 1, 3>},
+    {128, 128, 2, 106000, 66000, launch_tile<128, 128, 8, 16, 2, 2>},
+};
+
+const Form& form_for(int m, int n) {
+    const Form* best = nullptr;
+    int64_t least = 0;
+    for (const Form& f : kForms) {
+        const int64_t row_tiles = (m + f.rows - 1) / f.rows, column_tiles = (static_cast<int64_t>(n) + f.columns - 1) / f.columns;
+        // The second coordinate of a grid ends at 65,535: the rows' tiles in the forms along k, the columns' in the others.
+        // Tiles of up to 32 rows are for products that fill more than half of one; more than one would read the weights again.
+        if ((f.rows < 128 ? row_tiles : column_tiles) > 65535 || (f.rows < 32 && row_tiles > 1) ||
+            (f.columns > 16 && f.rows <= 32 && f.rows >= 2 * m)) {
+            continue;
+        }
+        const int64_t per_sm = (row_tiles * column_tiles + 147) / 148;
+        auto together = [&](int64_t ctas) { return ctas > 0 ? f.alone + (ctas - 1) * f.more : 0; };
+        const int64_t time = per_sm / f.resident * together(f.resident) + together(per_sm % f.resident);
+        if (best == nullptr || time < least) {
+            best = &f;
+            least = time;
+        }
+    }
+    return *best;  // (64-row tiles always fit: m is bounded by their count)
 }
 
 }  // namespace
@@ -402,44 +496,15 @@ PL_API int pl_gemm_f32(const float* a, const float* w, float* c, int m, int n, i
     const GemmF32Params p{a, w, c, m, n, k, lda, ldw, ldc, accumulate};
     const bool rows16 = (lda & 3) == 0 && (ldw & 3) == 0 &&
         ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
-    // Where the lines lie (us, measured alone with a cold L2; shapes N x K; the 64 x 64 tiles with a 4 x 4 block a
-    // thread that ran every size before are the last figure of each row):
-    //   2048 x 8192, 8 rows: few 44, 64 x 64 tiles 412, before 939; 16384 x 2048: 54, 134, 281
-    //   3072 x 2048, 64 rows (768 few CTAs): few 60, tiles 105; 128 rows (1,536): 102, 105, 221
-    //   16384 x 2048, 64 rows (2,048): few 228, tiles 139
-    //   2048 x 8192, 509 rows: 64 x 64 tiles 524 (256 of them), 128 x 64 tiles 516 (128), 128 x 128 tiles 868 (64)
-    //   3072 x 2048, 509 rows: 197 (384), 225 (192), 223 (96); 16384 x 2048: 852, 693, 733, before 1580
-    //   32000 x 2048, 509 rows: 1681, 1345, 1253 (1,000 tiles)
-    //   k of 64 and less is half a piece of the few-rows form: 3072 x 64, 128 rows, warm: few 9.6, before 7.4, tiles 4.9
-    const int64_t few_ctas = static_cast<int64_t>((n + kFewN - 1) / kFewN) * ((m + 31) / 32);
-    const int64_t tiles64 = static_cast<int64_t>((m + 63) / 64) * ((n + 63) / 64);
-    const int64_t tiles128x64 = static_cast<int64_t>((m + 127) / 128) * ((n + 63) / 64);
-    const bool padded = 2 * tiles128x64 > tiles64 + tiles64 / 4;  // (128-row tiles that would be a fifth empty and more)
-    cudaError_t few = cudaSuccess;
-    const bool tiles_fit = (static_cast<int64_t>(n) + 63) / 64 <= 65535;  // (the tiles' columns are the grid's y)
-    if (!rows16 || (!tiles_fit && m > 16)) {
+    if (!rows16) {
         const dim3 grid((n + kTileN - 1) / kTileN, (m + kTileM - 1) / kTileM);
         gemm_f32_any_kernel<<<grid, 256, 0, stream>>>(p);
-    } else if (m <= 4) {
-        few = launch_few<4, 1>(p, stream);
-    } else if (m <= 8 && few_ctas <= 148) {
-        few = launch_few<8, 1>(p, stream);
-    } else if (m <= 8 || (m <= 16 && n < 8192)) {
-        few = launch_few<4, 2>(p, stream);
-    } else if (m <= 16) {
-        few = launch_few<8, 2>(p, stream);
-    } else if (k > 64 && (m <= 32 || few_ctas <= 768)) {
-        few = launch_few<8, 4>(p, stream);
-    } else if (k <= 64 || padded || tiles64 <= 148 || (tiles128x64 > 148 && tiles64 <= 448)) {
-        launch_tile<64, 64, 4, 8, 1, 4>(p, stream);
-    } else if (tiles128x64 < 1500) {
-        launch_tile<128, 64, 8, 8, 1, 3>(p, stream);
-    } else {
-        launch_tile<128, 128, 8, 16, 2, 2>(p, stream);
+        PL_CHECK_LAUNCH("gemm_f32");
+        return 0;
     }
-    if (few != cudaSuccess) {
-        return pl_fail(3, "gemm_f32: launch failed: %s", cudaGetErrorString(few));
+    const cudaError_t err = form_for(m, n).launch(p, stream);
+    if (err != cudaSuccess) {
+        return pl_fail(3, "gemm_f32: launch failed: %s", cudaGetErrorString(err));
     }
-    PL_CHECK_LAUNCH("gemm_f32");
     return 0;
 }
