@@ -36,6 +36,15 @@
 // round both to bfloat16 (as a product that stored them would)
 // and apply the activation (or the clamped unit of gate_units.cuh: a build of its own).
 //
+// Grouped mode: the rows of X belong to experts, one run of rows each (`ends`, made on the device), and W stacks the
+// experts' matrices. A tile is 256 features (gated: 128) of one expert by up to 256 of its rows; an expert's rows are
+// split evenly over as few tiles as hold them, and a tile's MMAs are only as wide as its rows (in steps of 32), so little
+// is spent on padding. Rows of the next expert that a tile's last rows of 32 bring in are columns nobody stores. What bounds
+// it: the loads where experts have few rows (16 KB of weights a CTA and k block, whatever the width), the MMAs from about
+// 256 rows an expert on. 2,048 tokens, 4 of 32 experts, 2,048 wide, 1,024 features: gated 75.7 us, down 47.0; the
+// library's grouped products took 81.2 and 49.9, and a SwiGLU kernel between them (16 rows an expert 48.8 and 28.6, 68.7 and 43.3;
+// 1,024 rows 54.6 and 35.7, 56.0 and 35.1).
+//
 // Every wait on an mbarrier is bounded: after the limit the CTA raises bit 8 of the
 // status word, stops issuing work, lets what is in flight land, meets its partner,
 // frees its tensor memory and returns.
@@ -68,7 +77,18 @@ struct PairParams {
     int t_tiles;  // tiles along T (256 tokens each)
     int k_blocks;
     int total_tiles;
+    int act;  // grouped, not gated: the plain activation of the rounded product (gate_units.cuh's codes, 0: none)
+    const int32_t* ends;  // grouped: the row after each expert's last
+    int n_experts;
     int32_t* status;
+};
+
+constexpr int kMostExperts = 512;  // of a grouped product (their tiles' running counts sit in shared memory)
+
+// The rows of X one load brings in: half a tile's; grouped: boxes of 128, 64, 32 and 16 rows, of which a tile's half is made up.
+template <bool GROUPED>
+struct RowMaps {
+    CUtensorMap box[GROUPED ? 4 : 1];
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -122,8 +142,8 @@ __device__ __forceinline__ void arrive_on_first(uint64_t* bar) {
 constexpr int kGateRow = 17;  // 16 token columns handed over per thread and chunk, padded against bank conflicts
 constexpr int kGateBytes = 2 * 2 * (kTileM / 2) * kGateRow * 4;  // two buffers of [gate side, up side][64][17] floats
 
-// An epilogue's chunk of 32 tokens on its way out: [32][PER features] of fp32 at most, two of them.
-constexpr int out_bytes(int per) { return 2 * 32 * per * 4; }
+// An epilogue's chunk of 32 tokens on its way out: [32][PER features] of fp32 at most (grouped: bfloat16), two of them.
+constexpr int out_bytes(int per, bool grouped) { return 2 * 32 * per * (grouped ? 2 : 4); }
 
 template <typename T>
 __device__ __forceinline__ T out_value(float v) {
@@ -156,15 +176,45 @@ __device__ __forceinline__ void store_rows(const T* rows, T* y, int64_t ldy, int
     }
 }
 
+// One tile: the features from n0 on (of the pair), the rows of W from w0 on are its first, rows t0 .. t_end of X, MMAs
+// `wide` tokens wide.
+struct PairTile {
+    int n0, w0, t0, t_end, wide;
+};
+
+// Walks the tiles in ascending order. Grouped: expert by expert, within one the row tiles fastest, as in a plain product.
+template <bool GROUPED, int PER_PAIR, int MOST>
+struct PairTiles {
+    const PairParams& p;
+    const int* first;  // grouped: [n_experts + 1] tiles before each expert's, then rows before each expert's
+    int expert = 0;
+    __device__ __forceinline__ PairTiles(const PairParams& params, const int* counts): p(params), first(counts) {}
+    __device__ __forceinline__ PairTile at(int tile) {
+        if constexpr (!GROUPED) {
+            const int n0 = (tile / p.t_tiles) * PER_PAIR;
+            return {n0, n0, (tile % p.t_tiles) * MOST, p.t, MOST};
+        } else {
+            while (tile >= first[expert + 1]) {
+                ++expert;
+            }
+            const int* row = first + kMostExperts + 1;
+            const int begin = row[expert], end = row[expert + 1];
+            const int row_tiles = (end - begin + MOST - 1) / MOST, in = tile - first[expert];
+            const int rows = ((end - begin + row_tiles - 1) / row_tiles + 31) / 32 * 32;
+            const int n0 = in / row_tiles * PER_PAIR, t0 = begin + in % row_tiles * rows, t_end = min(end, t0 + rows);
+            return {n0, expert * p.n * (PER_PAIR == kTileM ? 2 : 1) + n0, t0, t_end, (t_end - t0 + 31) / 32 * 32};
+        }
+    }
+};
+
 // GATED: 0 the product alone, 1 silu(gate) * up, 2 the clamped unit of gate and up.
-template <int GATED, int kPairN>
+template <int GATED, int kPairN, bool GROUPED>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ RowMaps<GROUPED> map_x,
                  const PairParams p) {
     constexpr uint32_t kColumns = 2 * kMostTokens;  // two accumulators, kPairN columns of each half (a power of two is allotted)
     constexpr int kStageBytes = stage_bytes(kPairN);
-    constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kPairN >> 3) << 17) |
-        (static_cast<uint32_t>((2 * kTileM) >> 4) << 24);
+    constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>((2 * kTileM) >> 4) << 24);
 
     extern __shared__ unsigned char raw_smem[];
     unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) &
@@ -178,6 +228,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     __shared__ __align__(8) uint64_t acc_empty[2];         // waited on in the first CTA only
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
+    __shared__ int first_tile[GROUPED ? 2 * (kMostExperts + 1) : 1];
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = static_cast<int>(cluster_rank());
@@ -185,7 +236,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     pl_grid_trigger();
     if (threadIdx.x == 0) {
         tensormap_prefetch(&map_w);
-        tensormap_prefetch(&map_x);
+        tensormap_prefetch(&map_x.box[0]);
         for (int s = 0; s < kStages; ++s) {
             mbar_init(&full_bar[s], 1);
             mbar_init(&empty_bar[s], 1);
@@ -208,7 +259,36 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     cluster_wait_all();
     pl_grid_wait();
 
-    const int tile_begin = pair, tile_end = p.total_tiles, tile_step = gridDim.x >> 1;
+    if constexpr (GROUPED) {
+        if (warp == 0) {
+            int before = 0;
+            for (int base = 0; base < p.n_experts; base += 32) {
+                const int e = base + lane;
+                int upto = 0;
+                if (e < p.n_experts) {
+                    const int end = p.ends[e], rows = end - (e > 0 ? p.ends[e - 1] : 0);
+                    first_tile[kMostExperts + 2 + e] = end;
+                    upto = (rows + kPairN - 1) / kPairN * p.n_tiles;
+                }
+#pragma unroll
+                for (int offset = 1; offset < 32; offset <<= 1) {
+                    const int other = __shfl_up_sync(0xffffffffu, upto, offset);
+                    upto += lane >= offset ? other : 0;
+                }
+                if (e < p.n_experts) {
+                    first_tile[e + 1] = before + upto;
+                }
+                before += __shfl_sync(0xffffffffu, upto, 31);
+            }
+            if (lane == 0) {
+                first_tile[0] = 0;
+                first_tile[kMostExperts + 1] = 0;
+            }
+        }
+        __syncthreads();
+    }
+    const int tile_begin = pair, tile_end = GROUPED ? first_tile[p.n_experts] : p.total_tiles, tile_step = gridDim.x >> 1;
+    PairTiles<GROUPED, 2 * kPer, kPairN> places(p, first_tile);
 
     if (warp == 0) {
         // ------------------------------------------------ producer (both CTAs)
@@ -216,8 +296,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         uint32_t phase = 0;
         bool ok = true;
         for (int tile = tile_begin; ok && tile < tile_end; tile += tile_step) {
-            const int n0 = (tile / p.t_tiles) * (2 * kPer) + rank * kPer;
-            const int t0 = (tile % p.t_tiles) * kPairN + rank * (kPairN / 2);
+            const PairTile place = places.at(tile);
+            const int w0 = place.w0 + rank * kPer;
+            const int t0 = place.t0 + rank * (place.wide / 2);
             for (int kb = 0; kb < p.k_blocks; ++kb) {
                 if (!mbar_wait(&empty_bar[stage], phase ^ 1u, &abort_flag)) {
                     ok = false;
@@ -226,13 +307,24 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                 unsigned char* a = tiles + stage * kStageBytes;
                 if (elect_one()) {
                     if (rank == 0) {
-                        mbar_expect_tx(&full_bar[stage], 2 * kStageBytes);  // both CTAs' loads of this stage
+                        mbar_expect_tx(&full_bar[stage], 2 * stage_bytes(place.wide));  // both CTAs' loads of this stage
                     }
-                    tma_load_2d_pair(a, &map_w, kb * kBlockK, n0, &full_bar[stage]);
+                    tma_load_2d_pair(a, &map_w, kb * kBlockK, w0, &full_bar[stage]);
                     if (GATED) {  // the up rows of the same features under the gate rows
-                        tma_load_2d_pair(a + kBytesA / 2, &map_w, kb * kBlockK, p.n + n0, &full_bar[stage]);
+                        tma_load_2d_pair(a + kBytesA / 2, &map_w, kb * kBlockK, p.n + w0, &full_bar[stage]);
                     }
-                    tma_load_2d_pair(a + kBytesA, &map_x, kb * kBlockK, t0, &full_bar[stage]);
+                    if constexpr (GROUPED) {
+                        int row = 0;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            if (place.wide / 2 & (kMostTokens / 2 >> i)) {
+                                tma_load_2d_pair(a + kBytesA + row * kBlockK * 2, &map_x.box[i], kb * kBlockK, t0 + row, &full_bar[stage]);
+                                row += kMostTokens / 2 >> i;
+                            }
+                        }
+                    } else {
+                        tma_load_2d_pair(a + kBytesA, &map_x.box[0], kb * kBlockK, t0, &full_bar[stage]);
+                    }
                 }
                 __syncwarp();
                 if (++stage == kStages) {
@@ -254,6 +346,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             }
             tcgen05_fence_after();
             const uint32_t tmem_d = tmem_base + acc * kMostTokens;
+            const uint32_t idesc = kIdesc | (static_cast<uint32_t>(GROUPED ? places.at(tile).wide >> 3 : kPairN >> 3) << 17);
             for (int kb = 0; kb < p.k_blocks; ++kb) {
                 if (!mbar_wait(&full_bar[stage], phase, &abort_flag)) {
                     ok = false;
@@ -265,7 +358,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                 if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < kBlockK / 16; ++k) {
-                        tcgen05_mma_pair(tmem_d, desc_a + 2 * k, desc_b + 2 * k, kIdesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        tcgen05_mma_pair(tmem_d, desc_a + 2 * k, desc_b + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
                     }
                     tcgen05_commit_pair(&empty_bar[stage]);  // frees the stage in both CTAs
                 }
@@ -303,12 +396,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                 break;
             }
             tcgen05_fence_after();
-            const int n_first = (tile / p.t_tiles) * (2 * kPer) + rank * kPer;
-            const int n = (tile / p.t_tiles) * (2 * kPer) + rank * kPer + (GATED ? feature % kPer : feature);
-            const int t0 = (tile % p.t_tiles) * kPairN;
+            const PairTile place = places.at(tile);
+            const int n_first = place.n0 + rank * kPer;
+            const int n = n_first + (GATED ? feature % kPer : feature);
+            const int t0 = place.t0, t_end = place.t_end;
             const uint32_t tmem_row = tmem_base + (static_cast<uint32_t>(lane_group * 32) << 16) + acc * kMostTokens;
 #pragma unroll 1
-            for (int c0 = 0; c0 < kPairN && t0 + c0 < p.t; c0 += 32) {
+            for (int c0 = 0; c0 < kPairN && t0 + c0 < t_end; c0 += 32) {
                 uint32_t v[32];
                 tcgen05_ld32_nowait(tmem_row + c0, v);
                 tcgen05_wait_ld();
@@ -350,7 +444,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                                 rows[(mine + c) * kPer + feature % kPer] = out_value<T>(act[c]);
                             }
                         };
-                        if (p.out_f32) {
+                        if (!GROUPED && p.out_f32) {
                             put(reinterpret_cast<float*>(leaving) + ((c0 >> 5) & 1) * 32 * kPer);
                         } else {
                             put(reinterpret_cast<__nv_bfloat16*>(leaving) + ((c0 >> 5) & 1) * 32 * kPer);
@@ -361,22 +455,26 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                         using T = std::remove_reference_t<decltype(*rows)>;
 #pragma unroll
                         for (int c = 0; c < 32; ++c) {
-                            rows[c * kPer + feature] = out_value<T>(__uint_as_float(v[c]));
+                            float z = __uint_as_float(v[c]);
+                            if (GROUPED && p.act != 0) {  // (of the product rounded as one that stored it would round it)
+                                z = pl_plain_activation(__bfloat162float(__float2bfloat16_rn(z)), p.act);
+                            }
+                            rows[c * kPer + feature] = out_value<T>(z);
                         }
                     };
-                    if (p.out_f32) {
+                    if (!GROUPED && p.out_f32) {
                         put(reinterpret_cast<float*>(leaving) + ((c0 >> 5) & 1) * 32 * kPer);
                     } else {
                         put(reinterpret_cast<__nv_bfloat16*>(leaving) + ((c0 >> 5) & 1) * 32 * kPer);
                     }
                 }
                 asm volatile("bar.sync 1, 128;" ::: "memory");  // (two chunks' places: one barrier per chunk is enough)
-                if (p.out_f32) {
+                if (!GROUPED && p.out_f32) {
                     store_rows<kPer>(reinterpret_cast<const float*>(leaving) + ((c0 >> 5) & 1) * 32 * kPer,
-                                     static_cast<float*>(p.y), p.ldy, t0 + c0, p.t, n_first, p.n, vectors, thread);
+                                     static_cast<float*>(p.y), p.ldy, t0 + c0, t_end, n_first, p.n, vectors, thread);
                 } else {
                     store_rows<kPer>(reinterpret_cast<const __nv_bfloat16*>(leaving) + ((c0 >> 5) & 1) * 32 * kPer,
-                                     static_cast<__nv_bfloat16*>(p.y), p.ldy, t0 + c0, p.t, n_first, p.n, vectors, thread);
+                                     static_cast<__nv_bfloat16*>(p.y), p.ldy, t0 + c0, t_end, n_first, p.n, vectors, thread);
                 }
             }
             tcgen05_fence_before();
@@ -432,19 +530,13 @@ PL_API int pl_gemm_bf16_pair_supports(int t, int n, int k, int64_t ldx, int64_t 
 
 namespace {
 
-template <int GATED, int TOKENS>
-int launch_pair(const CUtensorMap& map_w, const CUtensorMap& map_x, const PairParams& p, int used_pairs,
+template <int GATED, int TOKENS, bool GROUPED = false>
+int launch_pair(const CUtensorMap& map_w, const RowMaps<GROUPED>& map_x, const PairParams& p, int used_pairs,
                 cudaStream_t stream) {
     constexpr int smem =
-        kStages * stage_bytes(TOKENS) + (GATED ? kGateBytes : 0) + out_bytes(GATED ? kTileM / 2 : kTileM) + 1024;
-    static bool configured = false;
-    if (!configured) {
-        const cudaError_t err = cudaFuncSetAttribute(gemm_pair_kernel<GATED, TOKENS>,
-                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (err != cudaSuccess) {
-            return pl_fail(3, "gemm_bf16_pair: cannot set shared memory size: %s", cudaGetErrorString(err));
-        }
-        configured = true;
+        kStages * stage_bytes(TOKENS) + (GATED ? kGateBytes : 0) + out_bytes(GATED ? kTileM / 2 : kTileM, GROUPED) + 1024;
+    if (const cudaError_t err = pl_allow_smem<gemm_pair_kernel<GATED, TOKENS, GROUPED>>(smem); err != cudaSuccess) {
+        return pl_fail(3, "gemm_bf16_pair: cannot set shared memory size: %s", cudaGetErrorString(err));
     }
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(2 * used_pairs);
@@ -460,7 +552,7 @@ int launch_pair(const CUtensorMap& map_w, const CUtensorMap& map_x, const PairPa
     attributes[1].val.programmaticStreamSerializationAllowed = 1;
     config.attrs = attributes;
     config.numAttrs = pl_overlap_enabled() ? 2 : 1;
-    const cudaError_t err = cudaLaunchKernelEx(&config, gemm_pair_kernel<GATED, TOKENS>, map_w, map_x, p);
+    const cudaError_t err = cudaLaunchKernelEx(&config, gemm_pair_kernel<GATED, TOKENS, GROUPED>, map_w, map_x, p);
     if (err != cudaSuccess) {
         return pl_fail(3, "gemm_bf16_pair: launch failed: %s", cudaGetErrorString(err));
     }
@@ -497,16 +589,17 @@ static int run_pair(const void* x, const void* w, void* y, int t, int n, int k, 
                "gemm_bf16_pair: operands must be 16-byte aligned");
     PL_REQUIRE(ldy >= n, "gemm_bf16_pair: ldy=%lld is smaller than n=%d", static_cast<long long>(ldy), n);
     const int per_pair = gated ? kTileM : 2 * kTileM;  // output features of a tile
-    CUtensorMap map_w, map_x;
+    CUtensorMap map_w;
+    RowMaps<false> map_x;
     if (const int code = make_map(&map_w, w, gated ? 2 * static_cast<int64_t>(n) : n, k, ldw,
                                   gated ? kTileM / 2 : kTileM, kBlockK)) {
         return code;
     }
     const int tokens = tile_tokens(t, (n + per_pair - 1) / per_pair);
-    if (const int code = make_map(&map_x, x, t, k, ldx, tokens / 2, kBlockK)) {
+    if (const int code = make_map(&map_x.box[0], x, t, k, ldx, tokens / 2, kBlockK)) {
         return code;
     }
-    PairParams p;
+    PairParams p = {};
     p.y = y;
     p.t = t;
     p.n = n;
@@ -539,4 +632,58 @@ PL_API int pl_gemm_bf16_pair(const void* x, const void* w, void* y, int t, int n
 PL_API int pl_gemm_bf16_pair_clamped(const void* x, const void* w, void* y, int t, int n, int k, int64_t ldx, int64_t ldw,
                                      int64_t ldy, int out_f32, float limit, int32_t* status, cudaStream_t stream) {
     return run_pair(x, w, y, t, n, k, ldx, ldw, ldy, out_f32, 2, limit, status, stream);
+}
+
+// 1 when pl_gemm_bf16_grouped takes these sizes (all operands contiguous, on 16-byte boundaries).
+PL_API int pl_gemm_bf16_grouped_supports(int n, int k, int n_experts) {
+    return n >= 1 && k >= 8 && k % 8 == 0 && n_experts >= 1 && n_experts <= kMostExperts;
+}
+
+// Rows of experts by their matrices: y[r] = x[r] w[e]^T for the rows r of expert e, ends[e - 1] <= r < ends[e] (ends int32
+// [n_experts] on the device, ascending, the last at most `rows`). x bf16 [rows, k]; w bf16 [n_experts, n, k], gated
+// [n_experts, 2n, k] (an expert's gate matrix over its up matrix); y bf16 [rows, n]. gated: 1 silu(gate) * up, 2 the clamped
+// unit with `limit`, of the two products rounded to bfloat16; 0 with `act`: the plain activation of the rounded product.
+PL_API int pl_gemm_bf16_grouped(const void* x, const void* w, void* y, const int32_t* ends, int rows, int n, int k, int n_experts,
+                                int gated, float limit, int act, int32_t* status, cudaStream_t stream) {
+    PL_REQUIRE(pl_gemm_bf16_grouped_supports(n, k, n_experts) && rows >= 0 && gated >= 0 && gated <= 2,
+               "gemm_bf16_grouped: unsupported sizes rows=%d n=%d k=%d experts=%d", rows, n, k, n_experts);
+    PL_REQUIRE(act == 0 || (gated == 0 && act >= 1 && act <= 3), "gemm_bf16_grouped: unknown activation %d", act);
+    PL_REQUIRE(((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0,
+               "gemm_bf16_grouped: operands must be 16-byte aligned");
+    if (rows == 0) {
+        return 0;
+    }
+    const int per_pair = gated ? kTileM : 2 * kTileM;
+    const int64_t w_rows = static_cast<int64_t>(n_experts) * n * (gated ? 2 : 1);
+    PL_REQUIRE(w_rows + 2 * kTileM <= INT32_MAX, "gemm_bf16_grouped: %lld rows of weights are too many",
+               static_cast<long long>(w_rows));
+    CUtensorMap map_w;
+    RowMaps<true> map_x;
+    if (const int code = make_map(&map_w, w, w_rows, k, k, gated ? kTileM / 2 : kTileM, kBlockK)) {
+        return code;
+    }
+    for (int i = 0; i < 4; ++i) {
+        if (const int code = make_map(&map_x.box[i], x, rows, k, k, kMostTokens / 2 >> i, kBlockK)) {
+            return code;
+        }
+    }
+    PairParams p = {};
+    p.y = y;
+    p.t = rows;
+    p.n = n;
+    p.k = k;
+    p.ldy = n;
+    p.limit = limit;
+    p.n_tiles = (n + per_pair - 1) / per_pair;
+    p.k_blocks = (k + kBlockK - 1) / kBlockK;
+    p.act = act;
+    p.ends = ends;
+    p.n_experts = n_experts;
+    p.status = status;
+    // (how many tiles there are is known on the device: at most this many)
+    const int64_t most = static_cast<int64_t>(p.n_tiles) * (static_cast<int64_t>(n_experts) + rows / kMostTokens);
+    const int used_pairs = most < pair_count() ? static_cast<int>(most) : pair_count();
+    return gated == 2 ? launch_pair<2, kMostTokens, true>(map_w, map_x, p, used_pairs, stream)
+        : gated       ? launch_pair<1, kMostTokens, true>(map_w, map_x, p, used_pairs, stream)
+                      : launch_pair<0, kMostTokens, true>(map_w, map_x, p, used_pairs, stream);
 }

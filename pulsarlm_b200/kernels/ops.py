@@ -90,6 +90,8 @@ _SIGNATURES = {
     "pl_gemm_bf16_skinny": [_PTR, _PTR, _PTR, _I32, _I32, _I32, _I64, _I64, _I64, _I32, _PTR, _PTR],
     "pl_gemm_bf16_skinny_max_tokens": [],
     "pl_gemm_bf16_pair": [_PTR, _PTR, _PTR, _I32, _I32, _I32, _I64, _I64, _I64, _I32, _I32, _PTR, _PTR],
+    "pl_gemm_bf16_grouped_supports": [_I32, _I32, _I32],
+    "pl_gemm_bf16_grouped": [_PTR, _PTR, _PTR, _PTR, _I32, _I32, _I32, _I32, _I32, _F32, _I32, _PTR, _PTR],
     "pl_gemm_bf16_pair_clamped": [_PTR, _PTR, _PTR, _I32, _I32, _I32, _I64, _I64, _I64, _I32, _F32, _PTR, _PTR],
     "pl_attention_decode_resident_clusters": [_I32, _I32, _I32],
     "pl_gemm_bf16_skinny_splits": [_I32, _I32, _I32],
@@ -1310,6 +1312,28 @@ def gemm_bf16(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status: torch
               int(out.dtype == torch.float32), int(gated), _p(status), _stream())
         return
     raise ValueError(f"gemm_bf16: unknown kernel {kernel!r}")
+
+
+def gemm_bf16_grouped_supports(n: int, k: int, n_experts: int) -> bool:
+    """Whether gemm_bf16_grouped takes matrices [n, k] of so many experts."""
+    return bool(library().pl_gemm_bf16_grouped_supports(n, k, n_experts))
+
+
+def gemm_bf16_grouped(x: torch.Tensor, w: torch.Tensor, ends: torch.Tensor, out: torch.Tensor, act: str | None = None,
+                      limit: float = 0.0, status: torch.Tensor | None = None) -> None:
+    """out[r] = act(x[r] @ w[e]^T) for the rows r of expert e (`ends`, int32 [E] as moe_sort makes it), bfloat16, on the tcgen05
+    tensor cores. act None: the product; "silu" or "clamped" (with `limit`): w holds a gate matrix over an up matrix per
+    expert and out is the gated unit of the two rounded products; "relu2" or "gelu": that of the rounded product."""
+    _dev(x, w, ends, out, status)
+    rows, k = x.shape
+    experts, n = w.shape[0], out.shape[1]
+    gated = {"silu": 1, "clamped": 2}.get(act, 0)
+    assert x.dtype == w.dtype == out.dtype == torch.bfloat16 and ends.dtype == torch.int32 and ends.shape == (experts,)
+    assert out.shape[0] == rows and w.shape == (experts, 2 * n if gated else n, k)
+    assert x.is_contiguous() and w.is_contiguous() and ends.is_contiguous() and out.is_contiguous()
+    _call("pl_gemm_bf16_grouped", _p(x), _p(w), _p(out), _p(ends), rows, n, k, experts, gated, float(limit),
+          {"relu2": 1, "gelu": 3}[act] if act is not None and not gated else 0, _p(status), _stream())
+
 
 GEMM_GATED_IN_MAX_TOKENS = 16
 

@@ -135,7 +135,12 @@ class RoutedExperts(Part):
 
     def _grouped(self, h: torch.Tensor) -> bool:
         return (h.dtype == torch.bfloat16 and h.shape[0] >= GROUPED_MIN_TOKENS and self.hidden % 8 == 0
-                and self.ff % 8 == 0 and hasattr(torch.nn.functional, "grouped_mm"))
+                and self.ff % 8 == 0 and (self._own_products() or hasattr(torch.nn.functional, "grouped_mm")))
+
+    def _own_products(self) -> bool:
+        """Whether the experts' grouped products are the package's own kernel's (else the library's)."""
+        return ops.gemm_bf16_grouped_supports(self.ff, self.hidden, self.n_experts) and ops.gemm_bf16_grouped_supports(
+            self.hidden, self.ff, self.n_experts)
 
     def _route(self, h: torch.Tensor) -> tuple:
         """(ids, weights on the experts' inputs, weights on their outputs, weight of the shared expert); weights None: 1."""
@@ -170,14 +175,27 @@ class RoutedExperts(Part):
                 batch, h.device, lambda: self._units(h), shared_expert=lambda: self._shared(h))
             ops.moe_down(act, self.down, ids, weights, shared, out, shared_weights)
             return out
-        # Pairs in expert order; each projection one grouped product over the sorted rows (the library's: operands
-        # [rows, K] and [E, K, N] with the experts' last rows as offsets).
+        # Pairs in expert order; each projection one grouped product over the sorted rows, the activation in the first
+        # one's epilogue (csrc/gemm_pair.cu; an expert's weight on its input keeps the activation a kernel of its own).
         ids, in_weights, weights, shared_weights = self._route(h)
         shared = self._shared(h)
         ends, row_of_pair, pair_of_row = ops.moe_sort(ids, self.n_experts)
         x = ops.moe_gather(h, pair_of_row, self.top)
-        gate_up = torch.nn.functional.grouped_mm(x, self.gate_up.transpose(1, 2), offs=ends)
         act = torch.empty((x.shape[0], self.ff), dtype=h.dtype, device=h.device)
+        if self._own_products():
+            if in_weights is None:
+                unit = ("silu" if self.limit is None else "clamped") if self.gated else self.plain_act
+                ops.gemm_bf16_grouped(x, self.gate_up, ends, act, unit, self.limit or 0.0)
+            else:
+                gate_up = torch.empty((x.shape[0], 2 * self.ff), dtype=h.dtype, device=h.device)
+                ops.gemm_bf16_grouped(x, self.gate_up, ends, gate_up)
+                ops.gated_act(gate_up, act, "clamped", self.limit, in_weights, pair_of_row)
+            y = torch.empty((x.shape[0], self.hidden), dtype=h.dtype, device=h.device)
+            ops.gemm_bf16_grouped(act, self.down, ends, y)
+            ops.moe_combine(y, row_of_pair, weights, shared, out, shared_weights)
+            return out
+        # More experts than that kernel counts: the library's (operands [rows, K] and [E, K, N], the experts' ends as offsets).
+        gate_up = torch.nn.functional.grouped_mm(x, self.gate_up.transpose(1, 2), offs=ends)
         if self.limit is not None:
             ops.gated_act(gate_up, act, "clamped", self.limit, in_weights, pair_of_row)
         elif self.gated:
