@@ -20,8 +20,7 @@
 
 #include <climits>
 
-#include "common.cuh"
-
+#include "cluster_helpers.cuh"
 #include "mma_helpers.cuh"
 
 namespace {
@@ -188,6 +187,24 @@ __device__ __forceinline__ bool delta_find_chunk(const int32_t* counts, const De
     return false;
 }
 
+// Up to 32 entries: the place in the entries' order of the `nth` longest of those that go in chunks. (By a whole warp.) Chains
+// of several lengths then start with the longest.
+__device__ __forceinline__ int delta_nth_longest(const int32_t* counts, const DeltaPass& p, int nth) {
+    if (p.n_entries > 32) {
+        return nth;
+    }
+    const int lane = threadIdx.x & 31;
+    const int count = lane < p.n_entries ? counts[lane] : 0;
+    const uint32_t longer = __ballot_sync(0xffffffffu, count >= p.least);
+    int rank = 0;
+    for (int other = 0; other < p.n_entries; ++other) {
+        const int theirs = __shfl_sync(0xffffffffu, count, other);
+        rank += theirs > count || (theirs == count && other < lane);
+    }
+    const uint32_t found = __ballot_sync(0xffffffffu, count >= p.least && rank == nth);
+    return found == 0 ? nth : __popc(longer & ((1u << (__ffs(found) - 1)) - 1u));
+}
+
 // The `nth` entry that goes in chunks, and how many chunks of this pass come before its own; false past the last. (By a whole
 // warp.)
 __device__ __forceinline__ bool delta_find_entry(const int32_t* counts, const DeltaPass& p, int nth, int& entry, int& before) {
@@ -259,32 +276,37 @@ __device__ __forceinline__ void mma_terms(float (&d0)[4], float (&d1)[4], const 
     }
 }
 
-// What a lane needs of a chunk, a chunk ahead of its use in registers (through shared memory it would pass the same ports
-// twice, which bound a first form of this kernel).
-template <bool GENERAL>
-struct DeltaLane {
-    TermsB wm, qg, kd, m, kv;
-    float4 zi[2], g;
-    uint4 vv;
+// A CTA's chunk in shared memory, in floats: the operands and M as they lie in the scratch, and of the rest the CTA's columns.
+template <int DIM, bool GENERAL>
+struct DeltaRing {
+    static constexpr DeltaChunkLayout kAt{DIM, 0, GENERAL};  // (the places up to zi hold for any vdim)
+    static constexpr int kZi = kAt.zi, kOi = kZi + 256, kVv = kOi + (GENERAL ? 256 : 0), kG = kVv + (GENERAL ? 128 : 0);
+    static constexpr int kFloats = kG + DIM;
+    static constexpr int kSlots = DIM == 128 || GENERAL ? 3 : 4;  // (two CTAs of 64 rows an SM)
+    static constexpr int kBytes = kSlots * kFloats * 4 + 2 * 2 * DIM / 16 * 32 * 16;
 };
 
-// grid (entries that go in chunks, heads, vdim / 16), NW = dim / 16 warps. On the path from a chunk to the next are only Z's products,
-// their sum over the warps, and the state's update; O's products fill the waits between and are added up a chunk later. Bound by
-// that path (one CTA of four warps an SM, 0.85 us a chunk; the chunks' 24 to 38 KB come from memory once and three times out of L2).
-// One prompt of 2,048 tokens, 32 heads of 64 x 64: 116 us a decay per channel behind 73 us for the chunks' matrices, 106 the general
-// rule behind 87; five portions of 1,283 tokens in all, the longest 584, 63 behind 60. The walks took 681 us for the first and 567
-// for the last. Slower: the matrices through shared memory (122 to 135 us), 32 columns a CTA (140), their lines asked into L1 a
-// chunk ahead (no gain).
+// grid (entries that go in chunks x heads, vdim / 16), 2 NW warps, NW = dim / 16. On the path from a chunk to the next are only
+// Z's products, their sum over the warps, and the state's update: the first NW warps do nothing else. They leave the state that
+// a chunk starts from in shared memory, where the other NW take it up for O's products, a barrier behind, and add those up a
+// chunk later. The chunks' matrices come into shared memory by bulk copies, three or four chunks in flight. Bound by the path's
+// instructions, each of which waits for the one before it (0.74 us a chunk; 0.85 where NW warps made the outputs too, with what
+// a lane needs of a chunk in registers, up to 250 a thread). In the part, beside the kernels around it, us, before and now: one
+// prompt of 2,048 tokens, 32 heads of 64 x 64: 128 and 95 a decay per channel, 175 and 101 the general rule; 16 heads of 128 x
+// 128 206 and 177 the general rule; twelve portions of 1,500 tokens in all 100 and 70. Slower: 32 columns a CTA (140); lines
+// asked into L1 or L2 chunks ahead change nothing.
 template <int NW, bool GENERAL>
-__global__ void __launch_bounds__(NW * 32) delta_chain_kernel(const DeltaChainParams p) {
+__global__ void __launch_bounds__(NW * 64, NW >= 8 ? 1 : 8 / NW) delta_chain_kernel(const DeltaChainParams p) {
     pl_grid_trigger();
     pl_grid_wait();
     constexpr int kDim = NW * 16;
-    __shared__ float4 shares[2][4][NW][32];  // by chunk parity: two tiles of Z, two of O
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const int head = blockIdx.y, ct = blockIdx.z;
+    __shared__ float4 shares[2][2][NW][32];     // by chunk parity: two tiles of Z,
+    __shared__ float4 o_shares[2][2][NW][32];   // two of O,
+    const int tid = threadIdx.x, lane = tid & 31, w = (tid >> 5) % NW;
+    const bool outputs = tid >= NW * 32;
+    const int head = blockIdx.x % p.n_heads, ct = blockIdx.y;
     int e, before;
-    if (!delta_find_entry(p.counts, p.pass, blockIdx.x, e, before)) {
+    if (!delta_find_entry(p.counts, p.pass, delta_nth_longest(p.counts, p.pass, blockIdx.x / p.n_heads), e, before)) {
         return;
     }
     const int count = p.counts[e];
@@ -292,60 +314,169 @@ __global__ void __launch_bounds__(NW * 32) delta_chain_kernel(const DeltaChainPa
     if (n_chunks == 0) {
         return;
     }
+    using Ring = DeltaRing<kDim, GENERAL>;
     const DeltaChunkLayout at(kDim, p.vdim, GENERAL);
-    constexpr DeltaChunkLayout kAt(kDim, 0, GENERAL);  // (the places up to zi hold for any vdim)
     const int64_t step = static_cast<int64_t>(p.n_heads) * at.floats;
     const float* chunk0 = p.scratch + (static_cast<int64_t>(before) * p.n_heads + head) * at.floats;
-    const float* src = chunk0 + w * 384 + lane * 4;
-    const float* src_m = chunk0 + kAt.m + lane * 4;
-    const float* src_zi = chunk0 + kAt.zi + (ct * 2 * 32 + lane) * 4;
-    const float* src_oi = chunk0 + at.oi + ((ct * 2 + w) * 32 + lane) * 4;
-    const float* src_vv = chunk0 + at.vv + (ct * 32 + lane) * 4;
-    const float* src_g = chunk0 + at.g + w * 16 + (lane & 3) * 4;
+    extern __shared__ __align__(128) float ring[];   // [slots][Ring::kFloats], and the state before the chunk, by its parity
+    auto states = reinterpret_cast<float4(*)[2][NW][32]>(ring + Ring::kSlots * Ring::kFloats);
+    __shared__ __align__(8) uint64_t landed[Ring::kSlots];
+    __shared__ int lost;
+    // One thread of the outputs' warps brings a chunk in, kSlots of them in flight.
+    const bool brings = tid == blockDim.x - 32;
+    auto bring = [&](int c) {
+        const float* from = chunk0 + c * step;
+        float* to = ring + c % Ring::kSlots * Ring::kFloats;
+        uint64_t* bar = &landed[c % Ring::kSlots];
+        auto copy = [&](int dst, int src, int floats) {
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                             smem_u32(to + dst)),
+                         "l"(from + src), "r"(floats * 4), "r"(smem_u32(bar))
+                         : "memory");
+        };
+        mbar_expect_tx(bar, Ring::kFloats * 4);
+        copy(0, 0, Ring::kZi);
+        copy(Ring::kZi, at.zi + ct * 256, 256);
+        if constexpr (GENERAL) {
+            copy(Ring::kOi, at.oi + ct * 256, 256);
+            copy(Ring::kVv, at.vv + ct * 128, 128);
+        }
+        copy(Ring::kG, at.g, kDim);
+    };
+    if (brings) {
+        lost = 0;
+        for (int i = 0; i < Ring::kSlots; ++i) {
+            mbar_init(&landed[i], 1);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    if (brings) {
+        for (int c = 0; c < min(Ring::kSlots, n_chunks); ++c) {
+            bring(c);
+        }
+    }
+    // A chunk's place once it is there. (One that never comes leaves numbers that are none: see the state's end.)
+    int slot = 0;
+    uint32_t phase = 0;
+    const float* cur = ring;
+    auto wait_for_chunk = [&] { mbar_wait(&landed[slot], phase, &lost); };
+    auto next_chunk = [&] {
+        cur += Ring::kFloats;
+        if (++slot == Ring::kSlots) {
+            slot = 0;
+            phase ^= 1u;
+            cur = ring;
+        }
+    };
     auto terms = [](TermsB& b, const float* from) {
 #pragma unroll
         for (int term = 0; term < 3; ++term) {
             b.t[term] = *reinterpret_cast<const uint4*>(from + term * 128);
         }
     };
-    auto fetch_m = [&](TermsB& m) {
-        terms(m, src_m);
-        src_m += step;
-    };
-    auto fetch = [&](DeltaLane<GENERAL>& in) {
-        terms(in.wm, src);
-        terms(in.qg, src + kAt.qg);
-        if constexpr (!GENERAL) {
-            terms(in.kd, src + kAt.kd);
+    const int own = w * 384 + lane * 4;
+    // The sum of the warps' shares of Z and its start: every warp makes it whole.
+    auto z_of = [&](float (&z)[2][4], const float4 (&zi)[2], int parity) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            float4 sum = shares[parity][j][0][lane];
+#pragma unroll
+            for (int other = 1; other < NW; ++other) {
+                const float4 part = shares[parity][j][other][lane];
+                sum = make_float4(sum.x + part.x, sum.y + part.y, sum.z + part.z, sum.w + part.w);
+            }
+            z[j][0] = zi[j].x + sum.x;
+            z[j][1] = zi[j].y + sum.y;
+            z[j][2] = zi[j].z + sum.z;
+            z[j][3] = zi[j].w + sum.w;
         }
-        in.zi[0] = *reinterpret_cast<const float4*>(src_zi);
-        in.zi[1] = *reinterpret_cast<const float4*>(src_zi + 128);
-        in.g = *reinterpret_cast<const float4*>(src_g);
-        if constexpr (GENERAL) {
-            terms(in.kv, src + kAt.kv);
-            in.vv = *reinterpret_cast<const uint4*>(src_vv);
-            src_vv += step;
-        } else if (w < 2) {
-            fetch_m(in.m);
-        }
-        src += step;
-        src_zi += step;
-        src_g += step;
     };
-    DeltaLane<GENERAL> even = {}, odd = {};
-    fetch(even);
 
-    // S transposed: s[j][r] is column ct * 16 + lane / 4 (+ 8 for r >= 2), row w * 16 + 8 j + (lane % 4) * 2 + r % 2.
-    float s[2][4];
-    float* corner = p.state + ((static_cast<int64_t>(p.slots[e]) * p.n_heads + head) * kDim + w * 16 + (lane & 3) * 2) * p.vdim +
-        ct * kDeltaCols + (lane >> 2);
+    if (!outputs) {
+        // S transposed: s[j][r] is column ct * 16 + lane / 4 (+ 8 for r >= 2), row w * 16 + 8 j + (lane % 4) * 2 + r % 2.
+        float s[2][4];
+        float* corner = p.state + ((static_cast<int64_t>(p.slots[e]) * p.n_heads + head) * kDim + w * 16 + (lane & 3) * 2) * p.vdim +
+            ct * kDeltaCols + (lane >> 2);
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
+        for (int j = 0; j < 2; ++j) {
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            s[j][r] = corner[static_cast<int64_t>(8 * j + (r & 1)) * p.vdim + (r >> 1) * 8];
+            for (int r = 0; r < 4; ++r) {
+                s[j][r] = corner[static_cast<int64_t>(8 * j + (r & 1)) * p.vdim + (r >> 1) * 8];
+            }
         }
+        TermsB wm, kd, kv = {};
+        float4 zi[2], g;
+        uint4 vv = {};
+        auto read_chunk = [&] {
+            wait_for_chunk();
+            terms(wm, cur + own);
+            terms(kd, cur + Ring::kAt.kd + own);
+            zi[0] = *reinterpret_cast<const float4*>(cur + Ring::kZi + lane * 4);
+            zi[1] = *reinterpret_cast<const float4*>(cur + Ring::kZi + 128 + lane * 4);
+            g = *reinterpret_cast<const float4*>(cur + Ring::kG + w * 16 + (lane & 3) * 4);
+            if constexpr (GENERAL) {
+                terms(kv, cur + Ring::kAt.kv + own);
+                vv = *reinterpret_cast<const uint4*>(cur + Ring::kVv + lane * 4);
+            }
+            next_chunk();
+        };
+        read_chunk();
+        for (int c = 0; c < n_chunks; ++c) {
+            const int parity = c & 1;
+            TermsA a, az;
+            terms_of(a, s[0], s[1]);
+            float d[2][4];
+            mma_terms(d[0], d[1], a, wm);  // this warp's rows' share of S0's part of Z
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                states[parity][j][w][lane] = make_float4(s[j][0], s[j][1], s[j][2], s[j][3]);
+                shares[parity][j][w][lane] = make_float4(d[j][0], d[j][1], d[j][2], d[j][3]);
+            }
+            __syncthreads();
+            const float decay[2][2] = {{g.x, g.y}, {g.z, g.w}};
+            float written[2][4] = {};
+            if constexpr (GENERAL) {  // + Kv^T V: the values are bfloat16 as they are
+                const uint32_t v[4] = {vv.x, vv.y, vv.z, vv.w};
+#pragma unroll
+                for (int term = 2; term >= 0; --term) {
+                    mma_bf16(written[0], v, kv.t[term].x, kv.t[term].y);
+                    mma_bf16(written[1], v, kv.t[term].z, kv.t[term].w);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    s[j][r] = fmaf(s[j][r], decay[j][r & 1], written[j][r]);
+                }
+            }
+            float z[2][4], moved[2][4];
+            z_of(z, zi, parity);
+            terms_of(az, z[0], z[1]);
+            mma_terms(moved[0], moved[1], az, kd);
+            if (c + 1 < n_chunks) {
+                read_chunk();  // (under the products' latency)
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    s[j][r] += moved[j][r];
+                }
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                corner[static_cast<int64_t>(8 * j + (r & 1)) * p.vdim + (r >> 1) * 8] = lost ? NAN : s[j][r];
+            }
+        }
+        return;
     }
+
     // This lane's outputs: columns lane / 4 and 8 on, tokens 8 w + (lane % 4) * 2 and the next (of the first two warps).
     const int done = p.pass.pass * p.pass.window * kDeltaChunk;
     const int rows = count - done;
@@ -357,7 +488,7 @@ __global__ void __launch_bounds__(NW * 32) delta_chain_kernel(const DeltaChainPa
     auto finish = [&](int parity) {
 #pragma unroll
         for (int other = 0; other < NW; ++other) {
-            const float4 part = shares[parity][2 + w][other][lane];
+            const float4 part = o_shares[parity][w][other][lane];
             o[0] += part.x;
             o[1] += part.y;
             o[2] += part.z;
@@ -374,87 +505,53 @@ __global__ void __launch_bounds__(NW * 32) delta_chain_kernel(const DeltaChainPa
         token += kDeltaChunk;
         dst += kDeltaChunk * o_stride;
     };
-
-    auto advance = [&](const DeltaLane<GENERAL>& in, DeltaLane<GENERAL>& ahead, int c, const int parity) {
-        // (M, Oi and Kd, which the chunk's end reads: a chunk ahead too the general rule's registers would not hold them)
-        TermsB m = in.m;
-        TermsB kd_now = in.kd;
-        float4 oi = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if constexpr (GENERAL) {
-            terms(kd_now, src - step + kAt.kd);
-            if (w < 2) {
-                fetch_m(m);
-                oi = *reinterpret_cast<const float4*>(src_oi);
-                src_oi += step;
+    for (int c = 0; c < n_chunks; ++c) {
+        const int parity = c & 1;
+        __syncthreads();  // the chunk's state and shares of Z are there, and the chunk before it was read by everyone
+        if (brings && c > 0 && c - 1 + Ring::kSlots < n_chunks) {
+            bring(c - 1 + Ring::kSlots);
+        }
+        wait_for_chunk();
+        TermsB qg, m = {};
+        terms(qg, cur + Ring::kAt.qg + own);
+        float4 zi[2] = {}, oi = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (w < 2) {
+            terms(m, cur + Ring::kAt.m + lane * 4);
+            zi[0] = *reinterpret_cast<const float4*>(cur + Ring::kZi + lane * 4);
+            zi[1] = *reinterpret_cast<const float4*>(cur + Ring::kZi + 128 + lane * 4);
+            if constexpr (GENERAL) {
+                oi = *reinterpret_cast<const float4*>(cur + Ring::kOi + (w * 32 + lane) * 4);
             }
         }
-        if (c + 1 < n_chunks) {
-            fetch(ahead);
+        next_chunk();
+        float s[2][4], q[2][4];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const float4 part = states[parity][j][w][lane];
+            s[j][0] = part.x;
+            s[j][1] = part.y;
+            s[j][2] = part.z;
+            s[j][3] = part.w;
         }
-        TermsA a, az;
+        TermsA a;
         terms_of(a, s[0], s[1]);
-        float d[2][4];
-        mma_terms(d[0], d[1], a, in.wm);  // this warp's rows' share of S0's part of Z
+        mma_terms(q[0], q[1], a, qg);  // this warp's rows' share of S0's part of O, read after the next barrier
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
-            shares[parity][j][w][lane] = make_float4(d[j][0], d[j][1], d[j][2], d[j][3]);
-        }
-        const float decay[2][2] = {{in.g.x, in.g.y}, {in.g.z, in.g.w}};
-        float written[2][4] = {};
-        if constexpr (GENERAL) {  // + Kv^T V: the values are bfloat16 as they are
-            const uint32_t v[4] = {in.vv.x, in.vv.y, in.vv.z, in.vv.w};
-#pragma unroll
-            for (int term = 2; term >= 0; --term) {
-                mma_bf16(written[0], v, in.kv.t[term].x, in.kv.t[term].y);
-                mma_bf16(written[1], v, in.kv.t[term].z, in.kv.t[term].w);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                s[j][r] = fmaf(s[j][r], decay[j][r & 1], written[j][r]);
-            }
-        }
-        __syncthreads();
-        float z[2][4];
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            float4 sum = shares[parity][j][0][lane];
-#pragma unroll
-            for (int other = 1; other < NW; ++other) {
-                const float4 part = shares[parity][j][other][lane];
-                sum = make_float4(sum.x + part.x, sum.y + part.y, sum.z + part.z, sum.w + part.w);
-            }
-            z[j][0] = in.zi[j].x + sum.x;
-            z[j][1] = in.zi[j].y + sum.y;
-            z[j][2] = in.zi[j].z + sum.z;
-            z[j][3] = in.zi[j].w + sum.w;
-        }
-        float size = 0.0f;  // (less than infinity while all of Z is)
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            size += fabsf(z[0][r]) + fabsf(z[1][r]);
-        }
-        float q[2][4];
-        mma_terms(q[0], q[1], a, in.qg);  // (and of O: made while the sums of Z come in, read after the next barrier)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            shares[parity][2 + j][w][lane] = make_float4(q[j][0], q[j][1], q[j][2], q[j][3]);
-        }
-        terms_of(az, z[0], z[1]);
-        float moved[2][4];
-        mma_terms(moved[0], moved[1], az, kd_now);
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                s[j][r] += moved[j][r];
-            }
+            o_shares[parity][j][w][lane] = make_float4(q[j][0], q[j][1], q[j][2], q[j][3]);
         }
         if (w < 2) {
             if (c > 0) {
                 finish(parity ^ 1);  // the chunk before: its shares were written before this chunk's barrier
+            }
+            float z[2][4];
+            TermsA az;
+            z_of(z, zi, parity);
+            terms_of(az, z[0], z[1]);
+            float size = 0.0f;  // (less than infinity while all of Z is)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                size += fabsf(z[0][r]) + fabsf(z[1][r]);
             }
             float half[4] = {0.0f, 0.0f, 0.0f, 0.0f};
             o[0] = oi.x;
@@ -502,30 +599,28 @@ __global__ void __launch_bounds__(NW * 32) delta_chain_kernel(const DeltaChainPa
                 o[i] += half[i];
             }
         }
-    };
-    for (int c = 0; c < n_chunks; c += 2) {
-        advance(even, odd, c, 0);
-        if (c + 1 < n_chunks) {
-            advance(odd, even, c + 1, 1);
-        }
     }
     __syncthreads();
     if (w < 2) {
         finish((n_chunks - 1) & 1);
     }
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            corner[static_cast<int64_t>(8 * j + (r & 1)) * p.vdim + (r >> 1) * 8] = s[j][r];
-        }
+    for (int spin = 0; brings && lost && spin < (1 << 16); ++spin) {
+        __nanosleep(64);  // copies in flight land meanwhile
     }
 }
 
 template <int NW, bool GENERAL>
 cudaError_t launch_delta_chain(const DeltaChainParams& p, int n_long, cudaStream_t stream) {
-    return pl_launch_overlapped(delta_chain_kernel<NW, GENERAL>, dim3(n_long, p.n_heads, p.vdim / kDeltaCols), dim3(NW * 32), 0,
-                                stream, p);
+    using Ring = DeltaRing<NW * 16, GENERAL>;
+    // Where every CTA can have an SM to itself, more than half of one's shared memory sees to it: CTAs that come in while the
+    // chunks' matrices still hold some SMs would otherwise share the others (one prompt: 135 us so, 95 alone).
+    constexpr int kAlone = 120 * 1024, kMost = Ring::kBytes > kAlone ? Ring::kBytes : kAlone;
+    if (const cudaError_t set = pl_allow_smem<delta_chain_kernel<NW, GENERAL>>(kMost); set != cudaSuccess) {
+        return set;
+    }
+    const dim3 grid(n_long * p.n_heads, p.vdim / kDeltaCols);
+    const bool alone = static_cast<int64_t>(grid.x) * grid.y <= 148;
+    return pl_launch_overlapped(delta_chain_kernel<NW, GENERAL>, grid, dim3(NW * 64), alone ? kMost : Ring::kBytes, stream, p);
 }
 
 // The heads' norm over vdim, its weight and the gate: out = o * rsqrt(mean(o^2) + eps) * norm * sigmoid(gate), four values a
