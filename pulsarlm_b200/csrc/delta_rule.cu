@@ -712,7 +712,7 @@ struct RuleStepParams {
 };
 
 template <int DIM>
-__global__ void __launch_bounds__(kStepThreads) delta_rule_step_kernel(const RuleStepParams c) {
+__global__ void __launch_bounds__(kStepThreads, step_ctas(DIM, DIM)) delta_rule_step_kernel(const RuleStepParams c) {
     pl_grid_trigger();
     pl_grid_wait();
     __shared__ __align__(16) DeltaStepShared<DIM, DIM> s;

@@ -941,7 +941,7 @@ struct GatedStepParams {
 };
 
 template <int DIM, int VDIM>
-__global__ void __launch_bounds__(kStepThreads) gated_delta_step_kernel(const GatedStepParams c) {
+__global__ void __launch_bounds__(kStepThreads, step_ctas(DIM, VDIM)) gated_delta_step_kernel(const GatedStepParams c) {
     pl_grid_trigger();
     pl_grid_wait();
     __shared__ __align__(16) DeltaStepShared<DIM, VDIM> s;
