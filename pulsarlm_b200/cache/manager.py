@@ -303,6 +303,13 @@ class CacheManager:
     def length(self, request) -> int:
         return self._lib.plh_cache_length(self._book, self._known(request))
 
+    def lengths(self, requests: list) -> list[int]:
+        """The tokens each request holds, -1 for one that is not open, in one call of the host core."""
+        handles = np.array([self._handles.get(r, -1) for r in requests], dtype=np.int64)
+        lens = np.empty(len(requests), dtype=np.int64)
+        self._lib.plh_cache_lengths(self._book, handles.ctypes.data, len(requests), lens.ctypes.data)
+        return lens.tolist()
+
     def pages_needed(self, request, new_len: int) -> int:
         """Pages `reserve(request, new_len)` would take, summed over groups."""
         return self._lib.plh_cache_pages_needed(self._book, self._known(request), new_len)
@@ -377,20 +384,22 @@ class CacheManager:
     def table_rows(self, group: int, requests: list, width_multiple: int = 8) -> np.ndarray:
         """int32 [len(requests), W]: each request's page ids of `group`, -1 where it
         holds none; W is the longest row rounded up to `width_multiple`."""
-        handles = [self._known(r) for r in requests]
-        longest = 1
-        for h in handles:
-            longest = max(longest, self._lib.plh_cache_table_row(self._book, group, h, self._row, 0))
-        width = -(-longest // width_multiple) * width_multiple
+        handles = np.array([self._handles.get(r, -1) for r in requests], dtype=np.int64)
+        longest = self._lib.plh_cache_longest_row(self._book, group, handles.ctypes.data, len(requests))
+        if longest < 0:
+            for r in requests:
+                self._known(r)
+            raise CacheError(f"table_rows failed with code {longest}")
+        width = -(-max(1, longest) // width_multiple) * width_multiple
         table = np.empty((len(handles), width), dtype=np.int32)
         self.fill_tables(group, handles, table, None)
         return table
 
-    def fill_tables(self, group: int, handles: list[int], table: np.ndarray, slots: np.ndarray | None) -> int:
+    def fill_tables(self, group: int, handles: list[int] | np.ndarray, table: np.ndarray, slots: np.ndarray | None) -> int:
         """Writes the block-table rows of `handles` into `table` (int32 [n, W], C order;
         -1 where no page) and their slots into `slots`; returns the longest row."""
         n = len(handles)
-        ids = (ctypes.c_int64 * max(1, n))(*handles)
+        ids = handles.ctypes.data_as(ctypes.c_void_p) if isinstance(handles, np.ndarray) else (ctypes.c_int64 * max(1, n))(*handles)
         longest = self._lib.plh_cache_fill_tables(
             self._book, group, ids, n, table.ctypes.data_as(ctypes.c_void_p), table.shape[1],
             slots.ctypes.data_as(ctypes.c_void_p) if slots is not None else None)

@@ -474,7 +474,7 @@ using plh::CacheBook;
 using plh::PagePool;
 using plh::SchedulerCore;
 
-PLH_API int plh_abi_version() { return 5; }
+PLH_API int plh_abi_version() { return 6; }
 
 PLH_API void* plh_pool_create(int n_pages) { return new PagePool(n_pages); }
 PLH_API void plh_pool_destroy(void* pool) { delete static_cast<PagePool*>(pool); }
@@ -510,6 +510,13 @@ PLH_API int plh_cache_slot(void* cache, int64_t request) { return static_cast<Ca
 PLH_API int64_t plh_cache_length(void* cache, int64_t request) {
     return static_cast<CacheBook*>(cache)->length(request);
 }
+// Of `count` requests the tokens each holds, -1 for one that is not open.
+PLH_API void plh_cache_lengths(void* cache, const int64_t* requests, int count, int64_t* lens) {
+    const CacheBook* book = static_cast<CacheBook*>(cache);
+    for (int i = 0; i < count; ++i) {
+        lens[i] = book->is_open(requests[i]) ? book->length(requests[i]) : -1;
+    }
+}
 PLH_API int plh_cache_reserve(void* cache, int64_t request, int64_t new_len) {
     return static_cast<CacheBook*>(cache)->reserve(request, new_len);
 }
@@ -522,6 +529,22 @@ PLH_API int plh_cache_pages_needed(void* cache, int64_t request, int64_t new_len
 }
 PLH_API int plh_cache_table_row(void* cache, int group, int64_t request, int32_t* out, int capacity) {
     return static_cast<CacheBook*>(cache)->table_row(group, request, out, capacity);
+}
+// The longest block-table row of `count` open requests, or the code of one that is none.
+PLH_API int plh_cache_longest_row(void* cache, int group, const int64_t* requests, int count) {
+    const CacheBook* book = static_cast<CacheBook*>(cache);
+    int longest = 0;
+    for (int i = 0; i < count; ++i) {
+        if (!book->is_open(requests[i])) {
+            return plh::kUnknownRequest;
+        }
+        const int n = book->table_row(group, requests[i], nullptr, 0);
+        if (n < 0) {
+            return n;
+        }
+        longest = std::max(longest, n);
+    }
+    return longest;
 }
 PLH_API int plh_cache_held_pages(void* cache, int group, int64_t request, int32_t* out, int capacity) {
     return static_cast<CacheBook*>(cache)->held_pages(group, request, out, capacity);

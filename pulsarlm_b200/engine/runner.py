@@ -146,72 +146,74 @@ class ModelRunner:
         if len(sources) != len(entries) or any(s >= 0 and len(e.tokens) != 1 for s, e in zip(sources, entries)):
             raise ValueError("tokens taken from the device: one row per entry, and only for entries of one token")
         seen = set()
-        for e, source in zip(entries, sources):
+        counts = [len(e.tokens) for e in entries]
+        portions: dict[int, np.ndarray] = {}  # the tokens of entries of more than one, as an array
+        for i, (e, source, n) in enumerate(zip(entries, sources, counts)):
             if e.request in seen:
                 raise ValueError(f"request {e.request!r} appears twice in one step")
             seen.add(e.request)
-            n = len(e.tokens)
             if n == 0:
                 raise ValueError(f"request {e.request!r}: a step entry needs at least one token")
             if n == 1:
                 if source < 0 and not 0 <= int(e.tokens[0]) < self.vocab:
                     raise ValueError(f"request {e.request!r}: token id {e.tokens[0]} is outside [0, {self.vocab})")
             else:
-                ids = np.asarray(e.tokens)
+                ids = portions[i] = np.asarray(e.tokens)
                 if int(ids.min()) < 0 or int(ids.max()) >= self.vocab:
                     bad = [t for t in e.tokens if not 0 <= int(t) < self.vocab]
                     raise ValueError(f"request {e.request!r}: token id {bad[0]} is outside [0, {self.vocab})")
             if e.want and not all(0 <= w < n for w in e.want):
                 raise ValueError(f"request {e.request!r}: wanted places {e.want} are outside its {n} tokens")
         limit = self.model.spec.max_positions
-        if limit is not None:
-            for e in entries:
-                held = self.cache.length(e.request) if self.cache.is_open(e.request) else 0
-                if held + len(e.tokens) > limit:
-                    raise ValueError(f"request {e.request!r}: {held + len(e.tokens)} tokens exceed the model's {limit} positions")
-        for e in entries:
-            if not self.cache.is_open(e.request):
-                if self.cache.open(e.request) is None:
-                    raise OutOfPages(e.request, f"no free slot for request {e.request!r}")
         all_requests = [e.request for e in entries]
-        starts, all_slots, done = self.cache.reserve_many(all_requests, [len(e.tokens) for e in entries])
+        held = self.cache.lengths(all_requests)
+        if limit is not None:
+            for e, have, n in zip(entries, held, counts):
+                if max(have, 0) + n > limit:
+                    raise ValueError(f"request {e.request!r}: {max(have, 0) + n} tokens exceed the model's {limit} positions")
+        for e, have in zip(entries, held):
+            if have < 0 and self.cache.open(e.request) is None:
+                raise OutOfPages(e.request, f"no free slot for request {e.request!r}")
+        first_tokens, all_slots, done = self.cache.reserve_many(all_requests, counts)
         if done < len(entries):
             e = entries[done]
             raise OutOfPages(e.request, f"too few free pages for request {e.request!r} to reach "
-                                        f"{int(starts[done]) + len(e.tokens)} tokens")
-        new_lens = [int(starts[i]) + len(e.tokens) for i, e in enumerate(entries)]
+                                        f"{int(first_tokens[done]) + counts[done]} tokens")
+        starts = first_tokens.tolist()
+        new_lens = [start + n for start, n in zip(starts, counts)]
 
         if getattr(self, "_copy_done", None) is not None:
             self._copy_done.synchronize()
         # Entries of one token go first (StepBatch's contract: mixers may send the leading
         # single tokens to a kernel of their own); the wanted rows still come back in the
         # caller's order of entries.
-        order = sorted(range(len(entries)), key=lambda i: len(entries[i].tokens) != 1)
-        n_decode = sum(1 for e in entries if len(e.tokens) == 1)
-        n_tokens = sum(len(e.tokens) for e in entries)
+        order = [i for i, n in enumerate(counts) if n == 1]
+        n_decode = len(order)
+        order += [i for i, n in enumerate(counts) if n != 1]
+        n_tokens = sum(counts)
         tokens = np.empty(n_tokens, dtype=np.int32)
         pos = np.empty(n_tokens, dtype=np.int32)
         entry = np.empty(n_tokens, dtype=np.int32)
         first_row = [0] * len(entries)
+        # The single tokens' rows all at once, then the portions'.
+        tokens[:n_decode] = [int(entries[i].tokens[0]) if sources[i] < 0 else 0 for i in order[:n_decode]]
+        pos[:n_decode] = [starts[i] for i in order[:n_decode]]
+        entry[:n_decode] = np.arange(n_decode, dtype=np.int32)
         at = 0
         for place, i in enumerate(order):
-            e = entries[i]
-            n = len(e.tokens)
-            start = int(starts[i])
-            tokens[at : at + n] = e.tokens if sources[i] < 0 else 0
-            if n == 1:
-                pos[at] = start
-            else:
-                pos[at : at + n] = np.arange(start, start + n, dtype=np.int32)
-            entry[at : at + n] = place
+            n = counts[i]
             first_row[i] = at
+            if n != 1:
+                tokens[at : at + n] = portions[i]
+                pos[at : at + n] = np.arange(starts[i], starts[i] + n, dtype=np.int32)
+                entry[at : at + n] = place
             at += n
         want_rows = [first_row[i] + w for i, e in enumerate(entries) for w in e.want]
         requests = [entries[i].request for i in order]
         slots = all_slots[order]
         tables = [self.cache.table_rows(g.index, requests) for g in self.cache.groups]
         host = HostStep(n_entries=len(entries), n_tokens=n_tokens, n_decode=n_decode,
-                        query_lens=[len(entries[i].tokens) for i in order],
+                        query_lens=[counts[i] for i in order],
                         context_lens=[new_lens[i] for i in order],
                         first_rows=[first_row[i] for i in order], page_size=self.cache.page_size)
         arrays = [tokens, pos, entry, slots, np.array(want_rows, dtype=np.int32), *tables]

@@ -11,7 +11,7 @@ from ..kernels import build
 _I32, _I64, _PTR = ctypes.c_int, ctypes.c_int64, ctypes.c_void_p
 _lib = None
 _lock = threading.Lock()
-ABI_VERSION = 5
+ABI_VERSION = 6
 
 # return codes of csrc_host/host_core.hpp
 OK, NO_ROOM = 0, 1
@@ -32,6 +32,8 @@ _SIGNATURES = {
     "plh_cache_is_open": ([_PTR, _I64], _I32),
     "plh_cache_slot": ([_PTR, _I64], _I32),
     "plh_cache_length": ([_PTR, _I64], _I64),
+    "plh_cache_lengths": ([_PTR, _PTR, _I32, _PTR], None),
+    "plh_cache_longest_row": ([_PTR, _I32, _PTR, _I32], _I32),
     "plh_cache_reserve": ([_PTR, _I64, _I64], _I32),
     "plh_cache_commit": ([_PTR, _I64, _I64], _I32),
     "plh_cache_close": ([_PTR, _I64], _I32),
