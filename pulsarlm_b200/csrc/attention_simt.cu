@@ -538,6 +538,233 @@ __global__ void attention_f32_staged_kernel(const StagedParams a) {
     }
 }
 
+// The same walk for few tokens without a window, its parts side by side: a CTA has one token and HEADS heads of a kv head, and
+// KEYS keys at a time. A warp's 32 keys are one chunk of the walk: its threads make their keys' scores, then the chunk's largest; what
+// the walk's maximum was before and after every chunk follows from those; the weights, their sums and the corrections are made
+// chunk by chunk at once, and then a thread walks the keys for one column of one head. Every number is made by the same
+// operations in the same order. Left in line is only the chain of fmafs over the keys, four cycles each; the walk above had every
+// chunk's phases in it. What bounds it: shared memory's operands (a key and a query a fmaf of the scores, a value and a quarter of a
+// weight a fmaf of the outputs). 8 tokens of 600 keys, 32 heads of 64 over 8, cold, in an engine step: 33.5 -> 20.1 us.
+constexpr int kWideThreads = 256;
+
+template <int HEADS, int KEYS>
+inline constexpr int wide_smem_bytes(int hd) {
+    return (HEADS * hd + HEADS * KEYS + 3 * HEADS * (KEYS / 32) + 2 * KEYS * (2 * hd + 4)) * 4 + HEADS * (KEYS / 32) * 4 + 3 * KEYS * 8;
+}
+
+template <int HEADS, int KEYS, int ACC>
+__global__ void __launch_bounds__(kWideThreads) attention_f32_wide_kernel(const StagedParams a) {
+    constexpr int kChunks = KEYS / 32, kSets = kWideThreads / KEYS, kOwn = (HEADS + kSets - 1) / kSets;
+    extern __shared__ __align__(16) float wide_smem[];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int hd = a.head_dim, k_ld = hd + 4;
+    float* ks = wide_smem;                                    // [2][KEYS][hd + 4]
+    float* vs = ks + 2 * KEYS * k_ld;                         // [2][KEYS][hd]
+    float* qs = vs + 2 * KEYS * hd;                           // [HEADS][hd]
+    float* ps = qs + HEADS * hd;                              // [HEADS][KEYS]
+    float* largest = ps + HEADS * KEYS;                       // [HEADS][chunks]
+    float* sums = largest + HEADS * kChunks;
+    float* corrections = sums + HEADS * kChunks;
+    uint32_t* seen = reinterpret_cast<uint32_t*>(corrections + HEADS * kChunks);
+    int64_t* offsets = reinterpret_cast<int64_t*>(seen + HEADS * kChunks);  // [3][KEYS]
+    const int t = blockIdx.x, kv_head = blockIdx.y, head0 = kv_head * a.group + blockIdx.z * HEADS;
+    const int position = a.pos[t];
+    const int steps = position / KEYS + 1;
+    const int32_t* row = a.table + static_cast<int64_t>(a.entry[t]) * a.table_width;
+
+    for (int idx = tid; idx < HEADS * hd; idx += kWideThreads) {
+        qs[idx] = a.q[t * a.q_row_stride + static_cast<int64_t>(head0) * hd + idx];
+    }
+    auto locate = [&](int w) {  // where a step's keys lie (-1: no page, or past the last key)
+        const int j = w * KEYS + tid;
+        if (tid < KEYS && w < steps) {
+            const int page = j <= position ? row[j / a.page_size] : -1;
+            offsets[w % 3 * KEYS + tid] = page >= 0 && page < a.n_pages
+                ? page * a.page_stride + kv_head * a.head_stride + static_cast<int64_t>(j % a.page_size) * hd : -1;
+        }
+    };
+    auto load = [&](int w) {
+        if (w < steps) {
+            const int64_t* where = offsets + w % 3 * KEYS;
+            const int stage = w & 1, per = hd / 4;
+            for (int idx = tid; idx < KEYS * per; idx += kWideThreads) {
+                const int key = idx / per, c = (idx - key * per) * 4;
+                const int64_t offset = where[key];
+                const bool there = offset >= 0;
+                cp_async_16_or_zero(ks + (stage * KEYS + key) * k_ld + c, a.k_pool + (there ? offset + c : 0), there);
+                cp_async_16_or_zero(vs + (stage * KEYS + key) * hd + c, a.v_pool + (there ? offset + c : 0), there);
+            }
+        }
+        cp_async_commit();
+    };
+    const int key = tid % KEYS, set = tid / KEYS, chunk = key / 32;  // (this thread's heads: set, set + kSets, ...)
+    float m[kOwn], acc[ACC], l[ACC];
+#pragma unroll
+    for (int i = 0; i < kOwn; ++i) {
+        m[i] = -INFINITY;
+    }
+#pragma unroll
+    for (int n = 0; n < ACC; ++n) {
+        acc[n] = l[n] = 0.0f;
+    }
+    locate(0);
+    locate(1);
+    __syncthreads();
+    load(0);
+    for (int w = 0; w < steps; ++w) {
+        cp_async_wait<0>();
+        __syncthreads();  // the step's keys have landed; the one before it was read by everyone
+        load(w + 1);
+        locate(w + 2);
+        const int stage = w & 1, j = w * KEYS + key;
+        const bool paged = offsets[w % 3 * KEYS + key] >= 0;
+        const float* krow = ks + (stage * KEYS + key) * k_ld;
+        float s[kOwn];
+#pragma unroll
+        for (int i = 0; i < kOwn; ++i) {
+            s[i] = 0.0f;
+        }
+#pragma unroll 4
+        for (int d = 0; d < hd; d += 4) {
+            const float4 kv = *reinterpret_cast<const float4*>(krow + d);
+#pragma unroll
+            for (int i = 0; i < kOwn; ++i) {
+                const float4 qv = *reinterpret_cast<const float4*>(qs + min(set + i * kSets, HEADS - 1) * hd + d);
+                s[i] = fmaf(qv.x, kv.x, s[i]);
+                s[i] = fmaf(qv.y, kv.y, s[i]);
+                s[i] = fmaf(qv.z, kv.z, s[i]);
+                s[i] = fmaf(qv.w, kv.w, s[i]);
+            }
+        }
+        if (j <= position && !paged && set == 0 && a.status != nullptr) {
+            atomicOr(a.status, 4);
+        }
+        const bool valid = j <= position && paged;
+#pragma unroll
+        for (int i = 0; i < kOwn; ++i) {
+            const int h = set + i * kSets;
+            float score = -INFINITY;
+            if (valid && h < HEADS) {
+                score = s[i] * a.scale;
+                if (a.softcap > 0.0f) {
+                    score = a.softcap * tanhf(score / a.softcap);
+                }
+                if (a.distance_bias != nullptr) {
+                    score += a.distance_bias[static_cast<int64_t>(head0 + h) * a.bias_rows + min(position - j, a.bias_rows - 1)];
+                }
+                if (a.distance_slopes != nullptr) {
+                    score = fmaf(-a.distance_slopes[head0 + h], static_cast<float>(position - j), score);
+                }
+            }
+            s[i] = score;
+            const float top = pl_warp_max(score);
+            const uint32_t there = __ballot_sync(0xffffffffu, valid);
+            if (lane == 0 && h < HEADS) {
+                largest[h * kChunks + chunk] = top;
+                seen[h * kChunks + chunk] = there;
+            }
+        }
+        __syncthreads();
+        // Chunks past the last key are not walked.
+        const int chunks = min(kChunks, (position - w * KEYS) / 32 + 1);
+#pragma unroll
+        for (int i = 0; i < kOwn; ++i) {
+            const int h = set + i * kSets;
+            float before = m[i], after = m[i], running = m[i];
+            for (int c = 0; c < chunks && h < HEADS; ++c) {
+                const float next = fmaxf(running, largest[h * kChunks + c]);
+                if (c == chunk) {
+                    before = running;
+                    after = next;
+                }
+                running = next;
+            }
+            m[i] = running;
+            const bool any = after > -INFINITY;  // (-inf only if a bad block table hid every key so far)
+            const float weight = valid && any ? expf(s[i] - after) : 0.0f;
+            const float sum = pl_warp_sum(weight);
+            if (h < HEADS) {
+                ps[h * KEYS + key] = weight;
+                if (lane == 0) {
+                    sums[h * kChunks + chunk] = sum;
+                    corrections[h * kChunks + chunk] = any ? expf(before - after) : 1.0f;
+                }
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int n = 0; n < ACC; ++n) {
+            const int column = tid + n * kWideThreads, h = column / hd;
+            if (column < HEADS * hd) {
+                const float* values = vs + stage * KEYS * hd + column - h * hd;
+                for (int c = 0; c < chunks; ++c) {
+                    const float corr = corrections[h * kChunks + c];
+                    const uint32_t mask = seen[h * kChunks + c];
+                    l[n] = l[n] * corr + sums[h * kChunks + c];
+                    acc[n] *= corr;
+                    if (mask == 0xffffffffu) {
+#pragma unroll
+                        for (int j4 = 0; j4 < 32; j4 += 4) {
+                            const float4 p4 = *reinterpret_cast<const float4*>(ps + h * KEYS + c * 32 + j4);
+                            const float* v = values + (c * 32 + j4) * hd;
+                            acc[n] = fmaf(p4.x, v[0], acc[n]);
+                            acc[n] = fmaf(p4.y, v[hd], acc[n]);
+                            acc[n] = fmaf(p4.z, v[2 * hd], acc[n]);
+                            acc[n] = fmaf(p4.w, v[3 * hd], acc[n]);
+                        }
+                    } else {
+                        for (int jj = 0; jj < 32; ++jj) {
+                            if (mask >> jj & 1) {
+                                acc[n] = fmaf(ps[h * KEYS + c * 32 + jj], values[(c * 32 + jj) * hd], acc[n]);
+                            }
+                        }
+                    }
+                }
+            }
+        }
+    }
+    // (the walk's last maximum, for the sink: every thread of set h has it for head h; the columns' threads make it again)
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kOwn; ++i) {
+        if (key == 0 && set + i * kSets < HEADS) {
+            largest[set + i * kSets] = m[i];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int n = 0; n < ACC; ++n) {
+        const int column = tid + n * kWideThreads, h = column / hd;
+        if (column >= HEADS * hd) {
+            continue;
+        }
+        if (a.sinks != nullptr) {
+            const float sink = a.sinks[head0 + h], top = largest[h];
+            const float m_new = fmaxf(top, sink);
+            const float corr = top > -INFINITY ? expf(top - m_new) : 0.0f;
+            l[n] = l[n] * corr + expf(sink - m_new);
+            acc[n] *= corr;
+        }
+        float inv = l[n] > 0.0f ? 1.0f / l[n] : 0.0f;
+        if (a.gate != nullptr) {
+            inv *= 1.0f / (1.0f + expf(-a.gate[t * a.gate_row_stride + head0 + h]));
+        }
+        a.out[t * a.out_row_stride + static_cast<int64_t>(head0) * hd + column] = acc[n] * inv;
+    }
+}
+
+template <int HEADS, int KEYS, int ACC>
+cudaError_t launch_wide(const StagedParams& a, int n_kv_heads, cudaStream_t stream) {
+    constexpr auto kernel = attention_f32_wide_kernel<HEADS, KEYS, ACC>;
+    constexpr int kMost = wide_smem_bytes<HEADS, KEYS>(KEYS == 128 ? 64 : 128);
+    static_assert(kMost <= 227 * 1024, "shared memory");
+    if (const cudaError_t set = pl_allow_smem<kernel>(kMost); set != cudaSuccess) {
+        return set;
+    }
+    kernel<<<dim3(a.n_tokens, n_kv_heads, a.group / HEADS), kWideThreads, wide_smem_bytes<HEADS, KEYS>(a.head_dim), stream>>>(a);
+    return cudaGetLastError();
+}
+
 template <int P, int ACC, int DIM>
 cudaError_t launch_staged(const StagedParams& a, int n_kv_heads, cudaStream_t stream) {
     const int pairs = a.run * a.group;
@@ -617,6 +844,25 @@ PL_API int pl_attention_simt(const void* q, int64_t q_row_stride, const void* k_
                        gate_row_stride, distance_bias, bias_rows, distance_slopes, keep_first > 0 ? keep_first : 0,
                        status};
         cudaError_t failed = cudaSuccess;
+        // Steps of few tokens without a window: the form whose parts are side by side, as long as every one of its CTAs (135 KB of
+        // keys and values each) has an SM to itself, two heads a CTA where there are SMs for that, else four; and where the table has
+        // room for more keys than one of its steps takes. 300 and 1,000 keys, us before and now: 32 heads of 64 over 8, 8 tokens 20.9
+        // -> 13.7, 55.7 -> 29.6; 8 heads over 8, 8 tokens 27.0 -> 12.7, 74.1 -> 29.1; 32 heads of 128 over 8, 8 tokens 27.0 -> 21.6,
+        // 73.3 -> 59.8; 16 over 2, 32 tokens 22.1 -> 16.8, 57.2 -> 37.5. With more CTAs than SMs: 32 over 8, 32 tokens 22.9 and 29.5.
+        const int64_t pairs = static_cast<int64_t>(n_tokens) * n_kv_heads;
+        const int heads = group % 4 == 0 && pairs * (group / 2) > 148 ? 4 : group % 2 == 0 ? 2 : 1;
+        if (few && window <= 0 && pairs * (group / heads) <= 148 && static_cast<int64_t>(table_width) * page_size > 128) {
+            failed = head_dim <= 64 ? (heads == 4   ? launch_wide<4, 128, 1>(a, n_kv_heads, stream)
+                                       : heads == 2 ? launch_wide<2, 128, 1>(a, n_kv_heads, stream)
+                                                    : launch_wide<1, 128, 1>(a, n_kv_heads, stream))
+                                    : (heads == 4   ? launch_wide<4, 64, 2>(a, n_kv_heads, stream)
+                                       : heads == 2 ? launch_wide<2, 64, 1>(a, n_kv_heads, stream)
+                                                    : launch_wide<1, 64, 1>(a, n_kv_heads, stream));
+            if (failed != cudaSuccess) {
+                return pl_fail(3, "attention: launch failed: %s", cudaGetErrorString(failed));
+            }
+            return 0;
+        }
         if (!few) {
             failed = head_dim <= 64 ? launch_staged<4, 2, 0>(a, n_kv_heads, stream)
                                     : launch_staged<4, 4, 0>(a, n_kv_heads, stream);

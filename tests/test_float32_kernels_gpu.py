@@ -148,3 +148,34 @@ def test_a_page_outside_the_pool_is_flagged_and_its_keys_are_left_out():
         mass, weight = torch.zeros((4, 2), device=DEV), torch.zeros(4, device=DEV)
         ops.attention_simt(q[rows], pools[0], pools[1], table, pos[rows], entry[rows], want, 16, None, 0.125, None, mass, weight)
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("heads,kv,dim", [(8, 2, 64), (3, 3, 20), (16, 1, 128), (6, 1, 36), (4, 4, 128), (2, 1, 64)])
+@pytest.mark.parametrize("options", [{}, {"softcap": 3.0, "sinks": True, "gate": True, "bias": True, "slopes": True}])
+def test_few_tokens_of_many_keys_give_the_bits_of_the_plain_walk(heads, kv, dim, options):
+    """Single tokens whose keys end around a chunk's 32, a step's 64 and 128 and several steps on, a page that is missing in the middle
+    of one request and at the start of another (the plain walk is reached by asking for attention mass)."""
+    ops = _ops()
+    gen = torch.Generator().manual_seed(heads * dim)
+    page, ends = 16, [0, 30, 31, 32, 63, 64, 127, 128, 129, 255, 256, 500, 777]
+    width = ends[-1] // page + 1
+    pools = torch.randn((2, len(ends) * width, kv, page, dim), generator=gen).to(DEV)
+    table = torch.randperm(len(ends) * width, generator=gen).int().view(len(ends), width)
+    table[10, 5], table[11, 0], table[12, :9] = -1, -1, -1
+    more = {}
+    if options:
+        more = {"sinks": torch.randn(heads, generator=gen).to(DEV), "distance_bias": torch.randn((heads, 50), generator=gen).to(DEV),
+                "distance_slopes": torch.rand(heads, generator=gen).to(DEV) * 0.1, "softcap": 3.0}
+    for chosen in ([i] for i in range(len(ends))) if heads > 8 else (list(range(len(ends))), [9], [12]):
+        n = len(chosen)
+        q = torch.randn((n, heads, dim), generator=gen).to(DEV)
+        pos = torch.tensor([ends[i] for i in chosen], dtype=torch.int32, device=DEV)
+        entry = torch.arange(n, dtype=torch.int32, device=DEV)
+        gate = {"gate": torch.randn((n, heads), generator=gen).to(DEV)} if options else {}
+        args = (pools[0], pools[1], table[chosen].contiguous().to(DEV), pos, entry)
+        got, want = torch.empty_like(q), torch.empty_like(q)
+        mass, weight = torch.zeros((pools.shape[1], heads), device=DEV), torch.zeros(pools.shape[1], device=DEV)
+        status, plain_status = torch.zeros(1, dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+        ops.attention_simt(q, *args, got, page, None, dim ** -0.5, status, **more, **gate)
+        ops.attention_simt(q, *args, want, page, None, dim ** -0.5, plain_status, mass, weight, **more, **gate)
+        assert torch.equal(got, want) and int(status.item()) == int(plain_status.item())
