@@ -437,7 +437,7 @@ constexpr int rule_chunk_smem() {
 }
 
 template <int DIM>
-__global__ void __launch_bounds__(128) delta_rule_chunk_kernel(const RuleChunkParams c) {
+__global__ void __launch_bounds__(128, DIM == 32 ? 5 : 4) delta_rule_chunk_kernel(const RuleChunkParams c) {
     pl_grid_trigger();
     pl_grid_wait();
     constexpr int kLd = DIM + 4;
