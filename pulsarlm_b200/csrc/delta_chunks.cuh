@@ -376,6 +376,9 @@ __global__ void __launch_bounds__(NW * 64, NW >= 8 ? 1 : 8 / NW) delta_chain_ker
         }
     };
     const int own = w * 384 + lane * 4;
+    // Both halves of the CTA meet once a chunk and once after the last, each from a branch of its own: __syncthreads() is only for
+    // places that every thread comes by, a named barrier counts threads wherever they are.
+    auto meet = [] { asm volatile("bar.sync 1, %0;" ::"n"(NW * 64) : "memory"); };
     // The sum of the warps' shares of Z and its start: every warp makes it whole.
     auto z_of = [&](float (&z)[2][4], const float4 (&zi)[2], int parity) {
 #pragma unroll
@@ -433,7 +436,7 @@ __global__ void __launch_bounds__(NW * 64, NW >= 8 ? 1 : 8 / NW) delta_chain_ker
                 states[parity][j][w][lane] = make_float4(s[j][0], s[j][1], s[j][2], s[j][3]);
                 shares[parity][j][w][lane] = make_float4(d[j][0], d[j][1], d[j][2], d[j][3]);
             }
-            __syncthreads();
+            meet();
             const float decay[2][2] = {{g.x, g.y}, {g.z, g.w}};
             float written[2][4] = {};
             if constexpr (GENERAL) {  // + Kv^T V: the values are bfloat16 as they are
@@ -466,7 +469,7 @@ __global__ void __launch_bounds__(NW * 64, NW >= 8 ? 1 : 8 / NW) delta_chain_ker
                 }
             }
         }
-        __syncthreads();
+        meet();
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
 #pragma unroll
@@ -507,7 +510,7 @@ __global__ void __launch_bounds__(NW * 64, NW >= 8 ? 1 : 8 / NW) delta_chain_ker
     };
     for (int c = 0; c < n_chunks; ++c) {
         const int parity = c & 1;
-        __syncthreads();  // the chunk's state and shares of Z are there, and the chunk before it was read by everyone
+        meet();  // the chunk's state and shares of Z are there, and the chunk before it was read by everyone
         if (brings && c > 0 && c - 1 + Ring::kSlots < n_chunks) {
             bring(c - 1 + Ring::kSlots);
         }
@@ -600,7 +603,7 @@ __global__ void __launch_bounds__(NW * 64, NW >= 8 ? 1 : 8 / NW) delta_chain_ker
             }
         }
     }
-    __syncthreads();
+    meet();
     if (w < 2) {
         finish((n_chunks - 1) & 1);
     }
