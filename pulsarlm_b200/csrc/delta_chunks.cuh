@@ -239,6 +239,7 @@ struct DeltaChainParams {
     float* o_raw;
     int n_heads, vdim;
     DeltaPass pass;
+    int32_t* status;  // (bit 8 where a chunk did not come; may be nullptr)
 };
 
 struct TermsA {
@@ -321,7 +322,7 @@ __global__ void __launch_bounds__(NW * 64, NW >= 8 ? 1 : 8 / NW) delta_chain_ker
     extern __shared__ __align__(128) float ring[];   // [slots][Ring::kFloats], and the state before the chunk, by its parity
     auto states = reinterpret_cast<float4(*)[2][NW][32]>(ring + Ring::kSlots * Ring::kFloats);
     __shared__ __align__(8) uint64_t landed[Ring::kSlots];
-    __shared__ int lost;
+    __shared__ volatile int lost;
     // One thread of the outputs' warps brings a chunk in, kSlots of them in flight.
     const bool brings = tid == blockDim.x - 32;
     auto bring = [&](int c) {
@@ -356,7 +357,9 @@ __global__ void __launch_bounds__(NW * 64, NW >= 8 ? 1 : 8 / NW) delta_chain_ker
             bring(c);
         }
     }
-    // A chunk's place once it is there. (One that never comes leaves numbers that are none: see the state's end.)
+    // A chunk's place once it is there. (Where one never comes the wait gives up: the state's end, this chunk's outputs and all later
+    // ones are not a number, and the status word says so. Whoever gave up said it before the next meeting, and what was made
+    // of the chunk is stored behind that.)
     int slot = 0;
     uint32_t phase = 0;
     const float* cur = ring;
@@ -497,6 +500,9 @@ __global__ void __launch_bounds__(NW * 64, NW >= 8 ? 1 : 8 / NW) delta_chain_ker
             o[2] += part.z;
             o[3] += part.w;
         }
+        if (lost) {
+            o[0] = o[1] = o[2] = o[3] = NAN;
+        }
         if (token < rows) {
             dst[0] = o[0];
             dst[8] = o[2];
@@ -607,8 +613,13 @@ __global__ void __launch_bounds__(NW * 64, NW >= 8 ? 1 : 8 / NW) delta_chain_ker
     if (w < 2) {
         finish((n_chunks - 1) & 1);
     }
-    for (int spin = 0; brings && lost && spin < (1 << 16); ++spin) {
-        __nanosleep(64);  // copies in flight land meanwhile
+    if (brings && lost) {
+        if (p.status != nullptr) {
+            atomicOr(p.status, 8);
+        }
+        for (int spin = 0; spin < (1 << 16); ++spin) {
+            __nanosleep(64);  // copies in flight land meanwhile
+        }
     }
 }
 

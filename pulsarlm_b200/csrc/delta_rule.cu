@@ -429,6 +429,7 @@ struct RuleChunkParams {
     ScanParams in;
     DeltaPass pass;
     float* scratch;
+    int32_t* status;
 };
 
 template <int DIM>
@@ -697,7 +698,7 @@ cudaError_t launch_rule_chunks(const RuleChunkParams& c, int64_t slots, int n_lo
         return made;
     }
     const DeltaChainParams chain{c.scratch, c.in.state, c.in.first_rows, c.in.counts, c.in.slots, c.in.o_raw, c.in.n_heads,
-                                 DIM, c.pass};
+                                 DIM, c.pass, c.status};
     return launch_delta_chain<DIM / 16, true>(chain, n_long, stream);
 }
 
@@ -797,14 +798,15 @@ __global__ void delta_rule_finish_kernel(const float* __restrict__ o_raw, const 
 // cover all n_tokens rows. o_raw: fp32 scratch [n_tokens, heads * dim] (walks and chunks). out [T, heads * dim]
 // in the engine's dtype. What the entries need (DeltaStep; what pl_delta_rule_forms says goes by entry): singles, walk_longest, n_long,
 // n_chunks, longest_chunks; n_long 0: the walk takes every portion longer than the step form's. scratch:
-// pl_delta_rule_chunk_floats floats on 16 bytes for the chunks.
+// pl_delta_rule_chunk_floats floats on 16 bytes for the chunks. status: bit 8 where a wait of the chunks' chain gave up (may be
+// nullptr).
 PL_API int pl_delta_rule(const void* r, const void* k, const void* v, const void* g, const void* a_pre,
                          int64_t row_stride, const void* w_pre, int64_t w_row_stride, const float* w0,
                          const float* a0, const float* norm, float* state, const int32_t* first_rows,
                          const int32_t* counts, const int32_t* slots, float* o_raw, float* scratch, void* out,
                          int64_t out_row_stride, int n_tokens, int n_entries, int singles, int walk_longest, int n_long,
                          int n_chunks, int longest_chunks, int n_heads, int dim, float decay_scale, float unit_eps,
-                         float eps, int dtype, cudaStream_t stream) {
+                         float eps, int dtype, int32_t* status, cudaStream_t stream) {
     PL_REQUIRE(n_entries >= 0 && n_tokens >= 0 && n_heads > 0 && dim > 0,
                "delta_rule: bad sizes tokens=%d entries=%d heads=%d dim=%d", n_tokens, n_entries, n_heads, dim);
     PL_REQUIRE(n_heads <= 65535 && dim <= 32 * kRowsPerLane, "delta_rule: %d heads of size %d are too many or too "
@@ -859,7 +861,7 @@ PL_API int pl_delta_rule(const void* r, const void* k, const void* v, const void
         PL_REQUIRE(forms.chunk_least < INT_MAX, "delta_rule: dim=%d does not go in chunks", dim);
         PL_REQUIRE(scratch != nullptr && aligned(scratch), "delta_rule: the scratch must start on 16 bytes");
         const int window = delta_window(step, n_heads, DeltaChunkLayout(dim, dim, true).floats);
-        RuleChunkParams c{p, {n_entries, forms.chunk_least, window, 0}, scratch};
+        RuleChunkParams c{p, {n_entries, forms.chunk_least, window, 0}, scratch, status};
         const int64_t n_slots = delta_chunk_slots(step, window);
         cudaError_t made = cudaSuccess;
         for (; c.pass.pass < delta_passes(step, window) && made == cudaSuccess; ++c.pass.pass) {

@@ -692,6 +692,7 @@ struct GatedChunkParams {
     GatedDeltaParams in;
     DeltaPass pass;
     float* scratch;
+    int32_t* status;
 };
 
 template <int DIM>
@@ -927,7 +928,7 @@ cudaError_t launch_gated_chunks(const GatedChunkParams& c, int64_t slots, int n_
         return made;
     }
     const DeltaChainParams chain{c.scratch, c.in.state, c.in.first_rows, c.in.counts, c.in.slots, c.in.o_raw, c.in.n_heads,
-                                 c.in.vdim, c.pass};
+                                 c.in.vdim, c.pass, c.status};
     return launch_delta_chain<DIM / 16, false>(chain, n_long, stream);
 }
 
@@ -1039,7 +1040,7 @@ __global__ void gated_delta_finish_kernel(const float* __restrict__ o_raw, const
 // counts, slots int32 [entries]; o_raw fp32 [T, n_heads * vdim] scratch (walks and chunks); out [T, n_heads * vdim].
 // What the entries need (DeltaStep; what pl_gated_delta_forms says goes by entry): singles, walk_longest, n_long, n_chunks,
 // longest_chunks; n_long 0: the walk takes every portion longer than the step form's. scratch: pl_gated_delta_chunk_floats floats
-// on 16 bytes for the chunks.
+// on 16 bytes for the chunks. status: bit 8 where a wait of the chunks' chain gave up (may be nullptr).
 PL_API int pl_gated_delta(const void* q, const void* k, const void* v, int64_t qkv_stride, const void* b_pre,
                           int64_t b_stride, const void* a_pre, int64_t a_stride, const void* gate_pre,
                           int64_t gate_stride, const float* a_log, const float* dt_bias, const float* norm,
@@ -1047,7 +1048,7 @@ PL_API int pl_gated_delta(const void* q, const void* k, const void* v, int64_t q
                           float* o_raw, float* scratch, void* out, int64_t out_stride, int n_tokens, int n_entries,
                           int singles, int walk_longest, int n_long, int n_chunks, int longest_chunks, int n_heads,
                           int qk_heads, int dim, int vdim, float unit_eps, float q_scale, float eps, int dtype,
-                          cudaStream_t stream) {
+                          int32_t* status, cudaStream_t stream) {
     PL_REQUIRE(n_tokens >= 0 && n_entries >= 0 && n_heads > 0 && qk_heads > 0 && dim > 0 && vdim > 0,
                "gated_delta: bad sizes tokens=%d entries=%d heads=%d qk_heads=%d dim=%d vdim=%d", n_tokens, n_entries,
                n_heads, qk_heads, dim, vdim);
@@ -1114,7 +1115,7 @@ PL_API int pl_gated_delta(const void* q, const void* k, const void* v, int64_t q
         PL_REQUIRE(scratch != nullptr && (reinterpret_cast<uintptr_t>(scratch) & 15) == 0,
                    "gated_delta: the scratch must start on 16 bytes");
         const int window = delta_window(step, n_heads, DeltaChunkLayout(dim, vdim, false).floats);
-        GatedChunkParams c{p, {n_entries, forms.chunk_least, window, 0}, scratch};
+        GatedChunkParams c{p, {n_entries, forms.chunk_least, window, 0}, scratch, status};
         const int64_t n_slots = delta_chunk_slots(step, window);
         cudaError_t made = cudaSuccess;
         for (; c.pass.pass < delta_passes(step, window) && made == cudaSuccess; ++c.pass.pass) {

@@ -25,7 +25,7 @@ _PTR = ctypes.c_void_p
 _lib = None
 _lock = threading.Lock()
 
-ABI_VERSION = 35
+ABI_VERSION = 36
 
 DTYPE_CODE = {torch.float32: 0, torch.bfloat16: 1}
 
@@ -42,7 +42,7 @@ _SIGNATURES = {
     "pl_short_conv": [_PTR, _PTR, _PTR, _PTR, _PTR, _PTR, _I32, _I32, _I32, _I32, _PTR],
     "pl_short_conv_state": [_PTR, _PTR, _PTR, _PTR, _I32, _I32, _I32, _I32, _PTR],
     "pl_delta_rule": [_PTR, _PTR, _PTR, _PTR, _PTR, _I64, _PTR, _I64, _PTR, _PTR, _PTR, _PTR, _PTR, _PTR, _PTR, _PTR,
-                      _PTR, _PTR, _I64, _I32, _I32, _I32, _I32, _I32, _I32, _I32, _I32, _I32, _F32, _F32, _F32, _I32, _PTR],
+                      _PTR, _PTR, _I64, _I32, _I32, _I32, _I32, _I32, _I32, _I32, _I32, _I32, _F32, _F32, _F32, _I32, _PTR, _PTR],
     "pl_norm_write_paged": [_PTR, _I64, _PTR, _F32, _PTR, _PTR, _PTR, _I32, _PTR, _I64, _I32, _I32, _I32, _I32, _I32,
                             _PTR, _PTR],
     "pl_take_tokens": [_PTR, _PTR, _PTR, _I32, _I32, _PTR, _PTR],
@@ -105,7 +105,7 @@ _SIGNATURES = {
     "pl_short_conv_state_strided": [_PTR, _I64, _PTR, _PTR, _PTR, _I32, _I32, _I32, _I32, _PTR],
     "pl_gated_delta": [_PTR, _PTR, _PTR, _I64, _PTR, _I64, _PTR, _I64, _PTR, _I64, _PTR, _PTR, _PTR, _PTR, _PTR, _PTR,
                        _PTR, _PTR, _PTR, _PTR, _I64, _I32, _I32, _I32, _I32, _I32, _I32, _I32, _I32, _I32, _I32, _I32, _F32, _F32,
-                       _F32, _I32, _PTR],
+                       _F32, _I32, _PTR, _PTR],
     "pl_moe_route": [_PTR, _I64, _PTR, _PTR, _PTR, _PTR, _PTR, _I32, _I32, _I32, _I32, _I32, _I32, _I32, _I32, _I32, _PTR,
                      _I32, _PTR],
     "pl_moe_up": [_PTR, _I64, _PTR, _PTR, _PTR, _I32, _I32, _I32, _I32, _I32, _I32, _I32, _PTR],
@@ -502,11 +502,12 @@ def _delta_kernels(needs: tuple[int, int, int, int, int], passes: int) -> int:
 def delta_rule(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tensor, a_pre: torch.Tensor,
                w_pre: torch.Tensor, w0: torch.Tensor, a0: torch.Tensor, norm: torch.Tensor, state: torch.Tensor,
                first_rows: torch.Tensor, counts: torch.Tensor, slots: torch.Tensor, out: torch.Tensor, n_heads: int,
-               dim: int, decay_scale: float, unit_eps: float, eps: float, lens: list[int] | None = None) -> None:
+               dim: int, decay_scale: float, unit_eps: float, eps: float, lens: list[int] | None = None,
+               status: torch.Tensor | None = None) -> None:
     """The generalized delta rule over each entry's rows in order (see csrc/delta_rule.cu). r, k, v,
     g, a_pre [T, heads * dim] share one row stride; state fp32 [slots, heads, dim, dim] is updated. lens: what counts
     holds, where the host knows it (fewer launches, less scratch)."""
-    _dev(r, k, v, g, a_pre, w_pre, w0, a0, norm, state, first_rows, counts, slots, out)
+    _dev(r, k, v, g, a_pre, w_pre, w0, a0, norm, state, first_rows, counts, slots, out, status)
     width = n_heads * dim
     stride = r.stride(0)
     for t in (r, k, v, g, a_pre):
@@ -528,7 +529,7 @@ def delta_rule(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tenso
     _call("pl_delta_rule", _p(r), _p(k), _p(v), _p(g), _p(a_pre), stride, _p(w_pre), w_pre.stride(0), _p(w0), _p(a0),
           _p(norm), _p(state), _p(first_rows), _p(counts), _p(slots), _p(o_raw), _p(o_raw) + 4 * tokens * width if floats else None,
           _p(out), out.stride(0), tokens, n_entries, *needs, n_heads, dim, float(decay_scale), float(unit_eps), float(eps),
-          _code(out.dtype), _stream())
+          _code(out.dtype), _p(status), _stream())
     global _launches
     _launches += _delta_kernels(needs, passes.value) - 1
 
@@ -644,11 +645,11 @@ def gated_delta(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b_pre: torch.
                 gate_pre: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor, norm: torch.Tensor,
                 state: torch.Tensor, first_rows: torch.Tensor, counts: torch.Tensor, slots: torch.Tensor,
                 out: torch.Tensor, n_heads: int, qk_heads: int, dim: int, vdim: int, unit_eps: float, q_scale: float,
-                eps: float, lens: list[int] | None = None) -> None:
+                eps: float, lens: list[int] | None = None, status: torch.Tensor | None = None) -> None:
     """The gated delta rule with a decay per key channel over each entry's rows in order (see
     csrc/gated_delta.cu). q, k [T, qk_heads * dim] and v [T, heads * vdim] share one row stride; state fp32
     [slots, heads, dim, vdim] is updated. lens: what counts holds, where the host knows it (fewer launches, less scratch)."""
-    _dev(q, k, v, b_pre, a_pre, gate_pre, a_log, dt_bias, norm, state, first_rows, counts, slots, out)
+    _dev(q, k, v, b_pre, a_pre, gate_pre, a_log, dt_bias, norm, state, first_rows, counts, slots, out, status)
     tokens = q.shape[0]
     assert q.shape[1] == k.shape[1] == qk_heads * dim and v.shape[1] == n_heads * vdim
     assert q.stride(0) == k.stride(0) == v.stride(0) and q.stride(1) == k.stride(1) == v.stride(1) == 1
@@ -674,7 +675,8 @@ def gated_delta(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b_pre: torch.
     _call("pl_gated_delta", _p(q), _p(k), _p(v), stride(q), _p(b_pre), stride(b_pre), _p(a_pre), stride(a_pre),
           _p(gate_pre), stride(gate_pre), _p(a_log), _p(dt_bias), _p(norm), _p(state), _p(first_rows), _p(counts),
           _p(slots), _p(o_raw), _p(o_raw) + 4 * tokens * n_heads * vdim if floats else None, _p(out), stride(out), tokens, n_entries,
-          *needs, n_heads, qk_heads, dim, vdim, float(unit_eps), float(q_scale), float(eps), _code(out.dtype), _stream())
+          *needs, n_heads, qk_heads, dim, vdim, float(unit_eps), float(q_scale), float(eps), _code(out.dtype),
+          _p(status), _stream())
     global _launches
     _launches += _delta_kernels(needs, passes.value) - 1
 

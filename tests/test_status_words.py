@@ -1,0 +1,71 @@
+"""Kernels whose waits are bounded get the step's status word from the parts that launch them (no GPU: the launches are
+recorded instead of made)."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from pulsarlm_b200 import models as _models  # noqa: F401  (registers the parts)
+from pulsarlm_b200.cache.manager import StateBinding
+from pulsarlm_b200.kernels import ops
+from pulsarlm_b200.models.model import HostStep, StepBatch
+from pulsarlm_b200.parts.registry import BuildContext, build_part, part_class
+from pulsarlm_b200.parts.spec import PartSpec
+
+BF = torch.bfloat16
+
+
+@pytest.fixture
+def launches(monkeypatch):
+    """(name, arguments) of every entry point that is called; its last argument is the stream, the one before it the status word."""
+    made = []
+    monkeypatch.setattr(ops, "_call", lambda name, *args: made.append((name, args)))
+    monkeypatch.setattr(ops, "_dev", lambda *tensors: None)
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    return made
+
+
+def _part(kind, name, params, names):
+    """With weights of zeros, ranks that a checkpoint decides being 16."""
+    spec = PartSpec(name, params, names if isinstance(names, dict) else {n: n for n in names})
+    part = build_part(kind, spec, BuildContext(BF, torch.device("cpu")))
+    needs = part_class(kind, name).tensor_needs(spec)
+    part.load({n: torch.zeros([d if d >= 0 else 16 for d in need.shape], dtype=BF) for n, need in needs.items()})
+    return part
+
+
+def _batch(part, lengths):
+    n, total = len(lengths), sum(lengths)
+    first = [sum(lengths[:i]) for i in range(n)]
+    singles = sum(1 for v in lengths if v == 1)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32)  # noqa: E731
+    step = HostStep(n, total, singles, lengths, lengths, first, 16)
+    plans = {}
+    if part.plan_key() is not None:
+        plans[part.plan_key()] = {k: torch.from_numpy(v) for k, v in part.plan_step(step).items()}
+    return StepBatch(ints([0] * total), ints(range(total)), ints([i for i, v in enumerate(lengths) for _ in range(v)]), {},
+                     ints(range(n)), None, ints([0]), total, n, singles, lengths, lengths, plans=plans)
+
+
+def _check(launches, name, batch, count):
+    found = [args for called, args in launches if called == name]
+    assert len(found) == count and all(args[-2] == batch.status.data_ptr() for args in found)
+
+
+@pytest.mark.parametrize("lengths", [[40], [1, 1, 20]])
+def test_delta_rules_in_chunks(launches, lengths):
+    heads, dim, hidden, total = 2, 64, 128, sum(lengths)
+    states = torch.zeros((len(lengths), heads, dim, dim))
+    sizes = {"hidden_size": hidden, "n_heads": heads, "head_dim": dim, "eps": 1e-6}
+    channel = _part("mixer", "channel_delta", {**sizes, "value_dim": dim, "taps": 4},
+                    ("q", "k", "v", "b", "a1", "a2", "g1", "g2", "q_conv", "k_conv", "v_conv", "o", "A_log", "dt_bias", "norm"))
+    channel.bind_cache(StateBinding(states))
+    channel.state_holders()[0].bind_cache(StateBinding(torch.zeros((len(lengths), 3, heads * 3 * dim), dtype=BF)))
+    general = _part("mixer", "general_delta", sizes,
+                    ("r", "k", "v", "g", "a", "w1", "w2", "o", "a_bias", "w0", "norm"))
+    general.bind_cache(StateBinding(states))
+    for part, name in ((channel, "pl_gated_delta"), (general, "pl_delta_rule")):
+        batch = _batch(part, lengths)
+        part.forward(torch.zeros((total, hidden), dtype=BF), batch)
+        _check(launches, name, batch, 1)
