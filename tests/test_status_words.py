@@ -69,3 +69,14 @@ def test_delta_rules_in_chunks(launches, lengths):
         batch = _batch(part, lengths)
         part.forward(torch.zeros((total, hidden), dtype=BF), batch)
         _check(launches, name, batch, 1)
+
+
+@pytest.mark.parametrize("expert,weigh_input", [("gated_silu", False), ("relu2", False), ("clamped", True)])
+def test_grouped_products_of_experts(launches, expert, weigh_input):
+    params = {"hidden_size": 64, "expert_size": 64, "n_experts": 4, "top": 2, "shared_size": None, "expert": expert,
+              "weigh_input": weigh_input, "expert_limit": 7.0}
+    part = _part("feed_forward", "moe", params, {"router": "router", "expert_gate": "e{e}.gate", "expert_up": "e{e}.up",
+                                                 "expert_down": "e{e}.down"})
+    batch = _batch(part, [64])
+    part.forward(torch.zeros((64, 64), dtype=BF), batch)
+    _check(launches, "pl_gemm_bf16_grouped", batch, 2)
