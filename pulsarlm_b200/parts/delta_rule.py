@@ -8,7 +8,7 @@ import numpy as np
 import torch
 
 from ..kernels import ops
-from .linear import activated_linear, linear
+from .linear import activated_linear, linear, status_of
 from .registry import BuildContext, Part, register_part
 from .spec import PartSpec, StateNeed, TensorNeed
 
@@ -112,5 +112,5 @@ class GeneralDelta(Part):
         out = torch.empty((tokens, width), dtype=h.dtype, device=h.device)
         ops.delta_rule(r, k, v, g, a, w_pre, self.w0, self.a0, self.norm, self.binding.states, plan["first"],
                        plan["count"], batch.slots, out, self.n_heads, self.head_dim, self.decay_scale, self.unit_eps,
-                       self.eps, batch.host_query_lens, batch.status)
+                       self.eps, batch.host_query_lens, status_of(batch))
         return linear(out, self.o)

@@ -7,7 +7,7 @@ import torch
 
 from ..kernels import ops
 from .delta_rule import SEQUENCE_ROWS_KEY, sequence_rows_plan
-from .linear import linear
+from .linear import linear, status_of
 from .registry import BuildContext, Part, register_part
 from .spec import PartSpec, StateNeed, TensorNeed
 
@@ -134,7 +134,7 @@ class ChannelDelta(Part):
         ops.gated_delta(filtered[:, :qk * hd], filtered[:, qk * hd:2 * qk * hd], filtered[:, 2 * qk * hd:], b_pre,
                         a_pre, gate_pre, self.a_log, self.dt_bias, self.norm, self.states, plan["first"],
                         plan["count"], batch.slots, out, nh, qk, hd, vd, self.unit_eps, hd ** -0.5, self.eps,
-                        batch.host_query_lens, batch.status)
+                        batch.host_query_lens, status_of(batch))
         return linear(out, self.o)
 
 

@@ -52,6 +52,11 @@ if GEMM_ROUTE not in ("library", "tcgen05", "mixed"):
 _PAIRS: dict[torch.device, int] = {}
 
 
+def status_of(batch) -> torch.Tensor | None:
+    """The status word of a step's batch; None where a part runs without one (its kernels then have nowhere to report to)."""
+    return getattr(batch, "status", None)
+
+
 def own_kernel_for(tokens: int, n: int, device: torch.device, k: int = 0) -> str | None:
     """Which of the package's own tcgen05 kernels the route gives a [tokens, n] product
     over k to ("skinny", "pair"), or None for the library. (A gate/up projection, whose activation the pair kernel would form itself,

@@ -9,7 +9,7 @@ import torch
 
 from ..kernels import ops
 from .branches import run_branches
-from .linear import activated_linear, gated_feed_forward, linear
+from .linear import activated_linear, gated_feed_forward, linear, status_of
 from .registry import BuildContext, Part, register_part
 from .spec import PartSpec, TensorNeed
 
@@ -185,13 +185,13 @@ class RoutedExperts(Part):
         if self._own_products():
             if in_weights is None:
                 unit = ("silu" if self.limit is None else "clamped") if self.gated else self.plain_act
-                ops.gemm_bf16_grouped(x, self.gate_up, ends, act, unit, self.limit or 0.0, batch.status)
+                ops.gemm_bf16_grouped(x, self.gate_up, ends, act, unit, self.limit or 0.0, status_of(batch))
             else:
                 gate_up = torch.empty((x.shape[0], 2 * self.ff), dtype=h.dtype, device=h.device)
-                ops.gemm_bf16_grouped(x, self.gate_up, ends, gate_up, status=batch.status)
+                ops.gemm_bf16_grouped(x, self.gate_up, ends, gate_up, status=status_of(batch))
                 ops.gated_act(gate_up, act, "clamped", self.limit, in_weights, pair_of_row)
             y = torch.empty((x.shape[0], self.hidden), dtype=h.dtype, device=h.device)
-            ops.gemm_bf16_grouped(act, self.down, ends, y, status=batch.status)
+            ops.gemm_bf16_grouped(act, self.down, ends, y, status=status_of(batch))
             ops.moe_combine(y, row_of_pair, weights, shared, out, shared_weights)
             return out
         # More experts than that kernel counts: the library's (operands [rows, K] and [E, K, N], the experts' ends as offsets).

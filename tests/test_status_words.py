@@ -80,3 +80,5 @@ def test_grouped_products_of_experts(launches, expert, weigh_input):
     batch = _batch(part, [64])
     part.forward(torch.zeros((64, 64), dtype=BF), batch)
     _check(launches, "pl_gemm_bf16_grouped", batch, 2)
+    part.forward(torch.zeros((64, 64), dtype=BF), None)  # (no step, nowhere to report to)
+    assert [args[-2] for called, args in launches if called == "pl_gemm_bf16_grouped"][2:] == [None, None]
