@@ -8,6 +8,7 @@ through `bind_caches()`.
 from __future__ import annotations
 
 import dataclasses
+import inspect
 
 import torch
 
@@ -119,6 +120,9 @@ class Model:
         self.final_norm = build_part("norm", spec.final_norm, self.ctx)
         self.head = build_part("head", spec.head, self.ctx)
         self.join = build_part("join", spec.join, self.ctx) if spec.join is not None else None
+        # (a head or join of a program's own need not take the step's status word)
+        self._reports = {part: "status" in inspect.signature(part.forward).parameters
+                         for part in (self.head, self.join) if part is not None}
         self.loaded = False
         # The cache units, in the order the cache manager hears of them: one per layer, or
         # (spec.cache_per_run) one per entry of the order. `_unit_layer[u]` is the layer of unit u.
@@ -273,6 +277,9 @@ class Model:
         return x, delta
 
     # ------------------------------------------------------------------ forward
+    def _status_for(self, part, batch: StepBatch) -> dict:
+        return {"status": batch.status} if self._reports.get(part) else {}
+
     def forward(self, batch: StepBatch) -> torch.Tensor | None:
         """Runs the batch's tokens through every layer in order; returns fp32 logits
         [R, vocab] at `batch.want_rows`, or None when none are wanted."""
@@ -289,9 +296,9 @@ class Model:
             if run in self._rejoin:
                 x, delta = self._rejoin_stream(x, delta, entered)
             if run in self._join_runs:
-                x, delta = self.join.forward(x, delta, entered), None
+                x, delta = self.join.forward(x, delta, entered, **self._status_for(self.join, batch)), None
             x, delta = block.forward(x, delta, batch)
         if batch.want_rows is None or batch.want_rows.numel() == 0:
             return None
         h = self.final_norm.forward(x, delta, rows=batch.want_rows)
-        return self.head.forward(h)
+        return self.head.forward(h, **self._status_for(self.head, batch))

@@ -11,7 +11,7 @@ import torch
 
 from ..kernels import ops
 from ..kernels.device import describe as describe_device
-from .linear import linear
+from .linear import linear, status_of
 from .registry import BuildContext, Part, build_part, register_part
 from .spec import KVCacheNeed, PartSpec, TensorNeed
 
@@ -301,7 +301,7 @@ class Attention(Part):
         nh, nkv, hd = self.n_heads, self.n_kv, self.head_dim
         cache = self.cache
         table = batch.tables[cache.group]
-        qkv = linear(h, self.qkv)
+        qkv = linear(h, self.qkv, status=status_of(batch))
         q = qkv[:, : nh * hd].view(tokens, nh, hd)
         inv_freq, rotary = self.position.table()
         if self._folds_rope(tokens, batch, inv_freq, rotary):
@@ -311,7 +311,7 @@ class Attention(Part):
                     qkv[:, (nh + nkv) * hd :].view(tokens, nkv, hd), inv_freq, rotary)
             out = torch.empty((tokens, nh, hd), dtype=h.dtype, device=h.device)
             self.attend(q, out, table, batch, rope)
-            return linear(out.view(tokens, nh * hd), self.o)
+            return linear(out.view(tokens, nh * hd), self.o, status=status_of(batch))
         if self.cache_from is None:
             k = qkv[:, nh * hd : (nh + nkv) * hd].view(tokens, nkv, hd)
             v = qkv[:, (nh + nkv) * hd :].view(tokens, nkv, hd)
@@ -322,7 +322,7 @@ class Attention(Part):
                               rotary, batch.status, self.q_norm, None, self.qk_norm_eps)
         out = torch.empty((tokens, nh, hd), dtype=h.dtype, device=h.device)
         self.attend(q, out, table, batch)
-        return linear(out.view(tokens, nh * hd), self.o)
+        return linear(out.view(tokens, nh * hd), self.o, status=status_of(batch))
 
     def _folds_rope(self, tokens: int, batch, inv_freq, rotary: int) -> bool:
         """Whether this step's position encoding and cache write go into the decode

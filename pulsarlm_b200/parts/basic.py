@@ -12,7 +12,7 @@ import math
 import torch
 
 from ..kernels import ops
-from .linear import activated_linear, gated_feed_forward, linear
+from .linear import activated_linear, gated_feed_forward, linear, status_of
 from .registry import BuildContext, Part, register_part
 from .spec import PartSpec, StateNeed, TensorNeed
 
@@ -452,8 +452,8 @@ class Head(Part):
             raise ValueError(f"head: cannot tie to a table of shape {tuple(table.shape)}")
         self.weight = table
 
-    def forward(self, h: torch.Tensor) -> torch.Tensor:
-        logits = linear(h, self.weight, out_dtype=torch.float32)
+    def forward(self, h: torch.Tensor, status: torch.Tensor | None = None) -> torch.Tensor:
+        logits = linear(h, self.weight, out_dtype=torch.float32, status=status)
         if self.softcap:
             ops.capped_scale(logits, self.scale, self.softcap)
         elif self.scale != 1.0:
@@ -495,7 +495,7 @@ class GatedMLP(Part):
         self.down = tensors[t["down"]].contiguous()
 
     def forward(self, h: torch.Tensor, batch) -> torch.Tensor:
-        return gated_feed_forward(h, self.gate_up, self.down, self.activation, self.limit)
+        return gated_feed_forward(h, self.gate_up, self.down, self.activation, self.limit, status_of(batch))
 
 
 @register_part("feed_forward", "mlp")
@@ -539,7 +539,8 @@ class PlainMLP(Part):
 
     def forward(self, h: torch.Tensor, batch, bias_taken: bool = False) -> torch.Tensor:
         """bias_taken: the caller adds `down_bias` itself (inside the kernel that reads the output)."""
-        y = activated_linear(linear(h, self.up), self.up_bias, self.activation, self.down)
+        status = status_of(batch)
+        y = activated_linear(linear(h, self.up, status=status), self.up_bias, self.activation, self.down, status)
         if self.down_bias is not None and not bias_taken:
             ops.bias_act(y, self.down_bias, y, "none")
         return y

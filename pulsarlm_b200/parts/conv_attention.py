@@ -8,7 +8,7 @@ import torch
 from ..kernels import ops
 from .attention import Attention
 from .gated_delta import FilterState
-from .linear import linear
+from .linear import linear, status_of
 from .registry import BuildContext, register_part
 from .spec import KVCacheNeed, PartSpec, TensorNeed
 
@@ -114,7 +114,7 @@ class ConvAttention(Attention):
         nh, nkv, hd, c = self.n_heads, self.n_kv, self.head_dim, self.channels
         cache = self.cache
         table = batch.tables[cache.group]
-        proj = linear(h, self.qkv)                             # [T, c (+ nh * hd)]
+        proj = linear(h, self.qkv, status=status_of(batch))   # [T, c (+ nh * hd)]
         q = torch.empty((tokens, nh, hd), dtype=h.dtype, device=h.device)
         inv_freq, rotary = self.position.table()
         states = self.filter_state.states(h)
@@ -131,4 +131,4 @@ class ConvAttention(Attention):
         flat = out.view(tokens, nh * hd)
         if self.gate_rows:
             ops.sigmoid_gate(flat, proj[:, c:])
-        return linear(flat, self.o)
+        return linear(flat, self.o, status=status_of(batch))

@@ -105,12 +105,13 @@ class GeneralDelta(Part):
     def forward(self, h: torch.Tensor, batch) -> torch.Tensor:
         tokens = h.shape[0]
         width = self.n_heads * self.head_dim
-        proj = linear(h, self.stacked)                              # [T, 5 * width + inner]
+        proj = linear(h, self.stacked, status=status_of(batch))   # [T, 5 * width + inner]
         r, k, v, g, a = (proj[:, i * width:(i + 1) * width] for i in range(5))
-        w_pre = activated_linear(proj[:, 5 * width:], None, "tanh", self.w2)   # the decay's inner activation
+        # (the decay's inner activation)
+        w_pre = activated_linear(proj[:, 5 * width:], None, "tanh", self.w2, status=status_of(batch))
         plan = batch.plans[SEQUENCE_ROWS_KEY]
         out = torch.empty((tokens, width), dtype=h.dtype, device=h.device)
         ops.delta_rule(r, k, v, g, a, w_pre, self.w0, self.a0, self.norm, self.binding.states, plan["first"],
                        plan["count"], batch.slots, out, self.n_heads, self.head_dim, self.decay_scale, self.unit_eps,
                        self.eps, batch.host_query_lens, status_of(batch))
-        return linear(out, self.o)
+        return linear(out, self.o, status=status_of(batch))

@@ -9,7 +9,7 @@ import torch
 
 from ..kernels import ops
 from .attention import Attention
-from .linear import linear
+from .linear import linear, status_of
 from .registry import BuildContext, register_part
 from .spec import KVCacheNeed, PartSpec, TensorNeed
 
@@ -89,7 +89,7 @@ class DiffAttention(Attention):
         nh, nkv, hd, vd = self.true_heads, self.n_kv, self.map_dim, self.value_dim
         cache = self.cache
         table = batch.tables[cache.group]
-        qkv = linear(h, self.qkv)
+        qkv = linear(h, self.qkv, status=status_of(batch))
         q_end, k_end = nh * MAPS * hd, (nh + nkv) * MAPS * hd
         q = torch.empty((tokens, MAPS * nh, self.padded), dtype=h.dtype, device=h.device)
         inv_freq, rotary = self.position.table()
@@ -100,7 +100,7 @@ class DiffAttention(Attention):
         self.attend(q, maps, table, batch)
         out = torch.empty((tokens, nh * vd), dtype=h.dtype, device=h.device)
         ops.diff_combine(maps, out, nh, vd, self.lam, self.eps, 1.0 - self.diff)
-        return linear(out, self.o)
+        return linear(out, self.o, status=status_of(batch))
 
 
 def padded_row(map_dim: int, value_dim: int) -> int:

@@ -11,7 +11,7 @@ from ..kernels import ops
 from .attention import Attention
 from .delta_rule import sequence_rows_plan
 from .gated_delta import FilterState
-from .linear import linear
+from .linear import linear, status_of
 from .registry import BuildContext, register_part
 from .spec import KVCacheNeed, PartSpec, TensorNeed
 
@@ -177,11 +177,11 @@ class FilteredAttention(Attention):
             ops.filter_state(proj, row_stride, plan["first"], plan["count"], batch.slots, states)
         out = torch.empty((tokens, self.n_heads, self.row), dtype=proj.dtype, device=proj.device)
         self.attend(q, out, table, batch)
-        y = linear(out.view(tokens, self.n_heads * self.row), self.o)
+        y = linear(out.view(tokens, self.n_heads * self.row), self.o, status=status_of(batch))
         if self.output_bias is not None and not bias_taken:
             ops.bias_act(y, self.output_bias.to(y.dtype), y, "none")
         return y
 
     def forward(self, h: torch.Tensor, batch) -> torch.Tensor:
-        proj = linear(h, self.in_weight)
+        proj = linear(h, self.in_weight, status=status_of(batch))
         return self.forward_columns(proj, proj.stride(0), h, batch, False)

@@ -115,7 +115,7 @@ class ChannelDelta(Part):
     def forward(self, h: torch.Tensor, batch) -> torch.Tensor:
         tokens = h.shape[0]
         nh, qk, hd, vd, c = self.n_heads, self.qk_heads, self.dim, self.vdim, self.channels
-        proj = linear(h, self.stacked)                       # [T, c + nh + ra + rg]
+        proj = linear(h, self.stacked, status=status_of(batch))   # [T, c + nh + ra + rg]
         filtered = torch.empty((tokens, c), dtype=h.dtype, device=h.device)
         conv_states = self.filter_state.states(h)
         # (a step of single tokens: the convolution and its state's update in one launch)
@@ -127,15 +127,15 @@ class ChannelDelta(Part):
             if self.taps > 1:
                 ops.short_conv_state_strided(proj[:, :c], batch.entry, batch.slots, conv_states)
         b_pre = proj[:, c:c + nh]
-        a_pre = linear(proj[:, c + nh:c + nh + self.rank_a], self.a2)
-        gate_pre = linear(proj[:, c + nh + self.rank_a:], self.g2)
+        a_pre = linear(proj[:, c + nh:c + nh + self.rank_a], self.a2, status=status_of(batch))
+        gate_pre = linear(proj[:, c + nh + self.rank_a:], self.g2, status=status_of(batch))
         plan = batch.plans[SEQUENCE_ROWS_KEY]
         out = torch.empty((tokens, nh * vd), dtype=h.dtype, device=h.device)
         ops.gated_delta(filtered[:, :qk * hd], filtered[:, qk * hd:2 * qk * hd], filtered[:, 2 * qk * hd:], b_pre,
                         a_pre, gate_pre, self.a_log, self.dt_bias, self.norm, self.states, plan["first"],
                         plan["count"], batch.slots, out, nh, qk, hd, vd, self.unit_eps, hd ** -0.5, self.eps,
                         batch.host_query_lens, status_of(batch))
-        return linear(out, self.o)
+        return linear(out, self.o, status=status_of(batch))
 
 
 class FilterState:

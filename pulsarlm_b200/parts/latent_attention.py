@@ -9,7 +9,7 @@ import torch
 
 from ..kernels import ops
 from .attention import KVBinding, decode_splits, prefill_splits
-from .linear import linear
+from .linear import linear, status_of
 from .registry import BuildContext, Part, build_part, register_part
 from .spec import KVCacheNeed, PartSpec, TensorNeed
 
@@ -149,7 +149,7 @@ class LatentAttention(Part):
         nh, hd, vd, rank, rot, row = self.n_heads, self.head_dim, self.value_dim, self.rank, self.rope_dim, self.row
         cache = self.cache
         table = batch.tables[cache.group]
-        proj = linear(h, self.stacked)
+        proj = linear(h, self.stacked, status=status_of(batch))
         stored = False
         if self.query_rank:
             # the queries' latent, normed into a dense operand of its own product
@@ -160,7 +160,7 @@ class LatentAttention(Part):
             ops.latent_norms(proj[:, :at], self.query_norm, c_q, z, self.latent_norm, self.eps, batch.pos, batch.entry, table,
                              cache.k_pool if z is not None else None, cache.page_size, batch.status)
             stored = z is not None
-            q = linear(c_q, self.query_up).view(tokens, nh, hd + rot)
+            q = linear(c_q, self.query_up, status=status_of(batch)).view(tokens, nh, hd + rot)
         else:
             q = proj[:, : nh * (hd + rot)].view(tokens, nh, hd + rot)
             at = nh * (hd + rot)
@@ -186,7 +186,7 @@ class LatentAttention(Part):
         flat = out.view(tokens, nh * vd)
         if self.gate_kind == "element":
             ops.sigmoid_gate(flat, gate)
-        return linear(flat, self.o)
+        return linear(flat, self.o, status=status_of(batch))
 
     # ------------------------------------------------------------------ planning a step
     def _kernels(self) -> tuple[bool, bool]:

@@ -80,8 +80,10 @@ def own_kernel_for(tokens: int, n: int, device: torch.device, k: int = 0) -> str
     return "pair" if tiles >= MIXED_MIN_TILES_PER_PAIR * _PAIRS[device] else None
 
 
-def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None = None) -> torch.Tensor:
-    """x [T, K] @ weight[N, K]^T -> [T, N] in x's dtype, or fp32 when asked."""
+def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None = None,
+           status: torch.Tensor | None = None) -> torch.Tensor:
+    """x [T, K] @ weight[N, K]^T -> [T, N] in x's dtype, or fp32 when asked. status: where a kernel whose bounded wait gave up
+    says so (status_of; here and below)."""
     if x.dtype != weight.dtype:
         raise ops.KernelError(f"linear: activation dtype {x.dtype} differs from weight dtype {weight.dtype}")
     tokens = x.shape[0]
@@ -97,7 +99,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None 
                 and weight.data_ptr() % 16 == 0 and ops.gemm_bf16_supports(
                 tokens, n, k, x.stride(0) if tokens > 1 else k, weight.stride(0) if n > 1 else k):
             out = torch.empty((tokens, n), dtype=out_dtype or torch.bfloat16, device=x.device)
-            ops.gemm_bf16(x, weight, out, kernel=kernel)
+            ops.gemm_bf16(x, weight, out, status, kernel=kernel)
             return out
         if out_dtype == torch.float32:
             # bf16 operands, fp32 accumulator written out unrounded.
@@ -106,7 +108,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None 
     raise ops.KernelError(f"linear: unsupported dtype {x.dtype}")
 
 
-def gated_linear(x: torch.Tensor, gate_up: torch.Tensor, limit: float | None = None) -> torch.Tensor:
+def gated_linear(x: torch.Tensor, gate_up: torch.Tensor, limit: float | None = None,
+                 status: torch.Tensor | None = None) -> torch.Tensor:
     """silu(x Wg^T) * (x Wu^T) for gate_up = [Wg; Wu] stacked [2I, K] -> [T, I]; with `limit` the
     clamped unit of the two products (ops.gated_act).
 
@@ -119,12 +122,12 @@ def gated_linear(x: torch.Tensor, gate_up: torch.Tensor, limit: float | None = N
     if (x.dtype == torch.bfloat16 == gate_up.dtype and own_kernel_for(tokens, 2 * inter, x.device, k) == "pair"
             and x.stride(1) == 1 and gate_up.stride(1) == 1
             and ops.gemm_bf16_supports(tokens, inter, k, x.stride(0) if tokens > 1 else k, gate_up.stride(0))):
-        ops.gemm_bf16(x, gate_up, act, kernel="pair", gated=True, limit=limit)
+        ops.gemm_bf16(x, gate_up, act, status, kernel="pair", gated=True, limit=limit)
         return act
     if limit is not None:
-        ops.gated_act(linear(x, gate_up), act, "clamped", limit)
+        ops.gated_act(linear(x, gate_up, status=status), act, "clamped", limit)
     else:
-        ops.swiglu(linear(x, gate_up), act)
+        ops.swiglu(linear(x, gate_up, status=status), act)
     return act
 
 
@@ -132,7 +135,7 @@ GATED_IN = os.environ.get("PULSARLM_B200_GATED_IN", "1") != "0"  # (0: always th
 
 
 def gated_feed_forward(x: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, act: str = "silu",
-                       limit: float = 0.0) -> torch.Tensor:
+                       limit: float = 0.0, status: torch.Tensor | None = None) -> torch.Tensor:
     """(act(x Wg^T) * (x Wu^T)) Wd^T -> [T, H], act "silu", "gelu_tanh" or "clamped" (ops.gated_act, with its
     `limit`). With silu, for a handful
     of tokens in bfloat16 the down projection's skinny kernel forms the gated activation itself as it
@@ -145,8 +148,8 @@ def gated_feed_forward(x: torch.Tensor, gate_up: torch.Tensor, down: torch.Tenso
     inter = gate_up.shape[0] // 2
     if act not in ("silu", "clamped"):
         gated = torch.empty((tokens, inter), dtype=x.dtype, device=x.device)
-        ops.gated_act(linear(x, gate_up), gated, act)
-        return linear(gated, down)
+        ops.gated_act(linear(x, gate_up, status=status), gated, act)
+        return linear(gated, down, status=status)
     cap = limit if act == "clamped" else None
     if (GATED_IN and x.dtype == torch.bfloat16 == gate_up.dtype == down.dtype
             and tokens <= ops.GEMM_GATED_IN_MAX_TOKENS and down.stride(1) == 1 and cap is None
@@ -154,15 +157,16 @@ def gated_feed_forward(x: torch.Tensor, gate_up: torch.Tensor, down: torch.Tenso
             and own_kernel_for(tokens, 2 * inter, x.device, k) != "pair"
             and ops.gemm_bf16_supports(tokens, down.shape[0], inter, 2 * inter, down.stride(0))):
         out = torch.empty((tokens, down.shape[0]), dtype=x.dtype, device=x.device)
-        ops.gemm_bf16_gated_in(linear(x, gate_up), down, out)
+        ops.gemm_bf16_gated_in(linear(x, gate_up, status=status), down, out, status)
         return out
-    return linear(gated_linear(x, gate_up, cap), down)
+    return linear(gated_linear(x, gate_up, cap, status), down, status=status)
 
 
 ACT_IN = os.environ.get("PULSARLM_B200_ACT_IN", "1") != "0"  # (0: always the bias-and-activation kernel)
 
 
-def activated_linear(z: torch.Tensor, bias: torch.Tensor | None, act: str, weight: torch.Tensor) -> torch.Tensor:
+def activated_linear(z: torch.Tensor, bias: torch.Tensor | None, act: str, weight: torch.Tensor,
+                     status: torch.Tensor | None = None) -> torch.Tensor:
     """act(z + bias) W^T -> [T, N] for z [T, K] (a projection's output; its rows may be columns of a
     wider matrix), act "relu2", "tanh" or "gelu" (the exact one, always a kernel of its own: the skinny kernel
     would form it anew in every tile). Else, for a handful of tokens in bfloat16 the skinny kernel forms
@@ -174,8 +178,8 @@ def activated_linear(z: torch.Tensor, bias: torch.Tensor | None, act: str, weigh
             and own_kernel_for(tokens, weight.shape[0], z.device, k) == "skinny"
             and ops.gemm_bf16_supports(tokens, weight.shape[0], k, z.stride(0) if tokens > 1 else k, weight.stride(0))):
         out = torch.empty((tokens, weight.shape[0]), dtype=z.dtype, device=z.device)
-        ops.gemm_bf16_act_in(z, bias, weight, out, act)
+        ops.gemm_bf16_act_in(z, bias, weight, out, act, status)
         return out
     activated = torch.empty((tokens, k), dtype=z.dtype, device=z.device)
     ops.bias_act(z, bias, activated, act)
-    return linear(activated, weight)
+    return linear(activated, weight, status=status)

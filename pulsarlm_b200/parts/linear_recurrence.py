@@ -8,7 +8,7 @@ import torch
 from ..kernels import ops
 from .delta_rule import SEQUENCE_ROWS_KEY, sequence_rows_plan
 from .filtered_attention import stacked_rows
-from .linear import linear
+from .linear import linear, status_of
 from .registry import BuildContext, Part, register_part
 from .spec import PartSpec, StateNeed, TensorNeed
 
@@ -143,7 +143,7 @@ class LinearRecurrence(Part):
         if proj.dtype == torch.bfloat16 and int(batch.n_decode) == tokens:
             ops.linear_step(x, row_stride, self.x_bias, self.conv, self.conv_bias, ring, self.gates, self.ra_bias,
                             self.ri_bias, self.decay, y, self.y_bias, self.states, batch.entry, batch.slots, batch.pos, out)
-            return linear(out, self.o)
+            return linear(out, self.o, status=status_of(batch))
         plan = batch.plans[SEQUENCE_ROWS_KEY]
         u = torch.empty((tokens, self.width), dtype=proj.dtype, device=proj.device)
         ops.ring_conv(x, row_stride, self.x_bias, self.conv, self.conv_bias, ring, plan["first"], batch.entry, batch.slots,
@@ -151,8 +151,8 @@ class LinearRecurrence(Part):
         ops.linear_scan(self._gate_products(u), self.ra_bias, self.ri_bias, self.decay, u, y, self.y_bias, x, row_stride,
                         ring, self.states, plan["first"], plan["count"], batch.slots, batch.pos,
                         max(batch.host_query_lens, default=1), out)
-        return linear(out, self.o)
+        return linear(out, self.o, status=status_of(batch))
 
     def forward(self, h: torch.Tensor, batch) -> torch.Tensor:
-        proj = linear(h, self.in_weight)
+        proj = linear(h, self.in_weight, status=status_of(batch))
         return self.forward_columns(proj, proj.stride(0), h, batch, False)

@@ -8,7 +8,7 @@ import torch
 
 from ..kernels import ops
 from .filtered_attention import stacked_rows
-from .linear import linear
+from .linear import linear, status_of
 from .registry import BuildContext, Part, register_part
 from .spec import PartSpec, StateNeed, TensorNeed
 
@@ -104,7 +104,7 @@ class MatrixMemory(Part):
     def forward(self, h: torch.Tensor, batch) -> torch.Tensor:
         tokens = h.shape[0]
         nh, hd, vd = self.n_heads, self.dim, self.vdim
-        proj = linear(h, self.stacked)
+        proj = linear(h, self.stacked, status=status_of(batch))
         columns = tuple(proj[:, at: at + nh * width] for at, width in zip(self.starts, (hd, hd, vd, vd)))
         plan = batch.plans[self.plan_key()]
         out = torch.empty((tokens, nh * vd), dtype=h.dtype, device=h.device)
@@ -112,13 +112,15 @@ class MatrixMemory(Part):
         single = min(int(batch.n_decode), tokens)
         constants = (self.gate_bias, self.cap, self.norm, self.eps, hd ** -0.5, self.states)
         if (single and not in_steps) or (single < tokens and not in_chunks):
-            ops.matrix_memory_walk(columns, proj.stride(0), linear(h, self.gates, out_dtype=torch.float32), *constants,
+            gates = linear(h, self.gates, out_dtype=torch.float32, status=status_of(batch))
+            ops.matrix_memory_walk(columns, proj.stride(0), gates, *constants,
                                    plan["first"], plan["count"], batch.slots, batch.entry, out, nh, hd, vd)
-            return linear(out, self.o)
+            return linear(out, self.o, status=status_of(batch))
         if single:
             ops.matrix_memory_step(tuple(c[:single] for c in columns), proj.stride(0), h[:single], self.gates, *constants,
                                    batch.slots, batch.entry[:single], out[:single], nh, hd, vd)
         if single < tokens:
-            ops.matrix_memory_chunks(columns, proj.stride(0), linear(h, self.gates, out_dtype=torch.float32), *constants,
+            gates = linear(h, self.gates, out_dtype=torch.float32, status=status_of(batch))
+            ops.matrix_memory_chunks(columns, proj.stride(0), gates, *constants,
                                      batch.slots, plan["chunks"], plan["spans"], out, nh, hd, vd)
-        return linear(out, self.o)
+        return linear(out, self.o, status=status_of(batch))

@@ -149,14 +149,14 @@ class RoutedExperts(Part):
                                      self.sigmoid_scores, self.group_top, self.renormalise, shared, self.logit_bias)
         return (ids, weights, None, shared) if self.weigh_input else (ids, None, weights, shared)
 
-    def _shared(self, h: torch.Tensor) -> torch.Tensor | None:
+    def _shared(self, h: torch.Tensor, status: torch.Tensor | None) -> torch.Tensor | None:
         """The shared expert's output."""
         if not self.shared_size:
             return None
         if self.gated:
             act = "silu" if self.shared_limit is None else "clamped"
-            return gated_feed_forward(h, self.shared_gate_up, self.shared_down, act, self.shared_limit or 0.0)
-        return activated_linear(linear(h, self.shared_gate_up), None, self.plain_act, self.shared_down)
+            return gated_feed_forward(h, self.shared_gate_up, self.shared_down, act, self.shared_limit or 0.0, status)
+        return activated_linear(linear(h, self.shared_gate_up, status=status), None, self.plain_act, self.shared_down, status)
 
     def _units(self, h: torch.Tensor) -> tuple:
         """Router and first half of the chosen experts, pair by pair: (activations [T * top, F], what `_route` says)."""
@@ -170,28 +170,29 @@ class RoutedExperts(Part):
 
     def forward(self, h: torch.Tensor, batch) -> torch.Tensor:
         out = torch.empty((h.shape[0], self.hidden), dtype=h.dtype, device=h.device)
+        status = status_of(batch)
         if not self._grouped(h):
             (act, (ids, _, weights, shared_weights)), shared = run_branches(
-                batch, h.device, lambda: self._units(h), shared_expert=lambda: self._shared(h))
+                batch, h.device, lambda: self._units(h), shared_expert=lambda: self._shared(h, status))
             ops.moe_down(act, self.down, ids, weights, shared, out, shared_weights)
             return out
         # Pairs in expert order; each projection one grouped product over the sorted rows, the activation in the first
         # one's epilogue (csrc/gemm_pair.cu; an expert's weight on its input keeps the activation a kernel of its own).
         ids, in_weights, weights, shared_weights = self._route(h)
-        shared = self._shared(h)
+        shared = self._shared(h, status)
         ends, row_of_pair, pair_of_row = ops.moe_sort(ids, self.n_experts)
         x = ops.moe_gather(h, pair_of_row, self.top)
         act = torch.empty((x.shape[0], self.ff), dtype=h.dtype, device=h.device)
         if self._own_products():
             if in_weights is None:
                 unit = ("silu" if self.limit is None else "clamped") if self.gated else self.plain_act
-                ops.gemm_bf16_grouped(x, self.gate_up, ends, act, unit, self.limit or 0.0, status_of(batch))
+                ops.gemm_bf16_grouped(x, self.gate_up, ends, act, unit, self.limit or 0.0, status)
             else:
                 gate_up = torch.empty((x.shape[0], 2 * self.ff), dtype=h.dtype, device=h.device)
-                ops.gemm_bf16_grouped(x, self.gate_up, ends, gate_up, status=status_of(batch))
+                ops.gemm_bf16_grouped(x, self.gate_up, ends, gate_up, status=status)
                 ops.gated_act(gate_up, act, "clamped", self.limit, in_weights, pair_of_row)
             y = torch.empty((x.shape[0], self.hidden), dtype=h.dtype, device=h.device)
-            ops.gemm_bf16_grouped(act, self.down, ends, y, status=status_of(batch))
+            ops.gemm_bf16_grouped(act, self.down, ends, y, status=status)
             ops.moe_combine(y, row_of_pair, weights, shared, out, shared_weights)
             return out
         # More experts than that kernel counts: the library's (operands [rows, K] and [E, K, N], the experts' ends as offsets).

@@ -10,7 +10,7 @@ import torch
 
 from ..kernels import ops
 from .attention import Attention
-from .linear import linear
+from .linear import linear, status_of
 from .registry import BuildContext, register_part
 from .spec import KVCacheNeed, PartSpec, TensorNeed
 
@@ -192,7 +192,7 @@ class NormedAttention(Attention):
         nh, nkv, hd, vd, row = self.n_heads, self.n_kv, self.key_dim, self.value_dim, self.row
         cache = self.cache
         table = batch.tables[cache.group]
-        proj = linear(h, self.qkv)
+        proj = linear(h, self.qkv, status=status_of(batch))
         q_end, k_end, v_end = nh * hd, (nh + nkv) * hd, (nh + nkv) * hd + nkv * vd
         q = proj[:, :q_end].view(tokens, nh, hd)
         k = proj[:, q_end:k_end].view(tokens, nkv, hd)
@@ -219,4 +219,4 @@ class NormedAttention(Attention):
         self.attend(q_rows, out, table, batch, gate=gate if self.head_gate else None)
         if self.gated and not self.head_gate:
             ops.sigmoid_gate_heads(out, gate)
-        return linear(out.view(tokens, nh * row), self.o)
+        return linear(out.view(tokens, nh * row), self.o, status=status_of(batch))

@@ -7,7 +7,7 @@ import torch
 from ..kernels import ops
 from .basic import NormedSides
 from .branches import run_branches
-from .linear import linear
+from .linear import linear, status_of
 from .registry import BuildContext, Part, build_part, part_class, register_part
 from .spec import PartSpec, TensorNeed
 
@@ -79,7 +79,7 @@ class SideBySide(Part):
     # ------------------------------------------------------------------ forward
     def pending(self, h: torch.Tensor, batch) -> NormedSides:
         """Both mixers' outputs as a residual contribution that is normed on its way in."""
-        proj = linear(h, self.in_weight)
+        proj = linear(h, self.in_weight, status=status_of(batch))
         at, stride = self.left.channels, self.in_weight.shape[0]
         left, right = run_branches(batch, h.device,
                                    lambda: self.left.forward_columns(proj[:, :at], stride, h, batch, True),

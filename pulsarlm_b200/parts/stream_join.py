@@ -31,11 +31,11 @@ class ConcatLinear(Part):
     def load(self, tensors: dict[str, torch.Tensor]) -> None:
         self.weight = tensors[self.spec.tensors["weight"]].contiguous()
 
-    def forward(self, x: torch.Tensor, delta, entered: torch.Tensor) -> torch.Tensor:
+    def forward(self, x: torch.Tensor, delta, entered: torch.Tensor, status: torch.Tensor | None = None) -> torch.Tensor:
         both = torch.empty((x.shape[0], 2 * self.hidden), dtype=self.ctx.dtype, device=x.device)
         if isinstance(delta, NormedSides):
             ops.side_norm(x, delta.sides(), delta.factor, delta.eps, delta.y3, None, 0.0, both, entered=entered)
         else:
             settle_pending(x, delta)
             ops.side_norm(x, None, 0.0, 0.0, None, None, 0.0, both, entered=entered)
-        return linear(both, self.weight, out_dtype=torch.float32)
+        return linear(both, self.weight, out_dtype=torch.float32, status=status)

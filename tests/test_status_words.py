@@ -3,6 +3,9 @@ recorded instead of made)."""
 
 from __future__ import annotations
 
+import ast
+import pathlib
+
 import pytest
 import torch
 
@@ -10,6 +13,7 @@ from pulsarlm_b200 import models as _models  # noqa: F401  (registers the parts)
 from pulsarlm_b200.cache.manager import StateBinding
 from pulsarlm_b200.kernels import ops
 from pulsarlm_b200.models.model import HostStep, StepBatch
+from pulsarlm_b200.parts import linear
 from pulsarlm_b200.parts.registry import BuildContext, build_part, part_class
 from pulsarlm_b200.parts.spec import PartSpec
 
@@ -82,3 +86,27 @@ def test_grouped_products_of_experts(launches, expert, weigh_input):
     _check(launches, "pl_gemm_bf16_grouped", batch, 2)
     part.forward(torch.zeros((64, 64), dtype=BF), None)  # (no step, nowhere to report to)
     assert [args[-2] for called, args in launches if called == "pl_gemm_bf16_grouped"][2:] == [None, None]
+
+
+@pytest.mark.parametrize("tokens", [1, 8, 40, 100])
+def test_products_of_layers(launches, monkeypatch, tokens):
+    monkeypatch.setattr(linear, "GEMM_ROUTE", "tcgen05")
+    gated = _part("feed_forward", "gated_mlp", {"hidden_size": 64, "intermediate_size": 128}, ("gate", "up", "down"))
+    plain = _part("feed_forward", "mlp", {"hidden_size": 64, "intermediate_size": 128}, ("up", "down"))
+    head = _part("head", "linear", {"hidden_size": 64, "vocab_size": 96}, ("weight",))
+    h, batch = torch.zeros((tokens, 64), dtype=BF), _batch(gated, [tokens])
+    gated.forward(h, batch)
+    plain.forward(h, batch)
+    head.forward(h, batch.status)
+    products = [args for name, args in launches if name.startswith("pl_gemm_bf16")]
+    assert len(products) == 5 and all(args[-2] == batch.status.data_ptr() for args in products)
+
+
+def test_no_part_leaves_the_status_word_out():
+    """(the positional place of `status`, counted from 0, in each function of parts/linear.py)"""
+    places = {"linear": 3, "gated_linear": 3, "gated_feed_forward": 5, "activated_linear": 4}
+    for path in pathlib.Path(linear.__file__).parent.glob("*.py"):
+        for node in ast.walk(ast.parse(path.read_text())):
+            if isinstance(node, ast.Call) and isinstance(node.func, ast.Name) and node.func.id in places:
+                given = len(node.args) > places[node.func.id] or any(k.arg == "status" for k in node.keywords)
+                assert given, f"{path.name}:{node.lineno}"
