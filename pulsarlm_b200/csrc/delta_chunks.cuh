@@ -9,7 +9,7 @@
 //   Z = Zi + Wm S0        [16, vdim]      O = Oi + Qg S0 + M Z      S <- diag(gC) S0 + Kd^T Z (+ Kv^T V)
 //
 // A first kernel makes Zi, Wm, Qg, M, Kd, gC (Oi, Kv) of all chunks side by side, all in fp32, decays between two tokens
-// as running products (never as quotients, nor as differences of long sums of logarithms). The kernel below walks the
+// as running products (never as quotients, nor as differences of long sums of logarithms). The kernels below walk the
 // chunks: one chain step per 16 tokens instead of one per token. A CTA has a head's 16 value columns; warp w of
 // dim / 16 has their 16 state rows from 16 w on, transposed, in the accumulators of m16n8k16 products: that layout is
 // also the A operand's, so the state goes from one product into the next without leaving registers. Every product
@@ -277,6 +277,283 @@ __device__ __forceinline__ void mma_terms(float (&d0)[4], float (&d1)[4], const 
     }
 }
 
+// The sum of the warps' shares of Z and its start: every warp makes it whole.
+template <int N, int NW>
+__device__ __forceinline__ void sum_of_shares(float (&z)[2][4], const float4 (&zi)[2], const float4 (&shares)[N][NW][32], int lane) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        float4 sum = shares[j][0][lane];
+#pragma unroll
+        for (int other = 1; other < NW; ++other) {
+            const float4 part = shares[j][other][lane];
+            sum = make_float4(sum.x + part.x, sum.y + part.y, sum.z + part.z, sum.w + part.w);
+        }
+        z[j][0] = zi[j].x + sum.x;
+        z[j][1] = zi[j].y + sum.y;
+        z[j][2] = zi[j].z + sum.z;
+        z[j][3] = zi[j].w + sum.w;
+    }
+}
+
+// Less than infinity while all of Z is.
+__device__ __forceinline__ float size_of(const float (&z)[2][4]) {
+    float size = 0.0f;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        size += fabsf(z[0][r]) + fabsf(z[1][r]);
+    }
+    return size;
+}
+
+// A chunk's outputs o = Oi + M Z of warp w's eight tokens (S0's part joins later), from Z's terms. `size`: size_of(Z).
+__device__ __forceinline__ void chunk_outputs(float (&o)[4], float size, TermsA& az, const TermsB& m, const float4& oi, int w,
+                                              int lane) {
+    float half[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    o[0] = oi.x;
+    o[1] = oi.y;
+    o[2] = oi.z;
+    o[3] = oi.w;
+    // A row of Z that is not finite would reach the chunk's earlier tokens through the zeros above M's diagonal: it is
+    // left out of the product, and the tokens from its own on are not a number. (What this needs of Z is in its terms.)
+    if (!__all_sync(0xffffffffu, size < INFINITY)) {
+        uint32_t bad[2] = {0u, 0u};  // bit t: token t's row, at this lane's column and the one 8 on
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const uint32_t exponent = 0x7f80u << (16 * r);
+                if ((az.t[0][q] & exponent) == exponent) {
+                    bad[q & 1] |= 1u << (8 * (q >> 1) + (lane & 3) * 2 + r);
+#pragma unroll
+                    for (int term = 0; term < 3; ++term) {
+                        az.t[term][q] &= 0xffffu << (16 * (1 - r));
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            bad[h] |= __shfl_xor_sync(0xffffffffu, bad[h], 1);
+            bad[h] |= __shfl_xor_sync(0xffffffffu, bad[h], 2);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {  // (tokens 8 w + (lane % 4) * 2 and the next: bits 0 to its own)
+            if (bad[i >> 1] & ((2u << (w * 8 + (lane & 3) * 2 + (i & 1))) - 1u)) {
+                o[i] = NAN;
+            }
+        }
+    }
+    constexpr int kA[6] = {2, 0, 1, 1, 0, 0}, kB[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        const uint4 b = m.t[kB[i]];
+        mma_bf16(i % 2 ? o : half, az.t[kA[i]], w == 0 ? b.x : b.z, w == 0 ? b.y : b.w);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        o[i] += half[i];
+    }
+}
+
+// What a lane of the joint form needs of a chunk, a chunk ahead of its use in registers.
+template <bool GENERAL>
+struct DeltaLane {
+    TermsB wm, qg, kd, m, kv;
+    float4 zi[2], g;
+    uint4 vv;
+};
+
+// Outputs by the chain's warps. grid (entries that go in chunks, heads, vdim / 16), NW = dim / 16 warps. On the path from a chunk to the next are only Z's products,
+// their sum over the warps, and the state's update; O's products fill the waits between and are added up a chunk later. Bound by
+// that path where an SM has one CTA (0.85 us a chunk); many CTAs fill the waits of one another, and a step of their short chains begins
+// with plain loads and no set-up. The walks took 681 us for one prompt of 2,048 tokens, 32 heads of 64 x 64. Slower: 32 columns a CTA.
+template <int NW, bool GENERAL>
+__global__ void __launch_bounds__(NW * 32) delta_chain_joint_kernel(const DeltaChainParams p) {
+    pl_grid_trigger();
+    pl_grid_wait();
+    constexpr int kDim = NW * 16;
+    __shared__ float4 shares[2][4][NW][32];  // by chunk parity: two tiles of Z, two of O
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int head = blockIdx.y, ct = blockIdx.z;
+    int e, before;
+    if (!delta_find_entry(p.counts, p.pass, blockIdx.x, e, before)) {
+        return;
+    }
+    const int count = p.counts[e];
+    const int n_chunks = delta_chunks_of(count, p.pass);
+    if (n_chunks == 0) {
+        return;
+    }
+    const DeltaChunkLayout at(kDim, p.vdim, GENERAL);
+    constexpr DeltaChunkLayout kAt(kDim, 0, GENERAL);  // (the places up to zi hold for any vdim)
+    const int64_t step = static_cast<int64_t>(p.n_heads) * at.floats;
+    const float* chunk0 = p.scratch + (static_cast<int64_t>(before) * p.n_heads + head) * at.floats;
+    const float* src = chunk0 + w * 384 + lane * 4;
+    const float* src_m = chunk0 + kAt.m + lane * 4;
+    const float* src_zi = chunk0 + kAt.zi + (ct * 2 * 32 + lane) * 4;
+    const float* src_oi = chunk0 + at.oi + ((ct * 2 + w) * 32 + lane) * 4;
+    const float* src_vv = chunk0 + at.vv + (ct * 32 + lane) * 4;
+    const float* src_g = chunk0 + at.g + w * 16 + (lane & 3) * 4;
+    auto terms = [](TermsB& b, const float* from) {
+#pragma unroll
+        for (int term = 0; term < 3; ++term) {
+            b.t[term] = *reinterpret_cast<const uint4*>(from + term * 128);
+        }
+    };
+    auto fetch_m = [&](TermsB& m) {
+        terms(m, src_m);
+        src_m += step;
+    };
+    auto fetch = [&](DeltaLane<GENERAL>& in) {
+        terms(in.wm, src);
+        terms(in.qg, src + kAt.qg);
+        if constexpr (!GENERAL) {
+            terms(in.kd, src + kAt.kd);
+        }
+        in.zi[0] = *reinterpret_cast<const float4*>(src_zi);
+        in.zi[1] = *reinterpret_cast<const float4*>(src_zi + 128);
+        in.g = *reinterpret_cast<const float4*>(src_g);
+        if constexpr (GENERAL) {
+            terms(in.kv, src + kAt.kv);
+            in.vv = *reinterpret_cast<const uint4*>(src_vv);
+            src_vv += step;
+        } else if (w < 2) {
+            fetch_m(in.m);
+        }
+        src += step;
+        src_zi += step;
+        src_g += step;
+    };
+    DeltaLane<GENERAL> even = {}, odd = {};
+    fetch(even);
+
+    // S transposed: s[j][r] is column ct * 16 + lane / 4 (+ 8 for r >= 2), row w * 16 + 8 j + (lane % 4) * 2 + r % 2.
+    float s[2][4];
+    float* corner = p.state + ((static_cast<int64_t>(p.slots[e]) * p.n_heads + head) * kDim + w * 16 + (lane & 3) * 2) * p.vdim +
+        ct * kDeltaCols + (lane >> 2);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            s[j][r] = corner[static_cast<int64_t>(8 * j + (r & 1)) * p.vdim + (r >> 1) * 8];
+        }
+    }
+    // This lane's outputs: columns lane / 4 and 8 on, tokens 8 w + (lane % 4) * 2 and the next (of the first two warps).
+    const int done = p.pass.pass * p.pass.window * kDeltaChunk;
+    const int rows = count - done;
+    const int64_t o_stride = static_cast<int64_t>(p.n_heads) * p.vdim;
+    int token = w * 8 + (lane & 3) * 2;
+    float* dst = p.o_raw + (p.first_rows[e] + done + token) * o_stride +
+        static_cast<int64_t>(head) * p.vdim + ct * kDeltaCols + (lane >> 2);
+    float o[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    auto finish = [&](int parity) {
+#pragma unroll
+        for (int other = 0; other < NW; ++other) {
+            const float4 part = shares[parity][2 + w][other][lane];
+            o[0] += part.x;
+            o[1] += part.y;
+            o[2] += part.z;
+            o[3] += part.w;
+        }
+        if (token < rows) {
+            dst[0] = o[0];
+            dst[8] = o[2];
+        }
+        if (token + 1 < rows) {
+            dst[o_stride] = o[1];
+            dst[o_stride + 8] = o[3];
+        }
+        token += kDeltaChunk;
+        dst += kDeltaChunk * o_stride;
+    };
+
+    auto advance = [&](const DeltaLane<GENERAL>& in, DeltaLane<GENERAL>& ahead, int c, const int parity) {
+        // (M, Oi and Kd, which the chunk's end reads: a chunk ahead too the general rule's registers would not hold them)
+        TermsB m = in.m;
+        TermsB kd_now = in.kd;
+        float4 oi = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if constexpr (GENERAL) {
+            terms(kd_now, src - step + kAt.kd);
+            if (w < 2) {
+                fetch_m(m);
+                oi = *reinterpret_cast<const float4*>(src_oi);
+                src_oi += step;
+            }
+        }
+        if (c + 1 < n_chunks) {
+            fetch(ahead);
+        }
+        TermsA a, az;
+        terms_of(a, s[0], s[1]);
+        float d[2][4];
+        mma_terms(d[0], d[1], a, in.wm);  // this warp's rows' share of S0's part of Z
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            shares[parity][j][w][lane] = make_float4(d[j][0], d[j][1], d[j][2], d[j][3]);
+        }
+        const float decay[2][2] = {{in.g.x, in.g.y}, {in.g.z, in.g.w}};
+        float written[2][4] = {};
+        if constexpr (GENERAL) {  // + Kv^T V: the values are bfloat16 as they are
+            const uint32_t v[4] = {in.vv.x, in.vv.y, in.vv.z, in.vv.w};
+#pragma unroll
+            for (int term = 2; term >= 0; --term) {
+                mma_bf16(written[0], v, in.kv.t[term].x, in.kv.t[term].y);
+                mma_bf16(written[1], v, in.kv.t[term].z, in.kv.t[term].w);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                s[j][r] = fmaf(s[j][r], decay[j][r & 1], written[j][r]);
+            }
+        }
+        __syncthreads();
+        float z[2][4];
+        sum_of_shares(z, in.zi, shares[parity], lane);
+        const float size = size_of(z);
+        float q[2][4];
+        mma_terms(q[0], q[1], a, in.qg);  // (and of O: made while the sums of Z come in, read after the next barrier)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            shares[parity][2 + j][w][lane] = make_float4(q[j][0], q[j][1], q[j][2], q[j][3]);
+        }
+        terms_of(az, z[0], z[1]);
+        float moved[2][4];
+        mma_terms(moved[0], moved[1], az, kd_now);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                s[j][r] += moved[j][r];
+            }
+        }
+        if (w < 2) {
+            if (c > 0) {
+                finish(parity ^ 1);  // the chunk before: its shares were written before this chunk's barrier
+            }
+            chunk_outputs(o, size, az, m, oi, w, lane);
+        }
+    };
+    for (int c = 0; c < n_chunks; c += 2) {
+        advance(even, odd, c, 0);
+        if (c + 1 < n_chunks) {
+            advance(odd, even, c + 1, 1);
+        }
+    }
+    __syncthreads();
+    if (w < 2) {
+        finish((n_chunks - 1) & 1);
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            corner[static_cast<int64_t>(8 * j + (r & 1)) * p.vdim + (r >> 1) * 8] = s[j][r];
+        }
+    }
+}
+
 // A CTA's chunk in shared memory, in floats: the operands and M as they lie in the scratch, and of the rest the CTA's columns.
 template <int DIM, bool GENERAL>
 struct DeltaRing {
@@ -287,7 +564,7 @@ struct DeltaRing {
     static constexpr int kBytes = kSlots * kFloats * 4 + 2 * 2 * DIM / 16 * 32 * 16;
 };
 
-// grid (entries that go in chunks x heads, vdim / 16), 2 NW warps, NW = dim / 16. On the path from a chunk to the next are only
+// Outputs by warps of their own. grid (entries that go in chunks x heads, vdim / 16), 2 NW warps, NW = dim / 16. On the path from a chunk to the next are only
 // Z's products, their sum over the warps, and the state's update: the first NW warps do nothing else. They leave the state that
 // a chunk starts from in shared memory, where the other NW take it up for O's products, a barrier behind, and add those up a
 // chunk later. The chunks' matrices come into shared memory by bulk copies, three or four chunks in flight. Bound by the path's
@@ -382,22 +659,6 @@ __global__ void __launch_bounds__(NW * 64, NW >= 8 ? 1 : 8 / NW) delta_chain_ker
     // Both halves of the CTA meet once a chunk and once after the last, each from a branch of its own: __syncthreads() is only for
     // places that every thread comes by, a named barrier counts threads wherever they are.
     auto meet = [] { asm volatile("bar.sync 1, %0;" ::"n"(NW * 64) : "memory"); };
-    // The sum of the warps' shares of Z and its start: every warp makes it whole.
-    auto z_of = [&](float (&z)[2][4], const float4 (&zi)[2], int parity) {
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            float4 sum = shares[parity][j][0][lane];
-#pragma unroll
-            for (int other = 1; other < NW; ++other) {
-                const float4 part = shares[parity][j][other][lane];
-                sum = make_float4(sum.x + part.x, sum.y + part.y, sum.z + part.z, sum.w + part.w);
-            }
-            z[j][0] = zi[j].x + sum.x;
-            z[j][1] = zi[j].y + sum.y;
-            z[j][2] = zi[j].z + sum.z;
-            z[j][3] = zi[j].w + sum.w;
-        }
-    };
 
     if (!outputs) {
         // S transposed: s[j][r] is column ct * 16 + lane / 4 (+ 8 for r >= 2), row w * 16 + 8 j + (lane % 4) * 2 + r % 2.
@@ -458,7 +719,7 @@ __global__ void __launch_bounds__(NW * 64, NW >= 8 ? 1 : 8 / NW) delta_chain_ker
                 }
             }
             float z[2][4], moved[2][4];
-            z_of(z, zi, parity);
+            sum_of_shares(z, zi, shares[parity], lane);
             terms_of(az, z[0], z[1]);
             mma_terms(moved[0], moved[1], az, kd);
             if (c + 1 < n_chunks) {
@@ -555,58 +816,9 @@ __global__ void __launch_bounds__(NW * 64, NW >= 8 ? 1 : 8 / NW) delta_chain_ker
             }
             float z[2][4];
             TermsA az;
-            z_of(z, zi, parity);
+            sum_of_shares(z, zi, shares[parity], lane);
             terms_of(az, z[0], z[1]);
-            float size = 0.0f;  // (less than infinity while all of Z is)
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                size += fabsf(z[0][r]) + fabsf(z[1][r]);
-            }
-            float half[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            o[0] = oi.x;
-            o[1] = oi.y;
-            o[2] = oi.z;
-            o[3] = oi.w;
-            // A row of Z that is not finite would reach the chunk's earlier tokens through the zeros above M's diagonal: it is
-            // left out of the product, and the tokens from its own on are not a number. (What this needs of Z is in its terms.)
-            if (!__all_sync(0xffffffffu, size < INFINITY)) {
-                uint32_t bad[2] = {0u, 0u};  // bit t: token t's row, at this lane's column and the one 8 on
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-#pragma unroll
-                    for (int r = 0; r < 2; ++r) {
-                        const uint32_t exponent = 0x7f80u << (16 * r);
-                        if ((az.t[0][q] & exponent) == exponent) {
-                            bad[q & 1] |= 1u << (8 * (q >> 1) + (lane & 3) * 2 + r);
-#pragma unroll
-                            for (int term = 0; term < 3; ++term) {
-                                az.t[term][q] &= 0xffffu << (16 * (1 - r));
-                            }
-                        }
-                    }
-                }
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    bad[h] |= __shfl_xor_sync(0xffffffffu, bad[h], 1);
-                    bad[h] |= __shfl_xor_sync(0xffffffffu, bad[h], 2);
-                }
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {  // (tokens 8 w + (lane % 4) * 2 and the next: bits 0 to its own)
-                    if (bad[i >> 1] & ((2u << (w * 8 + (lane & 3) * 2 + (i & 1))) - 1u)) {
-                        o[i] = NAN;
-                    }
-                }
-            }
-            constexpr int kA[6] = {2, 0, 1, 1, 0, 0}, kB[6] = {0, 2, 1, 0, 1, 0};
-#pragma unroll
-            for (int i = 0; i < 6; ++i) {
-                const uint4 b = m.t[kB[i]];
-                mma_bf16(i % 2 ? o : half, az.t[kA[i]], w == 0 ? b.x : b.z, w == 0 ? b.y : b.w);
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                o[i] += half[i];
-            }
+            chunk_outputs(o, size_of(z), az, m, oi, w, lane);
         }
     }
     meet();
@@ -623,9 +835,32 @@ __global__ void __launch_bounds__(NW * 64, NW >= 8 ? 1 : 8 / NW) delta_chain_ker
     }
 }
 
+// Whether the outputs go to warps of their own (delta_chain_kernel) or the chain's warps make them too (delta_chain_joint_kernel).
+// The former shortens the path from chunk to chunk, for chains that have an SM each, and keeps more copies in flight, for scratch
+// that does not stay in L2; it needs twice the warps and a ring of shared memory, which many short chains wait for. Both give the same
+// bits. Whole calls, 32 heads of 64 x 64, us, joint and apart: one entry of 8, 16, 32, 128 chunks 24 and 23, 38 and 32, 60 and 53,
+// 225 and 167; 12 entries of 1, 3, 8 (75 MB of scratch), 12 (112 MB) chunks 33 and 37, 55 and 60, 124 and 123, 192 and 171; the general
+// rule, 5 entries of 4, 12 (70 MB), 16 (94 MB), 32 chunks 42 and 45, 99 and 100, 138 and 128, 277 and 238. Never ahead with more
+// CTAs than SMs: 64 heads of 32 x 128 with a decay per channel (two entries of 32 chunks 146 and 169, one of 128 276 and 364), and
+// at most even where values are wider than keys.
+constexpr int64_t kDeltaKept = 88 << 20;  // (of scratch: about what of L2 the chunks' matrices keep)
 template <int NW, bool GENERAL>
-cudaError_t launch_delta_chain(const DeltaChainParams& p, int n_long, cudaStream_t stream) {
+inline bool delta_chain_apart(const DeltaChainParams& p, int64_t ctas, int64_t slots, int n_long) {
+    if (ctas <= 148) {
+        return slots / n_long >= 8;
+    }
+    const int64_t bytes = slots * p.n_heads * DeltaChunkLayout(NW * 16, p.vdim, GENERAL).floats * 4;
+    return bytes >= kDeltaKept && p.vdim <= NW * 16 && (GENERAL || NW > 2);
+}
+
+template <int NW, bool GENERAL>
+cudaError_t launch_delta_chain(const DeltaChainParams& p, int n_long, int64_t slots, cudaStream_t stream) {
     using Ring = DeltaRing<NW * 16, GENERAL>;
+    const int64_t ctas = static_cast<int64_t>(n_long) * p.n_heads * (p.vdim / kDeltaCols);
+    if (!delta_chain_apart<NW, GENERAL>(p, ctas, slots, n_long)) {
+        return pl_launch_overlapped(delta_chain_joint_kernel<NW, GENERAL>, dim3(n_long, p.n_heads, p.vdim / kDeltaCols),
+                                    dim3(NW * 32), 0, stream, p);
+    }
     // Where every CTA can have an SM to itself, more than half of one's shared memory sees to it: CTAs that come in while the
     // chunks' matrices still hold some SMs would otherwise share the others (one prompt: 135 us so, 95 alone).
     constexpr int kAlone = 120 * 1024, kMost = Ring::kBytes > kAlone ? Ring::kBytes : kAlone;
@@ -633,7 +868,7 @@ cudaError_t launch_delta_chain(const DeltaChainParams& p, int n_long, cudaStream
         return set;
     }
     const dim3 grid(n_long * p.n_heads, p.vdim / kDeltaCols);
-    const bool alone = static_cast<int64_t>(grid.x) * grid.y <= 148;
+    const bool alone = ctas <= 148;
     return pl_launch_overlapped(delta_chain_kernel<NW, GENERAL>, grid, dim3(NW * 64), alone ? kMost : Ring::kBytes, stream, p);
 }
 

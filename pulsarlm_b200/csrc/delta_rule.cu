@@ -699,7 +699,7 @@ cudaError_t launch_rule_chunks(const RuleChunkParams& c, int64_t slots, int n_lo
     }
     const DeltaChainParams chain{c.scratch, c.in.state, c.in.first_rows, c.in.counts, c.in.slots, c.in.o_raw, c.in.n_heads,
                                  DIM, c.pass, c.status};
-    return launch_delta_chain<DIM / 16, true>(chain, n_long, stream);
+    return launch_delta_chain<DIM / 16, true>(chain, n_long, slots, stream);
 }
 
 // ---------------------------------------------------------------------------- steps of single tokens

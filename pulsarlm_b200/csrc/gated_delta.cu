@@ -929,7 +929,7 @@ cudaError_t launch_gated_chunks(const GatedChunkParams& c, int64_t slots, int n_
     }
     const DeltaChainParams chain{c.scratch, c.in.state, c.in.first_rows, c.in.counts, c.in.slots, c.in.o_raw, c.in.n_heads,
                                  c.in.vdim, c.pass, c.status};
-    return launch_delta_chain<DIM / 16, false>(chain, n_long, stream);
+    return launch_delta_chain<DIM / 16, false>(chain, n_long, slots, stream);
 }
 
 // ---------------------------------------------------------------------------- steps of single tokens
