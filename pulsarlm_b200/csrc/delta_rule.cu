@@ -712,8 +712,8 @@ struct RuleStepParams {
     float eps;
 };
 
-template <int DIM>
-__global__ void __launch_bounds__(kStepThreads, step_ctas(DIM, DIM)) delta_rule_step_kernel(const RuleStepParams c) {
+template <int DIM, int CTAS = step_ctas(DIM, DIM)>
+__global__ void __launch_bounds__(kStepThreads, CTAS) delta_rule_step_kernel(const RuleStepParams c) {
     pl_grid_trigger();
     pl_grid_wait();
     __shared__ __align__(16) DeltaStepShared<DIM, DIM> s;
@@ -900,7 +900,10 @@ PL_API int pl_delta_rule(const void* r, const void* k, const void* v, const void
         p.most = forms.step_most;
         const RuleStepParams c{p, static_cast<const __nv_bfloat16*>(g), norm, static_cast<__nv_bfloat16*>(out), out_row_stride,
                                eps};
-        auto kernel = dim == 32 ? delta_rule_step_kernel<32> : dim == 64 ? delta_rule_step_kernel<64> : delta_rule_step_kernel<128>;
+        static_assert(step_has_two_builds(64, 64) && !step_has_two_builds(32, 32) && !step_has_two_builds(128, 128), "builds");
+        const bool many = step_many(static_cast<int64_t>(n_entries) * n_heads, dim, dim, true);
+        auto kernel = dim == 32 ? delta_rule_step_kernel<32> : dim == 128 ? delta_rule_step_kernel<128>
+                    : many      ? delta_rule_step_kernel<64, kStepMany> : delta_rule_step_kernel<64>;
         pl_launch_overlapped(kernel, dim3(n_entries, n_heads), dim3(kStepThreads), 0, stream, c);
         PL_CHECK_LAUNCH("delta_rule");
     }

@@ -11,11 +11,23 @@
 namespace {
 
 constexpr int kStepThreads = 256;
-// CTAs an SM holds: a CTA's loads answer once, so the state's stream is as wide as the CTAs in flight. Left to the compiler, heads
-// of 64 x 64 took 62 registers a thread and four CTAs an SM (64 entries of 32 heads 19.0 us, now 18.2; of 16 heads
-// of 128 x 128, a part 57.5 and 53.6); larger heads
-// keep what their rows need.
-constexpr int step_ctas(int dim, int vdim) { return dim * vdim <= 4096 ? 6 : dim * vdim <= 8192 ? 3 : 2; }
+// CTAs an SM holds: a CTA's loads answer once, so the state's stream is as wide as the CTAs in flight. Heads of 1,024 to 4,096 values
+// (without the least) have two builds: with the registers that the compiler takes (48 to 69 a thread: four CTAs an SM, three of 128 x
+// 32, five of 32 x 64), and with 40, a few of them in memory, and six. The latter takes 2 to 26 % longer for a CTA and is for steps that then go in
+// fewer rounds; the general rule, whose rows need more, for those with a good third fewer. us, four and six CTAs: 32 heads of 64 x 64, 16
+// entries 8.3 and 9.7, 24 entries 12.4 and 10.6, 32 entries 13.6 and 14.7, 64 entries 23.2 and 22.5, 256 entries 77.8 and 68.6 (the
+// general rule 9.0 and 11.0, 13.6 and 11.9, 14.9 and 17.4, 26.4 and 27.1, 89.6 and 85.5); 16 heads of 128 x 32, 24 entries 7.7 and 9.1,
+// 32 entries 11.7 and 9.9; 64 heads of 32 x 128, 16 entries 13.4 and 14.9, 256 entries 144 and 124. 128 x 128 is told of the two that it
+// has anyway: 128 registers for 126, 64 entries of 16 heads 33.6 and 32.8. Others as the compiler has them (64 x 128 held to
+// three: 36.0 and 37.3).
+constexpr int kStepMany = 6;
+constexpr bool step_has_two_builds(int dim, int vdim) { return dim * vdim > 1024 && dim * vdim <= 4096; }
+constexpr int step_ctas(int dim, int vdim) { return dim * vdim == 128 * 128 ? 2 : 0; }  // (0: nothing asked; one asked is not the same, 88 to 115 registers)
+inline bool step_many(int64_t ctas, int dim, int vdim, bool general) {
+    const int few = dim == 128 ? 3 : dim == 32 && vdim == 64 ? 5 : 4;
+    const int64_t rounds = (ctas + few * 148 - 1) / (few * 148), fewer = (ctas + kStepMany * 148 - 1) / (kStepMany * 148);
+    return general ? 5 * rounds >= 7 * fewer : rounds > fewer;
+}
 
 // A token's vectors of a head, made by the first DIM threads, and its scalars.
 template <int DIM, int VDIM>

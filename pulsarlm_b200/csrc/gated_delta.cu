@@ -943,8 +943,8 @@ struct GatedStepParams {
     float eps;
 };
 
-template <int DIM, int VDIM>
-__global__ void __launch_bounds__(kStepThreads, step_ctas(DIM, VDIM)) gated_delta_step_kernel(const GatedStepParams c) {
+template <int DIM, int VDIM, int CTAS>
+__global__ void __launch_bounds__(kStepThreads, CTAS) gated_delta_step_kernel(const GatedStepParams c) {
     pl_grid_trigger();
     pl_grid_wait();
     __shared__ __align__(16) DeltaStepShared<DIM, VDIM> s;
@@ -997,10 +997,20 @@ __global__ void __launch_bounds__(kStepThreads, step_ctas(DIM, VDIM)) gated_delt
     delta_step_walk<DIM, VDIM, false>(s, state, count, c.eps, vectors, store);
 }
 
+template <int DIM, int VDIM>
+auto gated_step_build(bool many) {
+    auto kernel = gated_delta_step_kernel<DIM, VDIM, step_ctas(DIM, VDIM)>;
+    if constexpr (step_has_two_builds(DIM, VDIM)) {
+        kernel = many ? gated_delta_step_kernel<DIM, VDIM, kStepMany> : kernel;
+    }
+    return kernel;
+}
+
 template <int DIM>
 void launch_gated_step(const GatedStepParams& c, int n_entries, cudaStream_t stream) {
-    auto kernel = c.in.vdim == 32 ? gated_delta_step_kernel<DIM, 32>
-                : c.in.vdim == 64 ? gated_delta_step_kernel<DIM, 64> : gated_delta_step_kernel<DIM, 128>;
+    const bool many = step_many(static_cast<int64_t>(n_entries) * c.in.n_heads, DIM, c.in.vdim, false);
+    auto kernel = c.in.vdim == 32   ? gated_step_build<DIM, 32>(many)
+                  : c.in.vdim == 64 ? gated_step_build<DIM, 64>(many) : gated_step_build<DIM, 128>(many);
     pl_launch_overlapped(kernel, dim3(n_entries, c.in.n_heads), dim3(kStepThreads), 0, stream, c);
 }
 
