@@ -838,26 +838,29 @@ __global__ void __launch_bounds__(NW * 64, NW >= 8 ? 1 : 8 / NW) delta_chain_ker
 // Whether the outputs go to warps of their own (delta_chain_kernel) or the chain's warps make them too (delta_chain_joint_kernel).
 // The former shortens the path from chunk to chunk, for chains that have an SM each, and keeps more copies in flight, for scratch
 // that does not stay in L2; it needs twice the warps and a ring of shared memory, which many short chains wait for. Both give the same
-// bits. Whole calls, 32 heads of 64 x 64, us, joint and apart: one entry of 8, 16, 32, 128 chunks 24 and 23, 38 and 32, 60 and 53,
-// 225 and 167; 12 entries of 1, 3, 8 (75 MB of scratch), 12 (112 MB) chunks 33 and 37, 55 and 60, 124 and 123, 192 and 171; the general
-// rule, 5 entries of 4, 12 (70 MB), 16 (94 MB), 32 chunks 42 and 45, 99 and 100, 138 and 128, 277 and 238. Never ahead with more
-// CTAs than SMs: 64 heads of 32 x 128 with a decay per channel (two entries of 32 chunks 146 and 169, one of 128 276 and 364), and
-// at most even where values are wider than keys.
-constexpr int64_t kDeltaKept = 88 << 20;  // (of scratch: about what of L2 the chunks' matrices keep)
+// bits. Whole calls, 32 heads of 64 x 64, us, joint and apart: one entry of 1, 4, 12, 32, 64 chunks 15.4 and 16.8, 19.0 and 19.8, 28.4 and
+// 24.7, 58.5 and 50.3, 107.5 and 88.2 (the general rule 16.4 and 13.3, 21.8 and 20.1, 33.5 and 28.8, 65.6 and 55.1, 120 and 104; 12
+// heads 0.76 to 1.15 times as long up to 4 chunks); 12 entries of 1, 3, 8 (75 MB of scratch), 12 (112 MB) chunks 33 and 37, 55 and 60,
+// 124 and 123, 192 and 171; the general rule, 5 entries of 4, 12 (70 MB), 16 (94 MB), 32 chunks 42 and 45, 99 and 100, 138 and 128, 277 and 238.
+// Never ahead with more CTAs than SMs: 64 heads of 32 x 128 with a decay per channel (two entries of 32 chunks 144 and 167),
+// and at most even where values are wider than keys.
 template <int NW, bool GENERAL>
-inline bool delta_chain_apart(const DeltaChainParams& p, int64_t ctas, int64_t slots, int n_long) {
+inline bool delta_chain_apart(int n_heads, int vdim, int64_t slots, int n_long, int64_t longest) {
+    const int64_t ctas = static_cast<int64_t>(n_long) * n_heads * (vdim / kDeltaCols), chunks = slots / n_long;
     if (ctas <= 148) {
-        return slots / n_long >= 8;
+        return chunks >= (NW == 8 ? 6 : GENERAL ? 4 : 10);
     }
-    const int64_t bytes = slots * p.n_heads * DeltaChunkLayout(NW * 16, p.vdim, GENERAL).floats * 4;
-    return bytes >= kDeltaKept && p.vdim <= NW * 16 && (GENERAL || NW > 2);
+    const int64_t bytes = slots * n_heads * DeltaChunkLayout(NW * 16, vdim, GENERAL).floats * 4;
+    const int64_t kept = (chunks >= 8 && vdim >= 64 ? 54 : 92) << 20;  // about what of L2 the matrices keep
+    // (a chain much longer than the others is a path again, on an SM that it shares: 1,500 tokens beside eight portions of 20, 16 heads
+    // of 128 x 128, the general rule 344 and 367)
+    return bytes >= kept && vdim <= NW * 16 && (NW > 2 ? longest < 4 * chunks : GENERAL);
 }
 
 template <int NW, bool GENERAL>
-cudaError_t launch_delta_chain(const DeltaChainParams& p, int n_long, int64_t slots, cudaStream_t stream) {
+cudaError_t launch_delta_chain(const DeltaChainParams& p, int n_long, bool apart, cudaStream_t stream) {
     using Ring = DeltaRing<NW * 16, GENERAL>;
-    const int64_t ctas = static_cast<int64_t>(n_long) * p.n_heads * (p.vdim / kDeltaCols);
-    if (!delta_chain_apart<NW, GENERAL>(p, ctas, slots, n_long)) {
+    if (!apart) {
         return pl_launch_overlapped(delta_chain_joint_kernel<NW, GENERAL>, dim3(n_long, p.n_heads, p.vdim / kDeltaCols),
                                     dim3(NW * 32), 0, stream, p);
     }
@@ -868,7 +871,7 @@ cudaError_t launch_delta_chain(const DeltaChainParams& p, int n_long, int64_t sl
         return set;
     }
     const dim3 grid(n_long * p.n_heads, p.vdim / kDeltaCols);
-    const bool alone = ctas <= 148;
+    const bool alone = static_cast<int64_t>(grid.x) * grid.y <= 148;
     return pl_launch_overlapped(delta_chain_kernel<NW, GENERAL>, grid, dim3(NW * 64), alone ? kMost : Ring::kBytes, stream, p);
 }
 

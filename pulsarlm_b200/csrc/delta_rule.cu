@@ -437,8 +437,11 @@ constexpr int rule_chunk_smem() {
     return (5 * 16 * (DIM + 4) + 4 * 256 + DeltaStageLayout(DIM, DIM, true).floats) * 4;
 }
 
-template <int DIM>
-__global__ void __launch_bounds__(128, DIM == 32 ? 5 : 4) delta_rule_chunk_kernel(const RuleChunkParams c) {
+// CTAS an SM: heads of 32 have a build for five, with 96 registers a thread and 20 bytes of them in memory, for launches of more CTAs
+// than the four that the compiler's registers (118; 0: nothing asked) allow: whole calls of 64 heads 2 to 4 % shorter, below that
+// line 2 % longer. Larger heads are held to four and two by shared memory.
+template <int DIM, int CTAS>
+__global__ void __launch_bounds__(128, CTAS) delta_rule_chunk_kernel(const RuleChunkParams c) {
     pl_grid_trigger();
     pl_grid_wait();
     constexpr int kLd = DIM + 4;
@@ -685,21 +688,33 @@ __global__ void __launch_bounds__(128, DIM == 32 ? 5 : 4) delta_rule_chunk_kerne
     send_chunk(out, c.scratch + (static_cast<int64_t>(blockIdx.x) * p.n_heads + head) * sent.floats, at, DIM);
 }
 
-template <int DIM>
-cudaError_t launch_rule_chunks(const RuleChunkParams& c, int64_t slots, int n_long, cudaStream_t stream) {
+template <int DIM, int CTAS>
+cudaError_t launch_rule_matrices(const RuleChunkParams& c, int64_t slots, cudaStream_t stream) {
     constexpr int kSmem = rule_chunk_smem<DIM>();
-    const cudaError_t set = pl_allow_smem<delta_rule_chunk_kernel<DIM>>(kSmem);
+    const cudaError_t set = pl_allow_smem<delta_rule_chunk_kernel<DIM, CTAS>>(kSmem);
     if (set != cudaSuccess) {
         return set;
     }
-    const cudaError_t made = pl_launch_overlapped(delta_rule_chunk_kernel<DIM>, dim3(static_cast<unsigned>(slots), c.in.n_heads),
-                                                  dim3(128), kSmem, stream, c);
+    return pl_launch_overlapped(delta_rule_chunk_kernel<DIM, CTAS>, dim3(static_cast<unsigned>(slots), c.in.n_heads), dim3(128), kSmem,
+                                stream, c);
+}
+
+template <int DIM>
+cudaError_t launch_rule_chunks(const RuleChunkParams& c, int64_t slots, int n_long, int longest, cudaStream_t stream) {
+    const bool apart = delta_chain_apart<DIM / 16, true>(c.in.n_heads, DIM, slots, n_long, longest);
+    cudaError_t made;
+    if constexpr (DIM == 32) {
+        made = slots * c.in.n_heads > 4 * 148 ? launch_rule_matrices<DIM, 5>(c, slots, stream)
+                                              : launch_rule_matrices<DIM, 0>(c, slots, stream);
+    } else {
+        made = launch_rule_matrices<DIM, 0>(c, slots, stream);
+    }
     if (made != cudaSuccess) {
         return made;
     }
     const DeltaChainParams chain{c.scratch, c.in.state, c.in.first_rows, c.in.counts, c.in.slots, c.in.o_raw, c.in.n_heads,
                                  DIM, c.pass, c.status};
-    return launch_delta_chain<DIM / 16, true>(chain, n_long, slots, stream);
+    return launch_delta_chain<DIM / 16, true>(chain, n_long, apart, stream);
 }
 
 // ---------------------------------------------------------------------------- steps of single tokens
@@ -863,11 +878,12 @@ PL_API int pl_delta_rule(const void* r, const void* k, const void* v, const void
         const int window = delta_window(step, n_heads, DeltaChunkLayout(dim, dim, true).floats);
         RuleChunkParams c{p, {n_entries, forms.chunk_least, window, 0}, scratch, status};
         const int64_t n_slots = delta_chunk_slots(step, window);
+        const int longest = min(longest_chunks, window);
         cudaError_t made = cudaSuccess;
         for (; c.pass.pass < delta_passes(step, window) && made == cudaSuccess; ++c.pass.pass) {
-            made = dim == 32 ? launch_rule_chunks<32>(c, n_slots, n_long, stream)
-                 : dim == 64 ? launch_rule_chunks<64>(c, n_slots, n_long, stream)
-                             : launch_rule_chunks<128>(c, n_slots, n_long, stream);
+            made = dim == 32 ? launch_rule_chunks<32>(c, n_slots, n_long, longest, stream)
+                 : dim == 64 ? launch_rule_chunks<64>(c, n_slots, n_long, longest, stream)
+                             : launch_rule_chunks<128>(c, n_slots, n_long, longest, stream);
         }
         if (made != cudaSuccess) {
             return pl_fail(3, "delta_rule: launch failed: %s", cudaGetErrorString(made));

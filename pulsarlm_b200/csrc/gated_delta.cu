@@ -700,10 +700,15 @@ constexpr int gated_chunk_smem(int vdim) {
     return (3 * 16 * (DIM + 4) + 2 * 256 + 16 + DeltaStageLayout(DIM, vdim, false).floats) * 4;
 }
 
-// (Its warps wait for shared memory and for one another's results more than they issue: six CTAs an SM, which 80 registers a thread
-// allow, 64.7 us for 2,048 tokens of 32 heads of 64 x 64, five 67, four with the compiler's 99 registers 73.)
-template <int DIM>
-__global__ void __launch_bounds__(128, DIM <= 64 ? 6 : 4) gated_delta_chunk_kernel(const GatedChunkParams c) {
+// Its warps wait for shared memory and for one another's results more than they issue. CTAS an SM: key sizes up to 64 have a build for
+// six, with 80 registers a thread and up to 28 bytes of them in memory, beside the compiler's (99; 0: nothing asked), which lets four
+// in. 2,048 tokens of 32 heads of 64 x 64 73 and 64.7 us. It is for launches of more CTAs than four an SM (64 heads of 32 x 64:
+// whole calls 4 to 10 % shorter), key sizes of 64 for those that then go in about two thirds of the rounds (36 chunks of 32 heads,
+// two rounds either way, 52 and 55 us a call) and, with values of 64, lead to a chain whose outputs go to warps of their own or go in
+// one round (48 entries of two chunks, behind which the joint chain comes, 143 and 152). Launches that fit lose 3 to 5 % of a call,
+// values of 256 leave no shared memory for six. Larger keys are held to four: calls 1 % shorter.
+template <int DIM, int CTAS>
+__global__ void __launch_bounds__(128, CTAS) gated_delta_chunk_kernel(const GatedChunkParams c) {
     pl_grid_trigger();
     pl_grid_wait();
     constexpr int kLd = DIM + 4;
@@ -915,21 +920,40 @@ __global__ void __launch_bounds__(128, DIM <= 64 ? 6 : 4) gated_delta_chunk_kern
     send_chunk(out, c.scratch + (static_cast<int64_t>(blockIdx.x) * p.n_heads + head) * sent.floats, at, DIM);
 }
 
-template <int DIM>
-cudaError_t launch_gated_chunks(const GatedChunkParams& c, int64_t slots, int n_long, cudaStream_t stream) {
-    const int smem = gated_chunk_smem<DIM>(c.in.vdim);
-    const cudaError_t set = pl_allow_smem<gated_delta_chunk_kernel<DIM>>(gated_chunk_smem<DIM>(256));
+template <int DIM, int CTAS>
+cudaError_t launch_gated_matrices(const GatedChunkParams& c, int64_t slots, cudaStream_t stream) {
+    const cudaError_t set = pl_allow_smem<gated_delta_chunk_kernel<DIM, CTAS>>(gated_chunk_smem<DIM>(256));
     if (set != cudaSuccess) {
         return set;
     }
-    const cudaError_t made = pl_launch_overlapped(gated_delta_chunk_kernel<DIM>, dim3(static_cast<unsigned>(slots), c.in.n_heads),
-                                                  dim3(128), smem, stream, c);
+    return pl_launch_overlapped(gated_delta_chunk_kernel<DIM, CTAS>, dim3(static_cast<unsigned>(slots), c.in.n_heads), dim3(128),
+                                gated_chunk_smem<DIM>(c.in.vdim), stream, c);
+}
+
+// Whether the matrices' launch takes the build for six CTAs an SM.
+template <int DIM>
+bool gated_matrices_many(int64_t ctas, int vdim, bool apart) {
+    const int64_t rounds = (ctas + 4 * 148 - 1) / (4 * 148), fewer = (ctas + 6 * 148 - 1) / (6 * 148);
+    return DIM == 32 ? rounds > 1 && vdim <= 128
+                     : vdim <= 128 && 3 * fewer <= 2 * rounds + 1 && rounds > 1 && (apart || vdim != 64 || fewer == 1);
+}
+
+template <int DIM>
+cudaError_t launch_gated_chunks(const GatedChunkParams& c, int64_t slots, int n_long, int longest, cudaStream_t stream) {
+    const bool apart = delta_chain_apart<DIM / 16, false>(c.in.n_heads, c.in.vdim, slots, n_long, longest);
+    cudaError_t made;
+    if constexpr (DIM > 64) {
+        made = launch_gated_matrices<DIM, 4>(c, slots, stream);
+    } else {
+        made = gated_matrices_many<DIM>(slots * c.in.n_heads, c.in.vdim, apart) ? launch_gated_matrices<DIM, 6>(c, slots, stream)
+                                                                                : launch_gated_matrices<DIM, 0>(c, slots, stream);
+    }
     if (made != cudaSuccess) {
         return made;
     }
     const DeltaChainParams chain{c.scratch, c.in.state, c.in.first_rows, c.in.counts, c.in.slots, c.in.o_raw, c.in.n_heads,
                                  c.in.vdim, c.pass, c.status};
-    return launch_delta_chain<DIM / 16, false>(chain, n_long, slots, stream);
+    return launch_delta_chain<DIM / 16, false>(chain, n_long, apart, stream);
 }
 
 // ---------------------------------------------------------------------------- steps of single tokens
@@ -1127,11 +1151,12 @@ PL_API int pl_gated_delta(const void* q, const void* k, const void* v, int64_t q
         const int window = delta_window(step, n_heads, DeltaChunkLayout(dim, vdim, false).floats);
         GatedChunkParams c{p, {n_entries, forms.chunk_least, window, 0}, scratch, status};
         const int64_t n_slots = delta_chunk_slots(step, window);
+        const int longest = min(longest_chunks, window);
         cudaError_t made = cudaSuccess;
         for (; c.pass.pass < delta_passes(step, window) && made == cudaSuccess; ++c.pass.pass) {
-            made = dim == 32 ? launch_gated_chunks<32>(c, n_slots, n_long, stream)
-                 : dim == 64 ? launch_gated_chunks<64>(c, n_slots, n_long, stream)
-                             : launch_gated_chunks<128>(c, n_slots, n_long, stream);
+            made = dim == 32 ? launch_gated_chunks<32>(c, n_slots, n_long, longest, stream)
+                 : dim == 64 ? launch_gated_chunks<64>(c, n_slots, n_long, longest, stream)
+                             : launch_gated_chunks<128>(c, n_slots, n_long, longest, stream);
         }
         if (made != cudaSuccess) {
             return pl_fail(3, "gated_delta: launch failed: %s", cudaGetErrorString(made));
