@@ -428,58 +428,66 @@ cudaError_t launch_rows(const GemmF32Params& p, cudaStream_t stream) {
 }
 
 // ---------------------------------------------------------------------------- which form
-// A form's tile, how many of its CTAs an SM holds, the time of a CTA alone on its SM and what each further one adds, in ps a k.
-// Measured with weights that are not in L2, 2048 to 32000 columns of 2048 to 8192 k. What is chosen decides time alone.
-// Picked form / the one before these (us): 8 rows, 12288 x 2048: 32 / 47; 16 rows,
-// 8192 x 2048: 33 / 59; 32 rows, 6144 x 4096: 90 / 119; 64 rows, 4096 x 2048: 47 / 69; 128 rows, 3072 x 2048: 76 / 99;
-// 200 rows, 2048 x 8192: 301 / 389; 300 rows, 32000 x 2048: 904 / 1065; 700 rows, 4096 x 2048: 281 / 312. Within 4 % of
-// even: up to 4 rows of 4096 columns and fewer, 509 rows of 16384 and 32000 (the 128-row tiles as before).
+// A form's tile, the k of one of its pieces, how many tiles of rows it is for (0: any), how many of its CTAs an SM holds, the time of a CTA
+// alone on its SM and what each further one adds, in ps a k. Measured with weights that are not in L2, 2048 to 32000 columns of 2048 to
+// 8192 k. k counts in whole pieces. What is chosen decides time alone. Tiles of up to 16 rows are for one of them, more would read
+// the weights again; the 8-row form is also for two, which read them from L2 (16 rows, 3072 x 8192: 87 us by 16-row tiles, 72 so). The
+// last 64-row form goes through registers in pieces of 16 k: for k up to 64 alone (200 rows, 3072 x 16: 3.7 us, by 32 x 32 tiles 7.4; at
+// 2048 k a third slower than the one along k).
+// Picked form / those before the table (us): 8 rows, 12288 x 2048: 32 / 47; 16 rows, 8192 x 2048: 33 / 59; 32 rows, 6144 x 4096: 90 /
+// 119; 64 rows, 4096 x 2048: 47 / 69; 128 rows, 3072 x 2048: 76 / 99; 200 rows, 2048 x 8192: 301 / 389; 300 rows, 32000 x 2048: 904 /
+// 1065; 700 rows, 4096 x 2048: 281 / 312. Within 5 % of even: up to 4 rows of 4096 columns and fewer, 509 rows of 16384 and 32000.
 struct Form {
-    int rows, columns, resident, alone, more;
+    int rows, columns, piece, row_tiles, resident, alone, more;
     cudaError_t (*launch)(const GemmF32Params&, cudaStream_t);
 };
 const Form kForms[] = {
-    {1, 32, 3, 5700, 2900, launch_rows<32, 1, 1, 1, 128, 4, 4, 4>},
-    {2, 16, 2, 4060, 1500, launch_rows<16, 1, 2, 1, 128, 4, 8, 8>},
-    {2, 32, 3, 5700, 2900, launch_rows<32, 1, 1, 2, 128, 4, 4, 4>},
-    {4, 16, 5, 4030, 1600, launch_rows<16, 1, 4, 1, 128, 4, 8, 4>},
-    {4, 32, 5, 9000, 2500, launch_rows<16, 2, 2, 2, 64, 2, 4, 4>},
-    {8, 16, 4, 4800, 3300, launch_rows<16, 1, 4, 2, 128, 4, 8, 4>},
-    {8, 32, 5, 9100, 3500, launch_rows<16, 2, 4, 2, 64, 2, 4, 4>},
-    {16, 16, 3, 6800, 6300, launch_rows<16, 1, 8, 2, 128, 4, 8, 4>},
-    {16, 32, 2, 10500, 7500, launch_rows<16, 2, 8, 2, 64, 2, 8, 8>},
-    {16, 32, 4, 13100, 4000, launch_rows<16, 2, 4, 4, 64, 2, 4, 4>},
-    {16, 64, 2, 20100, 4200, launch_rows<16, 4, 4, 4, 64, 1, 4, 4>},
-    {32, 16, 2, 9800, 8300, launch_rows<16, 1, 8, 4, 128, 2, 4, 4>},
-    {32, 32, 1, 14000, 14000, launch_rows<16, 2, 8, 4, 128, 1, 4, 4>},
-    {32, 32, 3, 15100, 9500, launch_rows<16, 2, 8, 4, 64, 2, 4, 4>},
-    {32, 64, 2, 23000, 15600, launch_rows<16, 4, 8, 4, 64, 1, 4, 4>},
-    {32, 64, 2, 36600, 400, launch_rows<16, 4, 4, 8, 32, 1, 6, 6>},
-    {64, 64, 4, 37000, 24300, launch_rows<16, 4, 8, 8, 32, 1, 3, 3, 2>},
-    {128, 64, 3, 62500, 39000, launch_tile<128, 64, 8, 8, 1, 3>},
-    {128, 128, 2, 106000, 66000, launch_tile<128, 128, 8, 16, 2, 2>},
+    {1, 32, 128, 1, 3, 5700, 2900, launch_rows<32, 1, 1, 1, 128, 4, 4, 4>},
+    {2, 16, 128, 1, 2, 4060, 1500, launch_rows<16, 1, 2, 1, 128, 4, 8, 8>},
+    {2, 32, 128, 1, 3, 5700, 2900, launch_rows<32, 1, 1, 2, 128, 4, 4, 4>},
+    {4, 16, 128, 1, 5, 4030, 1600, launch_rows<16, 1, 4, 1, 128, 4, 8, 4>},
+    {4, 32, 64, 1, 5, 9000, 2500, launch_rows<16, 2, 2, 2, 64, 2, 4, 4>},
+    {8, 16, 128, 1, 4, 4800, 3300, launch_rows<16, 1, 4, 2, 128, 4, 8, 4>},
+    {8, 16, 128, 2, 4, 5400, 1750, launch_rows<16, 1, 4, 2, 128, 4, 8, 4>},
+    {8, 32, 64, 1, 5, 9100, 3500, launch_rows<16, 2, 4, 2, 64, 2, 4, 4>},
+    {16, 16, 128, 1, 3, 6800, 6300, launch_rows<16, 1, 8, 2, 128, 4, 8, 4>},
+    {16, 32, 64, 1, 2, 10500, 7500, launch_rows<16, 2, 8, 2, 64, 2, 8, 8>},
+    {16, 32, 64, 1, 4, 13100, 4000, launch_rows<16, 2, 4, 4, 64, 2, 4, 4>},
+    {16, 64, 64, 1, 2, 20100, 4200, launch_rows<16, 4, 4, 4, 64, 1, 4, 4>},
+    {32, 16, 128, 0, 2, 9800, 8300, launch_rows<16, 1, 8, 4, 128, 2, 4, 4>},
+    {32, 32, 128, 0, 1, 14000, 14000, launch_rows<16, 2, 8, 4, 128, 1, 4, 4>},
+    {32, 32, 64, 0, 3, 15100, 9500, launch_rows<16, 2, 8, 4, 64, 2, 4, 4>},
+    {32, 64, 64, 0, 2, 23000, 15600, launch_rows<16, 4, 8, 4, 64, 1, 4, 4>},
+    {32, 64, 32, 0, 2, 36600, 400, launch_rows<16, 4, 4, 8, 32, 1, 6, 6>},
+    {64, 64, 32, 0, 4, 37000, 24300, launch_rows<16, 4, 8, 8, 32, 1, 3, 3, 2>},
+    {64, 64, 16, 0, 4, 37000, 24300, launch_tile<64, 64, 4, 8, 1, 4>},
+    {128, 64, 16, 0, 3, 62500, 39000, launch_tile<128, 64, 8, 8, 1, 3>},
+    {128, 128, 16, 0, 2, 106000, 66000, launch_tile<128, 128, 8, 16, 2, 2>},
 };
 
-const Form& form_for(int m, int n) {
+const Form& form_for(int m, int n, int k) {
     const Form* best = nullptr;
-    int64_t least = 0;
+    double least = 0.0;
     for (const Form& f : kForms) {
         const int64_t row_tiles = (m + f.rows - 1) / f.rows, column_tiles = (static_cast<int64_t>(n) + f.columns - 1) / f.columns;
-        // The second coordinate of a grid ends at 65,535: the rows' tiles in the forms along k, the columns' in the others.
-        // Tiles of up to 32 rows are for products that fill more than half of one; more than one would read the weights again.
-        if ((f.rows < 128 ? row_tiles : column_tiles) > 65535 || (f.rows < 32 && row_tiles > 1) ||
-            (f.columns > 16 && f.rows <= 32 && f.rows >= 2 * m)) {
+        // The second coordinate of a grid ends at 65,535: the rows' tiles in the forms along k, the columns' in those through
+        // registers (pieces of 16). Tiles of 32 columns and more are for products that fill more than half of their rows, a
+        // quarter of 64 and 128.
+        const bool along = f.piece > 16, shortest = !along && f.rows == 64;
+        if ((along ? row_tiles : column_tiles) > 65535 || (f.row_tiles != 0 && row_tiles != f.row_tiles) ||
+            (f.columns > 16 && f.rows <= 32 && f.rows >= 2 * m) || (f.rows > 32 && m <= 16) || (shortest && k > 64)) {
             continue;
         }
         const int64_t per_sm = (row_tiles * column_tiles + 147) / 148;
         auto together = [&](int64_t ctas) { return ctas > 0 ? f.alone + (ctas - 1) * f.more : 0; };
-        const int64_t time = per_sm / f.resident * together(f.resident) + together(per_sm % f.resident);
+        const int64_t k_whole = (static_cast<int64_t>(k) + f.piece - 1) / f.piece * f.piece;
+        const double time = static_cast<double>(per_sm / f.resident * together(f.resident) + together(per_sm % f.resident)) * k_whole;
         if (best == nullptr || time < least) {
             best = &f;
             least = time;
         }
     }
-    return *best;  // (64-row tiles always fit: m is bounded by their count)
+    return *best;  // (64-row tiles along k take any m from 17 on, 16-row and 8-row ones any below)
 }
 
 }  // namespace
@@ -502,7 +510,7 @@ PL_API int pl_gemm_f32(const float* a, const float* w, float* c, int m, int n, i
         PL_CHECK_LAUNCH("gemm_f32");
         return 0;
     }
-    const cudaError_t err = form_for(m, n).launch(p, stream);
+    const cudaError_t err = form_for(m, n, k).launch(p, stream);
     if (err != cudaSuccess) {
         return pl_fail(3, "gemm_f32: launch failed: %s", cudaGetErrorString(err));
     }

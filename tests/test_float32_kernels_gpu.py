@@ -39,6 +39,25 @@ def test_every_form_of_the_product_gives_the_same_bits(m, n, k, accumulate):
     assert bool(((got.double() - exact).abs() <= bound).all())
 
 
+# One size and more for every line of the forms' table, with CTAs alone on their SMs and with several: k over twice around the longest ring
+# (eight pieces of 128) and off the pieces; k of one piece through registers.
+@pytest.mark.parametrize("m,n,k", [
+    (2, 100, 2180), (2, 2500, 2180), (1, 8200, 2180), (2, 8200, 2180), (3, 2000, 2180), (3, 12300, 2180), (8, 100, 2180), (8, 2500, 2180),
+    (7, 8200, 2180), (16, 100, 2180), (16, 2500, 2180), (15, 2000, 2180), (9, 4100, 2180), (16, 12300, 2180), (9, 16400, 2180),
+    (31, 100, 2180), (17, 2000, 2180), (17, 2500, 2180), (31, 12300, 2180), (17, 6000, 2180), (31, 16400, 2180), (40, 12300, 2180),
+    (130, 6000, 2180), (300, 8200, 2180), (65, 33000, 132), (40, 5000, 16), (65, 6000, 4), (130, 100, 13 * 4)])
+def test_every_tile_gives_the_bits_of_the_general_form(m, n, k):
+    ops = _ops()
+    gen = torch.Generator(device=DEV).manual_seed(m + n + k)
+    a, w = torch.randn((m, k), generator=gen, device=DEV), torch.randn((n, k), generator=gen, device=DEV)
+    off = torch.zeros((m, k + 1), device=DEV)
+    off[:, 1:] = a
+    got, want = torch.empty((m + 1, n), device=DEV).fill_(7.0), torch.empty((m, n), device=DEV)
+    ops.gemm_f32(a, w, got[:m])
+    ops.gemm_f32(off[:, 1:], w, want)
+    assert torch.equal(got[:m], want) and bool((got[m] == 7.0).all())
+
+
 @pytest.mark.parametrize("heads,kv,dim", [(8, 2, 64), (3, 3, 20), (16, 1, 128), (5, 1, 36), (4, 4, 128)])
 @pytest.mark.parametrize("portions", [[1] * 3 + [5], [1] * 40 + [90, 1], [150], [1] * 70, [3] * 30, [70, 45, 2], [40]])
 @pytest.mark.parametrize("options", [{}, {"window": 37}, {"window": 37, "keep_first": 5},
@@ -89,7 +108,7 @@ def test_staged_attention_gives_the_bits_of_the_plain_walk(heads, kv, dim, porti
 
 
 def test_more_columns_than_the_tiles_grid_holds():
-    """65,535 tiles of 64 columns are one grid's; what is wider takes the general form."""
+    """65,535 tiles of 64 columns are one grid's; what is wider goes by the forms whose columns are its first coordinate."""
     ops = _ops()
     n, k, m = 65535 * 64 + 5, 4, 33
     a, w = torch.randn((m, k), device=DEV), torch.randn((n, k), device=DEV)
