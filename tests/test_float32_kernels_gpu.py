@@ -198,3 +198,29 @@ def test_few_tokens_of_many_keys_give_the_bits_of_the_plain_walk(heads, kv, dim,
         ops.attention_simt(q, *args, got, page, None, dim ** -0.5, status, **more, **gate)
         ops.attention_simt(q, *args, want, page, None, dim ** -0.5, plain_status, mass, weight, **more, **gate)
         assert torch.equal(got, want) and int(status.item()) == int(plain_status.item())
+
+
+# Steps whose CTAs of two heads outnumber the SMs take four heads each, of one and of two columns a thread.
+@pytest.mark.parametrize("heads,kv,dim,tokens", [(32, 8, 64, 13), (8, 2, 128, 39), (8, 2, 100, 39), (16, 1, 128, 26), (16, 4, 36, 26)])
+@pytest.mark.parametrize("options", [{}, {"softcap": 3.0}])
+def test_four_heads_a_cta_give_the_bits_of_the_plain_walk(heads, kv, dim, tokens, options):
+    ops = _ops()
+    gen = torch.Generator().manual_seed(heads * dim + tokens)
+    page, ends = 16, [0, 30, 31, 32, 63, 64, 127, 128, 129, 255, 256, 500, 777]
+    width = ends[-1] // page + 1
+    pools = torch.randn((2, tokens * width, kv, page, dim), generator=gen)
+    table = torch.randperm(tokens * width, generator=gen).int().view(tokens, width)
+    pos = [ends[i % len(ends)] for i in range(tokens)]
+    for e in range(tokens):  # (keys past a request's last are not written yet)
+        pools[:, table[e, pos[e] // page].item(), :, pos[e] % page + 1:] = float("nan")
+    table[10, 5], table[12, :9] = -1, -1
+    pools, table, pos = pools.to(DEV), table.to(DEV), torch.tensor(pos, dtype=torch.int32, device=DEV)
+    entry = torch.arange(tokens, dtype=torch.int32, device=DEV)
+    q = torch.randn((tokens, heads, dim), generator=gen).to(DEV)
+    more = {"gate": torch.randn((tokens, heads), generator=gen).to(DEV), "sinks": torch.randn(heads, generator=gen).to(DEV)} if options else {}
+    got, want = torch.empty_like(q), torch.empty_like(q)
+    mass, weight = torch.zeros((pools.shape[1], heads), device=DEV), torch.zeros(pools.shape[1], device=DEV)
+    status, plain_status = torch.zeros(1, dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops.attention_simt(q, pools[0], pools[1], table, pos, entry, got, page, None, dim ** -0.5, status, **options, **more)
+    ops.attention_simt(q, pools[0], pools[1], table, pos, entry, want, page, None, dim ** -0.5, plain_status, mass, weight, **options, **more)
+    assert bool(torch.isfinite(want).all()) and torch.equal(got, want) and int(status.item()) == int(plain_status.item())
