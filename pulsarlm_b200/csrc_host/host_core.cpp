@@ -474,7 +474,7 @@ using plh::CacheBook;
 using plh::PagePool;
 using plh::SchedulerCore;
 
-PLH_API int plh_abi_version() { return 6; }
+PLH_API int plh_abi_version() { return 7; }
 
 PLH_API void* plh_pool_create(int n_pages) { return new PagePool(n_pages); }
 PLH_API void plh_pool_destroy(void* pool) { delete static_cast<PagePool*>(pool); }
@@ -526,9 +526,6 @@ PLH_API int plh_cache_commit(void* cache, int64_t request, int64_t new_len) {
 PLH_API int plh_cache_close(void* cache, int64_t request) { return static_cast<CacheBook*>(cache)->close(request); }
 PLH_API int plh_cache_pages_needed(void* cache, int64_t request, int64_t new_len) {
     return static_cast<CacheBook*>(cache)->pages_needed(request, new_len);
-}
-PLH_API int plh_cache_table_row(void* cache, int group, int64_t request, int32_t* out, int capacity) {
-    return static_cast<CacheBook*>(cache)->table_row(group, request, out, capacity);
 }
 // The longest block-table row of `count` open requests, or the code of one that is none.
 PLH_API int plh_cache_longest_row(void* cache, int group, const int64_t* requests, int count) {

@@ -11,7 +11,7 @@ from ..kernels import build
 _I32, _I64, _PTR = ctypes.c_int, ctypes.c_int64, ctypes.c_void_p
 _lib = None
 _lock = threading.Lock()
-ABI_VERSION = 6
+ABI_VERSION = 7
 
 # return codes of csrc_host/host_core.hpp
 OK, NO_ROOM = 0, 1
@@ -38,7 +38,6 @@ _SIGNATURES = {
     "plh_cache_commit": ([_PTR, _I64, _I64], _I32),
     "plh_cache_close": ([_PTR, _I64], _I32),
     "plh_cache_pages_needed": ([_PTR, _I64, _I64], _I32),
-    "plh_cache_table_row": ([_PTR, _I32, _I64, _PTR, _I32], _I32),
     "plh_cache_held_pages": ([_PTR, _I32, _I64, _PTR, _I32], _I32),
     "plh_cache_take_fresh": ([_PTR, _I32, _PTR, _I32], _I32),
     "plh_cache_free_pages": ([_PTR], _I32),
