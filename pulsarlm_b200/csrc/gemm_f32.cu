@@ -471,8 +471,8 @@ const Form& form_for(int m, int n, int k) {
     for (const Form& f : kForms) {
         const int64_t row_tiles = (m + f.rows - 1) / f.rows, column_tiles = (static_cast<int64_t>(n) + f.columns - 1) / f.columns;
         // The second coordinate of a grid ends at 65,535: the rows' tiles in the forms along k, the columns' in those through
-        // registers (pieces of 16). Tiles of 32 columns and more are for products that fill more than half of their rows, a
-        // quarter of 64 and 128.
+        // registers (pieces of 16). Tiles of 32 columns and more are for products that fill more than half of their rows,
+        // those of 64 and 128 rows for more than 16.
         const bool along = f.piece > 16, shortest = !along && f.rows == 64;
         if ((along ? row_tiles : column_tiles) > 65535 || (f.row_tiles != 0 && row_tiles != f.row_tiles) ||
             (f.columns > 16 && f.rows <= 32 && f.rows >= 2 * m) || (f.rows > 32 && m <= 16) || (shortest && k > 64)) {

@@ -41,9 +41,11 @@
 // split evenly over as few tiles as hold them, and a tile's MMAs are only as wide as its rows (in steps of 32), so little
 // is spent on padding. Rows of the next expert that a tile's last rows of 32 bring in are columns nobody stores. What bounds
 // it: the loads where experts have few rows (16 KB of weights a CTA and k block, whatever the width), the MMAs from about
-// 256 rows an expert on. 2,048 tokens, 4 of 32 experts, 2,048 wide, 1,024 features: gated 75.7 us, down 47.0; the
-// library's grouped products took 81.2 and 49.9, and a SwiGLU kernel between them (16 rows an expert 48.8 and 28.6, 68.7 and 43.3;
-// 1,024 rows 54.6 and 35.7, 56.0 and 35.1).
+// 256 rows an expert on where k is long, the epilogue (0.9 us a chunk of 32 tokens) where it is not. us beside the library's grouped
+// products (and a SwiGLU kernel behind the first), gated and down: 32 experts, 2,048 wide, 1,024 features, 64 rows an expert 58 and 35, 74
+// and 45; 256 rows 69 and 44, 84 and 47; 1,024 rows 206 and 123, 234 and 107. 64 experts, 1,024 wide, 512 features, 64 rows 37 and 25,
+// 48 and 28; 1,024 rows 143 and 106, 141 and 76: products over 1,024 and fewer features are behind the library's from about 512 rows an expert
+// on, which the whole part shows past 4,096 tokens (8 of 64 experts, 8,192 tokens 489 and 514).
 //
 // Every wait on an mbarrier is bounded: after the limit the CTA raises bit 8 of the
 // status word, stops issuing work, lets what is in flight land, meets its partner,

@@ -133,14 +133,14 @@ class RoutedExperts(Part):
                                    if self.gated else tensors[t["shared_up"]].contiguous())
             self.shared_down = tensors[t["shared_down"]].contiguous()
 
-    def _grouped(self, h: torch.Tensor) -> bool:
-        return (h.dtype == torch.bfloat16 and h.shape[0] >= GROUPED_MIN_TOKENS and self.hidden % 8 == 0
-                and self.ff % 8 == 0 and (self._own_products() or hasattr(torch.nn.functional, "grouped_mm")))
-
-    def _own_products(self) -> bool:
-        """Whether the experts' grouped products are the package's own kernel's (else the library's)."""
-        return ops.gemm_bf16_grouped_supports(self.ff, self.hidden, self.n_experts) and ops.gemm_bf16_grouped_supports(
-            self.hidden, self.ff, self.n_experts)
+    def _grouped(self, h: torch.Tensor) -> str | None:
+        """Whose grouped products the experts are: "own", the package's kernel, or "library"; None: pair by pair."""
+        if h.dtype != torch.bfloat16 or h.shape[0] < GROUPED_MIN_TOKENS or self.hidden % 8 or self.ff % 8:
+            return None
+        if ops.gemm_bf16_grouped_supports(self.ff, self.hidden, self.n_experts) and ops.gemm_bf16_grouped_supports(
+                self.hidden, self.ff, self.n_experts):
+            return "own"
+        return "library" if hasattr(torch.nn.functional, "grouped_mm") else None
 
     def _route(self, h: torch.Tensor) -> tuple:
         """(ids, weights on the experts' inputs, weights on their outputs, weight of the shared expert); weights None: 1."""
@@ -171,7 +171,8 @@ class RoutedExperts(Part):
     def forward(self, h: torch.Tensor, batch) -> torch.Tensor:
         out = torch.empty((h.shape[0], self.hidden), dtype=h.dtype, device=h.device)
         status = status_of(batch)
-        if not self._grouped(h):
+        products = self._grouped(h)
+        if products is None:
             (act, (ids, _, weights, shared_weights)), shared = run_branches(
                 batch, h.device, lambda: self._units(h), shared_expert=lambda: self._shared(h, status))
             ops.moe_down(act, self.down, ids, weights, shared, out, shared_weights)
@@ -183,7 +184,7 @@ class RoutedExperts(Part):
         ends, row_of_pair, pair_of_row = ops.moe_sort(ids, self.n_experts)
         x = ops.moe_gather(h, pair_of_row, self.top)
         act = torch.empty((x.shape[0], self.ff), dtype=h.dtype, device=h.device)
-        if self._own_products():
+        if products == "own":
             if in_weights is None:
                 unit = ("silu" if self.limit is None else "clamped") if self.gated else self.plain_act
                 ops.gemm_bf16_grouped(x, self.gate_up, ends, act, unit, self.limit or 0.0, status)
