@@ -363,8 +363,9 @@ struct DeltaLane {
     uint4 vv;
 };
 
-// Outputs by the chain's warps. grid (entries that go in chunks, heads, vdim / 16), NW = dim / 16 warps. On the path from a chunk to the next are only Z's products,
-// their sum over the warps, and the state's update; O's products fill the waits between and are added up a chunk later. Bound by
+// Outputs by the chain's warps. grid (entries that go in chunks, heads, vdim / 16), NW = dim / 16 warps. On the path from a chunk to the
+// next are only Z's products, their sum over the warps, and the state's update; O's products fill the waits between and are added up a
+// chunk later. Bound by
 // that path where an SM has one CTA (0.85 us a chunk); many CTAs fill the waits of one another, and a step of their short chains begins
 // with plain loads and no set-up. The walks took 681 us for one prompt of 2,048 tokens, 32 heads of 64 x 64. Slower: 32 columns a CTA.
 template <int NW, bool GENERAL>
@@ -564,8 +565,8 @@ struct DeltaRing {
     static constexpr int kBytes = kSlots * kFloats * 4 + 2 * 2 * DIM / 16 * 32 * 16;
 };
 
-// Outputs by warps of their own. grid (entries that go in chunks x heads, vdim / 16), 2 NW warps, NW = dim / 16. On the path from a chunk to the next are only
-// Z's products, their sum over the warps, and the state's update: the first NW warps do nothing else. They leave the state that
+// Outputs by warps of their own. grid (entries that go in chunks x heads, vdim / 16), 2 NW warps, NW = dim / 16. On the path from a
+// chunk to the next are only Z's products, their sum over the warps, and the state's update: the first NW warps do nothing else. They leave the state that
 // a chunk starts from in shared memory, where the other NW take it up for O's products, a barrier behind, and add those up a
 // chunk later. The chunks' matrices come into shared memory by bulk copies, three or four chunks in flight. Bound by the path's
 // instructions, each of which waits for the one before it (0.74 us a chunk; 0.85 where NW warps made the outputs too, with what
@@ -852,8 +853,8 @@ inline bool delta_chain_apart(int n_heads, int vdim, int64_t slots, int n_long, 
     }
     const int64_t bytes = slots * n_heads * DeltaChunkLayout(NW * 16, vdim, GENERAL).floats * 4;
     const int64_t kept = (chunks >= 8 && vdim >= 64 ? 54 : 92) << 20;  // about what of L2 the matrices keep
-    // (a chain much longer than the others is a path again, on an SM that it shares: 1,500 tokens beside eight portions of 20, 16 heads
-    // of 128 x 128, the general rule 344 and 367)
+    // (a chain much longer than the others, in all its passes, is a path again, on an SM that it shares: 1,500 tokens beside eight
+    // portions of 20, 16 heads of 128 x 128, the general rule 344 and 367)
     return bytes >= kept && vdim <= NW * 16 && (NW > 2 ? longest < 4 * chunks : GENERAL);
 }
 

@@ -878,12 +878,11 @@ PL_API int pl_delta_rule(const void* r, const void* k, const void* v, const void
         const int window = delta_window(step, n_heads, DeltaChunkLayout(dim, dim, true).floats);
         RuleChunkParams c{p, {n_entries, forms.chunk_least, window, 0}, scratch, status};
         const int64_t n_slots = delta_chunk_slots(step, window);
-        const int longest = min(longest_chunks, window);
         cudaError_t made = cudaSuccess;
         for (; c.pass.pass < delta_passes(step, window) && made == cudaSuccess; ++c.pass.pass) {
-            made = dim == 32 ? launch_rule_chunks<32>(c, n_slots, n_long, longest, stream)
-                 : dim == 64 ? launch_rule_chunks<64>(c, n_slots, n_long, longest, stream)
-                             : launch_rule_chunks<128>(c, n_slots, n_long, longest, stream);
+            made = dim == 32 ? launch_rule_chunks<32>(c, n_slots, n_long, longest_chunks, stream)
+                 : dim == 64 ? launch_rule_chunks<64>(c, n_slots, n_long, longest_chunks, stream)
+                             : launch_rule_chunks<128>(c, n_slots, n_long, longest_chunks, stream);
         }
         if (made != cudaSuccess) {
             return pl_fail(3, "delta_rule: launch failed: %s", cudaGetErrorString(made));

@@ -22,7 +22,8 @@ constexpr int kStepThreads = 256;
 // three: 36.0 and 37.3).
 constexpr int kStepMany = 6;
 constexpr bool step_has_two_builds(int dim, int vdim) { return dim * vdim > 1024 && dim * vdim <= 4096; }
-constexpr int step_ctas(int dim, int vdim) { return dim * vdim == 128 * 128 ? 2 : 0; }  // (0: nothing asked; one asked is not the same, 88 to 115 registers)
+// (0: nothing asked; asked for one the compiler takes 88 to 115 registers)
+constexpr int step_ctas(int dim, int vdim) { return dim * vdim == 128 * 128 ? 2 : 0; }
 inline bool step_many(int64_t ctas, int dim, int vdim, bool general) {
     const int few = dim == 128 ? 3 : dim == 32 && vdim == 64 ? 5 : 4;
     const int64_t rounds = (ctas + few * 148 - 1) / (few * 148), fewer = (ctas + kStepMany * 148 - 1) / (kStepMany * 148);
